@@ -339,46 +339,6 @@ __device__ __forceinline__ double adj_b1_terms(const inst_view<double> &v, const
     return val;
 }
 
-// Gather: cross-line right-hand-side adjoints of an S stage into UB (and Y2B for KIND 2), the
-// lo/hi adjoints of the S lines (lsum / hsum of column q, added on rows 0 / nx-1), and for
-// KIND 1 the adjoint of the explicit v = v_lo boundary column (B1^T) with its parameter
-// sensitivities.  One grid point (p, q) per call.
-template <int KIND>
-__device__ __forceinline__ void adj_gather_point(const inst_view<double> &v, const bdesc &d, const double *__restrict__ U,
-                                                 const double *__restrict__ FB, const double *__restrict__ LV,
-                                                 double *__restrict__ UB, double *__restrict__ Y2B, adj_acc &acc,
-                                                 double tau, int p, int q, double lsum, double hsum)
-{
-    const int nx = v.nx, ny = v.ny;
-    auto F = [&](int a, int b) -> double {
-        return (a >= 1 && a <= nx - 2 && b >= 1 && b <= ny - 2) ? FB[(long long)a * ny + b] : 0.0;
-    };
-    auto W = [&](int slot, int a, int b) -> double {
-        return (a >= 1 && a <= nx - 2 && b >= 1 && b <= ny - 2) ? __ldg(v.S(slot) + (long long)a * ny + b) : 0.0;
-    };
-    const long long o = (long long)p * ny + q;
-    double val = 0.0;
-    if constexpr (KIND == 2) {
-        double db = W(SL_S2MZ, p + 1, q + 1) * F(p + 1, q + 1) - W(SL_S2MZ, p + 1, q - 1) * F(p + 1, q - 1) -
-                    W(SL_S2MZ, p - 1, q + 1) * F(p - 1, q + 1) + W(SL_S2MZ, p - 1, q - 1) * F(p - 1, q - 1);
-        if (d.scheme != LSS_ADI_CRAIG_SNEYD)
-            db += W(SL_X1, p + 1, q) * F(p + 1, q) + W(SL_X2, p, q) * F(p, q) + W(SL_X3, p - 1, q) * F(p - 1, q) +
-                  W(SL_X4, p, q + 1) * F(p, q + 1) + W(SL_X5, p, q - 1) * F(p, q - 1);
-        // HV: rows 1..nx-2 already hold the last v stage's adjoint of its input Y2
-        if (d.scheme == LSS_ADI_HUNDSDORFER_VERWER && p >= 1 && p <= nx - 2) Y2B[o] += db; else Y2B[o] = db;
-        val -= db;
-    } else {
-        val += W(SL_WW, p + 1, q) * F(p + 1, q) + W(SL_WE, p - 1, q) * F(p - 1, q) + W(SL_WS, p, q + 1) * F(p, q + 1) +
-               W(SL_WN, p, q - 1) * F(p, q - 1) + W(SL_WC, p, q) * F(p, q) + W(SL_WG, p + 1, q + 1) * F(p + 1, q + 1) -
-               W(SL_WG, p + 1, q - 1) * F(p + 1, q - 1) - W(SL_WG, p - 1, q + 1) * F(p - 1, q + 1) +
-               W(SL_WG, p - 1, q - 1) * F(p - 1, q - 1);
-        if (q <= 2) val += adj_b1_terms(v, d, U, LV, acc, tau, p, q);
-    }
-    if (p == 0) val += lsum;
-    if (p == nx - 1) val += hsum;
-    UB[o] += val;
-}
-
 // lo / hi adjoints of the S lines whose Dirichlet values come from column q (index_of remap)
 __device__ __forceinline__ void adj_line_ends(const inst_view<double> &v, const double *__restrict__ LS,
                                               const double *__restrict__ HS, int q, double &lsum, double &hsum)

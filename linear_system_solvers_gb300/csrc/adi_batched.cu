@@ -59,16 +59,6 @@ struct bdesc {
 // order[cls_start[c] .. cls_start[c] + cls_count[c]), longest first, pulled through counter[c].
 constexpr int MAX_GROUP_WARPS = 4;
 
-// Most chunks per line of the partitioned line solves of one large instance (wide path): a CTA
-// holds L lines x P chunks (L * P <= 1024 threads) and composes the chunks' carries through two
-// shared arrays of 1024 values, indexed [chunk][line] (carry2d).
-constexpr int MAX_CHUNKS = 128;
-template <typename T> struct carry2d {
-    T *p;
-    int L; // lines per CTA (blockDim.x)
-    __device__ __forceinline__ T *operator[](int c) const { return p + c * L; }
-};
-
 template <typename T> struct bparams {
     const bdesc *desc;
     const int *order;
@@ -285,71 +275,6 @@ __global__ void k_setup_v_lines(setup_params sp, T *V0, long long slot_stride, T
         s[VL_VN * slot_stride] = static_cast<T>(c * ib);
         s[VL_IB * slot_stride] = static_cast<T>(ib);
         if (t == e) chV_arena[d.ox + i] = static_cast<T>(c * ib);
-    }
-}
-
-// ------------------------------------------------------------------------------------------
-// time-dependent coefficients of one instance (SABR with r != 0 on the wide kernels)
-// ------------------------------------------------------------------------------------------
-// a and c carry D(t)^(2(1-beta)) and D(t)^(1-beta), D(t) = exp(-r (T - t)); b, d, e, f do not.
-// Before each step the S-direction base tables M, P, Z, C are re-evaluated at the step's powers
-// da, dc (general_heston_equation_coefficients, coefficients.hpp:89-98, on the transformed data
-// of lss_heat_data_transform.hpp:174-214) and the S lines re-factorised (k_tdep_s_factor,
-// k_tdep_s_slots); the v-direction tables do not change.  The same kernel scales the S-factors of the adjoint's
-// D(t) terms (X_HA, X_HDD by da, X_HC by dc) and the boundary-column weights that carry d^ on
-// the v = v_lo line (XB_M, XB_P), so that the adjoint steps see this step's a^ and c^.
-struct tdep_params {
-    const double *a_static, *c_static, *ab; // n each: ((0.5 v) v) S^(2 beta), ((rho nu) v) v S^beta, A B
-    const double *per_i;                    // 5 nx: A, A^2, A^3, A'', user d
-    const double *xs;                       // 3 nx: X_HA, X_HDD, X_HC at D = 1
-    double *base;                           // 7 n: M, P, Z, Mt, Pt, W, C
-    long long n;
-    int nx, ny;
-    double alpha, delta, two_alpha, half_rho_f;
-};
-
-// The S-line factorisation of the time-dependent instance in two kernels: the recurrence
-// beta_t = b_t - a_t gamma_{t-1} for 1/beta and gamma (k_tdep_s_factor, partitioned along the
-// lines), then every slot of every point in parallel (s_line_slots, the same formulas as
-// k_setup_s_lines).
-template <typename T>
-__global__ void k_tdep_s_slots(const double *__restrict__ base, long long n, int nx, int ny, int scheme, double th,
-                               double ze, double gm, T *S0, T *chS)
-{
-    const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    const int e = nx - 2;
-    if (q >= (long long)e * (ny - 2)) return;
-    const int t = 1 + static_cast<int>(q / (ny - 2)), j = 1 + static_cast<int>(q % (ny - 2));
-    const long long o = (long long)t * ny + j;
-    const double M = base[o], P = base[n + o], Z = base[2 * n + o], Mt = base[3 * n + o], Pt = base[4 * n + o],
-                 W = base[5 * n + o], C = base[6 * n + o];
-    const double ib = static_cast<double>(S0[SL_IB * n + o]), gam = static_cast<double>(S0[SL_G * n + o]);
-    s_line_slots<T>(S0 + o, n, scheme, th, ze, gm, M, P, Z, Mt, Pt, W, C, ib, gam);
-    if (t == e) chS[j] = static_cast<T>(-th * P * ib);
-}
-
-template <typename T>
-__global__ void k_tdep_refresh(tdep_params tp, double da, double dc, T *xarena, long long total_x)
-{
-    const long long o = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (o >= tp.n) return;
-    const int nx = tp.nx, ny = tp.ny;
-    const int i = static_cast<int>(o / ny), j = static_cast<int>(o % ny);
-    const double aval = tp.per_i[i], aa = tp.per_i[nx + i], aaa = tp.per_i[2 * nx + i];
-    const double gc = tp.per_i[3 * nx + i], ud = tp.per_i[4 * nx + i];
-    const double A = tp.a_static[o] * da;
-    const double ah = A / aa;
-    const double dh = ud / aval - (A * gc) / aaa;
-    tp.base[o] = tp.alpha * ah - tp.delta * dh;
-    tp.base[tp.n + o] = tp.alpha * ah + tp.delta * dh;
-    tp.base[2 * tp.n + o] = tp.two_alpha * ah - tp.half_rho_f;
-    tp.base[6 * tp.n + o] = (tp.c_static[o] * dc) / tp.ab[o];
-    if (j == 0) {
-        xarena[XB_M * total_x + i] = static_cast<T>(-tp.delta * dh);
-        xarena[XB_P * total_x + i] = static_cast<T>(tp.delta * dh);
-        xarena[X_HA * total_x + i] = static_cast<T>(tp.xs[i] * da);
-        xarena[X_HDD * total_x + i] = static_cast<T>(tp.xs[nx + i] * da);
-        xarena[X_HC * total_x + i] = static_cast<T>(tp.xs[2 * nx + i] * dc);
     }
 }
 
@@ -599,116 +524,6 @@ __device__ __forceinline__ void v_stage(const inst_view<T> &v, const T *__restri
     }
 }
 
-// v-line sweep through shared-memory tiles.  The lines of a v sweep are rows of the row-major
-// state, so lane r of a warp reading its own row walks memory 8 * ny bytes away from its
-// neighbours: every load of the plain sweep touches 32 sectors.  Here the warp's 32 consecutive
-// lines (lane r owns line i0 + r) move through a per-warp tile of VT columns: the whole warp loads
-// `in` (VT + 2 columns, the window's halo included) and `inh`, and stores `out`, as a few
-// contiguous row segments per instruction; each lane then runs its line's recurrence from the
-// tile.  The per-line arithmetic is that of v_stage, operation for operation (same bits).
-constexpr int VT = 4;
-template <typename T> struct vtile {
-    T in[32][VT + 3]; // columns t-1 .. t+VT of `in` (odd row stride: conflict-free lane reads)
-    T io[32][VT + 1]; // `inh`, overwritten by the recurrence's values, stored to `out`
-};
-
-// Copies `cols` columns starting at column c0 of rows i0 .. i0+nrows-1 (row stride ny) between
-// global memory and the tile rows 0 .. nrows-1 (row stride W), all 32 lanes of the warp
-// cooperating (`lane`: this thread's lane in its warp).
-template <int W, int CMAX, bool LOAD, typename T>
-__device__ __forceinline__ void vtile_copy(T *tile, const T *src, T *dst, long long i0, int ny, int nrows, int c0,
-                                           int cols, int lane)
-{
-#pragma unroll
-    for (int q = 0; q < CMAX; ++q) {
-        const int idx = lane + 32 * q, r = idx / CMAX, c = idx % CMAX;
-        if (r < nrows && c < cols) {
-            const long long g = (i0 + r) * ny + c0 + c;
-            if constexpr (LOAD) tile[r * W + c] = src[g];
-            else dst[g] = tile[r * W + c];
-        }
-    }
-}
-
-template <typename T>
-__device__ __forceinline__ void v_lines_tiled(const inst_view<T> &v, const T *__restrict__ in, const T *__restrict__ inh,
-                                              const T *__restrict__ sb0, T *__restrict__ out, int i0, vtile<T> &tl)
-{
-    const int lane = threadIdx.x & 31; // one-dimensional blocks of whole warps
-    const int nx = v.nx, ny = v.ny, e = v.e_v;
-    const int i = i0 + lane;
-    const bool act = i <= nx - 2;
-    const int nrows = min(32, nx - 1 - i0);
-    T lo = T(0), hi = T(0), y = T(0);
-    if (act) {
-        const int ii = ldg(v.imap() + i);
-        lo = sb0[ii];
-        hi = ldg(v.X(X_VHI) + ii);
-        y = lo;
-    }
-    const T chv = act ? ldg(v.X(X_CHV) + i) : T(0);
-    // forward recurrence y_t = f_t - la_t y_{t-1}, tiles left to right
-    for (int tb = 1; tb <= e; tb += VT) {
-        const int kk = min(VT, e - tb + 1);
-        vtile_copy<VT + 3, VT + 2, true>(&tl.in[0][0], in, (T *)nullptr, i0, ny, nrows, tb - 1, kk + 2, lane);
-        vtile_copy<VT + 1, VT, true>(&tl.io[0][0], inh, (T *)nullptr, i0, ny, nrows, tb, kk, lane);
-        __syncwarp();
-        if (act) {
-#pragma unroll
-            for (int k = 0; k < VT; ++k) {
-                if (k < kk) {
-                    const int t = tb + k;
-                    const long long ot = (long long)t * nx + i;
-                    y = v_point<T>(ldg(v.Vt(VL_LA) + ot), ldg(v.Vt(VL_VC) + ot), ldg(v.Vt(VL_VN) + ot),
-                                   ldg(v.Vt(VL_IB) + ot), tl.in[lane][k], tl.in[lane][k + 1], tl.in[lane][k + 2],
-                                   tl.io[lane][k], y);
-                    if (t == e) y = fma_x(-chv, hi, y);
-                    tl.io[lane][k] = y;
-                }
-            }
-        }
-        __syncwarp();
-        vtile_copy<VT + 1, VT, false>(&tl.io[0][0], (const T *)nullptr, out, i0, ny, nrows, tb, kk, lane);
-        __syncwarp();
-    }
-    // back substitution x_t = y_t - g_t x_{t+1} (x_e = y_e), tiles right to left
-    T x = y;
-    for (int te = e - 1; te >= 1; te -= VT) {
-        const int kk = min(VT, te), ts = te - kk + 1;
-        vtile_copy<VT + 1, VT, true>(&tl.io[0][0], out, (T *)nullptr, i0, ny, nrows, ts, kk, lane);
-        __syncwarp();
-        if (act) {
-#pragma unroll
-            for (int k = VT - 1; k >= 0; --k) {
-                if (k < kk) {
-                    const int t = ts + k;
-                    x = fma_x(-ldg(v.Vt(VL_G) + (long long)t * nx + i), x, tl.io[lane][k]);
-                    tl.io[lane][k] = x;
-                }
-            }
-        }
-        __syncwarp();
-        vtile_copy<VT + 1, VT, false>(&tl.io[0][0], (const T *)nullptr, out, i0, ny, nrows, ts, kk, lane);
-        __syncwarp();
-    }
-    if (act) {
-        const long long row = (long long)i * ny;
-        out[row] = lo;
-        out[row + ny - 1] = hi;
-    }
-}
-
-// v_stage through the warp tiles: the warp of lane (l0 mod 32) takes lines i0 = 1 + (l0 - lane),
-// i0 + ls, ... (ls a multiple of 32, all lanes of a warp in the same work split).
-template <typename T>
-__device__ __forceinline__ void v_stage_tiled(const inst_view<T> &v, const T *__restrict__ in, const T *__restrict__ inh,
-                                              const T *__restrict__ sb0, T *__restrict__ out, int l0, int ls,
-                                              vtile<T> &tl)
-{
-    const int nx = v.nx;
-    for (int i0 = 1 + (l0 & ~31); i0 <= nx - 2; i0 += ls) v_lines_tiled<T>(v, in, inh, sb0, out, i0, tl);
-}
-
 template <typename T> __device__ __forceinline__ inst_view<T> make_view(const bparams<T> &p, const bdesc &d)
 {
     inst_view<T> v;
@@ -944,8 +759,8 @@ __global__ void __launch_bounds__(BATCH_CTA, LSS_FWDADJ_MIN_CTAS) k_batch_fwdadj
 }
 
 // ------------------------------------------------------------------------------------------
-// wide path: one (large) instance, one kernel per stage over all threads of the grid, same
-// stage arithmetic as the batched kernel (bit-identical results for the same instance)
+// wide path: one instance, a thread per line and one kernel per stage over all threads of the grid,
+// the batched kernel's stage arithmetic (bit-identical results; LSS_ADI_OPT_LINE_PER_THREAD)
 // ------------------------------------------------------------------------------------------
 __device__ __forceinline__ int gtid() { return blockIdx.x * blockDim.x + threadIdx.x; }
 __device__ __forceinline__ int gstride() { return gridDim.x * blockDim.x; }
@@ -963,19 +778,12 @@ __global__ void k_wide_s(const __grid_constant__ bparams<T> p, const T *U, const
     const inst_view<T> v = make_view(p, d);
     with_scheme(d.scheme, [&](auto sch) { s_stage<T, KIND, decltype(sch)::value>(v, U, Y1, Y2, Y, gtid(), gstride()); });
 }
-// thread-per-line v sweep of the wide path, rows through shared-memory tiles (TILED) or read in
-// place; the two give the same bits, the autotuner keeps the faster for the instance
-template <typename T, bool TILED>
+template <typename T>
 __global__ void k_wide_v(const __grid_constant__ bparams<T> p, const T *in, const T *inh, const T *b0, T *out)
 {
     const bdesc d = p.desc[0];
     const inst_view<T> v = make_view(p, d);
-    if constexpr (TILED) {
-        __shared__ vtile<T> s_vt[1]; // blocks of one warp
-        v_stage_tiled<T>(v, in, inh, b0, out, gtid(), gstride(), s_vt[0]);
-    } else {
-        v_stage<T>(v, in, inh, b0, out, gtid(), gstride());
-    }
+    v_stage<T>(v, in, inh, b0, out, gtid(), gstride());
 }
 template <typename T> __global__ void k_wide_b2(const __grid_constant__ bparams<T> p, T *Vn)
 {
@@ -983,743 +791,6 @@ template <typename T> __global__ void k_wide_b2(const __grid_constant__ bparams<
     const inst_view<T> v = make_view(p, d);
     b2_stage<T>(v, Vn, gtid(), gstride());
 }
-// Partitioned line solves of the wide path.  A large single instance has only Nx or Ny
-// lines per sweep -- a few warps per SM, far below what the FP64 pipe needs -- so each line
-// is cut into P chunks solved concurrently (CTA: L = 8, 16 or 32 lines x P chunks).  Both recurrences
-// of the factorised solve are first order and linear:
-//   y_t = f_t - la_t y_{t-1}:  y_t = yhat_t + hf_t y_in,  hf_t = prod_{s=t0..t} (-la_s)
-//   x_t = y_t - g_t x_{t+1}:   x_t = xhat_t + hb_t x_in,  hb_t = prod_{s=t..t1} (-g_s)
-// where yhat / xhat are the chunk-local solutions from a zero start and hf / hb the
-// time-invariant chunk products (k_wide_spikes).  A chunk's incoming value is composed
-// from the other chunks' end values in shared memory.  Three passes over the chunk: local
-// forward solve; forward fix-up fused with the local back substitution; back fix-up.
-__device__ __forceinline__ void chunk_range(int e, int P, int c, int &t0, int &t1)
-{
-    t0 = 1 + static_cast<int>((static_cast<long long>(c) * e) / P);
-    t1 = static_cast<int>((static_cast<long long>(c + 1) * e) / P);
-}
-
-// The recurrence of the time-dependent S-line factorisation, partitioned like the line solves
-// (CTA: L lines x P chunks).  beta_t = b_t - a_t c_{t-1} / beta_{t-1} is the Moebius map of the
-// matrix [[b_t, -a_t c_{t-1}], [1, 0]] applied to beta_{t-1}: each chunk forms the product of its
-// rows' matrices (rescaled every 8 rows: only the ratio matters), a chunk composes the maps of
-// the chunks before it to get its incoming beta, then runs its own rows' recurrence from it
-// (1/beta and gamma = c/beta), so the serial chain is a chunk long instead of a line long.
-// Same values as the serial recurrence up to the rounding of the incoming beta of each chunk.
-template <typename T>
-__global__ void __launch_bounds__(1024) k_tdep_s_factor(const double *__restrict__ base, long long n, int nx, int ny,
-                                                        double th, T *S0)
-{
-    __shared__ double sm[4][1024]; // each chunk's map [[m11, m12], [m21, m22]], indexed [c * L + line]
-    const int L = blockDim.x, P = blockDim.y, lane = threadIdx.x, c = threadIdx.y;
-    const int j = 1 + blockIdx.x * L + lane;
-    const bool act = j <= ny - 2;
-    const int e = nx - 2, k = c * L + lane;
-    int t0, t1;
-    chunk_range(e, P, c, t0, t1);
-    const double *__restrict__ bM = base, *__restrict__ bP = base + n, *__restrict__ bZ = base + 2 * n;
-    if (act) {
-        double m11 = 1.0, m12 = 0.0, m21 = 0.0, m22 = 1.0;
-        double pprev = t0 > 1 ? bP[(long long)(t0 - 1) * ny + j] : 0.0; // P of row t-1 (c_{t-1} = -theta P)
-        for (int t = t0; t <= t1; ++t) {
-            const long long o = (long long)t * ny + j;
-            const double b = 1.0 + th * bZ[o];
-            const double ac = t > 1 ? (-th * bM[o]) * (-th * pprev) : 0.0; // a_t c_{t-1}
-            pprev = bP[o];
-            const double n11 = b * m11 - ac * m21, n12 = b * m12 - ac * m22;
-            m21 = m11;
-            m22 = m12;
-            m11 = n11;
-            m12 = n12;
-            if (((t - t0) & 7) == 7) {
-                const double sc = 1.0 / fmax(fabs(m11), fabs(m21));
-                m11 *= sc; m12 *= sc; m21 *= sc; m22 *= sc;
-            }
-        }
-        sm[0][k] = m11; sm[1][k] = m12; sm[2][k] = m21; sm[3][k] = m22;
-    }
-    __syncthreads();
-    if (!act) return;
-    // beta_{t0-1}: the maps of chunks 0 .. c-1 applied in order (chunk 0 starts at row 1, whose
-    // map ignores its argument: a_1 c_0 = 0)
-    double x = 1.0;
-    for (int q = 0; q < c; ++q) {
-        const int kq = q * L + lane;
-        x = (sm[0][kq] * x + sm[1][kq]) / (sm[2][kq] * x + sm[3][kq]);
-    }
-    double gam = t0 > 1 ? (-th * bP[(long long)(t0 - 1) * ny + j]) / x : 0.0;
-    for (int t = t0; t <= t1; ++t) {
-        const long long o = (long long)t * ny + j;
-        const double a = -th * bM[o], b = 1.0 + th * bZ[o], cc = -th * bP[o];
-        const double beta = (t == 1) ? b : b - a * gam;
-        S0[SL_IB * n + o] = static_cast<T>(1.0 / beta);
-        if (t < e) gam = cc / beta;
-        S0[SL_G * n + o] = static_cast<T>(t < e ? gam : 0.0);
-    }
-}
-
-// hf / hb of every chunk of every line; lines along j ([t][j] tables, S) or i ([t][i], v)
-template <typename T>
-__global__ void k_wide_spikes(const T *__restrict__ la, const T *__restrict__ g, T *__restrict__ hf,
-                              T *__restrict__ hb, int lines, int stride, int e, int P)
-{
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= (lines - 2) * P) return;
-    const int l = 1 + q / P, c = q % P;
-    int t0, t1;
-    chunk_range(e, P, c, t0, t1);
-    T pr = T(1);
-    for (int t = t0; t <= t1; ++t) {
-        const long long o = (long long)t * stride + l;
-        pr *= -la[o];
-        hf[o] = pr;
-    }
-    pr = T(1);
-    for (int t = t1; t >= t0; --t) {
-        const long long o = (long long)t * stride + l;
-        pr *= -g[o];
-        hb[o] = pr;
-    }
-}
-
-template <typename T, int KIND>
-__global__ void __launch_bounds__(1024) k_wide_s_chunk(const __grid_constant__ bparams<T> p, const T *U, const T *Y1,
-                                                        const T *Y2, T *Y, const T *__restrict__ hf,
-                                                        const T *__restrict__ hb)
-{
-    __shared__ T sa_s[1024], sb_s[1024];
-    const carry2d<T> sa{sa_s, static_cast<int>(blockDim.x)}, sb{sb_s, static_cast<int>(blockDim.x)};
-    const bdesc d = p.desc[0];
-    const inst_view<T> v = make_view(p, d);
-    const int nx = d.nx, ny = d.ny, e = nx - 2, P = blockDim.y, c = threadIdx.y, lane = threadIdx.x;
-    const int j = 1 + blockIdx.x * blockDim.x + lane;
-    const bool act = j <= ny - 2;
-    int t0, t1;
-    chunk_range(e, P, c, t0, t1);
-    T lo = T(0), hi = T(0);
-    if (act) {
-        const int jj = ldg(v.jmap() + j);
-        lo = U[jj];
-        hi = U[(long long)(nx - 1) * ny + jj];
-        with_scheme(d.scheme, [&](auto sch) {
-            sb[c][lane] = s_line_fwd<T, KIND, decltype(sch)::value>(v, U, Y1, Y2, Y, j, t0, t1, c == 0 ? lo : T(0), hi);
-        });
-        sa[c][lane] = hf[(long long)t1 * ny + j];
-    }
-    __syncthreads();
-    T xh = T(0);
-    if (act) {
-        T yin = T(0);
-        if (c > 0) {
-            yin = sb[0][lane];
-            for (int q = 1; q < c; ++q) yin = sb[q][lane] + sa[q][lane] * yin;
-        }
-        for (int t = t1; t >= t0; --t) {
-            const long long o = (long long)t * ny + j;
-            const T y = (c > 0) ? Y[o] + hf[o] * yin : Y[o];
-            xh = y - ldg(v.S(SL_G) + o) * xh;
-            Y[o] = xh;
-        }
-    }
-    __syncthreads();
-    if (act) {
-        sb[c][lane] = xh;
-        sa[c][lane] = hb[(long long)t0 * ny + j];
-    }
-    __syncthreads();
-    if (act) {
-        if (c < P - 1) {
-            T xin = sb[P - 1][lane];
-            for (int q = P - 2; q > c; --q) xin = sb[q][lane] + sa[q][lane] * xin;
-            for (int t = t0; t <= t1; ++t) {
-                const long long o = (long long)t * ny + j;
-                Y[o] += hb[o] * xin;
-            }
-        }
-        if (c == 0) Y[j] = lo;
-        if (c == P - 1) Y[(long long)(nx - 1) * ny + j] = hi;
-    }
-}
-
-// Partitioned v sweep with the rows read in place (see k_wide_s_chunk; same bits as
-// k_wide_v_chunk, whose rows go through shared-memory tiles).
-template <typename T>
-__global__ void __launch_bounds__(1024) k_wide_v_chunk_plain(const __grid_constant__ bparams<T> p, const T *in, const T *inh,
-                                                        const T *b0, T *out, const T *__restrict__ hf,
-                                                        const T *__restrict__ hb)
-{
-    __shared__ T sa_s[1024], sb_s[1024];
-    const carry2d<T> sa{sa_s, static_cast<int>(blockDim.x)}, sb{sb_s, static_cast<int>(blockDim.x)};
-    const bdesc d = p.desc[0];
-    const inst_view<T> v = make_view(p, d);
-    const int nx = d.nx, ny = d.ny, e = ny - 2, P = blockDim.y, c = threadIdx.y, lane = threadIdx.x;
-    const int i = 1 + blockIdx.x * blockDim.x + lane;
-    const bool act = i <= nx - 2;
-    const long long row = (long long)i * ny;
-    int t0, t1;
-    chunk_range(e, P, c, t0, t1);
-    T lo = T(0), hi = T(0);
-    if (act) {
-        const int ii = ldg(v.imap() + i);
-        lo = b0[ii];
-        hi = ldg(v.X(X_VHI) + ii);
-        sb[c][lane] = v_line_fwd<T>(v, in, inh, out, i, t0, t1, c == 0 ? lo : T(0), hi);
-        sa[c][lane] = hf[(long long)t1 * nx + i];
-    }
-    __syncthreads();
-    T xh = T(0);
-    if (act) {
-        T yin = T(0);
-        if (c > 0) {
-            yin = sb[0][lane];
-            for (int q = 1; q < c; ++q) yin = fma_x(sa[q][lane], yin, sb[q][lane]);
-        }
-        for (int t = t1; t >= t0; --t) {
-            const long long ot = (long long)t * nx + i;
-            const T y = (c > 0) ? fma_x(hf[ot], yin, out[row + t]) : out[row + t];
-            xh = fma_x(-ldg(v.Vt(VL_G) + ot), xh, y);
-            out[row + t] = xh;
-        }
-    }
-    __syncthreads();
-    if (act) {
-        sb[c][lane] = xh;
-        sa[c][lane] = hb[(long long)t0 * nx + i];
-    }
-    __syncthreads();
-    if (act) {
-        if (c < P - 1) {
-            T xin = sb[P - 1][lane];
-            for (int q = P - 2; q > c; --q) xin = fma_x(sa[q][lane], xin, sb[q][lane]);
-            for (int t = t0; t <= t1; ++t) out[row + t] = fma_x(hb[(long long)t * nx + i], xin, out[row + t]);
-        }
-        if (c == 0) out[row] = lo;
-        if (c == P - 1) out[row + ny - 1] = hi;
-    }
-}
-
-// Copy between global memory and a warp's tile where each tile row r has its own global offset
-// and length: owner(r, off, cnt) gives them (cnt = 0 for rows without work); `lane`: this
-// thread's lane in its warp.
-template <int W, int CMAX, bool LOAD, typename T, typename F>
-__device__ __forceinline__ void vtile_copy_rows(T *tile, const T *src, T *dst, F owner, int lane)
-{
-#pragma unroll
-    for (int q = 0; q < CMAX; ++q) {
-        const int idx = lane + 32 * q, r = idx / CMAX, c = idx % CMAX;
-        long long off;
-        int cnt;
-        owner(r, off, cnt);
-        if (c < cnt) {
-            if constexpr (LOAD) tile[r * W + c] = src[off + c];
-            else dst[off + c] = tile[r * W + c];
-        }
-    }
-}
-
-// Partitioned v sweep (see k_wide_s_chunk) with the rows of `in`, `inh` and `out` moved through
-// per-warp shared-memory tiles (v_lines_tiled): the CTA's threads are (lines x chunks) with the
-// line index fastest, so a warp holds 32 / L chunks of L lines (or one chunk of 32 lines), each
-// lane its own line and chunk.  Every tile row is a contiguous segment of one state row; the
-// arithmetic per point is that of the thread-per-line recurrences, operation for operation.
-// The CTA must be whole warps (L * P a multiple of 32, set_wide_chunks).  Dynamic shared memory:
-// one vtile per warp.
-template <typename T>
-__global__ void __launch_bounds__(1024) k_wide_v_chunk(const __grid_constant__ bparams<T> p, const T *in, const T *inh,
-                                                        const T *b0, T *out, const T *__restrict__ hf,
-                                                        const T *__restrict__ hb)
-{
-    __shared__ T sa_s[1024], sb_s[1024];
-    const carry2d<T> sa{sa_s, static_cast<int>(blockDim.x)}, sb{sb_s, static_cast<int>(blockDim.x)};
-    extern __shared__ unsigned char vt_raw[];
-    const bdesc d = p.desc[0];
-    const inst_view<T> v = make_view(p, d);
-    const int nx = d.nx, ny = d.ny, e = ny - 2, P = blockDim.y, c = threadIdx.y, lane = threadIdx.x, L = blockDim.x;
-    const int lin = c * L + lane, w = lin >> 5, wl = lin & 31;
-    vtile<T> &tl = reinterpret_cast<vtile<T> *>(vt_raw)[w];
-    const int i = 1 + blockIdx.x * L + lane;
-    const bool act = i <= nx - 2;
-    const long long row = (long long)i * ny;
-    int t0, t1;
-    chunk_range(e, P, c, t0, t1);
-    // tile row r of this warp: line and chunk of the warp's lane r
-    auto line_of = [&](int r, int &ir, int &cr) {
-        const int lr = (w << 5) + r;
-        cr = lr / L;
-        ir = 1 + blockIdx.x * L + lr % L;
-    };
-    const int steps = (t1 - t0 + VT) / VT; // tiles of this lane's chunk
-    int steps_max = steps;
-    for (int off = 16; off > 0; off >>= 1) steps_max = max(steps_max, __shfl_xor_sync(0xffffffffu, steps_max, off));
-    T lo = T(0), hi = T(0);
-    if (act) {
-        const int ii = ldg(v.imap() + i);
-        lo = b0[ii];
-        hi = ldg(v.X(X_VHI) + ii);
-    }
-    const T chv = act ? ldg(v.X(X_CHV) + i) : T(0);
-    // pass 1: local forward recurrence of the chunk (from lo on chunk 0, from 0 on the others)
-    T y = c == 0 ? lo : T(0);
-    for (int jt = 0; jt < steps_max; ++jt) {
-        auto own_in = [&](int r, long long &off, int &cnt) {
-            int ir, cr, a, b;
-            line_of(r, ir, cr);
-            chunk_range(e, P, cr, a, b);
-            const int tb = a + jt * VT, kk = min(VT, b - tb + 1);
-            cnt = (ir <= nx - 2 && kk > 0) ? kk + 2 : 0;
-            off = (long long)ir * ny + tb - 1;
-        };
-        auto own_h = [&](int r, long long &off, int &cnt) {
-            int ir, cr, a, b;
-            line_of(r, ir, cr);
-            chunk_range(e, P, cr, a, b);
-            const int tb = a + jt * VT, kk = min(VT, b - tb + 1);
-            cnt = (ir <= nx - 2 && kk > 0) ? kk : 0;
-            off = (long long)ir * ny + tb;
-        };
-        vtile_copy_rows<VT + 3, VT + 2, true>(&tl.in[0][0], in, (T *)nullptr, own_in, wl);
-        vtile_copy_rows<VT + 1, VT, true>(&tl.io[0][0], inh, (T *)nullptr, own_h, wl);
-        __syncwarp();
-        const int tb = t0 + jt * VT, kk = min(VT, t1 - tb + 1);
-        if (act) {
-#pragma unroll
-            for (int k = 0; k < VT; ++k) {
-                if (k < kk) {
-                    const int t = tb + k;
-                    const long long ot = (long long)t * nx + i;
-                    y = v_point<T>(ldg(v.Vt(VL_LA) + ot), ldg(v.Vt(VL_VC) + ot), ldg(v.Vt(VL_VN) + ot),
-                                   ldg(v.Vt(VL_IB) + ot), tl.in[wl][k], tl.in[wl][k + 1], tl.in[wl][k + 2],
-                                   tl.io[wl][k], y);
-                    if (t == e) y = fma_x(-chv, hi, y);
-                    tl.io[wl][k] = y;
-                }
-            }
-        }
-        __syncwarp();
-        vtile_copy_rows<VT + 1, VT, false>(&tl.io[0][0], (const T *)nullptr, out, own_h, wl);
-        __syncwarp();
-    }
-    if (act) {
-        sb[c][lane] = y;
-        sa[c][lane] = hf[(long long)t1 * nx + i];
-    }
-    __syncthreads();
-    // pass 2: forward fix-up y += hf yin with the incoming value composed from the chunks before,
-    // fused with the chunk's back substitution from a zero start
-    T yin = T(0);
-    if (act && c > 0) {
-        yin = sb[0][lane];
-        for (int q = 1; q < c; ++q) yin = fma_x(sa[q][lane], yin, sb[q][lane]);
-    }
-    T xh = T(0);
-    for (int jt = 0; jt < steps_max; ++jt) {
-        // tiles from the chunk's end: columns [b - (jt+1) VT + 1, b - jt VT] clipped to the chunk
-        auto own_b = [&](int r, long long &off, int &cnt) {
-            int ir, cr, a, b;
-            line_of(r, ir, cr);
-            chunk_range(e, P, cr, a, b);
-            const int te = b - jt * VT, ts = max(a, te - VT + 1);
-            cnt = (ir <= nx - 2 && te >= a) ? te - ts + 1 : 0;
-            off = (long long)ir * ny + ts;
-        };
-        vtile_copy_rows<VT + 1, VT, true>(&tl.io[0][0], out, (T *)nullptr, own_b, wl);
-        __syncwarp();
-        const int te = t1 - jt * VT, ts = max(t0, te - VT + 1);
-        if (act && te >= t0) {
-#pragma unroll
-            for (int k = VT - 1; k >= 0; --k) {
-                if (k <= te - ts) {
-                    const int t = ts + k;
-                    const long long ot = (long long)t * nx + i;
-                    const T yv = (c > 0) ? fma_x(hf[ot], yin, tl.io[wl][k]) : tl.io[wl][k];
-                    xh = fma_x(-ldg(v.Vt(VL_G) + ot), xh, yv);
-                    tl.io[wl][k] = xh;
-                }
-            }
-        }
-        __syncwarp();
-        vtile_copy_rows<VT + 1, VT, false>(&tl.io[0][0], (const T *)nullptr, out, own_b, wl);
-        __syncwarp();
-    }
-    __syncthreads();
-    if (act) {
-        sb[c][lane] = xh;
-        sa[c][lane] = hb[(long long)t0 * nx + i];
-    }
-    __syncthreads();
-    // pass 3: backward fix-up x += hb xin (all chunks but the last)
-    T xin = T(0);
-    if (act && c < P - 1) {
-        xin = sb[P - 1][lane];
-        for (int q = P - 2; q > c; --q) xin = fma_x(sa[q][lane], xin, sb[q][lane]);
-    }
-    for (int jt = 0; jt < steps_max; ++jt) {
-        auto own_f = [&](int r, long long &off, int &cnt) {
-            int ir, cr, a, b;
-            line_of(r, ir, cr);
-            chunk_range(e, P, cr, a, b);
-            const int tb = a + jt * VT, kk = min(VT, b - tb + 1);
-            cnt = (ir <= nx - 2 && kk > 0 && cr < P - 1) ? kk : 0;
-            off = (long long)ir * ny + tb;
-        };
-        vtile_copy_rows<VT + 1, VT, true>(&tl.io[0][0], out, (T *)nullptr, own_f, wl);
-        __syncwarp();
-        const int tb = t0 + jt * VT, kk = min(VT, t1 - tb + 1);
-        if (act && c < P - 1) {
-#pragma unroll
-            for (int k = 0; k < VT; ++k)
-                if (k < kk) tl.io[wl][k] = fma_x(hb[(long long)(tb + k) * nx + i], xin, tl.io[wl][k]);
-        }
-        __syncwarp();
-        vtile_copy_rows<VT + 1, VT, false>(&tl.io[0][0], (const T *)nullptr, out, own_f, wl);
-        __syncwarp();
-    }
-    if (act) {
-        if (c == 0) out[row] = lo;
-        if (c == P - 1) out[row + ny - 1] = hi;
-    }
-}
-
-// ------------------------------------------------------------------------------------------
-// wide forward + adjoint of one large FP64 instance: the adjoint stages of adi_adjoint.cuh as
-// one kernel each over all threads (thread per line / column), host-sequenced like the
-// forward; each thread's parameter sums live in `acc` (structure of arrays, 10 x nthr) between
-// kernels and are reduced once at the end.
-// ------------------------------------------------------------------------------------------
-__device__ __forceinline__ void acc_load(adj_acc &acc, const double *a, long long nthr, long long t)
-{
-    for (int q = 0; q < 5; ++q) acc.s[q] = a[q * nthr + t];
-    acc.vk = a[5 * nthr + t];
-    acc.vt = a[6 * nthr + t];
-    acc.vs1 = a[7 * nthr + t];
-    acc.vs2 = a[8 * nthr + t];
-    acc.vb = a[9 * nthr + t];
-}
-__device__ __forceinline__ void acc_store(const adj_acc &acc, double *a, long long nthr, long long t)
-{
-    for (int q = 0; q < 5; ++q) a[q * nthr + t] = acc.s[q];
-    a[5 * nthr + t] = acc.vk;
-    a[6 * nthr + t] = acc.vt;
-    a[7 * nthr + t] = acc.vs1;
-    a[8 * nthr + t] = acc.vs2;
-    a[9 * nthr + t] = acc.vb;
-}
-
-__global__ void k_wadj_b2(const __grid_constant__ bparams<double> p, double *VB, double *UB)
-{
-    const bdesc d = p.desc[0];
-    const inst_view<double> v = make_view(p, d);
-    adj_b2(v, VB, UB, d.scheme == LSS_ADI_HUNDSDORFER_VERWER, gtid(), gstride());
-}
-
-template <bool FIRST>
-__global__ void k_wadj_v(const __grid_constant__ bparams<double> p, const double *in, const double *out, const double *XB,
-                         double *INB, double *INHB, double *TMP, double *LV, double *acc_a, long long nacc)
-{
-    const bdesc d = p.desc[0];
-    const inst_view<double> v = make_view(p, d);
-    const long long t = gtid();
-    adj_acc acc;
-    acc_load(acc, acc_a, nacc, t);
-    adj_v<FIRST>(v, in, out, XB, INB, INHB, TMP, LV, acc, gtid(), gstride());
-    acc_store(acc, acc_a, nacc, t);
-}
-
-template <int KIND>
-__global__ void k_wadj_s(const __grid_constant__ bparams<double> p, const double *U, const double *Y1, const double *Y2,
-                         const double *Yo, const double *XB, double *FB, double *TMP, double *LS, double *HS, double *UB,
-                         double *Y1B, double *acc_a, long long nacc, double tau)
-{
-    const bdesc d = p.desc[0];
-    const inst_view<double> v = make_view(p, d);
-    const long long t = gtid();
-    adj_acc acc;
-    acc_load(acc, acc_a, nacc, t);
-    with_scheme(d.scheme, [&](auto sch) {
-        adj_s<KIND, decltype(sch)::value>(v, d, U, Y1, Y2, Yo, XB, FB, TMP, LS, HS, UB, Y1B, acc, tau, gtid(), gstride());
-    });
-    acc_store(acc, acc_a, nacc, t);
-}
-
-// Partitioned adjoint line solves (the wide adjoint's counterpart of k_wide_s_chunk /
-// k_wide_v_chunk): the transposed factorised solve
-//   z_t = xbar_t - g_{t-1} z_{t-1}  (t = 1..e),   w_t = z_t - la_{t+1} w_{t+1}  (t = e..1)
-// is cut into chunks with the chunk products hz_t = prod_{s=t0..t} (-g_{s-1}) and
-// hw_t = prod_{s=t..t1} (-la_{s+1}); after the final w of the whole line is in TMP, each chunk
-// applies the point-local terms (right-hand-side adjoints, parameter sums).
-template <typename T>
-__global__ void k_wadj_spikes(const T *__restrict__ la, const T *__restrict__ g, T *__restrict__ hz,
-                              T *__restrict__ hw, int lines, int stride, int e, int P)
-{
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= (lines - 2) * P) return;
-    const int l = 1 + q / P, c = q % P;
-    int t0, t1;
-    chunk_range(e, P, c, t0, t1);
-    T pr = T(1);
-    for (int t = t0; t <= t1; ++t) {
-        pr *= (t > 1) ? -g[(long long)(t - 1) * stride + l] : T(0);
-        hz[(long long)t * stride + l] = pr;
-    }
-    pr = T(1);
-    for (int t = t1; t >= t0; --t) {
-        pr *= (t < e) ? -la[(long long)(t + 1) * stride + l] : T(0);
-        hw[(long long)t * stride + l] = pr;
-    }
-}
-
-// z and w of one chunk of a line: element t of the line at base[t * st] in TMP, tables at
-// tab + t * ts; carries through the block's shared arrays (rows: chunks, columns: lines).
-__device__ __forceinline__ void adj_chunk_solve(double *__restrict__ TMP, long long base, long long st,
-                                                const double *__restrict__ XB, const double *__restrict__ G,
-                                                const double *__restrict__ LA, const double *__restrict__ hz,
-                                                const double *__restrict__ hw, long long tab, long long ts, int e,
-                                                int t0, int t1, int c, int P, int lane, bool act,
-                                                const carry2d<double> &sa, const carry2d<double> &sb)
-{
-    double z = 0.0;
-    if (act) {
-        for (int t = t0; t <= t1; ++t) {
-            const double gprev = (t > 1) ? __ldg(G + tab + (long long)(t - 1) * ts) : 0.0;
-            z = XB[base + t * st] - gprev * z;
-            TMP[base + t * st] = z;
-        }
-        sb[c][lane] = z;
-        sa[c][lane] = hz[tab + (long long)t1 * ts];
-    }
-    __syncthreads();
-    double w = 0.0;
-    if (act) {
-        double zin = 0.0;
-        if (c > 0) {
-            zin = sb[0][lane];
-            for (int q = 1; q < c; ++q) zin = sb[q][lane] + sa[q][lane] * zin;
-        }
-        double la_next = 0.0;
-        for (int t = t1; t >= t0; --t) {
-            const double zt = (c > 0) ? TMP[base + t * st] + hz[tab + (long long)t * ts] * zin : TMP[base + t * st];
-            w = zt - la_next * w;
-            TMP[base + t * st] = w;
-            la_next = __ldg(LA + tab + (long long)t * ts);
-        }
-    }
-    __syncthreads();
-    if (act) {
-        sb[c][lane] = w;
-        sa[c][lane] = hw[tab + (long long)t0 * ts];
-    }
-    __syncthreads();
-    if (act && c < P - 1) {
-        double win = sb[P - 1][lane];
-        for (int q = P - 2; q > c; --q) win = sb[q][lane] + sa[q][lane] * win;
-        for (int t = t0; t <= t1; ++t) TMP[base + t * st] += hw[tab + (long long)t * ts] * win;
-    }
-    __syncthreads();
-}
-
-template <bool FIRST>
-__global__ void __launch_bounds__(1024) k_wadj_v_chunk(const __grid_constant__ bparams<double> p, const double *in,
-                                                        const double *out, const double *XB, double *INB, double *INHB,
-                                                        double *TMP, double *LV, double *acc_a, long long nacc,
-                                                        const double *__restrict__ hz, const double *__restrict__ hw)
-{
-    __shared__ double sa_s[1024], sb_s[1024];
-    const carry2d<double> sa{sa_s, static_cast<int>(blockDim.x)}, sb{sb_s, static_cast<int>(blockDim.x)};
-    const bdesc d = p.desc[0];
-    const inst_view<double> v = make_view(p, d);
-    const int nx = d.nx, ny = d.ny, e = ny - 2, P = blockDim.y, c = threadIdx.y, lane = threadIdx.x;
-    const int i = 1 + blockIdx.x * blockDim.x + lane;
-    const bool act = i <= nx - 2;
-    const long long row = (long long)i * ny, tid = ((long long)blockIdx.x * P + c) * blockDim.x + lane;
-    int t0, t1;
-    chunk_range(e, P, c, t0, t1);
-    adj_chunk_solve(TMP, row, 1, XB, v.Vt(VL_G), v.Vt(VL_LA), hz, hw, i, nx, e, t0, t1, c, P, lane, act, sa, sb);
-    if (!act) return;
-    adj_acc acc;
-    acc_load(acc, acc_a, nacc, tid);
-    const double *LA = v.Vt(VL_LA), *VC = v.Vt(VL_VC), *VN = v.Vt(VL_VN), *IB = v.Vt(VL_IB);
-    for (int t = t1; t >= t0; --t) {
-        const long long ot = (long long)t * nx + i;
-        const double w0 = TMP[row + t];
-        const double w1 = (t + 1 <= e) ? TMP[row + t + 1] : 0.0, w2 = (t + 2 <= e) ? TMP[row + t + 2] : 0.0;
-        const double la2 = (t + 2 <= e) ? __ldg(LA + ot + 2LL * nx) : 0.0, vc1 = (t + 1 <= e) ? __ldg(VC + ot + nx) : 0.0;
-        const double fin = la2 * w2 + vc1 * w1 + __ldg(VN + ot) * w0; // adjoint of in(t+1)
-        if (FIRST) INB[row + t + 1] = fin; else INB[row + t + 1] += fin;
-        const double mu = __ldg(IB + ot) * w0;
-        if (FIRST) INHB[row + t] = mu; else INHB[row + t] += mu;
-        adj_v_sum(v, t, mu, in[row + t - 1] - out[row + t - 1], in[row + t] - out[row + t],
-                  in[row + t + 1] - out[row + t + 1], acc);
-    }
-    if (c == 0) {
-        const double w1 = TMP[row + 1], w2 = (2 <= e) ? TMP[row + 2] : 0.0;
-        const double la1 = __ldg(LA + nx + i), la2 = (2 <= e) ? __ldg(LA + 2LL * nx + i) : 0.0;
-        const double a1 = la2 * w2 + __ldg(VC + nx + i) * w1, a0 = la1 * w1;
-        if (FIRST) { INB[row + 1] = a1; INB[row] = a0; }
-        else { INB[row + 1] += a1; INB[row] += a0; }
-        const double lob = -la1 * w1 + XB[row];
-        if (FIRST) LV[i] = lob; else LV[i] += lob;
-    }
-    acc_store(acc, acc_a, nacc, tid);
-}
-
-template <int KIND>
-__global__ void __launch_bounds__(1024) k_wadj_s_chunk(const __grid_constant__ bparams<double> p, const double *U,
-                                                        const double *Y1, const double *Y2, const double *Yo,
-                                                        const double *XB, double *FB, double *TMP, double *LS, double *HS,
-                                                        double *UB, double *Y1B, double *acc_a, long long nacc, double tau,
-                                                        const double *__restrict__ hz, const double *__restrict__ hw)
-{
-    __shared__ double sa_s[1024], sb_s[1024];
-    const carry2d<double> sa{sa_s, static_cast<int>(blockDim.x)}, sb{sb_s, static_cast<int>(blockDim.x)};
-    const bdesc d = p.desc[0];
-    const inst_view<double> v = make_view(p, d);
-    const int nx = d.nx, ny = d.ny, e = nx - 2, P = blockDim.y, c = threadIdx.y, lane = threadIdx.x;
-    const int j = 1 + blockIdx.x * blockDim.x + lane;
-    const bool act = j <= ny - 2;
-    const long long tid = ((long long)blockIdx.x * P + c) * blockDim.x + lane;
-    int t0, t1;
-    chunk_range(e, P, c, t0, t1);
-    adj_chunk_solve(TMP, j, ny, XB, v.S(SL_G), v.S(SL_LA), hz, hw, j, ny, e, t0, t1, c, P, lane, act, sa, sb);
-    if (!act) return;
-    const bool sabr = d.model == LSS_ADI_SABR;
-    const double th = d.a_theta, omth = 1.0 - d.a_theta;
-    adj_acc acc;
-    acc_load(acc, acc_a, nacc, tid);
-    const double *LA = v.S(SL_LA), *IB = v.S(SL_IB);
-    with_scheme(d.scheme, [&](auto sch) {
-        constexpr int SCH = decltype(sch)::value;
-        constexpr bool hv = SCH == LSS_ADI_HUNDSDORFER_VERWER;
-        s_sums ps = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-        // three-row window over the chunk's rows (adj_s_row / adj_s_point)
-        s_row rh = adj_s_row<KIND, SCH>(U, Y1, Y2, Yo, (long long)(t1 + 1) * ny + j, th, omth);
-        s_row rc = adj_s_row<KIND, SCH>(U, Y1, Y2, Yo, (long long)t1 * ny + j, th, omth);
-        for (int t = t1; t >= t0; --t) {
-            const long long o = (long long)t * ny + j;
-            const s_row rl = adj_s_row<KIND, SCH>(U, Y1, Y2, Yo, o - ny, th, omth);
-            const double w0 = TMP[o];
-            FB[o] = w0;
-            const double mu = __ldg(IB + o) * w0;
-            if constexpr (KIND == 2) {
-                const double w1 = (t + 1 <= e) ? TMP[o + ny] : 0.0, w2 = (t + 2 <= e) ? TMP[o + 2LL * ny] : 0.0;
-                const double la2 = (t + 2 <= e) ? __ldg(LA + o + 2LL * ny) : 0.0;
-                const double sc1 = (t + 1 <= e) ? __ldg(v.S(SL_S2SC) + o + ny) : 0.0;
-                const double fin = la2 * w2 + sc1 * w1 + __ldg(v.S(SL_S2SE) + o) * w0;
-                if constexpr (hv) {
-                    Y1B[o + ny] = fin;
-                } else {
-                    UB[o + ny] += fin;
-                    Y1B[o] = mu;
-                }
-            }
-            const double muX = mu * __ldg(v.X(X_HX) + t);
-            const double muC = sabr ? mu * __ldg(v.X(X_HC) + t) : muX;
-            adj_s_point<KIND, SCH>(v, ps, rh, rc, rl, mu, muX, muC, t, sabr);
-            rh = rc;
-            rc = rl;
-        }
-        if (c == 0) {
-            const double w1 = TMP[(long long)ny + j], la1 = __ldg(LA + ny + j);
-            LS[j] = -la1 * w1 + XB[j];
-            if constexpr (KIND == 2) {
-                const double w2 = (2 <= e) ? TMP[2LL * ny + j] : 0.0, la2 = (2 <= e) ? __ldg(LA + 2LL * ny + j) : 0.0;
-                const double a1 = la2 * w2 + __ldg(v.S(SL_S2SC) + ny + j) * w1, a0 = la1 * w1;
-                if constexpr (hv) {
-                    Y1B[(long long)ny + j] = a1;
-                    Y1B[j] = a0;
-                } else {
-                    UB[(long long)ny + j] += a1;
-                    UB[j] += a0;
-                }
-            }
-        }
-        if (c == P - 1) HS[j] = -__ldg(v.Yv(Y_CHS) + j) * TMP[(long long)e * ny + j] + XB[(long long)(nx - 1) * ny + j];
-        adj_s_line<KIND, SCH>(v, d, j, ps, tau, sabr, acc);
-    });
-    acc_store(acc, acc_a, nacc, tid);
-}
-
-// Gather with one thread per grid point; the B1 parameter sums of column 0 go to acc slot p.
-template <int KIND>
-__global__ void k_wadj_gather2d(const __grid_constant__ bparams<double> p, const double *U, const double *FB,
-                                const double *LS, const double *HS, const double *LV, double *UB, double *Y2B,
-                                double *acc_a, long long nacc, double tau)
-{
-    const bdesc d = p.desc[0];
-    const inst_view<double> v = make_view(p, d);
-    const long long n = (long long)d.nx * d.ny;
-    const long long o = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (o >= n) return;
-    const int pr = static_cast<int>(o / d.ny), q = static_cast<int>(o % d.ny);
-    double lsum = 0.0, hsum = 0.0;
-    if (pr == 0 || pr == d.nx - 1) adj_line_ends(v, LS, HS, q, lsum, hsum);
-    adj_acc acc;
-    if (q == 0) {
-        acc_load(acc, acc_a, nacc, pr);
-    } else {
-        for (int k = 0; k < 5; ++k) acc.s[k] = 0.0;
-        acc.vk = acc.vt = acc.vs1 = acc.vs2 = acc.vb = 0.0;
-    }
-    adj_gather_point<KIND>(v, d, U, FB, LV, UB, Y2B, acc, tau, pr, q, lsum, hsum);
-    if (q == 0) acc_store(acc, acc_a, nacc, pr);
-}
-
-// final surface out, adjoint arrays cleared, finiteness of the final surface
-__global__ void k_wadj_begin(const __grid_constant__ bparams<double> p, const double *cur, double *VB, double *FB,
-                             double *Y1B, double *Y3B)
-{
-    const bdesc d = p.desc[0];
-    const long long n = (long long)d.nx * d.ny;
-    int bad = 0;
-    for (long long q = gtid(); q < n; q += gstride()) {
-        const double val = cur[q];
-        bad |= !isfinite(val);
-        p.U[q] = val;
-        VB[q] = 0.0;
-        FB[q] = 0.0;
-        Y1B[q] = 0.0;
-        Y3B[q] = 0.0;
-    }
-    if (bad) atomicOr(p.status, 1);
-}
-// value and its bilinear weights as the adjoint seed
-__global__ void k_wadj_seed(const __grid_constant__ bparams<double> p, const double *cur, double *VB)
-{
-    const bdesc d = p.desc[0];
-    const long long o = (long long)d.i0 * d.ny + d.j0;
-    p.values[0] = d.w00 * cur[o] + d.w10 * cur[o + d.ny] + d.w01 * cur[o + 1] + d.w11 * cur[o + d.ny + 1];
-    p.final_in_v[0] = 0;
-    VB[o] = d.w00;
-    VB[o + d.ny] = d.w10;
-    VB[o + 1] = d.w01;
-    VB[o + d.ny + 1] = d.w11;
-}
-// sum of the per-thread parameter sums; output order kappa, theta, sigma, rho, r
-__global__ void __launch_bounds__(256) k_wadj_reduce(const __grid_constant__ bparams<double> p, const double *acc_a,
-                                                     long long nthr)
-{
-    __shared__ double red[10][256];
-    for (int q = 0; q < 10; ++q) {
-        double sum = 0.0;
-        for (long long t = threadIdx.x; t < nthr; t += 256) sum += acc_a[q * nthr + t];
-        red[q][threadIdx.x] = sum;
-    }
-    __syncthreads();
-    for (int h = 128; h > 0; h >>= 1) {
-        if (threadIdx.x < h)
-            for (int q = 0; q < 10; ++q) red[q][threadIdx.x] += red[q][threadIdx.x + h];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        const bdesc d = p.desc[0];
-        const double th = d.a_theta, ni = d.a_ni;
-        p.grads[0] = red[1][0] + ni * th * red[5][0];
-        p.grads[1] = red[2][0] + ni * th * red[6][0];
-        p.grads[2] = red[3][0] + ni * th * red[7][0] + d.a_betat * th * red[8][0];
-        p.grads[3] = red[4][0];
-        p.grads[4] = red[0][0] + d.a_halfk * th * red[9][0];
-    }
-}
-
 // value, finiteness flag and final-array flag of the single instance
 // value at the evaluation point and finiteness of the final surface, grid-wide (the status word
 // is cleared before the time loop; any block that sees a non-finite point sets it)
@@ -1847,33 +918,9 @@ template <typename T> struct batch_typed {
     // wide path (count == 1)
     dbuf<T> d_b0;
     cudaGraphExec_t wide_graph = nullptr;
-    int wide_ps = 1, wide_pv = 1;   // chunks per S line / per v line (1: thread per line)
-    int wide_ls = 32, wide_lv = 32; // lines per CTA of the partitioned kernels (CTA: lines x chunks)
-    bool wide_vtile = true;         // v sweeps move their rows through shared-memory tiles (same bits)
-    dbuf<T> d_spk;                  // chunk products: S hf, S hb, v hf, v hb (n each)
-    int set_wide_chunks(int ps, int pv, cudaStream_t s, int ls = 0, int lv = 0); // ls, lv 0: by SM count
-    int autotune_wide(cudaStream_t s);
-    template <int KIND> void launch_wide_s(cudaStream_t s, const bparams<T> &p, const T *U, const T *Y1, const T *Y2, T *Y);
-    void launch_wide_v(cudaStream_t s, const bparams<T> &p, const T *in, const T *inh, const T *b0, T *out);
     void enqueue_wide_step(cudaStream_t s, const bparams<T> &p, const T *U, T *Y1, T *Y2, T *Y3, T *V);
     int enqueue_wide(cudaStream_t s);
     int run_wide(cudaStream_t s, bool use_graph);
-    // wide forward + adjoint (count == 1, FP64)
-    dbuf<double> d_wws;
-    long long wws_need = 0;
-    dbuf<T> d_aspk;                 // adjoint chunk products: S hz, S hw, v hz, v hw (n each)
-    int aspk_ps = 0, aspk_pv = 0;
-    int enqueue_wide_adjoint(cudaStream_t s);
-    // time-dependent coefficients (SABR with r != 0; one FP64 instance on the wide kernels):
-    // before each step, forward or adjoint, the S-line tables are rebuilt at the step's time
-    bool tdep = false;
-    dbuf<double> td_buf;            // base tables (7 n), a_static, c_static, ab (n each), per_i (5 nx), xs (3 nx)
-    tdep_params td{};
-    std::vector<double> td_da, td_dc; // D(t)^(2(1-beta)), D(t)^(1-beta) per step
-    double td_theta = 0.0, td_zeta = 0.0, td_gamma = 0.0;
-    int init_tdep(const lss_adi_problem &p);
-    // products: 1 = the forward chunk products of the S lines, 2 = the adjoint's
-    void refresh_step(cudaStream_t s, int step, int products);
     int enqueue(int mode, cudaStream_t s);
     int run(int mode, cudaStream_t s, bool use_graph);
 };
@@ -1939,32 +986,25 @@ template <typename T> int batch_typed<T>::create(const lss_adi_problem *ps, int 
                     }
                     const double h1 = tt.sc.h1;
                     {
-                        // coefficient derivatives (adjoint), double.  Heston: a = vS^2/2, b = sigma^2 v/2,
-                        // c = rho sigma v S, d = rS, e = kappa (theta - v), f = -r.  SABR (r = 0, D = 1):
-                        // a = v^2 F^(2 beta) D^(2(1-beta))/2, b = nu^2 v^2/2, c = rho nu v^2 F^beta D^(1-beta),
-                        // d = rF, e = 0, f = -r (sigma carries nu).
+                        // coefficient derivatives (adjoint), double
                         sinh_map<double> g;
                         g.init(ps[k]);
                         const double sg = ps[k].sigma, bt = ps[k].sabr_beta;
-                        const bool sabr = ps[k].model == LSS_ADI_SABR;
                         for (int i = 0; i < d.nx; ++i) {
-                            const double z = static_cast<double>(tt.sc.h1) * i;
-                            const double x = g.x(z), A = g.a_der(z), Add = g.c_der(z);
-                            xh[X_HX * total_x + d.ox + i] = static_cast<T>(x / A);
-                            xh[X_HC * total_x + d.ox + i] = static_cast<T>(sabr ? std::pow(x, bt) / A : x / A);
-                            xh[X_HA * total_x + d.ox + i] = static_cast<T>(sabr ? std::pow(x, 2.0 * bt) / (A * A) : 0.0);
-                            xh[X_HDD * total_x + d.ox + i] = static_cast<T>(sabr ? std::pow(x, 2.0 * bt) * Add / (A * A * A) : 0.0);
+                            const s_factors q = derivative_s(ps[k], g, static_cast<double>(tt.sc.h1) * i);
+                            xh[X_HX * total_x + d.ox + i] = static_cast<T>(q.hx);
+                            xh[X_HC * total_x + d.ox + i] = static_cast<T>(q.hc);
+                            xh[X_HA * total_x + d.ox + i] = static_cast<T>(q.ha);
+                            xh[X_HDD * total_x + d.ox + i] = static_cast<T>(q.hdd);
                         }
                         for (int j = 0; j < d.ny; ++j) {
-                            const double e = static_cast<double>(tt.sc.h2) * j;
-                            const double B = g.b_der(e), Bdd = g.d_der(e), vv = g.y(e);
-                            const double vb = sabr ? vv * vv : vv; // the v factor of b and c
-                            yh[Y_HY * total_y + d.oy + j] = static_cast<T>(vb / B);
-                            yh[Y_BS * total_y + d.oy + j] = static_cast<T>(sg * vb / (B * B));
-                            yh[Y_EK * total_y + d.oy + j] = static_cast<T>(sabr ? 0.0 : (ps[k].theta_v - vv) / B);
-                            yh[Y_ET * total_y + d.oy + j] = static_cast<T>(sabr ? 0.0 : ps[k].kappa / B);
-                            yh[Y_ES * total_y + d.oy + j] = static_cast<T>(-sg * vb * Bdd / (B * B * B));
-                            yh[Y_HV2 * total_y + d.oy + j] = static_cast<T>(sabr ? 0.5 * vv * vv : 0.0);
+                            const v_factors q = derivative_v(ps[k], g, static_cast<double>(tt.sc.h2) * j);
+                            yh[Y_HY * total_y + d.oy + j] = static_cast<T>(q.hy);
+                            yh[Y_BS * total_y + d.oy + j] = static_cast<T>(q.bs);
+                            yh[Y_EK * total_y + d.oy + j] = static_cast<T>(q.ek);
+                            yh[Y_ET * total_y + d.oy + j] = static_cast<T>(q.et);
+                            yh[Y_ES * total_y + d.oy + j] = static_cast<T>(q.es);
+                            yh[Y_HV2 * total_y + d.oy + j] = static_cast<T>(q.hv2);
                         }
                         desc[k].model = ps[k].model;
                         desc[k].a_alphat = static_cast<double>(tt.sc.alpha);
@@ -2094,84 +1134,7 @@ template <typename T> int batch_typed<T>::create(const lss_adi_problem *ps, int 
     LSS_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "SM count");
     this->sms = sms;
     if (n == 1) LSS_CUDA_TRY(d_b0.alloc(desc[0].nx), "batch: allocating the boundary column");
-    if (n == 1 && time_dependent(ps[0])) return init_tdep(ps[0]);
     return LSS_ADI_OK;
-}
-
-// Device copies of the time-independent factors of a time-dependent instance (FP64 only).
-template <typename T> int batch_typed<T>::init_tdep(const lss_adi_problem &p)
-{
-    if (!std::is_same<T, double>::value)
-        return set_error(LSS_ADI_EUNSUPPORTED, "batch: time-dependent coefficients on the wide kernels are FP64 only");
-    instance_tables<double> tt;
-    build_tables<double>(p, tt);
-    const bdesc &d = desc[0];
-    const long long n = total_n;
-    const int nx = d.nx;
-    const size_t off_stat = 7 * static_cast<size_t>(n), off_pi = off_stat + 3 * static_cast<size_t>(n),
-                 off_xs = off_pi + 5 * static_cast<size_t>(nx), total = off_xs + 3 * static_cast<size_t>(nx);
-    std::vector<double> h(total, 0.0);
-    std::copy(tt.coef.begin(), tt.coef.end(), h.begin());
-    std::copy(tt.a_static.begin(), tt.a_static.end(), h.begin() + off_stat);
-    std::copy(tt.c_static.begin(), tt.c_static.end(), h.begin() + off_stat + n);
-    std::copy(tt.ab.begin(), tt.ab.end(), h.begin() + off_stat + 2 * n);
-    std::copy(tt.per_i.begin(), tt.per_i.end(), h.begin() + off_pi);
-    // the adjoint's S-factors at D = 1 (the arena holds them as built by create)
-    std::vector<T> xa(X_COUNT * static_cast<size_t>(total_x));
-    LSS_CUDA_TRY(cudaMemcpy(xa.data(), xarena.p, xa.size() * sizeof(T), cudaMemcpyDeviceToHost), "batch: x arena");
-    for (int i = 0; i < nx; ++i) {
-        h[off_xs + i] = static_cast<double>(xa[X_HA * total_x + i]);
-        h[off_xs + nx + i] = static_cast<double>(xa[X_HDD * total_x + i]);
-        h[off_xs + 2 * nx + i] = static_cast<double>(xa[X_HC * total_x + i]);
-    }
-    LSS_CUDA_TRY(td_buf.alloc(total), "batch: allocating time-dependent tables");
-    LSS_CUDA_TRY(td_buf.upload(h.data(), total), "batch: uploading time-dependent tables");
-    td_theta = tt.sc.theta;
-    td_zeta = tt.sc.zeta;
-    td_gamma = tt.sc.gamma;
-    LSS_CUDA_TRY(cudaDeviceSynchronize(), "batch: time-dependent tables");
-    td.base = td_buf.p;
-    td.a_static = td_buf.p + off_stat;
-    td.c_static = td_buf.p + off_stat + n;
-    td.ab = td_buf.p + off_stat + 2 * n;
-    td.per_i = td_buf.p + off_pi;
-    td.xs = td_buf.p + off_xs;
-    td.n = n;
-    td.nx = nx;
-    td.ny = d.ny;
-    td.alpha = tt.sc.alpha;
-    td.delta = tt.sc.delta;
-    td.two_alpha = tt.two_alpha;
-    td.half_rho_f = tt.half_rho_f;
-    td_da = tt.step_da;
-    td_dc = tt.step_dc;
-    tdep = true;
-    return LSS_ADI_OK;
-}
-
-// The S-line tables (and with `products` the chunk products of the partitioned solves) of
-// step `step` of a time-dependent instance, enqueued on s before that step's kernels.
-template <typename T> void batch_typed<T>::refresh_step(cudaStream_t s, int step, int products)
-{
-    const bdesc &d = desc[0];
-    const long long n = total_n;
-    k_tdep_refresh<T><<<grid_for(n, 256), 256, 0, s>>>(td, td_da[step], td_dc[step], xarena.p, total_x);
-    {
-        // chunks of at least 4 rows, at most 32; 8 lines per CTA
-        int P = 1;
-        while (P < 32 && d.nx - 2 >= 8 * P) P *= 2;
-        k_tdep_s_factor<T><<<grid_for(d.ny - 2, 8), dim3(8, P), 0, s>>>(td.base, n, d.nx, d.ny, td_theta, stab.p);
-    }
-    k_tdep_s_slots<T><<<grid_for(static_cast<long long>(d.nx - 2) * (d.ny - 2), 256), 256, 0, s>>>(
-        td.base, n, d.nx, d.ny, d.scheme, td_theta, td_zeta, td_gamma, stab.p, yarena.p + Y_CHS * total_y);
-    if (wide_ps > 1) {
-        const bparams<T> p = params();
-        const int g = grid_for(static_cast<long long>(d.ny - 2) * wide_ps, 128);
-        if (products & 1)
-            k_wide_spikes<T><<<g, 128, 0, s>>>(p.S[SL_LA], p.S[SL_G], d_spk.p, d_spk.p + n, d.ny, d.ny, d.nx - 2, wide_ps);
-        if (products & 2)
-            k_wadj_spikes<T><<<g, 128, 0, s>>>(p.S[SL_LA], p.S[SL_G], d_aspk.p, d_aspk.p + n, d.ny, d.ny, d.nx - 2, wide_ps);
-    }
 }
 
 template <typename T> int batch_typed<T>::prepare_adjoint(cudaStream_t s)
@@ -2492,164 +1455,21 @@ template <typename T> int batch_typed<T>::autotune(int mode, int *chosen, cudaSt
     return LSS_ADI_OK;
 }
 
-// S and v sweeps of the wide path: thread per line (P = 1, bit-identical to the batched
-// kernel) or the partitioned solve with the autotuned chunk counts.
-template <typename T>
-template <int KIND>
-void batch_typed<T>::launch_wide_s(cudaStream_t s, const bparams<T> &p, const T *U, const T *Y1, const T *Y2, T *Y)
-{
-    const bdesc &d = desc[0];
-    if (wide_ps <= 1) {
-        k_wide_s<T, KIND><<<grid_for(d.ny - 2, 32), 32, 0, s>>>(p, U, Y1, Y2, Y);
-    } else {
-        const long long n = total_n;
-        k_wide_s_chunk<T, KIND><<<grid_for(d.ny - 2, wide_ls), dim3(wide_ls, wide_ps), 0, s>>>(p, U, Y1, Y2, Y, d_spk.p,
-                                                                                              d_spk.p + n);
-    }
-}
-
-template <typename T>
-void batch_typed<T>::launch_wide_v(cudaStream_t s, const bparams<T> &p, const T *in, const T *inh, const T *b0, T *out)
-{
-    const bdesc &d = desc[0];
-    if (wide_pv <= 1) {
-        if (wide_vtile)
-            k_wide_v<T, true><<<grid_for(d.nx - 2, 32), 32, 0, s>>>(p, in, inh, b0, out);
-        else
-            k_wide_v<T, false><<<grid_for(d.nx - 2, 32), 32, 0, s>>>(p, in, inh, b0, out);
-    } else {
-        const long long n = total_n;
-        if (wide_vtile) {
-            const size_t smem = sizeof(vtile<T>) * ((wide_lv * wide_pv) / 32);
-            k_wide_v_chunk<T><<<grid_for(d.nx - 2, wide_lv), dim3(wide_lv, wide_pv), smem, s>>>(
-                p, in, inh, b0, out, d_spk.p + 2 * n, d_spk.p + 3 * n);
-        } else {
-            k_wide_v_chunk_plain<T><<<grid_for(d.nx - 2, wide_lv), dim3(wide_lv, wide_pv), 0, s>>>(
-                p, in, inh, b0, out, d_spk.p + 2 * n, d_spk.p + 3 * n);
-        }
-    }
-}
-
-template <typename T> int batch_typed<T>::set_wide_chunks(int ps, int pv, cudaStream_t s, int ls, int lv)
-{
-    const bdesc &d = desc[0];
-    const long long n = total_n;
-    auto ok = [](int P, int e) { return P >= 1 && P <= MAX_CHUNKS && (P == 1 || e >= 4 * P); };
-    if (!ok(ps, d.nx - 2) || !ok(pv, d.ny - 2)) return set_error(LSS_ADI_EINVAL, "wide: chunk count out of range");
-    if ((ps > 1 || pv > 1) && !d_spk.p) LSS_CUDA_TRY(d_spk.alloc(4 * n), "wide: allocating chunk products");
-    const bparams<T> p = params();
-    if (ps > 1)
-        k_wide_spikes<T><<<grid_for((d.ny - 2) * ps, 128), 128, 0, s>>>(p.S[SL_LA], p.S[SL_G], d_spk.p, d_spk.p + n, d.ny,
-                                                                         d.ny, d.nx - 2, ps);
-    if (pv > 1)
-        k_wide_spikes<T><<<grid_for((d.nx - 2) * pv, 128), 128, 0, s>>>(p.Vt[VL_LA], p.Vt[VL_G], d_spk.p + 2 * n,
-                                                                         d_spk.p + 3 * n, d.nx, d.nx, d.ny - 2, pv);
-    LSS_CUDA_TRY(cudaGetLastError(), "wide: chunk products");
-    wide_ps = ps;
-    wide_pv = pv;
-    // the fewest lines per CTA (32, 16 or 8: a warp still reads whole 64-256 B row segments) that
-    // give every SM a CTA: with 1-2 k lines, 32 lines per CTA would leave most SMs idle
-    auto lines_per_cta = [&](int lines) {
-        for (int l : {32, 16})
-            if (grid_for(lines, l) >= sms) return l;
-        return 8;
-    };
-    wide_ls = (ls == 8 || ls == 16 || ls == 32) ? ls : lines_per_cta(d.ny - 2);
-    wide_lv = (lv == 8 || lv == 16 || lv == 32) ? lv : lines_per_cta(d.nx - 2);
-    // the partitioned v sweep works in whole warps (shared-memory tiles moved by all 32 lanes):
-    // lines x chunks must be a multiple of 32, which 32 lines per CTA always are
-    if (pv > 1 && (wide_lv * pv) % 32 != 0) wide_lv = 32;
-    // at most 1024 threads per CTA: 64 chunks take at most 16 lines
-    while (ps > 1 && wide_ls * ps > 1024) wide_ls >>= 1;
-    while (pv > 1 && wide_lv * pv > 1024) wide_lv >>= 1;
-    if (pv > 1) {
-        // the limit belongs to the kernel, shared by every solver of the process: set it to what a
-        // 1024-thread CTA needs, so that no solver lowers it under another one's launches
-        const int smem = static_cast<int>(sizeof(vtile<T>) * 32);
-        LSS_CUDA_TRY(cudaFuncSetAttribute(k_wide_v_chunk<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
-                     "wide: v-sweep tile memory");
-    }
-    if (wide_graph) cudaGraphExecDestroy(wide_graph);
-    wide_graph = nullptr;
-    return LSS_ADI_OK;
-}
-
-// Chunk counts and lines per CTA of the two sweeps, each timed on its own (first S stage,
-// first v stage) over P = 1, 2, 4, ..., MAX_CHUNKS (at least 4 rows per chunk) and L = 8, 16,
-// 32 (L * P <= 1024).
-template <typename T> int batch_typed<T>::autotune_wide(cudaStream_t s)
-{
-    const bdesc &d = desc[0];
-    bparams<T> p = params();
-    LSS_CUDA_TRY(cudaMemcpyAsync(p.U, d_payoff.p, total_n * sizeof(T), cudaMemcpyDeviceToDevice, s), "wide: tuning state");
-    cudaEvent_t e0, e1;
-    LSS_CUDA_TRY(cudaEventCreate(&e0), "wide: tuning events");
-    LSS_CUDA_TRY(cudaEventCreate(&e1), "wide: tuning events");
-    float best_s = 1e30f, best_v = 1e30f;
-    int ps = 1, pv = 1, ls = 32, lv = 32;
-    bool vt = true;
-    int rc = LSS_ADI_OK;
-    auto timed = [&](auto &&launch) {
-        launch();
-        cudaEventRecord(e0, s);
-        for (int r = 0; r < 3; ++r) launch();
-        cudaEventRecord(e1, s);
-        cudaEventSynchronize(e1);
-        float ms = 0.f;
-        cudaEventElapsedTime(&ms, e0, e1);
-        return ms;
-    };
-    for (int P = 1; P <= MAX_CHUNKS && rc == LSS_ADI_OK; P *= 2) {
-        const bool okS = (P == 1 || d.nx - 2 >= 4 * P), okV = (P == 1 || d.ny - 2 >= 4 * P);
-        if (!okS && !okV) break;
-        for (int L : {8, 16, 32}) {
-            if (P == 1 && L != 32) continue; // thread per line: L unused
-            if (L * P > 1024) continue;
-            rc = set_wide_chunks(okS ? P : 1, okV ? P : 1, s, L, L);
-            if (rc) break;
-            if (okS) {
-                const float ms = timed([&] { launch_wide_s<1>(s, p, p.U, nullptr, nullptr, p.Y1); });
-                if (ms < best_s) { best_s = ms; ps = P; ls = L; }
-            }
-            if (okV) {
-                k_wide_b1<T><<<grid_for(d.nx, 128), 128, 0, s>>>(p, p.U, d_b0.p);
-                for (bool tile : {true, false}) {
-                    wide_vtile = tile;
-                    const float ms = timed([&] { launch_wide_v(s, p, p.U, p.Y1, d_b0.p, p.Y2); });
-                    if (ms < best_v) { best_v = ms; pv = P; lv = L; vt = tile; }
-                }
-            }
-            const cudaError_t err = cudaGetLastError();
-            if (err != cudaSuccess) {
-                rc = set_error(LSS_ADI_ECUDA, std::string("wide: tuning: ") + cudaGetErrorString(err));
-                break;
-            }
-        }
-    }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    if (rc) return rc;
-    wide_vtile = vt;
-    return set_wide_chunks(ps, pv, s, ls, lv);
-}
-
 // One time step U -> V of the wide path (stage outputs in Y1, Y2, Y3).
 template <typename T>
 void batch_typed<T>::enqueue_wide_step(cudaStream_t s, const bparams<T> &p, const T *U, T *Y1, T *Y2, T *Y3, T *V)
 {
     const bdesc &d = desc[0];
     T *b0 = d_b0.p;
+    const int gs = grid_for(d.ny - 2, 32), gv = grid_for(d.nx - 2, 32);
     k_wide_b1<T><<<grid_for(d.nx, 128), 128, 0, s>>>(p, U, b0);
-    launch_wide_s<1>(s, p, U, nullptr, nullptr, Y1);
+    k_wide_s<T, 1><<<gs, 32, 0, s>>>(p, U, nullptr, nullptr, Y1);
     if (d.scheme == LSS_ADI_DOUGLAS_RACHFORD) {
-        launch_wide_v(s, p, U, Y1, b0, V);
+        k_wide_v<T><<<gv, 32, 0, s>>>(p, U, Y1, b0, V);
     } else {
-        launch_wide_v(s, p, U, Y1, b0, Y2);
-        launch_wide_s<2>(s, p, U, Y1, Y2, Y3);
-        if (d.scheme == LSS_ADI_HUNDSDORFER_VERWER)
-            launch_wide_v(s, p, Y2, Y3, b0, V);
-        else
-            launch_wide_v(s, p, U, Y3, b0, V);
+        k_wide_v<T><<<gv, 32, 0, s>>>(p, U, Y1, b0, Y2);
+        k_wide_s<T, 2><<<gs, 32, 0, s>>>(p, U, Y1, Y2, Y3);
+        k_wide_v<T><<<gv, 32, 0, s>>>(p, d.scheme == LSS_ADI_HUNDSDORFER_VERWER ? Y2 : U, Y3, b0, V);
     }
     k_wide_b2<T><<<grid_for(d.ny, 128), 128, 0, s>>>(p, V);
 }
@@ -2662,12 +1482,7 @@ template <typename T> int batch_typed<T>::enqueue_wide(cudaStream_t s)
     LSS_CUDA_TRY(cudaMemcpyAsync(U, d_payoff.p, total_n * sizeof(T), cudaMemcpyDeviceToDevice, s), "wide: initial state");
     LSS_CUDA_TRY(cudaMemsetAsync(d_status.p, 0, sizeof(int), s), "wide: clearing the status");
     long long nl = 0;
-    const int per_refresh = 3 + (wide_ps > 1 ? 1 : 0);
     for (int step = 0; step < d.steps; ++step) {
-        if (tdep) {
-            refresh_step(s, step, 1);
-            nl += per_refresh;
-        }
         enqueue_wide_step(s, p, U, Y1, Y2, Y3, V);
         nl += d.scheme == LSS_ADI_DOUGLAS_RACHFORD ? 4 : 6;
         std::swap(U, V);
@@ -2676,170 +1491,6 @@ template <typename T> int batch_typed<T>::enqueue_wide(cudaStream_t s)
     LSS_CUDA_TRY(cudaGetLastError(), "wide: launching the time loop");
     launches = nl + 1;
     return LSS_ADI_OK;
-}
-
-// Forward + adjoint of the single instance with the wide kernels: forward pass keeping a
-// checkpoint every d.ck steps, then per segment (last first) a forward recomputation keeping
-// every step's stage values and the adjoint steps in reverse order (as k_batch_fwdadj).
-template <typename T> int batch_typed<T>::enqueue_wide_adjoint(cudaStream_t s)
-{
-    if constexpr (!std::is_same<T, double>::value) {
-        (void)s;
-        return set_error(LSS_ADI_EUNSUPPORTED, "wide adjoint: FP64 only");
-    } else {
-        if (count != 1) return set_error(LSS_ADI_EINVAL, "wide adjoint: one instance only");
-        if (!adjoint_ok) return set_error(LSS_ADI_EUNSUPPORTED, "wide adjoint: " + adjoint_why);
-        bdesc &d = desc[0];
-        const int c0 = ck_override > 0 ? std::min(ck_override, d.steps) : d.ck;
-        if (c0 != d.ck) {
-            d.ck = c0;
-            LSS_CUDA_TRY(cudaMemcpy(d_desc.p, &d, sizeof(bdesc), cudaMemcpyHostToDevice), "wide adjoint: descriptor");
-        }
-        const int nx = d.nx, ny = d.ny, c = d.ck;
-        const long long n = total_n;
-        const int nseg = (d.steps + c - 1) / c;
-        const int threads = 128, grid = grid_for(std::max(nx, ny), threads);
-        const long long nthr = static_cast<long long>(grid) * threads;
-        // partitioned adjoint solves with the forward's chunk counts
-        const int ps = wide_ps, pv = wide_pv, ls = wide_ls, lv = wide_lv;
-        const int gS = grid_for(ny - 2, ls), gV = grid_for(nx - 2, lv);
-        const long long nacc = std::max({nthr, 1LL * ls * gS * ps, 1LL * lv * gV * pv, static_cast<long long>(nx)});
-        if ((ps > 1 || pv > 1) && (aspk_ps != ps || aspk_pv != pv)) {
-            if (!d_aspk.p) LSS_CUDA_TRY(d_aspk.alloc(4 * n), "wide adjoint: allocating chunk products");
-            const bparams<double> q = params();
-            if (ps > 1)
-                k_wadj_spikes<double><<<grid_for((ny - 2) * ps, 128), 128, 0, s>>>(q.S[SL_LA], q.S[SL_G], d_aspk.p,
-                                                                                   d_aspk.p + n, ny, ny, nx - 2, ps);
-            if (pv > 1)
-                k_wadj_spikes<double><<<grid_for((nx - 2) * pv, 128), 128, 0, s>>>(q.Vt[VL_LA], q.Vt[VL_G], d_aspk.p + 2 * n,
-                                                                                   d_aspk.p + 3 * n, nx, nx, ny - 2, pv);
-            LSS_CUDA_TRY(cudaGetLastError(), "wide adjoint: chunk products");
-            aspk_ps = ps;
-            aspk_pv = pv;
-        }
-        const double *hzS = d_aspk.p, *hwS = d_aspk.p + n, *hzV = d_aspk.p + 2 * n, *hwV = d_aspk.p + 3 * n;
-        const long long need = (nseg + 4LL * (c + 1) + 9) * n + nx + 2LL * ny + 10 * nacc;
-        if (!d_wws.p || wws_need != need) {
-            LSS_CUDA_TRY(d_wws.alloc(need), "wide adjoint: allocating workspace");
-            wws_need = need;
-        }
-        double *CK = d_wws.p;
-        double *SEG = CK + static_cast<long long>(nseg) * n;
-        double *W0 = SEG + (c + 1) * 4LL * n, *W1 = W0 + n;
-        double *UB = W1 + n, *VB = UB + n, *Y1B = VB + n, *Y2B = Y1B + n, *Y3B = Y2B + n, *FB = Y3B + n, *TMP = FB + n;
-        double *LV = TMP + n, *LS = LV + nx, *HS = LS + ny, *ACC = HS + ny;
-        auto slot = [&](int m, int a) -> double * { return SEG + (static_cast<long long>(m) * 4 + a) * n; };
-        const bparams<double> p = params();
-        // stage arrays start at zero (rows 0 and nx-1 of Y2 are never written by the sweeps)
-        LSS_CUDA_TRY(cudaMemsetAsync(SEG, 0, (c + 1) * 4LL * n * sizeof(double), s), "wide adjoint: clearing");
-        LSS_CUDA_TRY(cudaMemsetAsync(ACC, 0, 10 * nacc * sizeof(double), s), "wide adjoint: clearing");
-        LSS_CUDA_TRY(cudaMemsetAsync(d_status.p, 0, sizeof(int), s), "wide adjoint: clearing");
-        LSS_CUDA_TRY(cudaMemcpyAsync(CK, d_payoff.p, n * sizeof(double), cudaMemcpyDeviceToDevice, s), "wide adjoint: initial state");
-        long long nl = 0;
-        const int per_step = d.scheme == LSS_ADI_DOUGLAS_RACHFORD ? 4 : 6;
-        const double *cur = CK;
-        const int n0_last = (nseg - 1) * c; // the last segment keeps its stage values: no recomputation
-        const int per_refresh = 3 + (ps > 1 ? 1 : 0);
-        for (int step = 0; step < d.steps; ++step) {
-            if (tdep) {
-                refresh_step(s, step, 1);
-                nl += per_refresh;
-            }
-            if (step >= n0_last) {
-                const int m = step - n0_last;
-                enqueue_wide_step(s, p, cur, slot(m, 1), slot(m, 2), slot(m, 3), slot(m + 1, 0));
-                nl += per_step;
-                cur = slot(m + 1, 0);
-                continue;
-            }
-            double *next = ((step + 1) % c == 0 && step + 1 < d.steps) ? CK + static_cast<long long>((step + 1) / c) * n
-                                                                        : ((step & 1) ? W1 : W0);
-            enqueue_wide_step(s, p, cur, slot(0, 1), slot(0, 2), slot(0, 3), next);
-            nl += per_step;
-            cur = next;
-        }
-        k_wadj_begin<<<grid_for(n, 256), 256, 0, s>>>(p, cur, VB, FB, Y1B, Y3B);
-        k_wadj_seed<<<1, 1, 0, s>>>(p, cur, VB);
-        nl += 2;
-        double *ub = UB, *vb = VB;
-        for (int sgi = nseg - 1; sgi >= 0; --sgi) {
-            const int n0 = sgi * c;
-            const int L = std::min(c, d.steps - n0);
-            const double *u0 = CK + static_cast<long long>(sgi) * n;
-            for (int m = 0; m < L && sgi < nseg - 1; ++m) {
-                const double *um = (m == 0) ? u0 : slot(m, 0);
-                if (tdep) {
-                    refresh_step(s, n0 + m, 1);
-                    nl += per_refresh;
-                }
-                enqueue_wide_step(s, p, um, slot(m, 1), slot(m, 2), slot(m, 3), slot(m + 1, 0));
-                nl += per_step;
-            }
-            for (int m = L - 1; m >= 0; --m) {
-                const double *um = (m == 0) ? u0 : slot(m, 0);
-                if (tdep) { // this step's S-line tables and the adjoint's D(t) factors
-                    refresh_step(s, n0 + m, 2);
-                    nl += per_refresh;
-                }
-                const double *Y1 = slot(m, 1), *Y2 = slot(m, 2), *Y3 = slot(m, 3), *Vo = slot(m + 1, 0);
-                const double tau = d.a_tau0 + d.a_dtau * (n0 + m);
-                // v stages: (in, out, output adjoint, adjoint of in, adjoint of inh), first or accumulating
-                auto adj_v_stage = [&](bool first, const double *in, const double *out, const double *XB, double *INB,
-                                       double *INHB) {
-                    if (pv > 1) {
-                        if (first)
-                            k_wadj_v_chunk<true><<<gV, dim3(lv, pv), 0, s>>>(p, in, out, XB, INB, INHB, TMP, LV, ACC, nacc, hzV, hwV);
-                        else
-                            k_wadj_v_chunk<false><<<gV, dim3(lv, pv), 0, s>>>(p, in, out, XB, INB, INHB, TMP, LV, ACC, nacc, hzV, hwV);
-                    } else {
-                        if (first)
-                            k_wadj_v<true><<<grid, threads, 0, s>>>(p, in, out, XB, INB, INHB, TMP, LV, ACC, nacc);
-                        else
-                            k_wadj_v<false><<<grid, threads, 0, s>>>(p, in, out, XB, INB, INHB, TMP, LV, ACC, nacc);
-                    }
-                };
-                auto adj_s_stage = [&](int kind, const double *Yo, const double *XB) {
-                    if (ps > 1) {
-                        if (kind == 2)
-                            k_wadj_s_chunk<2><<<gS, dim3(ls, ps), 0, s>>>(p, um, Y1, Y2, Yo, XB, FB, TMP, LS, HS, ub, Y1B, ACC,
-                                                                          nacc, tau, hzS, hwS);
-                        else
-                            k_wadj_s_chunk<1><<<gS, dim3(ls, ps), 0, s>>>(p, um, Y1, Y2, Yo, XB, FB, TMP, LS, HS, ub, Y1B, ACC,
-                                                                          nacc, tau, hzS, hwS);
-                    } else {
-                        if (kind == 2)
-                            k_wadj_s<2><<<grid, threads, 0, s>>>(p, um, Y1, Y2, Yo, XB, FB, TMP, LS, HS, ub, Y1B, ACC, nacc, tau);
-                        else
-                            k_wadj_s<1><<<grid, threads, 0, s>>>(p, um, Y1, Y2, Yo, XB, FB, TMP, LS, HS, ub, Y1B, ACC, nacc, tau);
-                    }
-                };
-                const int gG = grid_for(n, 256);
-                k_wadj_b2<<<grid, threads, 0, s>>>(p, vb, ub);
-                if (d.scheme == LSS_ADI_DOUGLAS_RACHFORD) {
-                    adj_v_stage(true, um, Vo, vb, ub, Y1B);
-                    nl += 2;
-                } else {
-                    if (d.scheme == LSS_ADI_HUNDSDORFER_VERWER)
-                        adj_v_stage(true, Y2, Vo, vb, Y2B, Y3B);
-                    else
-                        adj_v_stage(true, um, Vo, vb, ub, Y3B);
-                    adj_s_stage(2, Y3, Y3B);
-                    k_wadj_gather2d<2><<<gG, 256, 0, s>>>(p, um, FB, LS, HS, LV, ub, Y2B, ACC, nacc, tau);
-                    adj_v_stage(false, um, Y2, Y2B, ub, Y1B);
-                    nl += 5;
-                }
-                adj_s_stage(1, Y1, Y1B);
-                k_wadj_gather2d<1><<<gG, 256, 0, s>>>(p, um, FB, LS, HS, LV, ub, Y2B, ACC, nacc, tau);
-                nl += 2;
-                std::swap(ub, vb);
-            }
-        }
-        k_wadj_reduce<<<1, 256, 0, s>>>(p, ACC, nacc);
-        LSS_CUDA_TRY(cudaMemcpyAsync(p.V, vb, n * sizeof(double), cudaMemcpyDeviceToDevice, s), "wide adjoint: payoff gradient");
-        LSS_CUDA_TRY(cudaGetLastError(), "wide adjoint: launching");
-        launches = nl + 1;
-        return LSS_ADI_OK;
-    }
 }
 
 template <typename T> int batch_typed<T>::run_wide(cudaStream_t s, bool use_graph)
@@ -2892,29 +1543,26 @@ template <typename T> int batch_typed<T>::run(int mode, cudaStream_t s, bool use
     return LSS_ADI_OK;
 }
 
+// One thread per line (LSS_ADI_OPT_LINE_PER_THREAD).
 template <typename T> struct wide_solver : wide_solver_base {
     batch_typed<T> b;
+    lss_adi_problem prob{};
     std::vector<T> x, y, pay0;
+    std::unique_ptr<wide_solver_base> parts; // partitioned, once lss_adi_line_chunks asks for it
 
     int init(const lss_adi_problem &p)
     {
+        prob = p;
         instance_tables<T> tt;
         build_tables_for<T>(p, tt);
         x = tt.x;
         y = tt.y;
         pay0 = tt.payoff;
-        int rc = b.create(&p, 1);
-        if (rc) return rc;
-        if (p.options & LSS_ADI_OPT_LINE_PER_THREAD) return LSS_ADI_OK;
-        LSS_CUDA_TRY(cudaMemcpy(b.d_payoff.p, pay0.data(), pay0.size() * sizeof(T), cudaMemcpyHostToDevice),
-                     "wide: initial state");
-        rc = b.autotune_wide(nullptr);
-        if (rc) return rc;
-        LSS_CUDA_TRY(cudaDeviceSynchronize(), "wide: tuning");
-        return LSS_ADI_OK;
+        return b.create(&p, 1);
     }
     int forward(const void *payoff, void *out_surface, double *out_value, int flags, void *stream, bool use_graph) override
     {
+        if (parts) return parts->forward(payoff, out_surface, out_value, flags, stream, use_graph);
         cudaStream_t s = static_cast<cudaStream_t>(stream);
         const bool dev = (flags & LSS_ADI_DEVICE_POINTERS) != 0;
         const size_t n = static_cast<size_t>(b.total_n);
@@ -2942,36 +1590,27 @@ template <typename T> struct wide_solver : wide_solver_base {
     }
     int chunks(int s_chunks, int v_chunks, int *out_s, int *out_v, void *stream) override
     {
-        cudaStream_t s = static_cast<cudaStream_t>(stream);
-        if (s_chunks < 0 || v_chunks < 0) return set_error(LSS_ADI_EINVAL, "lss_adi_line_chunks: negative chunk count");
-        int rc = LSS_ADI_OK;
-        if (s_chunks == 0 || v_chunks == 0) {
-            LSS_CUDA_TRY(cudaMemcpyAsync(b.d_payoff.p, pay0.data(), pay0.size() * sizeof(T), cudaMemcpyHostToDevice, s),
-                         "wide: initial state");
-            rc = b.autotune_wide(s);
-            if (rc) return rc;
+        if (!parts) {
+            std::unique_ptr<wide_solver_base> w;
+            int rc = make_partitioned_solver(prob, w);
+            if (!rc) rc = w->chunks(s_chunks, v_chunks, out_s, out_v, stream);
+            if (!rc) parts = std::move(w);
+            return rc;
         }
-        if (s_chunks || v_chunks) { // a direction left at 0 keeps its tuned chunks and lines per CTA
-            rc = b.set_wide_chunks(s_chunks ? s_chunks : b.wide_ps, v_chunks ? v_chunks : b.wide_pv, s,
-                                   s_chunks ? 0 : b.wide_ls, v_chunks ? 0 : b.wide_lv);
-            if (rc) return rc;
-        }
-        LSS_CUDA_TRY(cudaStreamSynchronize(s), "lss_adi_line_chunks");
-        if (out_s) *out_s = b.wide_ps;
-        if (out_v) *out_v = b.wide_pv;
-        return LSS_ADI_OK;
+        return parts->chunks(s_chunks, v_chunks, out_s, out_v, stream);
     }
-    void current_chunks(int &s_chunks, int &v_chunks, int &s_lines, int &v_lines) const override
+    void current_chunks(int &s_chunks, int &v_chunks) const override
     {
-        s_chunks = b.wide_ps;
-        v_chunks = b.wide_pv;
-        s_lines = b.wide_ls;
-        v_lines = b.wide_lv;
+        s_chunks = v_chunks = 1;
+        if (parts) parts->current_chunks(s_chunks, v_chunks);
     }
 };
 
 int make_wide_solver(const lss_adi_problem &p, std::unique_ptr<wide_solver_base> &out)
 {
+    // time-dependent coefficients (no batched kernel to agree with) run partitioned, in one chunk per line
+    // where a thread per line is asked for
+    if (!(p.options & LSS_ADI_OPT_LINE_PER_THREAD) || time_dependent(p)) return make_partitioned_solver(p, out);
     try {
         if (p.precision == LSS_ADI_FP64) {
             std::unique_ptr<wide_solver<double>> w(new wide_solver<double>());
@@ -2990,10 +1629,11 @@ int make_wide_solver(const lss_adi_problem &p, std::unique_ptr<wide_solver_base>
     return LSS_ADI_OK;
 }
 
-// lss_adi_adjoint: one parametric FP64 Heston instance through the batched forward+adjoint kernel.
+// lss_adi_adjoint: one parametric FP64 instance, on one warp group of the batched forward + adjoint
+// kernel or on the partitioned kernels over the whole GPU.
 struct adjoint_impl {
-    batch_typed<double> b;
-    bool wide = false; // large instance: the wide kernels instead of one CTA
+    std::unique_ptr<batch_typed<double>> b;
+    std::unique_ptr<wide_adjoint_base> wide;
 };
 
 adjoint_solver::adjoint_solver() = default;
@@ -3007,31 +1647,31 @@ int adjoint_solver::init(const lss_adi_problem &p)
     if (!impl) return set_error(LSS_ADI_ENOMEM, "host allocation failed");
     lss_adi_problem q = p;
     q.arith = LSS_ADI_ARITH_FAST;
-    int rc = impl->b.create(&q, 1);
-    if (rc) return rc;
-    // one CTA carries an instance of up to 256 x 160 points well; larger ones run wide, and so
-    // do time-dependent coefficients (SABR with r != 0), whose S-line tables the host-sequenced
-    // wide kernels rebuild before every step
-    impl->wide = p.nx > 256 || static_cast<long long>(p.nx) * p.ny > 40960 || (p.options & LSS_ADI_OPT_WIDE_ADJOINT) ||
-                 time_dependent(p);
-    if (impl->wide && !(p.options & LSS_ADI_OPT_LINE_PER_THREAD)) {
-        rc = impl->b.autotune_wide(nullptr);
-        if (rc) return rc;
-        LSS_CUDA_TRY(cudaDeviceSynchronize(), "lss_adi_adjoint: tuning");
-    }
-    return LSS_ADI_OK;
+    // one warp group carries an instance of up to 256 x 160 points (the same bits as a member of a
+    // batch); larger ones run wide, and so do time-dependent coefficients (SABR with r != 0), whose
+    // S-line tables the host-sequenced wide kernels rebuild before every step
+    if (p.nx > 256 || static_cast<long long>(p.nx) * p.ny > 40960 || (p.options & LSS_ADI_OPT_WIDE_ADJOINT) || time_dependent(p))
+        return make_wide_adjoint(q, impl->wide);
+    impl->b.reset(new (std::nothrow) batch_typed<double>());
+    if (!impl->b) return set_error(LSS_ADI_ENOMEM, "host allocation failed");
+    return impl->b->create(&q, 1);
 }
 
-int adjoint_solver::set_chunks(int s_chunks, int v_chunks, int s_lines, int v_lines, void *stream)
+int adjoint_solver::set_chunks(int s_chunks, int v_chunks, void *stream)
 {
     if (!impl || !impl->wide) return LSS_ADI_OK;
-    return impl->b.set_wide_chunks(s_chunks, v_chunks, static_cast<cudaStream_t>(stream), s_lines, v_lines);
+    LSS_CUDA_TRY(cudaStreamSynchronize(static_cast<cudaStream_t>(stream)), "lss_adi_adjoint: chunk counts");
+    int rc = impl->wide->set_chunks(s_chunks, v_chunks);
+    if (rc) return rc;
+    LSS_CUDA_TRY(cudaDeviceSynchronize(), "lss_adi_adjoint: chunk counts");
+    return LSS_ADI_OK;
 }
 
 int adjoint_solver::run(const void *payoff, double *out_value, double *dv_dparams, void *dv_dpayoff, int checkpoint_every,
                         int flags, void *stream)
 {
-    batch_typed<double> &b = impl->b;
+    if (impl->wide) return impl->wide->run(payoff, out_value, dv_dparams, dv_dpayoff, checkpoint_every, flags, stream);
+    batch_typed<double> &b = *impl->b;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const bool dev = (flags & LSS_ADI_DEVICE_POINTERS) != 0;
     const size_t n = static_cast<size_t>(b.total_n);
@@ -3040,7 +1680,7 @@ int adjoint_solver::run(const void *payoff, double *out_value, double *dv_dparam
                                      dev ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s),
                      "lss_adi_adjoint: copying the terminal condition");
     b.ck_override = checkpoint_every;
-    int rc = impl->wide ? b.enqueue_wide_adjoint(s) : b.run(1, s, false);
+    int rc = b.run(1, s, false);
     if (rc) return rc;
     if (out_value)
         LSS_CUDA_TRY(cudaMemcpyAsync(out_value, b.d_values.p, sizeof(double), cudaMemcpyDeviceToHost, s), "lss_adi_adjoint: value");

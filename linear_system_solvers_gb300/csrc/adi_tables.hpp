@@ -228,6 +228,27 @@ template <typename T> inline void build_time_tables(const lss_adi_problem &p, co
     }
 }
 
+// Coefficient derivatives of the adjoint, split into S and v factors (double).  Heston: a = vS^2/2,
+// b = sigma^2 v/2, c = rho sigma v S, d = rS, e = kappa (theta - v), f = -r.  SABR (D = 1):
+// a = v^2 F^(2 beta) D^(2(1-beta))/2, b = nu^2 v^2/2, c = rho nu v^2 F^beta D^(1-beta), d = rF, e = 0,
+// f = -r (sigma carries nu).
+struct s_factors { double hx, hc, ha, hdd; };         // S/A; S-factor of c^; F^(2 beta)/A^2; F^(2 beta) A''/A^3
+struct v_factors { double hy, bs, ek, et, es, hv2; }; // v-factor of c^; db^/dsigma; de^/d(kappa, theta, sigma); v^2/2
+inline s_factors derivative_s(const lss_adi_problem &p, const sinh_map<double> &g, double zeta)
+{
+    const double x = g.x(zeta), A = g.a_der(zeta), Add = g.c_der(zeta), bt = p.sabr_beta;
+    if (p.model != LSS_ADI_SABR) return {x / A, x / A, 0.0, 0.0};
+    return {x / A, std::pow(x, bt) / A, std::pow(x, 2.0 * bt) / (A * A), std::pow(x, 2.0 * bt) * Add / (A * A * A)};
+}
+inline v_factors derivative_v(const lss_adi_problem &p, const sinh_map<double> &g, double eta)
+{
+    const bool sabr = p.model == LSS_ADI_SABR;
+    const double B = g.b_der(eta), Bdd = g.d_der(eta), vv = g.y(eta), sg = p.sigma;
+    const double vb = sabr ? vv * vv : vv; // the v factor of b and c
+    return {vb / B, sg * vb / (B * B), sabr ? 0.0 : (p.theta_v - vv) / B, sabr ? 0.0 : p.kappa / B, -sg * vb * Bdd / (B * B * B),
+            sabr ? 0.5 * vv * vv : 0.0};
+}
+
 // Builds the tables of a parametric problem at time t (coefficients) -- Heston
 // coefficients do not depend on t; SABR ones only through D(t) = exp(-r (T - t)).
 template <typename T> inline void build_tables(const lss_adi_problem &p, instance_tables<T> &it)
