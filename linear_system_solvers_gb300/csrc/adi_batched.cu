@@ -40,7 +40,9 @@ enum { Y_SLO = 0, Y_B2C, Y_CHS, Y_HY, Y_BS, Y_EK, Y_ET, Y_ES, Y_HV2, Y_COUNT };
 
 struct bdesc {
     int nx, ny, steps, scheme;
-    long long o2;  // offset of the instance in the nx*ny arenas
+    int ld, pad0_; // row pitch of the state (FP64: a multiple of 4; FP32: ny)
+    long long o2;  // offset of the instance in the nx*ld arenas
+    long long op;  // offset in the nx*ny arena of initial conditions
     int ox, oy;    // offsets in the nx- and ny-sized arenas
     double bnc;    // constant of the Neumann-corner boundary row
     int i0, j0;    // bilinear cell of (eval_s, eval_v)
@@ -278,6 +280,19 @@ __global__ void k_setup_v_lines(setup_params sp, T *V0, long long slot_stride, T
     }
 }
 
+// The same in delta form (FP64; the tables of adi_wide.cuh, v lines transposed to [t][i]).
+__device__ __forceinline__ int setup_instance(const setup_params &sp, long long g)
+{
+    int lo = 0, hi = sp.count - 1; // the instance owning global line g
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (sp.line_start[mid] <= g) lo = mid; else hi = mid - 1;
+    }
+    return lo;
+}
+static __global__ void k_setup_s_delta(setup_params sp, double *S0, long long stride);
+static __global__ void k_setup_v_delta(setup_params sp, double *V0, long long stride);
+
 // ------------------------------------------------------------------------------------------
 // the persistent time-loop kernel
 // ------------------------------------------------------------------------------------------
@@ -285,7 +300,7 @@ __global__ void k_setup_v_lines(setup_params sp, T *V0, long long slot_stride, T
 // space (__grid_constant__), so they cost no registers; only the offsets are carried.
 template <typename T> struct inst_view {
     const bparams<T> *p;
-    int nx, ny, e_s, e_v;
+    int nx, ny, ld, e_s, e_v;
     long long o2;
     int ox, oy;
     __device__ __forceinline__ const T *S(int k) const { return p->S[k] + o2; }
@@ -325,17 +340,17 @@ template <typename T>
 __device__ __forceinline__ void b1_stage(const inst_view<T> &v, const T *__restrict__ U, T *__restrict__ sb0, double bnc,
                                          int l0, int ls)
 {
-    const int nx = v.nx, ny = v.ny, N = nx - 1;
+    const int nx = v.nx, ld = v.ld, N = nx - 1;
     for (int i = l0; i < nx; i += ls) {
         T r;
         if (i == 0) {
             r = ldg(v.Yv(Y_SLO));
         } else if (i == N) {
-            r = ldg(v.X(XB_C) + i) * U[(long long)N * ny] + ldg(v.X(XB_1) + i) * U[(long long)N * ny + 1] +
-                ldg(v.X(XB_2) + i) * U[(long long)N * ny + 2] + static_cast<T>(bnc);
+            r = ldg(v.X(XB_C) + i) * U[(long long)N * ld] + ldg(v.X(XB_1) + i) * U[(long long)N * ld + 1] +
+                ldg(v.X(XB_2) + i) * U[(long long)N * ld + 2] + static_cast<T>(bnc);
         } else {
-            const long long o = (long long)i * ny;
-            r = ldg(v.X(XB_M) + i) * U[o - ny] + ldg(v.X(XB_C) + i) * U[o] + ldg(v.X(XB_P) + i) * U[o + ny] +
+            const long long o = (long long)i * ld;
+            r = ldg(v.X(XB_M) + i) * U[o - ld] + ldg(v.X(XB_C) + i) * U[o] + ldg(v.X(XB_P) + i) * U[o + ld] +
                 ldg(v.X(XB_2) + i) * U[o + 2] + ldg(v.X(XB_1) + i) * U[o + 1];
         }
         sb0[i] = r;
@@ -345,16 +360,19 @@ __device__ __forceinline__ void b1_stage(const inst_view<T> &v, const T *__restr
 // boundary#2: row S_lo and the S_max extrapolation row (explicit_boundary.hpp:202-238)
 template <typename T> __device__ __forceinline__ void b2_stage(const inst_view<T> &v, T *Vn, int l0, int ls)
 {
-    const int nx = v.nx, ny = v.ny, lri = nx - 1;
+    const int nx = v.nx, ny = v.ny, ld = v.ld, lri = nx - 1;
     const T four3 = T(4.0 / 3.0), third = T(1.0 / 3.0);
     for (int j = l0; j < ny; j += ls) {
         Vn[j] = ldg(v.Yv(Y_SLO) + j);
         const int jj = ldg(v.jmap() + j);
-        Vn[(long long)lri * ny + j] =
-            four3 * Vn[(long long)(lri - 1) * ny + jj] - third * Vn[(long long)(lri - 2) * ny + jj] - ldg(v.Yv(Y_B2C) + j);
+        Vn[(long long)lri * ld + j] =
+            four3 * Vn[(long long)(lri - 1) * ld + jj] - third * Vn[(long long)(lri - 2) * ld + jj] - ldg(v.Yv(Y_B2C) + j);
     }
 }
 
+// Stages of the FP32 instances, written on Y1, Y2, Y3 (their values keep that form's rounding; FP64
+// runs in delta form, adi_delta.cuh).
+//
 // S-line sweeps.  KIND 1: explicit operator on U (Y1).  KIND 2: second S stage of CS/MCS/HV
 // (scheme SCH) on U, Y1, Y2.  Thread per line j; every access of a warp is one coalesced row
 // segment.  The mixed difference (x(t-1,j-1) - x(t-1,j+1)) - (x(t+1,j-1) - x(t+1,j+1)) is formed
@@ -530,6 +548,7 @@ template <typename T> __device__ __forceinline__ inst_view<T> make_view(const bp
     v.p = &p;
     v.nx = d.nx;
     v.ny = d.ny;
+    v.ld = d.ld;
     v.e_s = d.nx - 2;
     v.e_v = d.ny - 2;
     v.o2 = d.o2;
@@ -537,6 +556,8 @@ template <typename T> __device__ __forceinline__ inst_view<T> make_view(const bp
     v.oy = d.oy;
     return v;
 }
+
+#include "adi_delta.cuh"
 
 // One time step U -> Vn of scheme SCH with stage outputs in Y1, Y2, Y3; ends with a group barrier.
 template <typename T, int SCH>
@@ -566,11 +587,22 @@ __device__ __forceinline__ void fwd_step(const inst_view<T> &v, const T *U, T *Y
 
 // Persistent forward kernel of the instances of scheme SCH: CTAs of 4 warps split into groups
 // (the layout word of the CTA), each group pulling instances of its class (warps per instance)
-// from the class counter.  Register budget 64 per thread (8 CTAs per SM).
+// from the class counter.  Register budget 128 per thread in FP64 (4 CTAs per SM: the sweeps hold
+// the rows that they load ahead), 64 in FP32 (8 CTAs).
 constexpr int BATCH_CTA = 32 * MAX_GROUP_WARPS;
 
+// initial condition into the pitched state
+template <typename T> __device__ __forceinline__ void load_payoff(const bparams<T> &p, const bdesc &d, T *U, const grp &g)
+{
+    for (int i = g.t / 32; i < d.nx; i += g.n / 32)
+        for (int j = g.t & 31; j < d.ny; j += 32) U[i * d.ld + j] = p.payoff[d.op + (long long)i * d.ny + j];
+}
+#ifndef LSS_FWD_MIN_CTAS
+#define LSS_FWD_MIN_CTAS 4
+#endif
+
 template <typename T, int SCH>
-__global__ void __launch_bounds__(BATCH_CTA, 8) k_batch_forward(const __grid_constant__ bparams<T> p)
+__global__ void __launch_bounds__(BATCH_CTA, sizeof(T) == 8 ? LSS_FWD_MIN_CTAS : 8) k_batch_forward(const __grid_constant__ bparams<T> p)
 {
     __shared__ int s_idx[MAX_GROUP_WARPS];
     __shared__ int s_bad[MAX_GROUP_WARPS];
@@ -586,8 +618,13 @@ __global__ void __launch_bounds__(BATCH_CTA, 8) k_batch_forward(const __grid_con
         const inst_view<T> v = make_view(p, d);
         T *U = p.U + d.o2, *Vn = p.V + d.o2, *Y1 = p.Y1 + d.o2, *Y2 = p.Y2 + d.o2, *Y3 = p.Y3 + d.o2;
         T *sb0 = p.B0 + d.ox;
+        if constexpr (sizeof(T) == 8) {
+            load_payoff(p, d, U, g);
+            g.sync();
+        }
         for (int step = 0; step < d.steps; ++step) {
-            fwd_step<T, SCH>(v, U, Y1, Y2, Y3, Vn, sb0, d.bnc, g);
+            if constexpr (sizeof(T) == 8) delta_step<SCH>(v, d, U, Y1, Y2, Y3, Vn, sb0, g);
+            else fwd_step<T, SCH>(v, U, Y1, Y2, Y3, Vn, sb0, d.bnc, g);
             T *tmp = U;
             U = Vn;
             Vn = tmp;
@@ -595,15 +632,15 @@ __global__ void __launch_bounds__(BATCH_CTA, 8) k_batch_forward(const __grid_con
         // value at (eval_s, eval_v) and a finiteness check of the final surface
         if (g.t == 0) s_bad[g.gi] = 0;
         g.sync();
-        const long long n = (long long)d.nx * d.ny;
+        const long long n = (long long)d.nx * d.ld; // the pitch's padding is zero
         int bad = 0;
         for (long long q = g.t; q < n; q += g.n) bad |= !isfinite(static_cast<double>(U[q]));
         if (bad) atomicOr(&s_bad[g.gi], 1);
         g.sync();
         if (g.t == 0) {
-            const long long o = (long long)d.i0 * d.ny + d.j0;
-            p.values[inst] = d.w00 * static_cast<double>(U[o]) + d.w10 * static_cast<double>(U[o + d.ny]) +
-                             d.w01 * static_cast<double>(U[o + 1]) + d.w11 * static_cast<double>(U[o + d.ny + 1]);
+            const long long o = (long long)d.i0 * d.ld + d.j0;
+            p.values[inst] = d.w00 * static_cast<double>(U[o]) + d.w10 * static_cast<double>(U[o + d.ld]) +
+                             d.w01 * static_cast<double>(U[o + 1]) + d.w11 * static_cast<double>(U[o + d.ld + 1]);
             p.status[inst] = s_bad[g.gi];
             p.final_in_v[inst] = d.steps & 1;
         }
@@ -611,18 +648,15 @@ __global__ void __launch_bounds__(BATCH_CTA, 8) k_batch_forward(const __grid_con
     }
 }
 
-#include "adi_adjoint.cuh"
-
 // Forward + adjoint of each instance of scheme SCH by one warp group: forward pass keeping a checkpoint every
 // d.ck steps (and the stage values of every step of the last segment), then per segment (last
 // first) a forward recomputation that keeps the stage values of every step (not needed for the
 // last segment), followed by the adjoint steps of the segment in reverse order.
 // Results: value, the 5 parameter sensitivities, the final surface (state U arena) and
 // dV/d(initial condition) (state V arena).  A group of w warps works in w consecutive workspace
-// slices.  Register budget 96 per thread (5 CTAs of 4 warps per SM): fewer spills than at 80, and
-// fewer resident CTAs leave each more workspace, so the plan recomputes fewer steps.
+// slices.  Register budget 128 per thread (4 CTAs of 4 warps per SM).
 #ifndef LSS_FWDADJ_MIN_CTAS
-#define LSS_FWDADJ_MIN_CTAS 5
+#define LSS_FWDADJ_MIN_CTAS 4
 #endif
 template <int SCH>
 __global__ void __launch_bounds__(BATCH_CTA, LSS_FWDADJ_MIN_CTAS) k_batch_fwdadj(const __grid_constant__ bparams<double> p)
@@ -643,49 +677,33 @@ __global__ void __launch_bounds__(BATCH_CTA, LSS_FWDADJ_MIN_CTAS) k_batch_fwdadj
         const bdesc d = p.desc[inst];
         const inst_view<double> v = make_view(p, d);
         const int nx = d.nx, ny = d.ny;
-        const long long n = (long long)nx * ny;
+        const long long n = (long long)nx * d.ld;
         const int c = d.ck;
         const int nseg = (d.steps + c - 1) / c;
         double *sb0 = p.B0 + d.ox;
         // workspace carve-up
         double *CK = ws;                                  // nseg * n
-        double *SEG = CK + (long long)nseg * n;           // (c + 1) * 4 * n
+        double *SEG = CK + (long long)nseg * n;           // (c + 1) * 4 * n: U, D1, D2, D3 of a step
         double *W0 = SEG + (long long)(c + 1) * 4 * n;    // n
         double *W1 = W0 + n;                              // n
-        double *UB = W1 + n, *VB = UB + n, *Y1B = VB + n, *Y2B = Y1B + n, *Y3B = Y2B + n, *FB = Y3B + n;
-        double *TMP = FB + n;
-        double *LV = TMP + n, *LS = LV + nx, *HS = LS + ny;
+        double *VB = W1 + n, *DB = VB + n, *FB = DB + n, *MU = FB + n, *DV = MU + n, *D2B = DV + n;
+        double *LV = D2B + n, *LS = LV + nx, *HS = LS + ny;
         auto slot = [&](int m, int a) -> double * { return SEG + ((long long)m * 4 + a) * n; };
 
-        // clear what must start at zero for this instance's shape
-        for (long long q = g.t; q < n; q += g.n) {
-            FB[q] = 0.0;
-            Y1B[q] = 0.0;
-            Y3B[q] = 0.0;
-            CK[q] = static_cast<double>(p.payoff[d.o2 + q]);
-        }
-        for (int m = 0; m < c; ++m) {
-            double *y2 = slot(m, 2);
-            for (int q = g.t; q < ny; q += g.n) {
-                y2[q] = 0.0;
-                y2[(long long)(nx - 1) * ny + q] = 0.0;
-            }
-        }
+        // FB's boundary rows and columns are read as zeros
+        for (long long q = g.t; q < n; q += g.n) FB[q] = VB[q] = 0.0;
+        load_payoff(p, d, CK, g);
         g.sync();
-        // forward pass with checkpoints; the steps of the last segment keep their stage values in
+        // forward pass with checkpoints; the steps of the last segment keep their stage increments in
         // the segment slots, so the reverse sweep starts without recomputing that segment
         const double *cur = CK;
         const int n0_last = (nseg - 1) * c;
         for (int step = 0; step < d.steps; ++step) {
-            if (step >= n0_last) {
-                const int m = step - n0_last;
-                fwd_step<double, SCH>(v, cur, slot(m, 1), slot(m, 2), slot(m, 3), slot(m + 1, 0), sb0, d.bnc, g);
-                cur = slot(m + 1, 0);
-                continue;
-            }
-            double *next = ((step + 1) % c == 0 && step + 1 < d.steps) ? CK + (long long)((step + 1) / c) * n
-                                                                        : ((step & 1) ? W1 : W0);
-            fwd_step<double, SCH>(v, cur, slot(0, 1), slot(0, 2), slot(0, 3), next, sb0, d.bnc, g);
+            const bool keep = step >= n0_last;
+            const int m = keep ? step - n0_last : 0;
+            double *next = keep ? slot(m + 1, 0)
+                                : (step + 1) % c == 0 ? CK + (long long)((step + 1) / c) * n : ((step & 1) ? W1 : W0);
+            delta_step<SCH>(v, d, cur, slot(m, 1), slot(m, 2), slot(m, 3), next, sb0, g);
             cur = next;
         }
         // value, finiteness, final surface
@@ -693,58 +711,42 @@ __global__ void __launch_bounds__(BATCH_CTA, LSS_FWDADJ_MIN_CTAS) k_batch_fwdadj
         g.sync();
         int bad = 0;
         double *outU = p.U + d.o2;
-        for (long long q = g.t; q < n; q += g.n) {
-            const double val = cur[q];
-            bad |= !isfinite(val);
-            outU[q] = val;
-            VB[q] = 0.0;
-        }
+        for (int i = g.t / 32; i < nx; i += g.n / 32)
+            for (int j = g.t & 31; j < ny; j += 32) {
+                const double val = cur[i * d.ld + j];
+                bad |= !isfinite(val);
+                outU[i * d.ld + j] = val;
+            }
         if (bad) atomicOr(&s_bad[g.gi], 1);
         g.sync();
         if (g.t == 0) {
-            const long long o = (long long)d.i0 * ny + d.j0;
-            p.values[inst] = d.w00 * cur[o] + d.w10 * cur[o + ny] + d.w01 * cur[o + 1] + d.w11 * cur[o + ny + 1];
+            const long long o = (long long)d.i0 * d.ld + d.j0;
+            p.values[inst] = d.w00 * cur[o] + d.w10 * cur[o + d.ld] + d.w01 * cur[o + 1] + d.w11 * cur[o + d.ld + 1];
             p.status[inst] = s_bad[g.gi];
             p.final_in_v[inst] = 0;
             VB[o] = d.w00;
-            VB[o + ny] = d.w10;
+            VB[o + d.ld] = d.w10;
             VB[o + 1] = d.w01;
-            VB[o + ny + 1] = d.w11;
+            VB[o + d.ld + 1] = d.w11;
         }
         g.sync();
         // reverse sweep over the segments
-        adj_acc acc;
-        for (int q = 0; q < 5; ++q) acc.s[q] = 0.0;
-        acc.vk = acc.vt = acc.vs1 = acc.vs2 = acc.vb = 0.0;
-        double *ub = UB, *vb = VB;
+        adj_acc acc = {{0.0, 0.0, 0.0, 0.0, 0.0}};
         for (int sgi = nseg - 1; sgi >= 0; --sgi) {
             const int n0 = sgi * c;
             const int L = min(c, d.steps - n0);
             const double *u0 = CK + (long long)sgi * n;
-            for (int m = 0; m < L && sgi < nseg - 1; ++m) {
-                const double *um = (m == 0) ? u0 : slot(m, 0);
-                fwd_step<double, SCH>(v, um, slot(m, 1), slot(m, 2), slot(m, 3), slot(m + 1, 0), sb0, d.bnc, g);
-            }
-            for (int m = L - 1; m >= 0; --m) {
-                const double *um = (m == 0) ? u0 : slot(m, 0);
-                adj_step<SCH>(v, d, um, slot(m, 1), slot(m, 2), slot(m, 3), slot(m + 1, 0), vb, ub, Y1B, Y2B, Y3B, FB,
-                              TMP, LV, LS, HS, acc, d.a_tau0 + d.a_dtau * (n0 + m), g);
-                double *t = ub;
-                ub = vb;
-                vb = t;
-            }
+            for (int m = 0; m < L && sgi < nseg - 1; ++m)
+                delta_step<SCH>(v, d, m == 0 ? u0 : slot(m, 0), slot(m, 1), slot(m, 2), slot(m, 3), slot(m + 1, 0), sb0, g);
+            for (int m = L - 1; m >= 0; --m)
+                delta_adjoint<SCH>(v, d, m == 0 ? u0 : slot(m, 0), slot(m, 1), slot(m, 2), slot(m, 3), slot(m + 1, 0), VB, DB, FB, MU, DV,
+                                   D2B, LV, LS, HS, acc, d.a_tau0 + d.a_dtau * (n0 + m), g);
         }
-        // vb = adjoint of the initial condition
+        // VB = adjoint of the initial condition
         double *outL = p.V + d.o2;
-        for (long long q = g.t; q < n; q += g.n) outL[q] = vb[q];
-        const double th = d.a_theta, ni = d.a_ni;
-        double gr[5];
+        for (long long q = g.t; q < n; q += g.n) outL[q] = VB[q];
         // order in the output: kappa, theta, sigma, rho, r
-        gr[0] = acc.s[1] + ni * th * acc.vk;
-        gr[1] = acc.s[2] + ni * th * acc.vt;
-        gr[2] = acc.s[3] + ni * th * acc.vs1 + d.a_betat * th * acc.vs2;
-        gr[3] = acc.s[4];
-        gr[4] = acc.s[0] + d.a_halfk * th * acc.vb;
+        double gr[5] = {acc.s[1], acc.s[2], acc.s[3], acc.s[4], acc.s[0]};
         // sum over the group: within each warp by shuffles, then the warps in order
         for (int q = 0; q < 5; ++q)
             for (int off = 16; off > 0; off >>= 1) gr[q] += __shfl_down_sync(0xffffffffu, gr[q], off);
@@ -765,25 +767,34 @@ __global__ void __launch_bounds__(BATCH_CTA, LSS_FWDADJ_MIN_CTAS) k_batch_fwdadj
 __device__ __forceinline__ int gtid() { return blockIdx.x * blockDim.x + threadIdx.x; }
 __device__ __forceinline__ int gstride() { return gridDim.x * blockDim.x; }
 
-template <typename T> __global__ void k_wide_b1(const __grid_constant__ bparams<T> p, const T *U, T *b0)
+template <typename T> __global__ void k_wide_b1(const __grid_constant__ bparams<T> p, const T *U, T *b0, T *Y2)
 {
     const bdesc d = p.desc[0];
     const inst_view<T> v = make_view(p, d);
     b1_stage<T>(v, U, b0, d.bnc, gtid(), gstride());
+    if constexpr (sizeof(T) == 8) d2_edges(v, U, Y2, gtid(), gstride());
 }
 template <typename T, int KIND>
 __global__ void k_wide_s(const __grid_constant__ bparams<T> p, const T *U, const T *Y1, const T *Y2, T *Y)
 {
     const bdesc d = p.desc[0];
     const inst_view<T> v = make_view(p, d);
-    with_scheme(d.scheme, [&](auto sch) { s_stage<T, KIND, decltype(sch)::value>(v, U, Y1, Y2, Y, gtid(), gstride()); });
+    with_scheme(d.scheme, [&](auto sch) {
+        if constexpr (sizeof(T) == 8) ds_stage<KIND, decltype(sch)::value>(v, d, U, KIND == 1 ? U : Y2, Y1, Y, gtid(), gstride());
+        else s_stage<T, KIND, decltype(sch)::value>(v, U, Y1, Y2, Y, gtid(), gstride());
+    });
 }
-template <typename T>
-__global__ void k_wide_v(const __grid_constant__ bparams<T> p, const T *in, const T *inh, const T *b0, T *out)
+// the v stage after the S stage with result `s` (LAST: the step's last one)
+template <typename T, bool LAST>
+__global__ void k_wide_v(const __grid_constant__ bparams<T> p, const T *U, const T *Y1, const T *Y2, const T *s, const T *b0, T *out)
 {
     const bdesc d = p.desc[0];
     const inst_view<T> v = make_view(p, d);
-    v_stage<T>(v, in, inh, b0, out, gtid(), gstride());
+    const bool hv = LAST && d.scheme == LSS_ADI_HUNDSDORFER_VERWER;
+    if constexpr (sizeof(T) == 4) v_stage<T>(v, hv ? Y2 : U, s, b0, out, gtid(), gstride());
+    else if constexpr (!LAST) dv_stage<V_FIRST>(v, U, s, nullptr, nullptr, b0, out, gtid(), gstride());
+    else if (hv) dv_stage<V_LAST_HV>(v, U, Y1, s, Y2, b0, out, gtid(), gstride());
+    else dv_stage<V_LAST>(v, U, s, nullptr, nullptr, b0, out, gtid(), gstride());
 }
 template <typename T> __global__ void k_wide_b2(const __grid_constant__ bparams<T> p, T *Vn)
 {
@@ -797,28 +808,91 @@ template <typename T> __global__ void k_wide_b2(const __grid_constant__ bparams<
 template <typename T> __global__ void k_wide_finish(const __grid_constant__ bparams<T> p, const T *U)
 {
     const bdesc d = p.desc[0];
-    const long long n = (long long)d.nx * d.ny;
+    const long long n = (long long)d.nx * d.ld;
     int b = 0;
     for (long long q = gtid(); q < n; q += gstride()) b |= !isfinite(static_cast<double>(U[q]));
     b = __syncthreads_or(b);
     if (b && threadIdx.x == 0) atomicOr(p.status, 1);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        const long long o = (long long)d.i0 * d.ny + d.j0;
-        p.values[0] = d.w00 * static_cast<double>(U[o]) + d.w10 * static_cast<double>(U[o + d.ny]) +
-                      d.w01 * static_cast<double>(U[o + 1]) + d.w11 * static_cast<double>(U[o + d.ny + 1]);
+        const long long o = (long long)d.i0 * d.ld + d.j0;
+        p.values[0] = d.w00 * static_cast<double>(U[o]) + d.w10 * static_cast<double>(U[o + d.ld]) +
+                      d.w01 * static_cast<double>(U[o + 1]) + d.w11 * static_cast<double>(U[o + d.ld + 1]);
         p.final_in_v[0] = d.steps & 1;
     }
+}
+
+static __global__ void k_setup_s_delta(setup_params sp, double *S0, long long stride)
+{
+    const long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (g >= sp.total_lines) return;
+    const int inst = setup_instance(sp, g);
+    const bdesc d = sp.desc[inst];
+    const int j = 1 + static_cast<int>(g - sp.line_start[inst]);
+    const int ld = d.ld, e = d.nx - 2;
+    const double th = sp.scal[3 * inst], gm = sp.scal[3 * inst + 2];
+    const long long N = sp.total_n;
+    // the next row's coefficients are loaded before this row's stores
+    double gam = 0.0, nv[7];
+    long long o = d.o2 + ld + j;
+    for (int k = 0; k < 7; ++k) nv[k] = sp.base[k * N + o];
+    for (int t = 1; t <= e; ++t, o += ld) {
+        const double M = nv[0], P = nv[1], Z = nv[2], Mt = nv[3], Pt = nv[4], W = nv[5], C = nv[6];
+        if (t < e)
+            for (int k = 0; k < 7; ++k) nv[k] = sp.base[k * N + o + ld];
+        const double a = -th * M, b = 1.0 + th * Z, c = -th * P;
+        const double ib = 1.0 / (b - a * gam);
+        gam = c * ib;
+        double *s = S0 + o;
+        s[DS_LA * stride] = a * ib;
+        s[DS_G * stride] = gam;
+        s[DS_WG * stride] = gm * C * ib;
+        s[DS_WW * stride] = M * ib;
+        s[DS_WS * stride] = Mt * ib;
+        s[DS_WQ * stride] = ((M + P - Z) - W) * ib;
+        s[DS_WC * stride] = -(Z + W) * ib;
+        s[DS_WN * stride] = Pt * ib;
+        s[DS_WE * stride] = P * ib;
+        s[DS_IB * stride] = ib;
+    }
+}
+static __global__ void k_setup_v_delta(setup_params sp, double *V0, long long stride)
+{
+    const long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (g >= sp.total_lines) return;
+    const int inst = setup_instance(sp, g);
+    const bdesc d = sp.desc[inst];
+    const int i = 1 + static_cast<int>(g - sp.line_start[inst]);
+    const int nx = d.nx, e = d.ny - 2;
+    const double th = sp.scal[3 * inst];
+    const long long N = sp.total_n, row = d.o2 + (long long)i * d.ld;
+    const double *Mt = sp.base + 3 * N + row, *Pt = sp.base + 4 * N + row, *W = sp.base + 5 * N + row;
+    double *L = V0 + d.o2 + i, *U = L + stride, *IB = U + stride;
+    double ib = 0.0, cp = 0.0;
+    for (int t = 1; t <= e; ++t) {
+        const double a = -th * Mt[t], b = 1.0 + th * W[t], c = -th * Pt[t];
+        const double l = t == 1 ? a : a * ib;
+        ib = 1.0 / (t == 1 ? b : b - l * cp);
+        L[(long long)t * nx] = l;
+        IB[(long long)t * nx] = ib;
+        if (t > 1) U[(long long)(t - 1) * nx] = cp * ib;
+        cp = c;
+    }
+    U[(long long)e * nx] = cp;
 }
 
 // ------------------------------------------------------------------------------------------
 // host side
 // ------------------------------------------------------------------------------------------
 template <typename T> struct batch_typed {
+    // line tables: delta form (FP64) or the stages on Y1, Y2, Y3 (FP32)
+    static constexpr bool DELTA = std::is_same<T, double>::value;
+    static constexpr int S_SLOTS = DELTA ? static_cast<int>(DS_COUNT) : static_cast<int>(SL_COUNT);
+    static constexpr int V_SLOTS = DELTA ? static_cast<int>(DV_COUNT) : static_cast<int>(VL_COUNT);
     int count = 0;
     std::vector<bdesc> desc;
     std::vector<int> order;
     std::vector<long long> gps;
-    long long total_n = 0, total_x = 0, total_y = 0;
+    long long total_n = 0, total_flat = 0, total_x = 0, total_y = 0; // sums of nx*ld, nx*ny, nx, ny
     dbuf<bdesc> d_desc;
     dbuf<int> d_order, d_counter, d_status, d_final, d_imap, d_jmap;
     dbuf<double> d_values;
@@ -874,8 +948,8 @@ template <typename T> struct batch_typed {
         p.Y1 = state.p + 2 * total_n;
         p.Y2 = state.p + 3 * total_n;
         p.Y3 = state.p + 4 * total_n;
-        for (int s = 0; s < SL_COUNT; ++s) p.S[s] = stab.p + s * total_n;
-        for (int s = 0; s < VL_COUNT; ++s) p.Vt[s] = vtab.p + s * total_n;
+        for (int s = 0; s < S_SLOTS; ++s) p.S[s] = stab.p + s * total_n;
+        for (int s = 0; s < V_SLOTS; ++s) p.Vt[s] = vtab.p + s * total_n;
         for (int s = 0; s < X_COUNT; ++s) p.X[s] = xarena.p + s * total_x;
         for (int s = 0; s < Y_COUNT; ++s) p.Yv[s] = yarena.p + s * total_y;
         p.imap = d_imap.p;
@@ -930,21 +1004,25 @@ template <typename T> int batch_typed<T>::create(const lss_adi_problem *ps, int 
     count = n;
     desc.resize(n);
     gps.resize(n);
-    long long on = 0, ox = 0, oy = 0;
+    long long on = 0, of = 0, ox = 0, oy = 0;
     for (int k = 0; k < n; ++k) {
         desc[k].nx = ps[k].nx;
         desc[k].ny = ps[k].ny;
         desc[k].steps = ps[k].nt - 1;
         desc[k].scheme = ps[k].scheme;
+        desc[k].ld = DELTA ? (ps[k].ny + 3) / 4 * 4 : ps[k].ny;
         desc[k].o2 = on;
+        desc[k].op = of;
         desc[k].ox = static_cast<int>(ox);
         desc[k].oy = static_cast<int>(oy);
         gps[k] = static_cast<long long>(ps[k].nx) * ps[k].ny * (ps[k].nt - 1);
-        on += static_cast<long long>(ps[k].nx) * ps[k].ny;
+        on += static_cast<long long>(ps[k].nx) * desc[k].ld;
+        of += static_cast<long long>(ps[k].nx) * ps[k].ny;
         ox += ps[k].nx;
         oy += ps[k].ny;
     }
     total_n = on;
+    total_flat = of;
     total_x = ox;
     total_y = oy;
     if (ox > (1LL << 31) || oy > (1LL << 31)) return set_error(LSS_ADI_EINVAL, "batch too large");
@@ -954,7 +1032,7 @@ template <typename T> int batch_typed<T>::create(const lss_adi_problem *ps, int 
     std::vector<T> xh(X_COUNT * static_cast<size_t>(total_x)), yh(Y_COUNT * static_cast<size_t>(total_y));
     std::vector<int> imh(total_x), jmh(total_y);
     std::vector<double> scal(3 * static_cast<size_t>(n));
-    std::vector<T> pay(static_cast<size_t>(total_n));
+    std::vector<T> pay(static_cast<size_t>(total_flat));
     const unsigned nthr = std::max(1u, std::min(32u, std::thread::hardware_concurrency()));
     std::vector<std::thread> pool;
     std::vector<int> errs(nthr, 0);
@@ -967,9 +1045,12 @@ template <typename T> int batch_typed<T>::create(const lss_adi_problem *ps, int 
                     const bdesc &d = desc[k];
                     const size_t nn = static_cast<size_t>(d.nx) * d.ny;
                     for (int s = 0; s < 7; ++s)
-                        for (size_t q = 0; q < nn; ++q)
-                            base[s * static_cast<size_t>(total_n) + d.o2 + q] = static_cast<double>(tt.coef[s * nn + q]);
-                    std::copy(tt.payoff.begin(), tt.payoff.end(), pay.begin() + d.o2);
+                        for (int i = 0; i < d.nx; ++i) {
+                            double *dst = base.data() + s * static_cast<size_t>(total_n) + d.o2 + static_cast<size_t>(i) * d.ld;
+                            const T *src = tt.coef.data() + s * nn + static_cast<size_t>(i) * d.ny;
+                            for (int j = 0; j < d.ny; ++j) dst[j] = static_cast<double>(src[j]);
+                        }
+                    std::copy(tt.payoff.begin(), tt.payoff.end(), pay.begin() + d.op);
                     const double th = tt.sc.theta, ni = tt.sc.ni, dl = tt.sc.delta, rk = tt.sc.rho;
                     scal[3 * k] = th;
                     scal[3 * k + 1] = static_cast<double>(tt.sc.zeta);
@@ -1074,10 +1155,10 @@ template <typename T> int batch_typed<T>::create(const lss_adi_problem *ps, int 
     LSS_CUDA_TRY(yarena.alloc(Y_COUNT * total_y), "batch: allocating v boundary arrays");
     LSS_CUDA_TRY(state.alloc(5 * total_n), "batch: allocating state");
     LSS_CUDA_TRY(cudaMemset(state.p, 0, state.n * sizeof(T)), "batch: clearing state");
-    LSS_CUDA_TRY(d_payoff.alloc(total_n), "batch: allocating initial conditions");
-    LSS_CUDA_TRY(d_payoff.upload(pay.data(), total_n), "batch: uploading initial conditions");
-    LSS_CUDA_TRY(stab.alloc(SL_COUNT * total_n), "batch: allocating S-line tables");
-    LSS_CUDA_TRY(vtab.alloc(VL_COUNT * total_n), "batch: allocating v-line tables");
+    LSS_CUDA_TRY(d_payoff.alloc(total_flat), "batch: allocating initial conditions");
+    LSS_CUDA_TRY(d_payoff.upload(pay.data(), total_flat), "batch: uploading initial conditions");
+    LSS_CUDA_TRY(stab.alloc(S_SLOTS * total_n), "batch: allocating S-line tables");
+    LSS_CUDA_TRY(vtab.alloc(V_SLOTS * total_n), "batch: allocating v-line tables");
     // boundary rows/columns of the line tables are read (as zeros) by the adjoint's gather
     LSS_CUDA_TRY(cudaMemset(stab.p, 0, stab.n * sizeof(T)), "batch: clearing S-line tables");
     LSS_CUDA_TRY(cudaMemset(vtab.p, 0, vtab.n * sizeof(T)), "batch: clearing v-line tables");
@@ -1118,14 +1199,16 @@ template <typename T> int batch_typed<T>::create(const lss_adi_problem *ps, int 
         for (int k = 0; k < n; ++k) { ls[k] = acc; acc += desc[k].ny - 2; }
         LSS_CUDA_TRY(d_ls.upload(ls.data(), n), "batch: line offsets");
         sp.total_lines = acc;
-        k_setup_s_lines<T><<<grid_for(acc, 128), 128>>>(sp, stab.p, total_n, yarena.p + Y_CHS * total_y);
+        if constexpr (DELTA) k_setup_s_delta<<<grid_for(acc, 128), 128>>>(sp, stab.p, total_n);
+        else k_setup_s_lines<T><<<grid_for(acc, 128), 128>>>(sp, stab.p, total_n, yarena.p + Y_CHS * total_y);
         LSS_CUDA_TRY(cudaGetLastError(), "batch: launching S-line set-up");
         LSS_CUDA_TRY(cudaDeviceSynchronize(), "batch: S-line set-up");
         acc = 0;
         for (int k = 0; k < n; ++k) { ls[k] = acc; acc += desc[k].nx - 2; }
         LSS_CUDA_TRY(d_ls.upload(ls.data(), n), "batch: line offsets");
         sp.total_lines = acc;
-        k_setup_v_lines<T><<<grid_for(acc, 128), 128>>>(sp, vtab.p, total_n, xarena.p + X_CHV * total_x);
+        if constexpr (DELTA) k_setup_v_delta<<<grid_for(acc, 128), 128>>>(sp, vtab.p, total_n);
+        else k_setup_v_lines<T><<<grid_for(acc, 128), 128>>>(sp, vtab.p, total_n, xarena.p + X_CHV * total_x);
         LSS_CUDA_TRY(cudaGetLastError(), "batch: launching v-line set-up");
         LSS_CUDA_TRY(cudaDeviceSynchronize(), "batch: v-line set-up");
     }
@@ -1145,13 +1228,13 @@ template <typename T> int batch_typed<T>::prepare_adjoint(cudaStream_t s)
 }
 
 // Workspace (doubles) of one instance checkpointed every c steps: nseg checkpoints, the stage
-// values of one segment (4 arrays per step plus the segment's end), two scratch states, seven
+// increments of one segment (4 arrays per step plus the segment's end), two scratch states, six
 // adjoint arrays and three line-end vectors.
 static long long adj_ws_need(const bdesc &d, int c)
 {
-    const long long nn = static_cast<long long>(d.nx) * d.ny;
+    const long long nn = static_cast<long long>(d.nx) * d.ld;
     const long long nseg = (d.steps + c - 1) / c;
-    return (nseg + 4LL * (c + 1) + 2 + 7) * nn + d.nx + 2LL * d.ny;
+    return (nseg + 4LL * (c + 1) + 2 + 6) * nn + d.nx + 2LL * d.ny;
 }
 
 // Bytes the adjoint workspace may take: the cap set by lss_adi_batch_set_workspace, by default
@@ -1393,8 +1476,9 @@ template <typename T> int batch_typed<T>::enqueue(int mode, cudaStream_t s)
     if (mode == 1) {
         rc = launch_fwdadj(s);
     } else {
-        LSS_CUDA_TRY(cudaMemcpyAsync(state.p, d_payoff.p, total_n * sizeof(T), cudaMemcpyDeviceToDevice, s),
-                     "batch: initial state");
+        if (!DELTA) // (the FP64 kernels read the initial conditions themselves)
+            LSS_CUDA_TRY(cudaMemcpyAsync(state.p, d_payoff.p, total_n * sizeof(T), cudaMemcpyDeviceToDevice, s),
+                         "batch: initial state");
         rc = launch_forward(s);
     }
     return rc;
@@ -1462,14 +1546,14 @@ void batch_typed<T>::enqueue_wide_step(cudaStream_t s, const bparams<T> &p, cons
     const bdesc &d = desc[0];
     T *b0 = d_b0.p;
     const int gs = grid_for(d.ny - 2, 32), gv = grid_for(d.nx - 2, 32);
-    k_wide_b1<T><<<grid_for(d.nx, 128), 128, 0, s>>>(p, U, b0);
+    k_wide_b1<T><<<grid_for(std::max(d.nx, d.ny), 128), 128, 0, s>>>(p, U, b0, Y2);
     k_wide_s<T, 1><<<gs, 32, 0, s>>>(p, U, nullptr, nullptr, Y1);
     if (d.scheme == LSS_ADI_DOUGLAS_RACHFORD) {
-        k_wide_v<T><<<gv, 32, 0, s>>>(p, U, Y1, b0, V);
+        k_wide_v<T, true><<<gv, 32, 0, s>>>(p, U, Y1, Y2, Y1, b0, V);
     } else {
-        k_wide_v<T><<<gv, 32, 0, s>>>(p, U, Y1, b0, Y2);
+        k_wide_v<T, false><<<gv, 32, 0, s>>>(p, U, Y1, Y2, Y1, b0, Y2);
         k_wide_s<T, 2><<<gs, 32, 0, s>>>(p, U, Y1, Y2, Y3);
-        k_wide_v<T><<<gv, 32, 0, s>>>(p, d.scheme == LSS_ADI_HUNDSDORFER_VERWER ? Y2 : U, Y3, b0, V);
+        k_wide_v<T, true><<<gv, 32, 0, s>>>(p, U, Y1, Y2, Y3, b0, V);
     }
     k_wide_b2<T><<<grid_for(d.ny, 128), 128, 0, s>>>(p, V);
 }
@@ -1479,7 +1563,8 @@ template <typename T> int batch_typed<T>::enqueue_wide(cudaStream_t s)
     const bdesc &d = desc[0];
     bparams<T> p = params();
     T *U = p.U, *V = p.V, *Y1 = p.Y1, *Y2 = p.Y2, *Y3 = p.Y3;
-    LSS_CUDA_TRY(cudaMemcpyAsync(U, d_payoff.p, total_n * sizeof(T), cudaMemcpyDeviceToDevice, s), "wide: initial state");
+    LSS_CUDA_TRY(cudaMemcpy2DAsync(U, d.ld * sizeof(T), d_payoff.p, d.ny * sizeof(T), d.ny * sizeof(T), d.nx,
+                                   cudaMemcpyDeviceToDevice, s), "wide: initial state");
     LSS_CUDA_TRY(cudaMemsetAsync(d_status.p, 0, sizeof(int), s), "wide: clearing the status");
     long long nl = 0;
     for (int step = 0; step < d.steps; ++step) {
@@ -1565,7 +1650,7 @@ template <typename T> struct wide_solver : wide_solver_base {
         if (parts) return parts->forward(payoff, out_surface, out_value, flags, stream, use_graph);
         cudaStream_t s = static_cast<cudaStream_t>(stream);
         const bool dev = (flags & LSS_ADI_DEVICE_POINTERS) != 0;
-        const size_t n = static_cast<size_t>(b.total_n);
+        const size_t n = static_cast<size_t>(b.total_flat);
         const void *src = payoff ? payoff : static_cast<const void *>(pay0.data());
         LSS_CUDA_TRY(cudaMemcpyAsync(b.d_payoff.p, src, n * sizeof(T),
                                      (payoff && dev) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s),
@@ -1576,7 +1661,9 @@ template <typename T> struct wide_solver : wide_solver_base {
             LSS_CUDA_TRY(cudaMemcpyAsync(out_value, b.d_values.p, sizeof(double), cudaMemcpyDeviceToHost, s), "wide: value");
         if (out_surface) {
             const T *fin = b.state.p + ((b.desc[0].steps & 1) ? b.total_n : 0);
-            LSS_CUDA_TRY(cudaMemcpyAsync(out_surface, fin, n * sizeof(T), dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, s),
+            const bdesc &d = b.desc[0];
+            LSS_CUDA_TRY(cudaMemcpy2DAsync(out_surface, d.ny * sizeof(T), fin, d.ld * sizeof(T), d.ny * sizeof(T), d.nx,
+                                           dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, s),
                          "wide: surface");
         }
         if (!dev || out_value) LSS_CUDA_TRY(cudaStreamSynchronize(s), "wide: time loop");
@@ -1674,7 +1761,8 @@ int adjoint_solver::run(const void *payoff, double *out_value, double *dv_dparam
     batch_typed<double> &b = *impl->b;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const bool dev = (flags & LSS_ADI_DEVICE_POINTERS) != 0;
-    const size_t n = static_cast<size_t>(b.total_n);
+    const size_t n = static_cast<size_t>(b.total_flat);
+    const bdesc &d = b.desc[0];
     if (payoff)
         LSS_CUDA_TRY(cudaMemcpyAsync(b.d_payoff.p, payoff, n * sizeof(double),
                                      dev ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s),
@@ -1688,8 +1776,8 @@ int adjoint_solver::run(const void *payoff, double *out_value, double *dv_dparam
         LSS_CUDA_TRY(cudaMemcpyAsync(dv_dparams, b.d_grads.p, 5 * sizeof(double), cudaMemcpyDeviceToHost, s),
                      "lss_adi_adjoint: gradients");
     if (dv_dpayoff)
-        LSS_CUDA_TRY(cudaMemcpyAsync(dv_dpayoff, b.state.p + b.total_n, n * sizeof(double),
-                                     dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, s),
+        LSS_CUDA_TRY(cudaMemcpy2DAsync(dv_dpayoff, d.ny * sizeof(double), b.state.p + b.total_n, d.ld * sizeof(double),
+                                       d.ny * sizeof(double), d.nx, dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, s),
                      "lss_adi_adjoint: payoff gradient");
     LSS_CUDA_TRY(cudaStreamSynchronize(s), "lss_adi_adjoint: run");
     return LSS_ADI_OK;
@@ -1713,8 +1801,8 @@ template <typename T> static int payoff_grad_t(batch_typed<T> &bt, int index, vo
     if (!std::is_same<T, double>::value) return set_error(LSS_ADI_EUNSUPPORTED, "lss_adi_batch_payoff_gradient: FP64 only");
     LSS_CUDA_TRY(cudaDeviceSynchronize(), "batch: synchronising");
     const bdesc &d = bt.desc[index];
-    LSS_CUDA_TRY(cudaMemcpy(out, bt.state.p + bt.total_n + d.o2, static_cast<size_t>(d.nx) * d.ny * sizeof(T),
-                            cudaMemcpyDeviceToHost),
+    LSS_CUDA_TRY(cudaMemcpy2D(out, d.ny * sizeof(T), bt.state.p + bt.total_n + d.o2, d.ld * sizeof(T), d.ny * sizeof(T), d.nx,
+                              cudaMemcpyDeviceToHost),
                  "batch: payoff gradient");
     return LSS_ADI_OK;
 }
@@ -1734,7 +1822,7 @@ template <typename T>
 static int run_host_t(batch_typed<T> &bt, int mode, const void *payoffs, double *values, double *grads, cudaStream_t s)
 {
     if (payoffs)
-        LSS_CUDA_TRY(cudaMemcpyAsync(bt.d_payoff.p, payoffs, bt.total_n * sizeof(T), cudaMemcpyHostToDevice, s),
+        LSS_CUDA_TRY(cudaMemcpyAsync(bt.d_payoff.p, payoffs, bt.total_flat * sizeof(T), cudaMemcpyHostToDevice, s),
                      "batch: uploading payoffs");
     int rc = bt.run(mode, s, true);
     if (rc) return rc;
@@ -1765,7 +1853,8 @@ template <typename T> static int surface_t(batch_typed<T> &bt, int index, void *
     LSS_CUDA_TRY(cudaMemcpy(&fin, bt.d_final.p + index, sizeof(int), cudaMemcpyDeviceToHost), "batch: flag");
     const bdesc &d = bt.desc[index];
     const T *src = bt.state.p + (fin ? bt.total_n : 0) + d.o2;
-    LSS_CUDA_TRY(cudaMemcpy(out, src, static_cast<size_t>(d.nx) * d.ny * sizeof(T), cudaMemcpyDeviceToHost), "batch: surface");
+    LSS_CUDA_TRY(cudaMemcpy2D(out, d.ny * sizeof(T), src, d.ld * sizeof(T), d.ny * sizeof(T), d.nx, cudaMemcpyDeviceToHost),
+                 "batch: surface");
     return LSS_ADI_OK;
 }
 

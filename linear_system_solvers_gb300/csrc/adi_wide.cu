@@ -87,7 +87,7 @@ template <typename T> struct line_solver {
         LSS_CUDA_TRY(state.alloc(5 * n), "wide: allocating state");
         LSS_CUDA_TRY(cudaMemset(state.p, 0, state.n * sizeof(T)), "wide: clearing state");
         U = state.p; Vn = U + n; D1 = U + 2 * n; D2 = U + 3 * n; D3 = U + 4 * n;
-        LSS_CUDA_TRY(stab.alloc(9 * n), "wide: allocating S-line tables");
+        LSS_CUDA_TRY(stab.alloc(W_COUNT * n), "wide: allocating S-line tables");
         LSS_CUDA_TRY(vtab.alloc(3 * n), "wide: allocating v-line tables");
         LSS_CUDA_TRY(cudaMemset(stab.p, 0, stab.n * sizeof(T)), "wide: clearing S-line tables");
         LSS_CUDA_TRY(cudaMemset(vtab.p, 0, vtab.n * sizeof(T)), "wide: clearing v-line tables");
@@ -150,7 +150,7 @@ template <typename T> struct line_solver {
         wp.zeta = static_cast<T>(tt.sc.zeta);
         wp.zt = static_cast<T>(static_cast<double>(tt.sc.zeta) - static_cast<double>(tt.sc.theta));
         wp.bnc = static_cast<T>(-dl * (2.0 * h1 * static_cast<double>(tt.s_hi_neu[0])) * static_cast<double>(tt.coef_v0[nx - 1]));
-        for (int k = 0; k < 9; ++k) wp.S[k] = stab.p + k * n;
+        for (int k = 0; k < W_COUNT; ++k) wp.S[k] = stab.p + k * n;
         for (int k = 0; k < 3; ++k) wp.V[k] = vtab.p + k * n;
         const T *x = xy.p;
         wp.xbm = x; wp.xbc = x + nx; wp.xbp = x + 2 * nx; wp.xb2 = x + 3 * nx; wp.xb1 = x + 4 * nx; wp.xvhi = x + 5 * nx;
