@@ -60,7 +60,7 @@ struct lss_adi_handle {
     std::unique_ptr<plain_solver<double>> s64;
     std::unique_ptr<plain_solver<float>> s32;
     std::unique_ptr<wide_solver_base> wide;
-    std::unique_ptr<adjoint_solver> adj;
+    std::unique_ptr<wide_adjoint_base> adj;
 };
 
 template <typename T> static void tables_from(const lss_adi_problem &p, instance_tables<T> &tab) { build_tables_for<T>(p, tab); }
@@ -182,9 +182,10 @@ int lss_adi_adjoint(lss_adi_handle *h, const void *payoff, double *out_value, do
         return set_error(LSS_ADI_EUNSUPPORTED, "lss_adi_adjoint: parametric FP64 problems only");
     if (checkpoint_every < 0) return set_error(LSS_ADI_EINVAL, "lss_adi_adjoint: checkpoint_every must be >= 0");
     if (!h->adj) {
-        std::unique_ptr<adjoint_solver> a(new (std::nothrow) adjoint_solver());
-        if (!a) return set_error(LSS_ADI_ENOMEM, "host allocation failed");
-        int rc = a->init(h->prob);
+        if (h->prob.scheme == LSS_ADI_EXPLICIT_EULER)
+            return set_error(LSS_ADI_EUNSUPPORTED, "lss_adi_adjoint: no adjoint for the explicit Euler scheme");
+        std::unique_ptr<wide_adjoint_base> a;
+        int rc = make_wide_adjoint(h->prob, a);
         if (rc) return rc;
         if (h->wide) { // the forward's chunk counts, so both passes solve alike
             int ps = 0, pv = 0;

@@ -591,6 +591,13 @@ __device__ __forceinline__ void fwd_step(const inst_view<T> &v, const T *U, T *Y
 // the rows that they load ahead), 64 in FP32 (8 CTAs).
 constexpr int BATCH_CTA = 32 * MAX_GROUP_WARPS;
 
+// value at (eval_s, eval_v), corner o of its cell
+template <typename T> __device__ __forceinline__ double bilinear_value(const bdesc &d, const T *U, long long o)
+{
+    const double a = U[o], b = U[o + d.ld], c = U[o + 1], e = U[o + d.ld + 1];
+    if (sizeof(T) == 8) return fma(d.w11, e, fma(d.w01, c, fma(d.w10, b, d.w00 * a)));
+    return d.w00 * a + d.w10 * b + d.w01 * c + d.w11 * e;
+}
 // initial condition into the pitched state
 template <typename T> __device__ __forceinline__ void load_payoff(const bparams<T> &p, const bdesc &d, T *U, const grp &g)
 {
@@ -639,8 +646,7 @@ __global__ void __launch_bounds__(BATCH_CTA, sizeof(T) == 8 ? LSS_FWD_MIN_CTAS :
         g.sync();
         if (g.t == 0) {
             const long long o = (long long)d.i0 * d.ld + d.j0;
-            p.values[inst] = d.w00 * static_cast<double>(U[o]) + d.w10 * static_cast<double>(U[o + d.ld]) +
-                             d.w01 * static_cast<double>(U[o + 1]) + d.w11 * static_cast<double>(U[o + d.ld + 1]);
+            p.values[inst] = bilinear_value(d, U, o);
             p.status[inst] = s_bad[g.gi];
             p.final_in_v[inst] = d.steps & 1;
         }
@@ -721,7 +727,7 @@ __global__ void __launch_bounds__(BATCH_CTA, LSS_FWDADJ_MIN_CTAS) k_batch_fwdadj
         g.sync();
         if (g.t == 0) {
             const long long o = (long long)d.i0 * d.ld + d.j0;
-            p.values[inst] = d.w00 * cur[o] + d.w10 * cur[o + d.ld] + d.w01 * cur[o + 1] + d.w11 * cur[o + d.ld + 1];
+            p.values[inst] = bilinear_value(d, cur, o);
             p.status[inst] = s_bad[g.gi];
             p.final_in_v[inst] = 0;
             VB[o] = d.w00;
@@ -771,8 +777,12 @@ template <typename T> __global__ void k_wide_b1(const __grid_constant__ bparams<
 {
     const bdesc d = p.desc[0];
     const inst_view<T> v = make_view(p, d);
-    b1_stage<T>(v, U, b0, d.bnc, gtid(), gstride());
-    if constexpr (sizeof(T) == 8) d2_edges(v, U, Y2, gtid(), gstride());
+    if constexpr (sizeof(T) == 8) {
+        db1_stage(v, d, U, b0, gtid(), gstride());
+        d2_edges(v, U, Y2, gtid(), gstride());
+    } else {
+        b1_stage<T>(v, U, b0, d.bnc, gtid(), gstride());
+    }
 }
 template <typename T, int KIND>
 __global__ void k_wide_s(const __grid_constant__ bparams<T> p, const T *U, const T *Y1, const T *Y2, T *Y)
@@ -800,7 +810,8 @@ template <typename T> __global__ void k_wide_b2(const __grid_constant__ bparams<
 {
     const bdesc d = p.desc[0];
     const inst_view<T> v = make_view(p, d);
-    b2_stage<T>(v, Vn, gtid(), gstride());
+    if constexpr (sizeof(T) == 8) db2_stage(v, Vn, gtid(), gstride());
+    else b2_stage<T>(v, Vn, gtid(), gstride());
 }
 // value, finiteness flag and final-array flag of the single instance
 // value at the evaluation point and finiteness of the final surface, grid-wide (the status word
@@ -815,8 +826,7 @@ template <typename T> __global__ void k_wide_finish(const __grid_constant__ bpar
     if (b && threadIdx.x == 0) atomicOr(p.status, 1);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         const long long o = (long long)d.i0 * d.ld + d.j0;
-        p.values[0] = d.w00 * static_cast<double>(U[o]) + d.w10 * static_cast<double>(U[o + d.ld]) +
-                      d.w01 * static_cast<double>(U[o + 1]) + d.w11 * static_cast<double>(U[o + d.ld + 1]);
+        p.values[0] = bilinear_value(d, U, o);
         p.final_in_v[0] = d.steps & 1;
     }
 }
@@ -840,7 +850,7 @@ static __global__ void k_setup_s_delta(setup_params sp, double *S0, long long st
         if (t < e)
             for (int k = 0; k < 7; ++k) nv[k] = sp.base[k * N + o + ld];
         const double a = -th * M, b = 1.0 + th * Z, c = -th * P;
-        const double ib = 1.0 / (b - a * gam);
+        const double ib = 1.0 / fma(-a, gam, b);
         gam = c * ib;
         double *s = S0 + o;
         s[DS_LA * stride] = a * ib;
@@ -871,7 +881,7 @@ static __global__ void k_setup_v_delta(setup_params sp, double *V0, long long st
     for (int t = 1; t <= e; ++t) {
         const double a = -th * Mt[t], b = 1.0 + th * W[t], c = -th * Pt[t];
         const double l = t == 1 ? a : a * ib;
-        ib = 1.0 / (t == 1 ? b : b - l * cp);
+        ib = 1.0 / (t == 1 ? b : fma(-l, cp, b));
         L[(long long)t * nx] = l;
         IB[(long long)t * nx] = ib;
         if (t > 1) U[(long long)(t - 1) * nx] = cp * ib;
@@ -1713,73 +1723,6 @@ int make_wide_solver(const lss_adi_problem &p, std::unique_ptr<wide_solver_base>
     } catch (const std::bad_alloc &) {
         return set_error(LSS_ADI_ENOMEM, "wide: host allocation failed");
     }
-    return LSS_ADI_OK;
-}
-
-// lss_adi_adjoint: one parametric FP64 instance, on one warp group of the batched forward + adjoint
-// kernel or on the partitioned kernels over the whole GPU.
-struct adjoint_impl {
-    std::unique_ptr<batch_typed<double>> b;
-    std::unique_ptr<wide_adjoint_base> wide;
-};
-
-adjoint_solver::adjoint_solver() = default;
-adjoint_solver::~adjoint_solver() = default;
-
-int adjoint_solver::init(const lss_adi_problem &p)
-{
-    if (p.scheme == LSS_ADI_EXPLICIT_EULER)
-        return set_error(LSS_ADI_EUNSUPPORTED, "lss_adi_adjoint: no adjoint for the explicit Euler scheme");
-    impl.reset(new (std::nothrow) adjoint_impl());
-    if (!impl) return set_error(LSS_ADI_ENOMEM, "host allocation failed");
-    lss_adi_problem q = p;
-    q.arith = LSS_ADI_ARITH_FAST;
-    // one warp group carries an instance of up to 256 x 160 points (the same bits as a member of a
-    // batch); larger ones run wide, and so do time-dependent coefficients (SABR with r != 0), whose
-    // S-line tables the host-sequenced wide kernels rebuild before every step
-    if (p.nx > 256 || static_cast<long long>(p.nx) * p.ny > 40960 || (p.options & LSS_ADI_OPT_WIDE_ADJOINT) || time_dependent(p))
-        return make_wide_adjoint(q, impl->wide);
-    impl->b.reset(new (std::nothrow) batch_typed<double>());
-    if (!impl->b) return set_error(LSS_ADI_ENOMEM, "host allocation failed");
-    return impl->b->create(&q, 1);
-}
-
-int adjoint_solver::set_chunks(int s_chunks, int v_chunks, void *stream)
-{
-    if (!impl || !impl->wide) return LSS_ADI_OK;
-    LSS_CUDA_TRY(cudaStreamSynchronize(static_cast<cudaStream_t>(stream)), "lss_adi_adjoint: chunk counts");
-    int rc = impl->wide->set_chunks(s_chunks, v_chunks);
-    if (rc) return rc;
-    LSS_CUDA_TRY(cudaDeviceSynchronize(), "lss_adi_adjoint: chunk counts");
-    return LSS_ADI_OK;
-}
-
-int adjoint_solver::run(const void *payoff, double *out_value, double *dv_dparams, void *dv_dpayoff, int checkpoint_every,
-                        int flags, void *stream)
-{
-    if (impl->wide) return impl->wide->run(payoff, out_value, dv_dparams, dv_dpayoff, checkpoint_every, flags, stream);
-    batch_typed<double> &b = *impl->b;
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const bool dev = (flags & LSS_ADI_DEVICE_POINTERS) != 0;
-    const size_t n = static_cast<size_t>(b.total_flat);
-    const bdesc &d = b.desc[0];
-    if (payoff)
-        LSS_CUDA_TRY(cudaMemcpyAsync(b.d_payoff.p, payoff, n * sizeof(double),
-                                     dev ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s),
-                     "lss_adi_adjoint: copying the terminal condition");
-    b.ck_override = checkpoint_every;
-    int rc = b.run(1, s, false);
-    if (rc) return rc;
-    if (out_value)
-        LSS_CUDA_TRY(cudaMemcpyAsync(out_value, b.d_values.p, sizeof(double), cudaMemcpyDeviceToHost, s), "lss_adi_adjoint: value");
-    if (dv_dparams)
-        LSS_CUDA_TRY(cudaMemcpyAsync(dv_dparams, b.d_grads.p, 5 * sizeof(double), cudaMemcpyDeviceToHost, s),
-                     "lss_adi_adjoint: gradients");
-    if (dv_dpayoff)
-        LSS_CUDA_TRY(cudaMemcpy2DAsync(dv_dpayoff, d.ny * sizeof(double), b.state.p + b.total_n, d.ld * sizeof(double),
-                                       d.ny * sizeof(double), d.nx, dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, s),
-                     "lss_adi_adjoint: payoff gradient");
-    LSS_CUDA_TRY(cudaStreamSynchronize(s), "lss_adi_adjoint: run");
     return LSS_ADI_OK;
 }
 

@@ -10,21 +10,6 @@
 
 namespace lss_gb300 {
 
-struct batch_impl;   // defined in adi_batched.cu
-struct adjoint_impl; // defined in adi_adjoint.cu
-
-// Forward + adjoint of one parametric FP64 Heston problem (behind lss_adi_adjoint).
-struct adjoint_solver {
-    std::unique_ptr<adjoint_impl> impl;
-    adjoint_solver();
-    ~adjoint_solver();
-    int init(const lss_adi_problem &p);
-    int run(const void *payoff, double *out_value, double *dv_dparams, void *dv_dpayoff, int checkpoint_every, int flags,
-            void *stream);
-    // chunk counts of the partitioned solves of a large instance (no effect on one-group instances)
-    int set_chunks(int s_chunks, int v_chunks, void *stream);
-};
-
 // Single instance on the factorised ("fast") arithmetic: one kernel per stage over the whole
 // GPU, graph-replayed time loop (behind lss_adi_create with LSS_ADI_ARITH_FAST).
 struct wide_solver_base {
@@ -39,10 +24,10 @@ int make_wide_solver(const lss_adi_problem &p, std::unique_ptr<wide_solver_base>
 // the same with the line solves partitioned over the whole GPU (adi_wide.cu)
 int make_partitioned_solver(const lss_adi_problem &p, std::unique_ptr<wide_solver_base> &out);
 
-// Forward + adjoint of one FP64 instance with the same partitioned solves (adi_wide.cu).
+// Forward + adjoint of one parametric FP64 instance (behind lss_adi_adjoint, adi_wide.cu).
 struct wide_adjoint_base {
     virtual ~wide_adjoint_base() = default;
-    virtual int set_chunks(int s_chunks, int v_chunks) = 0; // 0: chosen by the line's length
+    virtual int set_chunks(int s_chunks, int v_chunks, void *stream) = 0; // 0: chosen by the line's length
     virtual int run(const void *payoff, double *out_value, double *dv_dparams, void *dv_dpayoff, int checkpoint_every, int flags,
                     void *stream) = 0;
 };

@@ -40,6 +40,30 @@ enum { V_FIRST = 0, V_LAST = 1, V_LAST_HV = 2 };
 
 constexpr int BK = 8; // rows of a block of the one-instruction passes
 
+// The explicit v = v_lo column and the rows of S_lo and S_max (b1_stage, b2_stage) in the order of
+// adi_wide.cuh: a single instance in relay order has the same bits.
+__device__ __forceinline__ void db1_stage(const inst_view<double> &v, const bdesc &d, const double *U, double *sb0, int l0, int ls)
+{
+    const int nx = v.nx, ld = v.ld;
+    for (int i = l0; i < nx; i += ls) {
+        const double *u = U + i * ld;
+        double r = fma(__ldg(v.X(XB_2) + i), u[2], fma(__ldg(v.X(XB_1) + i), u[1], __ldg(v.X(XB_C) + i) * u[0]));
+        if (i == 0) r = __ldg(v.Yv(Y_SLO));
+        else if (i == nx - 1) r += d.bnc;
+        else r = fma(__ldg(v.X(XB_P) + i), u[ld], fma(__ldg(v.X(XB_M) + i), u[-ld], r));
+        sb0[i] = r;
+    }
+}
+__device__ __forceinline__ void db2_stage(const inst_view<double> &v, double *Vn, int l0, int ls)
+{
+    const int ny = v.ny, ld = v.ld, last = (v.nx - 1) * ld;
+    for (int j = l0; j < ny; j += ls) {
+        Vn[j] = __ldg(v.Yv(Y_SLO) + j);
+        const int jj = __ldg(v.jmap() + j);
+        Vn[last + j] = fma(4.0 / 3.0, Vn[last - ld + jj], fma(-1.0 / 3.0, Vn[last - 2 * ld + jj], -__ldg(v.Yv(Y_B2C) + j)));
+    }
+}
+
 // One S stage.  KIND 1: A = U.  KIND 2: A = D2.  Y: the increment, rows 0 and nx-1 included.
 template <int KIND, int SCH>
 __device__ __forceinline__ void ds_stage(const inst_view<double> &v, const bdesc &d, const double *U, const double *A, const double *D1,
@@ -265,8 +289,8 @@ __device__ __forceinline__ void da_b2(const inst_view<double> &v, double *VB, in
     for (int q = l0; q < ny; q += ls) {
         double add = __ldg(v.jmap() + q) == q ? VB[last + q] : 0.0;
         if (q + 1 < ny && __ldg(v.jmap() + q + 1) == q) add += VB[last + q + 1];
-        VB[last - ld + q] += (4.0 / 3.0) * add;
-        VB[last - 2 * ld + q] -= (1.0 / 3.0) * add;
+        VB[last - ld + q] = fma(4.0 / 3.0, add, VB[last - ld + q]);
+        VB[last - 2 * ld + q] = fma(-1.0 / 3.0, add, VB[last - 2 * ld + q]);
     }
 }
 // rows 0 and nx-1 of a step's output do not depend on its input
@@ -415,7 +439,7 @@ __device__ __forceinline__ void da_s(const inst_view<double> &v, const bdesc &d,
             }
             return r;
         };
-        double sY = 0, sB = 0, sE = 0, sA = 0, sC = 0, sQ = 0, sS = 0, sYa = 0, sYd = 0, sAa = 0, sDd = 0, vm = 0, v0 = 0, vp = 0;
+        double sY = 0, sB = 0, sE = 0, sA = 0, sC = 0, sQ = 0, sS = 0, sYa = 0, sYd = 0, sAa = 0, sDd = 0, vd = 0, v0 = 0, vm = 0;
         double xh = X[last + j], xc = X[last - ld + j], yh = Y[last + j], yc = Y[last - ld + j];
         double ddh = X[last + j - 1] - X[last + j + 1], ss = X[last - ld + j - 1], ddc = ss - X[last - ld + j + 1];
         double w = 0.0;
@@ -440,7 +464,7 @@ __device__ __forceinline__ void da_s(const inst_view<double> &v, const bdesc &d,
                 sA = fma(mx, dx, sA);
                 sC = fma(mu, xc, sC);
                 sQ = fma(mu, ddc, sQ);
-                sS = fma(mu, ss, sS);
+                sS = fma(mu, ss - xc, sS);
             }
             if (sabr) {
                 const double ma = mu * __ldg(v.X(X_HA) + t), md = mu * __ldg(v.X(X_HDD) + t);
@@ -451,9 +475,9 @@ __device__ __forceinline__ void da_s(const inst_view<double> &v, const bdesc &d,
                     sDd = fma(md, dx, sDd);
                 }
             }
-            vm = fma(r.m, r.x0, vm);
+            vd = fma(r.m, r.x2 - r.x0, vd);
             v0 = fma(r.m, r.x1, v0);
-            vp = fma(r.m, r.x2, vp);
+            vm = fma(r.m, r.x0 - r.x1, vm);
             xh = xc; xc = r.xc;
             yh = yc; yc = r.y;
             ddh = ddc; ddc = ddl;
@@ -472,7 +496,7 @@ __device__ __forceinline__ void da_s(const inst_view<double> &v, const bdesc &d,
         }
         // the line's sums: theta weighs the terms in Y, wx those in X
         const double th = d.a_theta, wx = KIND == 1 ? 1.0 : hv ? d.a_zeta : d.a_zeta - d.a_theta, we = KIND == 1 ? 1.0 : d.a_zeta;
-        const double A = th * sY + wx * sA, B = -(th * sB + 2.0 * wx * sC), Q = -wx * sQ, D = wx * (2.0 * sS - sQ - 2.0 * sC);
+        const double A = th * sY + wx * sA, B = -(th * sB + 2.0 * wx * sC), Q = -wx * sQ, D = wx * (2.0 * sS - sQ);
         const double E = we * d.a_gamma * sE;
         const double ek = __ldg(v.Yv(Y_EK) + j), et = __ldg(v.Yv(Y_ET) + j), es = __ldg(v.Yv(Y_ES) + j), bs = __ldg(v.Yv(Y_BS) + j);
         const double hy = __ldg(v.Yv(Y_HY) + j);
@@ -480,11 +504,11 @@ __device__ __forceinline__ void da_s(const inst_view<double> &v, const bdesc &d,
         if (sabr)
             g0 += tau * d.a_omb * (__ldg(v.Yv(Y_HV2) + j) * (2.0 * d.a_delta * (th * sYd + wx * sDd) - 2.0 * d.a_alphat * (th * sYa + wx * sAa)) -
                                    d.a_rho * d.a_sigma * hy * E);
-        const double nq = d.a_ni * (Q + th * (vp - vm));
+        const double nq = d.a_ni * (Q + th * vd);
         acc.s[0] += g0 - d.a_halfk * th * v0;
         acc.s[1] += ek * nq;
         acc.s[2] += et * nq;
-        acc.s[3] += es * nq + d.a_betat * bs * (D + th * (vm + vp - 2.0 * v0)) + d.a_rho * hy * E;
+        acc.s[3] += es * nq + d.a_betat * bs * (D + th * (2.0 * vm + vd)) + d.a_rho * hy * E;
         acc.s[4] += d.a_sigma * hy * E;
     }
 }
@@ -608,10 +632,10 @@ __device__ __forceinline__ void da_b1(const inst_view<double> &v, const bdesc &d
     for (int p = l0; p < nx; p += ls) {
         const int o = p * ld;
         const double bb = B0(p);
-        VB[o] += (p + 1 <= nx - 2 ? __ldg(v.X(XB_M) + p + 1) * B0(p + 1) : 0.0) + __ldg(v.X(XB_C) + p) * bb +
-                 (p >= 1 ? __ldg(v.X(XB_P) + p - 1) * B0(p - 1) : 0.0);
-        VB[o + 1] += __ldg(v.X(XB_1) + p) * bb;
-        VB[o + 2] += __ldg(v.X(XB_2) + p) * bb;
+        const double below = p >= 1 ? __ldg(v.X(XB_P) + p - 1) : 0.0, above = p + 1 <= nx - 2 ? __ldg(v.X(XB_M) + p + 1) : 0.0;
+        VB[o] += fma(below, B0(p - 1), fma(__ldg(v.X(XB_C) + p), bb, above * B0(p + 1)));
+        VB[o + 1] = fma(__ldg(v.X(XB_1) + p), bb, VB[o + 1]);
+        VB[o + 2] = fma(__ldg(v.X(XB_2) + p), bb, VB[o + 2]);
         if (bb != 0.0) {
             const double u0 = U[o], u1 = U[o + 1], u2 = U[o + 2];
             const double ee = d.a_ni * bb * (4.0 * u1 - 3.0 * u0 - u2);
@@ -631,7 +655,7 @@ __device__ __forceinline__ void delta_step(const inst_view<double> &v, const bde
                                            double *Vn, double *sb0, const grp &g)
 {
     const int l0 = g.t, ls = g.n;
-    b1_stage<double>(v, U, sb0, d.bnc, l0, ls);
+    db1_stage(v, d, U, sb0, l0, ls);
     ds_stage<1, SCH>(v, d, U, U, nullptr, D1, l0, ls);
     if constexpr (SCH != LSS_ADI_DOUGLAS_RACHFORD) d2_edges(v, U, D2, l0, ls);
     g.sync();
@@ -646,7 +670,7 @@ __device__ __forceinline__ void delta_step(const inst_view<double> &v, const bde
         else dv_stage<V_LAST>(v, U, D3, nullptr, nullptr, sb0, Vn, l0, ls);
     }
     g.sync();
-    b2_stage<double>(v, Vn, l0, ls);
+    db2_stage(v, Vn, l0, ls);
     g.sync();
 }
 

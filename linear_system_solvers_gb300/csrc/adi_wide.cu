@@ -56,6 +56,7 @@ template <typename T> struct line_solver {
     dbuf<double> value;
     bilinear bil{};
     wparams<T> wp{};
+    bool serial = false; // recurrences in relay order (FP64)
     T *U = nullptr, *Vn = nullptr, *D1 = nullptr, *D2 = nullptr, *D3 = nullptr;
     long long launches = 0;
     // time-dependent coefficients (FP64)
@@ -63,6 +64,10 @@ template <typename T> struct line_solver {
     dbuf<double> td_mem;
     tdep_tab td{};
     std::vector<double> td_da, td_dc;
+    dbuf<double> td_sets;
+    tdep_set td_set{};
+    int td_group = 1, td_have = -1; // steps per set-up launch; the group whose tables are held
+    bool td_adjoint = false;
     cudaGraphExec_t graph = nullptr;
 
     ~line_solver()
@@ -87,9 +92,10 @@ template <typename T> struct line_solver {
         LSS_CUDA_TRY(state.alloc(5 * n), "wide: allocating state");
         LSS_CUDA_TRY(cudaMemset(state.p, 0, state.n * sizeof(T)), "wide: clearing state");
         U = state.p; Vn = U + n; D1 = U + 2 * n; D2 = U + 3 * n; D3 = U + 4 * n;
-        LSS_CUDA_TRY(stab.alloc(W_COUNT * n), "wide: allocating S-line tables");
+        const bool td_case = time_dependent(p); // (S-line tables in sets: set_chunks)
+        if (!td_case) LSS_CUDA_TRY(stab.alloc(W_COUNT * n), "wide: allocating S-line tables");
         LSS_CUDA_TRY(vtab.alloc(3 * n), "wide: allocating v-line tables");
-        LSS_CUDA_TRY(cudaMemset(stab.p, 0, stab.n * sizeof(T)), "wide: clearing S-line tables");
+        if (!td_case) LSS_CUDA_TRY(cudaMemset(stab.p, 0, stab.n * sizeof(T)), "wide: clearing S-line tables");
         LSS_CUDA_TRY(cudaMemset(vtab.p, 0, vtab.n * sizeof(T)), "wide: clearing v-line tables");
         LSS_CUDA_TRY(pay.alloc(flat), "wide: allocating the initial condition");
         LSS_CUDA_TRY(surf.alloc(flat), "wide: allocating the surface");
@@ -142,7 +148,7 @@ template <typename T> struct line_solver {
             }
             LSS_CUDA_TRY(base.upload(hb.data(), hb.size()), "wide: uploading coefficient tables");
         }
-        k_wide_setup_s<T><<<grid_for(ny - 2, 32), 32>>>(base.p, n, nx, ny, ld, th, gm, stab.p);
+        if (!td_case) k_wide_setup_s<T><<<grid_for(ny - 2, 32), 32>>>(base.p, n, nx, ny, ld, th, gm, stab.p);
         k_wide_setup_v<T><<<grid_for(nx - 2, 32), 32>>>(base.p, n, nx, ny, ld, th, vtab.p);
         LSS_CUDA_TRY(cudaGetLastError(), "wide: launching the set-up");
         LSS_CUDA_TRY(cudaDeviceSynchronize(), "wide: set-up");
@@ -150,13 +156,13 @@ template <typename T> struct line_solver {
         wp.zeta = static_cast<T>(tt.sc.zeta);
         wp.zt = static_cast<T>(static_cast<double>(tt.sc.zeta) - static_cast<double>(tt.sc.theta));
         wp.bnc = static_cast<T>(-dl * (2.0 * h1 * static_cast<double>(tt.s_hi_neu[0])) * static_cast<double>(tt.coef_v0[nx - 1]));
-        for (int k = 0; k < W_COUNT; ++k) wp.S[k] = stab.p + k * n;
+        for (int k = 0; k < W_COUNT && !td_case; ++k) wp.S[k] = stab.p + k * n;
         for (int k = 0; k < 3; ++k) wp.V[k] = vtab.p + k * n;
         const T *x = xy.p;
         wp.xbm = x; wp.xbc = x + nx; wp.xbp = x + 2 * nx; wp.xb2 = x + 3 * nx; wp.xb1 = x + 4 * nx; wp.xvhi = x + 5 * nx;
         wp.yslo = x + 6 * nx; wp.yb2c = wp.yslo + ny;
         wp.imap = maps.p; wp.jmap = maps.p + nx;
-        if (time_dependent(p)) {
+        if (td_case) {
             int rc = init_tdep(tt);
             if (rc) return rc;
         }
@@ -235,19 +241,23 @@ template <typename T> struct line_solver {
         for (carry_tab<T> *c : {&wp.vf, &wp.vb}) carve(*c, wp.v, q);
         if (graph) cudaGraphExecDestroy(graph);
         graph = nullptr;
-        for (int dir = 0; dir < 2; ++dir) {
-            if (!tdep || dir == 1) products(nullptr, dir == 0);
+        if (tdep) {
+            const int rc = set_groups();
+            if (rc) return rc;
+        } else {
+            products(nullptr, true);
         }
+        products(nullptr, false);
         LSS_CUDA_TRY(cudaGetLastError(), "wide: chunk products");
         return LSS_ADI_OK;
     }
 
     // one launch with programmatic stream serialisation
     template <typename... P, typename... A>
-    void launch(cudaStream_t s, void (*k)(P...), int grid, dim3 block, size_t smem, A &&...args)
+    void launch(cudaStream_t s, void (*k)(P...), dim3 grid, dim3 block, size_t smem, A &&...args)
     {
         cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(grid);
+        cfg.gridDim = grid;
         cfg.blockDim = block;
         cfg.dynamicSmemBytes = smem;
         cfg.stream = s;
@@ -280,42 +290,102 @@ template <typename T> struct line_solver {
         }
     }
 
-    // the S-line tables of step `step` of a time-dependent instance
-    void refresh(cudaStream_t s, int step)
+    // Sets of S-line tables of a time-dependent instance: as many steps to a launch as keep its grid at
+    // four CTAs per SM, while the sets stay within half of L2 (64 MB).
+    int set_groups()
+    {
+        const long long chunks = static_cast<long long>(wp.s.tiles) * (2 * wp.s.PC + wp.s.groups()) * wp.ls;
+        const long long words = (W_COUNT * n + 2 * nx + (td_adjoint ? 4 : 2) * chunks + 3) / 4 * 4;
+        const long long fit = (64LL << 20) / (words * static_cast<long long>(sizeof(double))), ctas = grid_for(ny - 2, wp.s.L);
+        const long long fill = (4LL * sms + ctas - 1) / ctas;
+        td_group = static_cast<int>(std::max(1LL, std::min({fit, fill, static_cast<long long>(TDEP_STEPS), static_cast<long long>(steps)})));
+        LSS_CUDA_TRY(td_sets.alloc(td_group * words), "wide: allocating time-dependent tables");
+        LSS_CUDA_TRY(cudaMemset(td_sets.p, 0, td_sets.n * sizeof(double)), "wide: clearing time-dependent tables");
+        td_set = tdep_set{};
+        td_set.S = td_sets.p;
+        td_set.xb = td_sets.p + W_COUNT * n;
+        td_set.stride = words;
+        double *q = td_set.xb + 2 * nx;
+        carve_set(td_set.sf, q);
+        carve_set(td_set.sb, q);
+        if (td_adjoint) {
+            carve_set(td_set.sz, q);
+            carve_set(td_set.sw, q);
+        }
+        return LSS_ADI_OK;
+    }
+    void carve_set(carry_tab<double> &c, double *&q) const
+    {
+        const long long chunks = static_cast<long long>(wp.s.tiles) * wp.s.PC * wp.ls;
+        c.A = q; q += chunks;
+        c.PreG = q; q += chunks;
+        c.GA = q; q += static_cast<long long>(wp.s.tiles) * wp.s.groups() * wp.ls;
+    }
+    static carry_tab<double> shifted(const carry_tab<double> &c, long long o) { return {c.A + o, c.PreG + o, c.GA + o}; }
+
+    // Points wp (and an adjoint's sz, sw) at the S-line tables of time step `step`, made for its group
+    // of steps when they are not at hand.
+    void refresh(cudaStream_t s, int step, adj_params *ap = nullptr)
     {
         if constexpr (std::is_same<T, double>::value) {
-            int P = 1; // chunks of at least 4 rows, at most 32; 8 lines per CTA
-            while (P < 32 && nx - 2 >= 8 * P) P *= 2;
-            launch(s, k_wide_tdep_factor, grid_for(ny - 2, 8), dim3(8, P), 0, td, td_da[step], stab.p);
-            const long long pts = std::max<long long>(nx, static_cast<long long>(nx - 2) * (ny - 2));
-            launch(s, k_wide_tdep_slots, grid_for(pts, 256), dim3(256), 0, td, td_da[step], td_dc[step], stab.p,
-                   const_cast<double *>(wp.xbm), const_cast<double *>(wp.xbp));
+            const int group = step / td_group, first = group * td_group;
+            if (group != td_have) {
+                tdep_steps st{};
+                const int len = std::min(td_group, steps - first);
+                for (int k = 0; k < len; ++k) {
+                    st.da[k] = td_da[first + k];
+                    st.dc[k] = td_dc[first + k];
+                }
+                const split &sp = wp.s;
+                const size_t smem = sizeof(double) * sp.L * (4 * sp.PC + std::max(4 * sp.groups(), sp.PC));
+                const dim3 grid(grid_for(ny - 2, sp.L), len), block(sp.L * sp.PC);
+                if (sp.R == 5) launch(s, k_wide_tdep<5>, grid, block, smem, td, st, td_set, sp, wp.ls);
+                else if (sp.R == 8) launch(s, k_wide_tdep<8>, grid, block, smem, td, st, td_set, sp, wp.ls);
+                else launch(s, k_wide_tdep<16>, grid, block, smem, td, st, td_set, sp, wp.ls);
+                td_have = group;
+            }
+            const long long o = (step - first) * td_set.stride;
+            for (int k = 0; k < W_COUNT; ++k) wp.S[k] = td_set.S + o + k * n;
+            wp.xbm = td_set.xb + o;
+            wp.xbp = wp.xbm + nx;
+            wp.sf = shifted(td_set.sf, o);
+            wp.sb = shifted(td_set.sb, o);
+            if (ap) {
+                ap->sz = shifted(td_set.sz, o);
+                ap->sw = shifted(td_set.sw, o);
+            }
         }
     }
 
+    // f(R, SER) with the rows per chunk of a split and the order of the recurrences as constants
+    template <bool S_LINES, typename F> void shaped(F &&f)
+    {
+        const int R = S_LINES ? wp.s.R : wp.v.R;
+        auto with = [&](auto ser) {
+            if (R == 8) f(std::integral_constant<int, 8>{}, ser);
+            else if (R == 16) f(std::integral_constant<int, 16>{}, ser);
+            else f(std::integral_constant<int, S_LINES ? 5 : 4>{}, ser);
+        };
+        if constexpr (std::is_same<T, double>::value) {
+            if (serial) return with(std::true_type{});
+        }
+        with(std::false_type{});
+    }
     template <int KIND, int SCH> void s_stage(cudaStream_t s, const T *u, const T *a, const T *d1, T *y)
     {
         const split &sp = wp.s;
-        const int grid = grid_for(ny - 1, sp.L);
-        const dim3 block(sp.L * sp.PC);
-        const size_t smem = 2 * sizeof(T) * carry_words(sp);
-        switch (sp.R) {
-        case 5: launch(s, k_wide_s<T, 5, KIND, SCH>, grid, block, smem, wp, u, a, d1, y); break;
-        case 8: launch(s, k_wide_s<T, 8, KIND, SCH>, grid, block, smem, wp, u, a, d1, y); break;
-        default: launch(s, k_wide_s<T, 16, KIND, SCH>, grid, block, smem, wp, u, a, d1, y); break;
-        }
+        shaped<true>([&](auto r, auto ser) {
+            launch(s, k_wide_s<T, decltype(r)::value, KIND, SCH, decltype(ser)::value>, grid_for(ny - 1, sp.L), dim3(sp.L * sp.PC),
+                   2 * sizeof(T) * carry_words(sp), wp, u, a, d1, y);
+        });
     }
     template <int KIND> void v_stage(cudaStream_t s, const T *u, const T *d, const T *e, const T *d2, T *out)
     {
         const split &sp = wp.v;
-        const int grid = grid_for(nx - 2, sp.L);
-        const dim3 block(sp.L * sp.PC);
-        const size_t smem = 2 * sizeof(T) * carry_words(sp);
-        switch (sp.R) {
-        case 4: launch(s, k_wide_v<T, 4, KIND>, grid, block, smem, wp, u, d, e, d2, out); break;
-        case 8: launch(s, k_wide_v<T, 8, KIND>, grid, block, smem, wp, u, d, e, d2, out); break;
-        default: launch(s, k_wide_v<T, 16, KIND>, grid, block, smem, wp, u, d, e, d2, out); break;
-        }
+        shaped<false>([&](auto r, auto ser) {
+            launch(s, k_wide_v<T, decltype(r)::value, KIND, decltype(ser)::value>, grid_for(nx - 2, sp.L), dim3(sp.L * sp.PC),
+                   2 * sizeof(T) * carry_words(sp), wp, u, d, e, d2, out);
+        });
     }
     // one time step u -> next, stage increments in d1, d2, d3
     void step(cudaStream_t s, const T *u, T *d1, T *d2, T *d3, T *next)
@@ -339,16 +409,14 @@ template <typename T> struct line_solver {
     // the same at time step m (time-dependent tables rebuilt first)
     void forward_step(cudaStream_t s, int m, const T *u, T *d1, T *d2, T *d3, T *next)
     {
-        if (tdep) {
-            refresh(s, m);
-            products(s, true);
-        }
+        if (tdep) refresh(s, m);
         step(s, u, d1, d2, d3, next);
     }
 
     int enqueue(cudaStream_t s)
     {
         launches = 0;
+        td_have = -1;
         const long long flat = static_cast<long long>(nx) * ny;
         k_wide_begin<T><<<grid_for(flat, 256), 256, 0, s>>>(pay.p, U, nx, ny, ld, status.p);
         const T *u = U;
@@ -394,7 +462,7 @@ template <typename T> struct line_front : wide_solver_base {
         instance_tables<T> tt;
         build_tables_for<T>(p, tt);
         int rc = w.init(p, tt);
-        if (!rc && (p.options & LSS_ADI_OPT_LINE_PER_THREAD)) rc = w.set_chunks(1, 1);
+        if (p.options & LSS_ADI_OPT_LINE_PER_THREAD) w.serial = 1;
         x = std::move(tt.x);
         y = std::move(tt.y);
         pay0 = std::move(tt.payoff);
@@ -430,6 +498,7 @@ template <typename T> struct line_front : wide_solver_base {
         auto ok = [](int P, int e) { return P <= MAX_CHUNKS && (P <= 1 || e >= 4 * P); };
         if (!ok(s_chunks, w.nx - 2) || !ok(v_chunks, w.ny - 2)) return set_error(LSS_ADI_EINVAL, "wide: chunk count out of range");
         LSS_CUDA_TRY(cudaStreamSynchronize(static_cast<cudaStream_t>(stream)), "lss_adi_line_chunks");
+        w.serial = 0; // chunk counts ask for partitioned solves
         int rc = w.set_chunks(s_chunks, v_chunks);
         if (rc) return rc;
         LSS_CUDA_TRY(cudaDeviceSynchronize(), "lss_adi_line_chunks");
@@ -452,12 +521,12 @@ struct line_adjoint : wide_adjoint_base {
     dbuf<double> ws, factors, carry_adj, grads;
     adj_params ap{};
     long long held = 0, nacc = 0;
-    bool line_per_thread = false;
 
     int init(const lss_adi_problem &p)
     {
         instance_tables<double> tt;
         build_tables<double>(p, tt);
+        w.td_adjoint = true;
         int rc = w.init(p, tt);
         if (rc) return rc;
         LSS_CUDA_TRY(cudaMemcpy(w.pay.p, tt.payoff.data(), tt.payoff.size() * sizeof(double), cudaMemcpyHostToDevice),
@@ -489,13 +558,20 @@ struct line_adjoint : wide_adjoint_base {
         ap.sabr = p.model == LSS_ADI_SABR;
         tau0 = p.forward ? p.maturity - ap.k : ap.k;
         dtau = p.forward ? -ap.k : ap.k;
-        line_per_thread = (p.options & LSS_ADI_OPT_LINE_PER_THREAD) != 0;
-        return set_chunks(line_per_thread ? 1 : 0, line_per_thread ? 1 : 0);
+        // Up to 256 x 160 points the recurrences run in relay order: the value has the bits of the same
+        // instance in a batch.  (One warp group of the batched kernel took 119 ms for a 128 x 64 x 200
+        // Craig-Sneyd call with sensitivities.)  Larger ones, and those of LSS_ADI_OPT_WIDE_ADJOINT, are
+        // partitioned; LINE_PER_THREAD asks for relay order at any size.
+        const bool small = p.nx <= 256 && static_cast<long long>(p.nx) * p.ny <= 40960 && !time_dependent(p);
+        w.serial = (p.options & LSS_ADI_OPT_LINE_PER_THREAD) || (small && !(p.options & LSS_ADI_OPT_WIDE_ADJOINT));
+        return set_chunks(0, 0, nullptr);
     }
     double tau0 = 0.0, dtau = 0.0;
 
-    int set_chunks(int ps, int pv) override
+    int set_chunks(int ps, int pv, void *stream) override
     {
+        LSS_CUDA_TRY(cudaStreamSynchronize(static_cast<cudaStream_t>(stream)), "lss_adi_adjoint: chunk counts");
+        if (w.serial) ps = pv = 0; // (relay order: the same result for every count)
         int rc = w.set_chunks(ps, pv);
         if (rc) return rc;
         const long long need = w.carry_need();
@@ -507,6 +583,7 @@ struct line_adjoint : wide_adjoint_base {
         w.product(nullptr, false, w.wp.V[W_VU], 1, w.ny - 1, -1, true, ap.vz);
         w.product(nullptr, false, w.wp.V[W_VL], 0, w.ny - 2, 1, false, ap.vw);
         LSS_CUDA_TRY(cudaGetLastError(), "wide adjoint: chunk products");
+        LSS_CUDA_TRY(cudaDeviceSynchronize(), "wide adjoint: chunk products");
         return LSS_ADI_OK;
     }
     void s_products(cudaStream_t s)
@@ -518,14 +595,10 @@ struct line_adjoint : wide_adjoint_base {
     template <int KIND> void adj_v(cudaStream_t s, const double *XB, double *VB, double *DB, double *LV, int add)
     {
         const split &sp = w.wp.v;
-        const int grid = grid_for(w.nx - 2, sp.L);
-        const dim3 block(sp.L * sp.PC);
-        const size_t smem = 2 * sizeof(double) * carry_words(sp);
-        switch (sp.R) {
-        case 4: w.launch(s, k_wadj_v<4, KIND>, grid, block, smem, w.wp, ap, XB, VB, DB, LV, add); break;
-        case 8: w.launch(s, k_wadj_v<8, KIND>, grid, block, smem, w.wp, ap, XB, VB, DB, LV, add); break;
-        default: w.launch(s, k_wadj_v<16, KIND>, grid, block, smem, w.wp, ap, XB, VB, DB, LV, add); break;
-        }
+        w.shaped<false>([&](auto r, auto ser) {
+            w.launch(s, k_wadj_v<decltype(r)::value, KIND, decltype(ser)::value>, grid_for(w.nx - 2, sp.L), dim3(sp.L * sp.PC),
+                     2 * sizeof(double) * carry_words(sp), w.wp, ap, XB, VB, DB, LV, add);
+        });
     }
     struct arrays {
         double *VB, *DB, *FB, *MU, *DV, *D2B, *LV, *LS, *HS, *ACC;
@@ -535,14 +608,11 @@ struct line_adjoint : wide_adjoint_base {
                const double *XB, double tau, double da, double dc)
     {
         const split &sp = w.wp.s;
-        const int grid = grid_for(w.ny - 1, sp.L);
-        const dim3 block(sp.L * sp.PC);
-        const size_t smem = 2 * sizeof(double) * carry_words(sp);
-        switch (sp.R) {
-        case 5: w.launch(s, k_wadj_s<5, KIND, SCH>, grid, block, smem, w.wp, ap, U, Vn, D1, D2, Y, XB, a.DV, a.VB, a.FB, a.MU, a.LS, a.HS, a.ACC, nacc, tau, da, dc); break;
-        case 8: w.launch(s, k_wadj_s<8, KIND, SCH>, grid, block, smem, w.wp, ap, U, Vn, D1, D2, Y, XB, a.DV, a.VB, a.FB, a.MU, a.LS, a.HS, a.ACC, nacc, tau, da, dc); break;
-        default: w.launch(s, k_wadj_s<16, KIND, SCH>, grid, block, smem, w.wp, ap, U, Vn, D1, D2, Y, XB, a.DV, a.VB, a.FB, a.MU, a.LS, a.HS, a.ACC, nacc, tau, da, dc); break;
-        }
+        w.shaped<true>([&](auto r, auto ser) {
+            w.launch(s, k_wadj_s<decltype(r)::value, KIND, SCH, decltype(ser)::value>, grid_for(w.ny - 1, sp.L), dim3(sp.L * sp.PC),
+                     2 * sizeof(double) * carry_words(sp), w.wp, ap, U, Vn, D1, D2, Y, XB, a.DV, a.VB, a.FB, a.MU, a.LS, a.HS, a.ACC,
+                     nacc, tau, da, dc);
+        });
     }
     template <int KIND, int SCH> void gather(cudaStream_t s, const arrays &a, const double *U, double tau, double da)
     {
@@ -555,8 +625,7 @@ struct line_adjoint : wide_adjoint_base {
     {
         double da = 1.0, dc = 1.0;
         if (w.tdep) {
-            w.refresh(s, m);
-            s_products(s);
+            w.refresh(s, m, &ap);
             da = w.td_da[m];
             dc = w.td_dc[m];
         }
@@ -623,6 +692,7 @@ struct line_adjoint : wide_adjoint_base {
         auto slot = [&](int m, int k) { return SEG + (4LL * m + k) * n; };
         const long long flat = static_cast<long long>(w.nx) * w.ny;
         w.launches = 0;
+        w.td_have = -1;
         k_wide_begin<double><<<grid_for(flat, 256), 256, 0, s>>>(w.pay.p, CK, w.nx, w.ny, w.ld, w.status.p);
         const double *cur = CK;
         const int n0_last = (nseg - 1) * c;

@@ -120,6 +120,22 @@ template <typename T> __device__ __forceinline__ carry<T> make_carry(T *raw, con
     k.lane = lane; k.c = c;
     return k;
 }
+// The recurrence over the chunks one after the other, each from the value that the one before ended
+// with (run(y): this thread's rows from the incoming y, returning the last): the operations of a
+// thread that solves the whole line, so the same bits, while right-hand sides and everything
+// that does not hang on the recurrence stay spread over the chunks' threads.
+template <typename T, bool FWD, typename F> __device__ __forceinline__ void relay(const carry<T> &k, T &in, F run)
+{
+    for (int q = 0; q < k.PC; ++q) {
+        if (k.c == (FWD ? q : k.PC - 1 - q)) {
+            const T y = q == 0 ? in : k.gb[k.lane];
+            k.gb[k.lane] = run(y);
+        }
+        __syncthreads();
+    }
+    in = k.gb[k.lane]; // every thread: the value entering the next tile
+    __syncthreads();
+}
 // Products of this thread's chunk into shared memory; preg: of those before it in its group.
 template <typename T>
 __device__ __forceinline__ void carry_load(const carry<T> &k, const carry_tab<T> &t, int ls, int tile, int l, T &preg)
@@ -168,8 +184,9 @@ template <typename T, bool FWD> __device__ __forceinline__ T compose(const carry
 
 // ------------------------------------------------------------------------------------------
 // S stages.  KIND 1: D1 = S F(U) (A = U).  KIND 2: D3 or E (A = D2; D1: the first stage's increment).
+// SER: the recurrences in relay order (a thread-per-line solve's bits).
 // ------------------------------------------------------------------------------------------
-template <typename T, int R, int KIND, int SCH>
+template <typename T, int R, int KIND, int SCH, bool SER>
 __global__ void __launch_bounds__(MAX_CTA) k_wide_s(const __grid_constant__ wparams<T> p, const T *U, const T *A, const T *D1, T *Y)
 {
     extern __shared__ __align__(16) unsigned char raw[];
@@ -248,19 +265,23 @@ __global__ void __launch_bounds__(MAX_CTA) k_wide_s(const __grid_constant__ wpar
             f[r] = v;
             q[r] = p.S[W_LA][o];
             if constexpr (R <= 8) g[r] = p.S[W_G][o];
-            y = wfma(-q[r], y, v);
+            if constexpr (!SER) y = wfma(-q[r], y, v);
             a0c = a1c; a1c = a2c;
             a1m = a2m; a1p = a2p;
             q0 = q1; q1 = q2;
         }
         const bool more = tile + 1 < sp.tiles;
-        y = compose<T, true>(kf, y, preg, in);
+        auto sweep = [&](T z) -> T {
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-            y = wfma(-q[r], y, f[r]);
-            f[r] = y;
-            if (more && act && t0 + r <= e) Y[(long long)(t0 + r) * ld + j] = y;
-        }
+            for (int r = 0; r < R; ++r) {
+                z = wfma(-q[r], z, f[r]);
+                f[r] = z;
+                if (more && act && t0 + r <= e) Y[(long long)(t0 + r) * ld + j] = z;
+            }
+            return z;
+        };
+        if constexpr (SER) relay<T, true>(kf, in, sweep);
+        else sweep(compose<T, true>(kf, y, preg, in));
     }
     in = hi;
     for (int tile = sp.tiles - 1; tile >= 0; --tile) {
@@ -277,14 +298,18 @@ __global__ void __launch_bounds__(MAX_CTA) k_wide_s(const __grid_constant__ wpar
             const long long o = (long long)min(t, nx - 1) * ld + j;
             if (again) f[r] = t <= e ? Y[o] : hi;
             if (R > 8 || again) g[r] = p.S[W_G][o];
-            x = wfma(-g[r], x, f[r]);
+            if constexpr (!SER) x = wfma(-g[r], x, f[r]);
         }
-        x = compose<T, false>(kb, x, bpreg, in);
+        auto sweep = [&](T z) -> T {
 #pragma unroll
-        for (int r = R - 1; r >= 0; --r) {
-            x = wfma(-g[r], x, f[r]);
-            if (act && t0 + r <= e) Y[(long long)(t0 + r) * ld + j] = x;
-        }
+            for (int r = R - 1; r >= 0; --r) {
+                z = wfma(-g[r], z, f[r]);
+                if (act && t0 + r <= e) Y[(long long)(t0 + r) * ld + j] = z;
+            }
+            return z;
+        };
+        if constexpr (SER) relay<T, false>(kb, in, sweep);
+        else sweep(compose<T, false>(kb, x, bpreg, in));
     }
 }
 
@@ -294,9 +319,9 @@ template <typename T> __device__ __forceinline__ T boundary1(const wparams<T> &p
     const int N = p.nx - 1;
     const T *u = U + (long long)i * p.ld;
     if (i == 0) return p.yslo[0];
-    T r = p.xbc[i] * u[0] + p.xb1[i] * u[1] + p.xb2[i] * u[2];
+    const T r = wfma(p.xb2[i], u[2], wfma(p.xb1[i], u[1], p.xbc[i] * u[0]));
     if (i == N) return r + p.bnc;
-    return r + p.xbm[i] * u[-p.ld] + p.xbp[i] * u[p.ld];
+    return wfma(p.xbp[i], u[p.ld], wfma(p.xbm[i], u[-p.ld], r));
 }
 
 // ------------------------------------------------------------------------------------------
@@ -304,7 +329,7 @@ template <typename T> __device__ __forceinline__ T boundary1(const wparams<T> &p
 // Block 0 holds the last rows, so that the extrapolated row nx-1 (explicit_boundary.hpp:202-238)
 // follows in the same CTA.
 // ------------------------------------------------------------------------------------------
-template <typename T, int R, int KIND>
+template <typename T, int R, int KIND, bool SER>
 __global__ void __launch_bounds__(MAX_CTA) k_wide_v(const __grid_constant__ wparams<T> p, const T *U, const T *D, const T *E,
                                                     const T *D2, T *out)
 {
@@ -368,16 +393,20 @@ __global__ void __launch_bounds__(MAX_CTA) k_wide_v(const __grid_constant__ wpar
             if (t == 0) f[r] = KIND == V_LAST_HV ? T(0) : lo - u0;
             if (t == ny - 1) f[r] = KIND == V_LAST_HV ? T(0) : hi - un;
             if (t >= ny) f[r] = T(0);
-            y = wfma(-q[r], y, f[r]);
+            if constexpr (!SER) y = wfma(-q[r], y, f[r]);
         }
         const bool more = tile + 1 < sp.tiles;
-        y = compose<T, true>(kf, y, preg, in);
+        auto sweep = [&](T z) -> T {
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-            y = wfma(-q[r], y, f[r]);
-            f[r] = y;
-            if ((r & 3) == 3 && more && act && t0 + r < ld) st4(out + row + t0 + r - 3, f + r - 3);
-        }
+            for (int r = 0; r < R; ++r) {
+                z = wfma(-q[r], z, f[r]);
+                f[r] = z;
+                if ((r & 3) == 3 && more && act && t0 + r < ld) st4(out + row + t0 + r - 3, f + r - 3);
+            }
+            return z;
+        };
+        if constexpr (SER) relay<T, true>(kf, in, sweep);
+        else sweep(compose<T, true>(kf, y, preg, in));
     }
     in = T(0);
     for (int tile = sp.tiles - 1; tile >= 0; --tile) {
@@ -391,8 +420,10 @@ __global__ void __launch_bounds__(MAX_CTA) k_wide_v(const __grid_constant__ wpar
             for (int r = 0; r < R; r += 4) ld4(out + col(t0 + r), f + r);
         }
         T x = T(0);
+        if constexpr (!SER) {
 #pragma unroll
-        for (int r = R - 1; r >= 0; --r) x = wfma(-g[r], x, f[r]);
+            for (int r = R - 1; r >= 0; --r) x = wfma(-g[r], x, f[r]);
+        }
         // what the output needs is loaded before the composition waits
         T u[R];
         if constexpr (KIND != V_FIRST) {
@@ -407,7 +438,16 @@ __global__ void __launch_bounds__(MAX_CTA) k_wide_v(const __grid_constant__ wpar
                 }
             }
         }
-        x = compose<T, false>(kb, x, bpreg, in);
+        auto sweep = [&](T z) -> T {
+#pragma unroll
+            for (int r = R - 1; r >= 0; --r) {
+                z = wfma(-g[r], z, f[r]);
+                f[r] = z;
+            }
+            return z;
+        };
+        if constexpr (SER) relay<T, false>(kb, in, sweep);
+        else sweep(compose<T, false>(kb, x, bpreg, in));
 #pragma unroll
         for (int r = R - 4; r >= 0; r -= 4) {
             if (R > 8) ld4(p.V[W_VIB] + col(t0 + r), ib + r);
@@ -415,9 +455,8 @@ __global__ void __launch_bounds__(MAX_CTA) k_wide_v(const __grid_constant__ wpar
 #pragma unroll
             for (int z = 3; z >= 0; --z) {
                 const int t = t0 + r + z;
-                x = wfma(-g[r + z], x, f[r + z]);
-                if constexpr (KIND == V_FIRST) o[z] = ib[r + z] * x;
-                else o[z] = wfma(ib[r + z], x, u[r + z]);
+                if constexpr (KIND == V_FIRST) o[z] = ib[r + z] * f[r + z];
+                else o[z] = wfma(ib[r + z], f[r + z], u[r + z]);
                 if constexpr (KIND != V_FIRST) {
                     if (t == 0) o[z] = lo;
                     if (t == ny - 1) o[z] = hi;
@@ -440,7 +479,7 @@ __global__ void __launch_bounds__(MAX_CTA) k_wide_v(const __grid_constant__ wpar
             for (int t = w; t < ny; t += ws) {
                 out[t] = p.yslo[t];
                 const int tt = p.jmap[t];
-                out[lr + t] = four3 * __ldcg(out + lr - ld + tt) - third * __ldcg(out + lr - 2 * ld + tt) - p.yb2c[t];
+                out[lr + t] = wfma(four3, __ldcg(out + lr - ld + tt), wfma(-third, __ldcg(out + lr - 2 * ld + tt), -p.yb2c[t]));
             }
         }
     }
@@ -518,7 +557,7 @@ __global__ void k_wide_setup_s(const double *base, long long n, int nx, int ny, 
         if (t < e)
             for (int k = 0; k < 7; ++k) nv[k] = base[k * n + o + ld];
         const double a = -th * v[0], b = 1.0 + th * v[2], c = -th * v[1];
-        const double ib = 1.0 / (b - a * gam);
+        const double ib = 1.0 / fma(-a, gam, b);
         gam = c * ib;
         T *s = S + o;
         s[W_LA * n] = static_cast<T>(a * ib);
@@ -540,8 +579,7 @@ __global__ void k_wide_setup_v(const double *base, long long n, int nx, int ny, 
     for (int t = 1; t <= ny - 2; ++t) {
         const double a = -th * Mt[row + t], b = 1.0 + th * W[row + t], c = -th * Pt[row + t];
         const double l = t == 1 ? a : a * ib;
-        const double beta = t == 1 ? b : b - l * cp;
-        ib = 1.0 / beta;
+        ib = 1.0 / (t == 1 ? b : fma(-l, cp, b));
         L[t] = static_cast<T>(l);
         IB[t] = static_cast<T>(ib);
         if (t > 1) Uf[t - 1] = static_cast<T>(cp * ib);
@@ -564,79 +602,183 @@ struct tdep_tab {
     int nx, ny, ld;
     long long n;
 };
-// The S-line factorisation's recurrence, partitioned along the lines (CTA: L lines x P chunks).
-// beta_t = b_t - a_t c_{t-1} / beta_{t-1} is the Moebius map of the matrix [[b_t, -a_t c_{t-1}], [1, 0]]
-// applied to beta_{t-1}: each chunk forms the product of its rows' matrices (rescaled every 8 rows:
-// only the ratio matters), a chunk composes the maps of the chunks before it to get its incoming
-// beta, then runs its own rows' recurrence from it.
-static __global__ void __launch_bounds__(1024) k_wide_tdep_factor(tdep_tab q, double da, double *S)
+// One step's set of tables among those of a group: S-line tables, boundary weights, chunk products.
+struct tdep_set {
+    double *S, *xb;                // of the group's first step: W_COUNT n; XB_M and XB_P, nx each
+    carry_tab<double> sf, sb, sz, sw; // (sz, sw: the transposed solves', null A without them)
+    long long stride;              // doubles from one step's set to the next
+};
+constexpr int TDEP_STEPS = 16;
+struct tdep_steps {
+    double da[TDEP_STEPS], dc[TDEP_STEPS];
+};
+// 2^-e of the largest of four magnitudes (1 for zero): the exponent field's arithmetic, no FP64
+__device__ __forceinline__ double pow2_inverse(double a, double b, double c, double d)
 {
-    __shared__ double sm[4][1024];
-    const int L = blockDim.x, P = blockDim.y, lane = threadIdx.x, c = threadIdx.y;
-    const int j = 1 + blockIdx.x * L + lane;
+    const int top = 0x7fffffff;
+    const int m = max(max(__double2hiint(a) & top, __double2hiint(b) & top), max(__double2hiint(c) & top, __double2hiint(d) & top)) >> 20;
+    return m == 0 || m > 2044 ? 1.0 : __hiloint2double((2046 - m) << 20, 0);
+}
+// All S-line tables of a group of steps (blockIdx.y: the step) in the shape of the S stages' split: a
+// CTA factorises its lines, writes factors and right-hand-side slots and composes the chunks' products.
+// beta_t = b_t - a_t c_{t-1} / beta_{t-1} is the Moebius map of the matrix [[b_t, -a_t c_{t-1}], [1, 0]]
+// applied to beta_{t-1}: each chunk forms the product of its rows' matrices (scaled by powers of two:
+// only the ratio matters), the chunks' maps are composed like the solves' end maps, a chunk then runs
+// its own rows' recurrence from its incoming beta.
+// What bounds it: FP64 instructions (about 45 per point, one division among them) as long as the grid
+// fills the GPU, which the steps of a group are there for.  A launch per step of 32 CTAs, followed by
+// one for the slots and one for each sweep's products, took 115 to 240 us of a 512 x 256 step.
+template <int R>
+__global__ void __launch_bounds__(MAX_CTA) k_wide_tdep(const __grid_constant__ tdep_tab q, const __grid_constant__ tdep_steps steps,
+                                                       const __grid_constant__ tdep_set set, const __grid_constant__ split sp, int ls)
+{
+    extern __shared__ __align__(16) unsigned char raw[];
+    const int L = sp.L, PC = sp.PC, ng = sp.groups(), gs = sp.gs, lane = threadIdx.x % L, c = threadIdx.x / L;
+    const int j = 1 + blockIdx.x * L + lane, e = q.nx - 2, w = L * PC, at = c * L + lane;
     const bool act = j <= q.ny - 2;
-    const int e = q.nx - 2, k = c * L + lane;
-    const int t0 = 1 + static_cast<int>(static_cast<long long>(c) * e / P), t1 = static_cast<int>(static_cast<long long>(c + 1) * e / P);
-    const double th = q.th;
-    auto M = [&](long long o, int t) { return fma(da, q.ma[o], q.mb[t]); };
-    auto Pf = [&](long long o, int t) { return fma(da, q.pa[o], -q.mb[t]); };
+    double *sm = reinterpret_cast<double *>(raw), *gm = sm + 4 * w; // chunks' maps (later products), groups' maps
+    const double th = q.th, da = steps.da[blockIdx.y], dc = steps.dc[blockIdx.y];
+    const long long off = blockIdx.y * set.stride;
+    double *S = set.S + off;
     pdl_launch();
-    double cin = 0.0; // c of the row before the chunk
-    if (act) {
-        if (t0 > 1) cin = -th * Pf((long long)(t0 - 1) * q.ld + j, t0 - 1);
-        double m11 = 1.0, m12 = 0.0, m21 = 0.0, m22 = 1.0, cp = cin;
-        for (int t = t0; t <= t1; ++t) {
-            const long long o = (long long)t * q.ld + j;
-            const double m = M(o, t), pp = Pf(o, t);
-            const double b = fma(th, m + pp + q.z0, 1.0), ac = (-th * m) * cp;
-            cp = -th * pp;
-            const double n11 = b * m11 - ac * m21, n12 = b * m12 - ac * m22;
-            m21 = m11; m22 = m12; m11 = n11; m12 = n12;
-            if (((t - t0) & 7) == 7) {
-                const double sc = 1.0 / fmax(fabs(m11), fabs(m21));
-                m11 *= sc; m12 *= sc; m21 *= sc; m22 *= sc;
+    double in = 1.0; // beta of the row before the tile: row 1's map ignores it (a_1 c_0 = 0)
+    bool waited = false;
+    for (int tile = 0; tile < sp.tiles; ++tile) {
+        const int G = tile * PC + c, t0 = 1 + G * R;
+        double m[R], pp[R];
+        double cin = 0.0; // c of the row before the chunk
+        if (act) {
+            if (t0 > 1 && t0 <= e + 1) cin = -th * fma(da, q.pa[(long long)(t0 - 1) * q.ld + j], -q.mb[t0 - 1]);
+            double m11 = 1.0, m12 = 0.0, m21 = 0.0, m22 = 1.0, cp = cin;
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const int t = t0 + r;
+                m[r] = pp[r] = 0.0;
+                if (t > e) continue;
+                const long long o = (long long)t * q.ld + j;
+                m[r] = fma(da, q.ma[o], q.mb[t]);
+                pp[r] = fma(da, q.pa[o], -q.mb[t]);
+                const double b = fma(th, m[r] + pp[r] + q.z0, 1.0), ac = (-th * m[r]) * cp;
+                cp = -th * pp[r];
+                const double n11 = b * m11 - ac * m21, n12 = b * m12 - ac * m22;
+                m21 = m11; m22 = m12; m11 = n11; m12 = n12;
+                if ((r & 7) == 7 || r == R - 1 || t == e) {
+                    const double sc = pow2_inverse(m11, m12, m21, m22);
+                    m11 *= sc; m12 *= sc; m21 *= sc; m22 *= sc;
+                }
+            }
+            sm[at] = m11; sm[w + at] = m12; sm[2 * w + at] = m21; sm[3 * w + at] = m22;
+        }
+        __syncthreads();
+        if (act && c < ng) { // this thread's group: maps of the chunks before each one in the group
+            double m11 = 1.0, m12 = 0.0, m21 = 0.0, m22 = 1.0;
+            const int q1 = min((c + 1) * gs, PC);
+            for (int k = c * gs; k < q1; ++k) {
+                const int z = k * L + lane;
+                const double a11 = sm[z], a12 = sm[w + z], a21 = sm[2 * w + z], a22 = sm[3 * w + z];
+                sm[z] = m11; sm[w + z] = m12; sm[2 * w + z] = m21; sm[3 * w + z] = m22;
+                const double n11 = a11 * m11 + a12 * m21, n12 = a11 * m12 + a12 * m22;
+                const double n21 = a21 * m11 + a22 * m21, n22 = a21 * m12 + a22 * m22;
+                const double sc = pow2_inverse(n11, n12, n21, n22);
+                m11 = n11 * sc; m12 = n12 * sc; m21 = n21 * sc; m22 = n22 * sc;
+            }
+            const int z = 4 * (c * L + lane);
+            gm[z] = m11; gm[z + 1] = m12; gm[z + 2] = m21; gm[z + 3] = m22;
+        }
+        __syncthreads();
+        if (act && c == 0) { // beta as a ratio x / y through the groups
+            double x = in, y = 1.0;
+            for (int k = 0; k < ng; ++k) {
+                double *g = gm + 4 * (k * L + lane);
+                const double a11 = g[0], a12 = g[1], a21 = g[2], a22 = g[3];
+                g[0] = x; g[1] = y;
+                const double nx = a11 * x + a12 * y, ny = a21 * x + a22 * y;
+                const double sc = pow2_inverse(nx, ny, 0.0, 0.0);
+                x = nx * sc; y = ny * sc;
+            }
+            in = x / y;
+        }
+        __syncthreads();
+        double prl = 1.0, prb = 1.0, prz = 1.0; // products of this chunk's slopes (prl: la without its first row's)
+        double la1 = 0.0;                       // la of the chunk's first row
+        double gam = 0.0, la_next = 0.0;
+        if (act) {
+            const double x = gm[4 * (c / gs * L + lane)], y = gm[4 * (c / gs * L + lane) + 1];
+            // incoming beta; gamma of the row before the chunk
+            const double bx = sm[at] * x + sm[w + at] * y, by = sm[2 * w + at] * x + sm[3 * w + at] * y;
+            gam = cin != 0.0 ? cin * by / bx : 0.0;
+        }
+        if (!waited) pdl_wait(); // the stages that read the sets before are done
+        waited = true;
+        if (act) {
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const int t = t0 + r;
+                prz *= t <= e ? -gam : 0.0;
+                if (t > e) {
+                    prl = prb = 0.0;
+                    continue;
+                }
+                const long long o = (long long)t * q.ld + j;
+                const double z = m[r] + pp[r] + q.z0;
+                const double ib = 1.0 / fma(th * m[r], gam, fma(th, z, 1.0));
+                const double la = (-th * m[r]) * ib;
+                gam = (-th * pp[r]) * ib;
+                S[W_IB * q.n + o] = ib;
+                S[W_G * q.n + o] = gam;
+                S[W_LA * q.n + o] = la;
+                s_slots(S + o, q.n, m[r], pp[r], z, q.mt[o], q.pt[o], q.w[o], dc * q.cs[o], q.gm, ib);
+                if (r == 0) la1 = la;
+                else prl *= -la;
+                prb *= -gam;
+            }
+            // la of the row after the tile (the tile's last chunk): pivot from its own row
+            if (c == PC - 1 && t0 + R <= e) {
+                const long long o = (long long)(t0 + R) * q.ld + j;
+                const double mm = fma(da, q.ma[o], q.mb[t0 + R]), p1 = fma(da, q.pa[o], -q.mb[t0 + R]);
+                la_next = (-th * mm) / fma(th * mm, gam, fma(th, mm + p1 + q.z0, 1.0));
             }
         }
-        sm[0][k] = m11; sm[1][k] = m12; sm[2][k] = m21; sm[3][k] = m22;
+        __syncthreads(); // every thread has its incoming beta: the maps' arrays become the products'
+        if (act) {
+            sm[at] = -la1 * prl;
+            sm[w + at] = prb;
+            sm[2 * w + at] = prz;
+            gm[at] = la1;
+        }
+        __syncthreads();
+        if (act && set.sw.A) { // slopes of the transposed back sweep: la of the row after
+            sm[3 * w + at] = -(c < PC - 1 ? gm[at + L] : la_next) * prl;
+        }
+        __syncthreads();
+        // products of the chunks before each in its group, of the groups; sweep u / ng, group u % ng
+        const int sweeps = set.sw.A ? 4 : 2;
+        for (int u = c; act && u < sweeps * ng; u += PC) {
+            const int sw = u / ng, g = u % ng;
+            const carry_tab<double> &t = sw == 0 ? set.sf : sw == 1 ? set.sb : sw == 2 ? set.sz : set.sw;
+            const bool fwd = (sw & 1) == 0;
+            double pr = 1.0;
+            for (int k = g * gs; k < min((g + 1) * gs, PC); ++k) {
+                const int ch = fwd ? k : PC - 1 - k;
+                const long long o = (long long)(tile * PC + ch) * ls + j + off;
+                const double a = sm[sw * w + ch * L + lane];
+                const_cast<double *>(t.A)[o] = a;
+                const_cast<double *>(t.PreG)[o] = pr;
+                pr *= a;
+            }
+            const_cast<double *>(t.GA)[(long long)(tile * ng + g) * ls + j + off] = pr;
+        }
+        __syncthreads();
     }
-    __syncthreads();
-    pdl_wait(); // the stages that read the tables of the step before are done
-    if (!act) return;
-    // incoming beta of the chunk: chunk 0 starts at row 1, whose map ignores its argument (a_1 c_0 = 0)
-    double x = 1.0;
-    for (int r = 0; r < c; ++r) {
-        const int kr = r * L + lane;
-        x = (sm[0][kr] * x + sm[1][kr]) / (sm[2][kr] * x + sm[3][kr]);
+    // the boundary column's weights
+    if (blockIdx.x == 0) {
+        double *xb = set.xb + off;
+        for (int i = threadIdx.x; i < q.nx; i += blockDim.x) {
+            const double d = fma(da, q.am[i], q.bm[i]);
+            xb[i] = -d;
+            xb[q.nx + i] = d;
+        }
     }
-    double gam = t0 > 1 ? cin / x : 0.0;
-    for (int t = t0; t <= t1; ++t) {
-        const long long o = (long long)t * q.ld + j;
-        const double m = M(o, t), pp = Pf(o, t);
-        const double b = fma(th, m + pp + q.z0, 1.0);
-        const double ib = 1.0 / (b - (-th * m) * gam);
-        gam = (-th * pp) * ib;
-        S[W_IB * q.n + o] = ib;
-        S[W_G * q.n + o] = gam;
-        S[W_LA * q.n + o] = -th * m * ib;
-    }
-}
-// The right-hand-side slots of every point, and the boundary column's weights.
-static __global__ void k_wide_tdep_slots(tdep_tab q, double da, double dc, double *S, double *xbm, double *xbp)
-{
-    const long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    const int e = q.nx - 2, m = q.ny - 2;
-    pdl_launch();
-    pdl_wait();
-    if (k < q.nx) {
-        const double d = fma(da, q.am[k], q.bm[k]);
-        xbm[k] = -d;
-        xbp[k] = d;
-    }
-    if (k >= (long long)e * m) return;
-    const int t = 1 + static_cast<int>(k / m), j = 1 + static_cast<int>(k % m);
-    const long long o = (long long)t * q.ld + j;
-    const double M = fma(da, q.ma[o], q.mb[t]), P = fma(da, q.pa[o], -q.mb[t]);
-    s_slots(S + o, q.n, M, P, M + P + q.z0, q.mt[o], q.pt[o], q.w[o], dc * q.cs[o], q.gm, S[W_IB * q.n + o]);
 }
 
 // initial condition into the pitched state; final surface out of it, with its value and finiteness
@@ -663,8 +805,8 @@ __global__ void k_wide_end(const T *U, int nx, int ny, int ld, bilinear b, T *su
     if (bad && threadIdx.x == 0) atomicOr(status, 1);
     if (q == 0) {
         const long long o = (long long)b.i0 * ld + b.j0;
-        *value = b.w00 * static_cast<double>(U[o]) + b.w10 * static_cast<double>(U[o + ld]) + b.w01 * static_cast<double>(U[o + 1]) +
-                 b.w11 * static_cast<double>(U[o + ld + 1]);
+        *value = fma(b.w11, static_cast<double>(U[o + ld + 1]),
+                     fma(b.w01, static_cast<double>(U[o + 1]), fma(b.w10, static_cast<double>(U[o + ld]), b.w00 * static_cast<double>(U[o]))));
     }
 }
 
@@ -687,7 +829,7 @@ struct adj_params {
     carry_tab<double> sz, sw, vz, vw;
 };
 
-template <int R, int KIND>
+template <int R, int KIND, bool SER>
 __global__ void __launch_bounds__(MAX_CTA) k_wadj_v(const __grid_constant__ wparams<double> p, const __grid_constant__ adj_params q,
                                                     const double *XB, double *VB, double *DB, double *LV, int add_lv)
 {
@@ -745,16 +887,20 @@ __global__ void __launch_bounds__(MAX_CTA) k_wadj_v(const __grid_constant__ wpar
         for (int r = 0; r < R; ++r) {
             f[r] = t0 + r < ny ? ib[r] * f[r] : 0.0;
             if (t0 + r >= ny) g[r] = 0.0;
-            z = fma(-g[r], z, f[r]);
+            if constexpr (!SER) z = fma(-g[r], z, f[r]);
         }
-        z = compose<double, true>(kf, z, preg, in);
         const bool more = tile + 1 < sp.tiles;
+        auto sweep = [&](double y) -> double {
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-            z = fma(-g[r], z, f[r]);
-            f[r] = z;
-            if ((r & 3) == 3 && more && act && t0 + r < ld) st4(DB + row + t0 + r - 3, f + r - 3);
-        }
+            for (int r = 0; r < R; ++r) {
+                y = fma(-g[r], y, f[r]);
+                f[r] = y;
+                if ((r & 3) == 3 && more && act && t0 + r < ld) st4(DB + row + t0 + r - 3, f + r - 3);
+            }
+            return y;
+        };
+        if constexpr (SER) relay<double, true>(kf, in, sweep);
+        else sweep(compose<double, true>(kf, z, preg, in));
     }
     in = 0.0;
     for (int tile = sp.tiles - 1; tile >= 0; --tile) {
@@ -778,14 +924,24 @@ __global__ void __launch_bounds__(MAX_CTA) k_wadj_v(const __grid_constant__ wpar
             }
         }
         double w = 0.0;
+        if constexpr (!SER) {
 #pragma unroll
-        for (int r = R - 1; r >= 0; --r) w = fma(-g[r], w, f[r]);
-        w = compose<double, false>(kb, w, bpreg, in);
+            for (int r = R - 1; r >= 0; --r) w = fma(-g[r], w, f[r]);
+        }
+        auto sweep = [&](double y) -> double {
+#pragma unroll
+            for (int r = R - 1; r >= 0; --r) {
+                y = fma(-g[r], y, f[r]);
+                f[r] = y;
+            }
+            return y;
+        };
+        if constexpr (SER) relay<double, false>(kb, in, sweep);
+        else sweep(compose<double, false>(kb, w, bpreg, in));
 #pragma unroll
         for (int r = R - 1; r >= 0; --r) {
             const int t = t0 + r;
-            w = fma(-g[r], w, f[r]);
-            f[r] = w;
+            w = f[r];
             if constexpr (KIND != V_LAST_HV) {
                 if (act && t == ny - 1) VB[row + t] -= w;
                 if (act && t == 0) {
@@ -804,10 +960,10 @@ __global__ void __launch_bounds__(MAX_CTA) k_wadj_v(const __grid_constant__ wpar
 
 // Parameter sums of one thread (rows of one line) of an S kernel, before the line's v factors.
 struct s_acc {
-    double A, Y, E, B, C, Q, S, Aa, Ya, Dd, Yd, v0, vm, vp;
+    double A, Y, E, B, C, Q, S, Aa, Ya, Dd, Yd, v0, vm, vd;
 };
 
-template <int R, int KIND, int SCH>
+template <int R, int KIND, int SCH, bool SER>
 __global__ void __launch_bounds__(MAX_CTA) k_wadj_s(const __grid_constant__ wparams<double> p, const __grid_constant__ adj_params q,
                                                 const double *U, const double *Vn, const double *D1, const double *D2, const double *Y,
                                                 const double *XB, const double *DV, double *VB, double *FB, double *MU, double *LS,
@@ -847,14 +1003,22 @@ __global__ void __launch_bounds__(MAX_CTA) k_wadj_s(const __grid_constant__ wpar
             if constexpr (KIND == 1 && !dr) x += DV[o];
             f[r] = t0 + r <= e ? x : 0.0;
             g[r] = t0 + r <= e ? p.S[W_G][o - ld] : 0.0; // row 0 of the table is zero
-            z = fma(-g[r], z, f[r]);
+            if constexpr (!SER) z = fma(-g[r], z, f[r]);
         }
-        z = compose<double, true>(kf, z, preg, in);
         const bool more = tile + 1 < sp.tiles;
+        auto sweep = [&](double y) -> double {
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                y = fma(-g[r], y, f[r]);
+                f[r] = y;
+            }
+            return y;
+        };
+        if constexpr (SER) relay<double, true>(kf, in, sweep);
+        else sweep(compose<double, true>(kf, z, preg, in));
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-            z = fma(-g[r], z, f[r]);
-            f[r] = z;
+            z = f[r];
             if (more && act && t0 + r <= e) FB[at(t0 + r)] = z;
             if (act && t0 + r == e) { // adjoint of the upper value
                 const double h = -p.S[W_G][at(e)] * z;
@@ -877,9 +1041,18 @@ __global__ void __launch_bounds__(MAX_CTA) k_wadj_s(const __grid_constant__ wpar
         for (int r = R - 1; r >= 0; --r) {
             if (again) f[r] = t0 + r <= e ? FB[at(t0 + r)] : 0.0;
             g[r] = t0 + r < e ? p.S[W_LA][at(t0 + r + 1)] : 0.0;
-            w = fma(-g[r], w, f[r]);
+            if constexpr (!SER) w = fma(-g[r], w, f[r]);
         }
-        w = compose<double, false>(kb, w, bpreg, in);
+        auto sweep = [&](double y) -> double {
+#pragma unroll
+            for (int r = R - 1; r >= 0; --r) {
+                y = fma(-g[r], y, f[r]);
+                f[r] = y;
+            }
+            return y;
+        };
+        if constexpr (SER) relay<double, false>(kb, in, sweep);
+        else sweep(compose<double, false>(kb, w, bpreg, in));
         // X: the operand of the explicit terms (U, or D2), Y: the stage's result; rows t+1, t, t-1
         const double *X = KIND == 1 ? U : D2;
         double xh = X[at(t0 + R)], xc = X[at(t0 + R - 1)], yh = Y[at(t0 + R)], yc = Y[at(t0 + R - 1)];
@@ -890,7 +1063,7 @@ __global__ void __launch_bounds__(MAX_CTA) k_wadj_s(const __grid_constant__ wpar
         for (int r = R - 1; r >= 0; --r) {
             const int t = t0 + r;
             const long long o = at(t), ol = at(t - 1);
-            w = fma(-g[r], w, f[r]);
+            w = f[r];
             const double xl = X[ol], yl = Y[ol], sl = X[ol - 1], ddl = sl - X[ol + 1];
             if (t <= e) {
                 const double mu = p.S[W_IB][o] * w;
@@ -914,7 +1087,7 @@ __global__ void __launch_bounds__(MAX_CTA) k_wadj_s(const __grid_constant__ wpar
                     s.A = fma(mx, dx, s.A);
                     s.C = fma(mu, xc, s.C);
                     s.Q = fma(mu, ddc, s.Q);
-                    s.S = fma(mu, ss, s.S);
+                    s.S = fma(mu, ss - xc, s.S);
                 }
                 if (q.sabr) {
                     const double ma = mu * q.ha[t], md = mu * q.hdd[t];
@@ -936,9 +1109,9 @@ __global__ void __launch_bounds__(MAX_CTA) k_wadj_s(const __grid_constant__ wpar
                     x0 = Vn[o - 1] - U[o - 1]; x1 = Vn[o] - U[o]; x2 = Vn[o + 1] - U[o + 1];
                     if constexpr (hv) { x0 -= D2[o - 1]; x1 -= D2[o]; x2 -= D2[o + 1]; }
                 }
-                s.vm = fma(m, x0, s.vm);
+                s.vd = fma(m, x2 - x0, s.vd);
                 s.v0 = fma(m, x1, s.v0);
-                s.vp = fma(m, x2, s.vp);
+                s.vm = fma(m, x0 - x1, s.vm);
             }
             xh = xc; xc = xl;
             yh = yc; yc = yl;
@@ -951,14 +1124,14 @@ __global__ void __launch_bounds__(MAX_CTA) k_wadj_s(const __grid_constant__ wpar
     const double th = q.theta, wx = KIND == 1 ? 1.0 : q.dw, we = KIND == 1 ? 1.0 : q.zeta;
     const double A = th * s.Y + wx * s.A;
     const double B = -(th * s.B + 2.0 * wx * s.C);
-    const double Q = -wx * s.Q, D = wx * (2.0 * s.S - s.Q - 2.0 * s.C), E = we * q.gamma * dc * s.E;
+    const double Q = -wx * s.Q, D = wx * (2.0 * s.S - s.Q), E = we * q.gamma * dc * s.E;
     const double ek = q.ek[j], et = q.et[j], es = q.es[j], bs = q.bs[j], hy = q.hy[j];
     double g0 = q.delta * A + q.halfk * B;
     if (q.sabr) {
         const double Aa = da * (th * s.Ya + wx * s.Aa), Dd = da * (th * s.Yd + wx * s.Dd);
         g0 += tau * q.omb * (q.hv2[j] * (2.0 * q.delta * Dd - 2.0 * q.alphat * Aa) - q.rho * q.sigma * hy * E);
     }
-    const double vq = th * q.ni * (s.vp - s.vm), vs = th * q.betat * (s.vm + s.vp - 2.0 * s.v0);
+    const double vq = th * q.ni * s.vd, vs = th * q.betat * (2.0 * s.vm + s.vd);
     g0 -= q.halfk * th * s.v0;
     const double g1 = ek * (q.ni * Q + vq), g2 = et * (q.ni * Q + vq);
     const double g3 = es * (q.ni * Q + vq) + bs * (q.betat * D + vs) + q.rho * hy * E, g4 = q.sigma * hy * E;
@@ -987,42 +1160,55 @@ __global__ void __launch_bounds__(256) k_wadj_gather(const __grid_constant__ wpa
     if (id >= n) return;
     const int r = static_cast<int>(id / ny), q = static_cast<int>(id % ny);
     const long long o = (long long)r * ld + q;
-    // FB and the tables are zero on boundary rows and columns: only points outside need a guard
-    const bool up = r + 1 < nx, dn = r > 0, rt = q + 1 < ny, lf = q > 0;
-    auto prod = [&](int slot, bool ok, long long at) { return ok ? p.S[slot][at] * FB[at] : 0.0; };
-    double m = prod(W_WG, up && rt, o + ld + 1) - prod(W_WG, up && lf, o + ld - 1);
-    m -= prod(W_WG, dn && rt, o - ld + 1) - prod(W_WG, dn && lf, o - ld - 1);
-    double x = 0.0;
-    if constexpr (KIND == 1 || hv || mcs) {
-        const double east = prod(W_WE, dn, o - ld);
-        x = prod(W_WW, up, o + ld) + (KIND == 2 && mcs ? -east : east) + prod(W_WC, true, o) + prod(W_WS, rt, o + 1) + prod(W_WN, lf, o - 1);
+    // Row t contributes down (to t-1), up (to t+1) and mid (to t) terms from FB and the tables at
+    // columns q-1, q, q+1 (the operations of da_gather, in its order); FB and the tables are zero on
+    // boundary rows and columns, only points outside need a guard.
+    constexpr bool six = KIND == 1 || hv || mcs;
+    const bool lf = q >= 1, rt = q + 1 < ny;
+    auto F = [&](long long at, bool ok) { return ok ? FB[at] : 0.0; };
+    auto W = [&](int slot, long long at, bool ok) { return ok ? p.S[slot][at] : 0.0; };
+    auto mixed = [&](long long t) { return fma(W(W_WG, t + 1, rt), F(t + 1, rt), -W(W_WG, t - 1, lf) * F(t - 1, lf)); };
+    double dn = 0.0, up = 0.0, mid = 0.0;
+    if (r + 1 < nx) {
+        const long long t = o + ld;
+        const double g = mixed(t);
+        dn = !six ? g : KIND == 2 && mcs ? fma(p.zeta, g, p.zt * (p.S[W_WW][t] * FB[t])) : fma(p.S[W_WW][t], FB[t], g);
+    }
+    if (r > 0) {
+        const long long t = o - ld;
+        const double g = mixed(t);
+        up = !six ? -g : KIND == 2 && mcs ? -fma(p.zeta, g, p.zt * (p.S[W_WE][t] * FB[t])) : fma(p.S[W_WE][t], FB[t], -g);
+    }
+    double x = dn + up;
+    if constexpr (six) {
+        mid = fma(W(W_WS, o + 1, rt), F(o + 1, rt), fma(W(W_WN, o - 1, lf), F(o - 1, lf), p.S[W_WC][o] * FB[o]));
+        x += KIND == 2 && mcs ? p.zt * mid : mid;
     }
     if constexpr (KIND == 2) {
-        double d = mcs ? fma(p.zeta, m, p.zt * x) : hv ? p.zeta * (m + x) - prod(W_IB, true, o) : p.zeta * m;
+        const double d = hv ? fma(p.zeta, x, -(p.S[W_IB][o] * FB[o])) : mcs ? x : p.zeta * x;
         if (r == 0 || r == nx - 1) VB[o] -= d;
-        else D2B[o] = hv ? d + VB[o] : d;
+        else D2B[o] = hv ? VB[o] + d : d;
     } else {
-        double v = m + x;
         if (r == 0 || r == nx - 1) {
             const double *E = r == 0 ? LS : HS;
-            if (q >= 1 && q <= ny - 2) v += (p.jmap[q] == q ? E[q] : 0.0) - E[q];
-            if (q + 1 <= ny - 2 && p.jmap[q + 1] == q) v += E[q + 1];
+            double s = q >= 1 && q <= ny - 2 && p.jmap[q] != q ? -E[q] : 0.0;
+            if (q + 1 <= ny - 2 && p.jmap[q + 1] == q) s += E[q + 1];
+            x += s;
         }
+        double v = VB[o] + x;
         if (q <= 2) {
             auto B0 = [&](int i) -> double { // adjoint of the boundary value of row i
-                if (i < 0 || i > nx - 1) return 0.0;
-                double sum = 0.0;
-                if (i >= 1 && i <= nx - 2 && p.imap[i] == i) sum += LV[i];
-                if (i + 1 >= 1 && i + 1 <= nx - 2 && p.imap[i + 1] == i) sum += LV[i + 1];
-                return i >= 1 && i <= nx - 2 ? sum : 0.0; // the values of rows 0 and nx-1 are the S boundaries'
+                if (i < 1 || i > nx - 2) return 0.0;
+                double sum = p.imap[i] == i ? LV[i] : 0.0;
+                if (i + 1 <= nx - 2 && p.imap[i + 1] == i) sum += LV[i + 1];
+                return sum;
             };
-            if (q == 1) v += p.xb1[r] * B0(r);
-            else if (q == 2) v += p.xb2[r] * B0(r);
+            const double bb = B0(r);
+            if (q == 1) v = fma(p.xb1[r], bb, v);
+            else if (q == 2) v = fma(p.xb2[r], bb, v);
             else {
-                v += p.xbc[r] * B0(r);
-                if (r + 1 <= nx - 2) v += p.xbm[r + 1] * B0(r + 1);
-                if (r >= 1) v += p.xbp[r - 1] * B0(r - 1);
-                const double bb = B0(r);
+                const double below = r >= 1 ? p.xbp[r - 1] : 0.0, above = r + 1 <= nx - 2 ? p.xbm[r + 1] : 0.0;
+                v += fma(below, B0(r - 1), fma(p.xbc[r], bb, above * B0(r + 1)));
                 if (bb != 0.0) {
                     const double u0 = U[o], u1 = U[o + 1], u2 = U[o + 2];
                     const double ee = a.ni * bb * (4.0 * u1 - 3.0 * u0 - u2);
@@ -1035,7 +1221,7 @@ __global__ void __launch_bounds__(256) k_wadj_gather(const __grid_constant__ wpa
                 }
             }
         }
-        VB[o] += v;
+        VB[o] = v;
     }
 }
 
