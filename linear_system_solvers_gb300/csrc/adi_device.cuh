@@ -103,4 +103,86 @@ __device__ __forceinline__ T s_rhs(const dev_instance<T> &d, int t, int j, const
     }
 }
 
+// ------------------------------------------------------------------------------------------
+// boundary#1: explicit_heston_boundary_scheme::rhs (explicit_boundary.hpp:39-84) + v_hi column
+// ------------------------------------------------------------------------------------------
+// Results go to bcol0[i * stride], bcolN[i * stride]: the boundary columns of the v lines
+// (stride 1) or, for the explicit Euler step, columns 0 and ny-1 of the next state (stride ny).
+template <typename T, bool X>
+__device__ __forceinline__ void boundary1_row(const dev_instance<T> &d, const T *U, int i, T *bcol0, T *bcolN, int stride)
+{
+    using R = ar<X>;
+    const int nx = d.nx, ny = d.ny, N = nx - 1;
+    const T one = T(1), two = T(2), three = T(3), four = T(4);
+    const long long w = static_cast<long long>(i) * stride;
+    if (i == 0) {
+        bcol0[0] = d.s_lo[0];
+    } else if (i == N) {
+        const T D = d.D0[N], E = d.E0[N], F = d.F0[N];
+        const T dlt = R::mul(R::mul(two, d.h1), d.s_hi_neu[0]);
+        const T t1 = R::mul(R::add(R::sub(one, R::mul(R::mul(three, d.ni), E)), R::mul(d.rho, F)), U[N * ny]);
+        const T t2 = R::mul(R::mul(R::mul(four, d.ni), E), U[N * ny + 1]);
+        const T t3 = R::mul(R::mul(d.ni, E), U[N * ny + 2]);
+        const T t4 = R::mul(R::mul(d.delta, dlt), D);
+        bcol0[w] = R::sub(R::sub(R::add(t1, t2), t3), t4);
+    } else {
+        const T D = d.D0[i], E = d.E0[i], F = d.F0[i];
+        const T t1 = R::mul(R::mul(-d.delta, D), U[(i - 1) * ny]);
+        const T t2 = R::mul(R::add(R::sub(one, R::mul(R::mul(three, d.ni), E)), R::mul(d.rho, F)), U[i * ny]);
+        const T t3 = R::mul(R::mul(d.delta, D), U[(i + 1) * ny]);
+        const T t4 = R::mul(R::mul(d.ni, E), U[i * ny + 2]);
+        const T t5 = R::mul(R::mul(R::mul(four, d.ni), E), U[i * ny + 1]);
+        bcol0[w] = R::add(R::sub(R::add(R::add(t1, t2), t3), t4), t5);
+    }
+    bcolN[w] = d.v_hi[i];
+}
+
+// ------------------------------------------------------------------------------------------
+// HV full-grid stage rhs_intermed_3 (lss_heat_hundsdorfer_verwer_method.hpp:146-171).
+// ------------------------------------------------------------------------------------------
+template <typename T, bool X>
+__device__ __forceinline__ T hv3_value(const dev_instance<T> &d, const T *U, const T *Y1, const T *Y2, int o)
+{
+    using R = ar<X>;
+    const int ny = d.ny;
+    const T one = T(1);
+    const T th = d.theta;
+    const T M = d.M[o], Z = d.Z[o], P = d.P[o], W = d.W[o];
+    const T t1 = R::mul(R::mul(-th, M), Y1[o - ny]);
+    const T t2 = R::mul(R::add(one, R::mul(th, Z)), Y1[o]);
+    const T t3 = R::mul(R::mul(th, P), Y1[o + ny]);
+    const T t4 = R::mul(R::mul(th, M), U[o - ny]);
+    const T t5 = R::mul(R::mul(th, Z), U[o]);
+    const T t6 = R::mul(R::mul(th, P), U[o + ny]);
+    const T d1 = R::sub(Y2[o + ny + 1], U[o + ny + 1]);
+    const T d2 = R::sub(Y2[o + ny - 1], U[o + ny - 1]);
+    const T d3 = R::sub(Y2[o - ny + 1], U[o - ny + 1]);
+    const T d4 = R::sub(Y2[o - ny - 1], U[o - ny - 1]);
+    const T t7 = R::mul(R::mul(R::mul(d.zeta, d.gamma), d.C[o]), R::add(R::sub(R::sub(d1, d2), d3), d4));
+    const T e1 = R::mul(M, R::sub(Y2[o - ny], U[o - ny]));
+    const T e2 = R::mul(R::add(W, Z), R::sub(Y2[o], U[o]));
+    const T e3 = R::mul(P, R::sub(Y2[o + ny], U[o + ny]));
+    const T e4 = R::mul(d.Mt[o], R::sub(Y2[o - 1], U[o - 1]));
+    const T e5 = R::mul(d.Pt[o], R::sub(Y2[o + 1], U[o + 1]));
+    const T t8 = R::mul(d.zeta, R::add(R::add(R::add(R::sub(e1, e2), e3), e4), e5));
+    return R::add(R::add(R::add(R::sub(R::add(R::sub(R::add(t1, t2), t3), t4), t5), t6), t7), t8);
+}
+
+// ------------------------------------------------------------------------------------------
+// boundary#2 (explicit_boundary.hpp:202-238): row 0 Dirichlet, row nx-1 from the
+// one-sided Neumann extrapolation with the index_of-remapped column.
+// ------------------------------------------------------------------------------------------
+template <typename T, bool X> __device__ __forceinline__ void boundary2_column(const dev_instance<T> &d, T *V, int j)
+{
+    using R = ar<X>;
+    const int nx = d.nx, ny = d.ny;
+    const T two = T(2), three = T(3), four = T(4);
+    V[j] = d.s_lo[j];
+    const int jj = d.jmap[j];
+    const int lri = nx - 1;
+    V[lri * ny + j] = R::div(R::sub(R::sub(R::mul(four, V[(lri - 1) * ny + jj]), V[(lri - 2) * ny + jj]),
+                                    R::mul(R::mul(two, d.h1), d.s_hi_neu[j])),
+                             three);
+}
+
 } // namespace lss_gb300

@@ -11,46 +11,19 @@
 // container_2d<by_enum::Row>.
 #include "adi_plain.hpp"
 
+#include "adi_exact.cuh"
+
 #include <algorithm>
 #include <vector>
 
 namespace lss_gb300 {
 
-// ------------------------------------------------------------------------------------------
-// boundary#1: explicit_heston_boundary_scheme::rhs (explicit_boundary.hpp:39-84) + v_hi column
-// ------------------------------------------------------------------------------------------
-// Results go to bcol0[i * stride], bcolN[i * stride]: the boundary columns of the v lines
-// (stride 1) or, for the explicit Euler step, columns 0 and ny-1 of the next state (stride ny).
 template <typename T, bool X>
 __global__ void k_boundary1(dev_instance<T> d, const T *__restrict__ U, T *__restrict__ bcol0, T *__restrict__ bcolN,
                             int stride)
 {
-    using R = ar<X>;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int nx = d.nx, ny = d.ny, N = nx - 1;
-    if (i >= nx) return;
-    const T one = T(1), two = T(2), three = T(3), four = T(4);
-    const long long w = static_cast<long long>(i) * stride;
-    if (i == 0) {
-        bcol0[0] = d.s_lo[0];
-    } else if (i == N) {
-        const T D = d.D0[N], E = d.E0[N], F = d.F0[N];
-        const T dlt = R::mul(R::mul(two, d.h1), d.s_hi_neu[0]);
-        const T t1 = R::mul(R::add(R::sub(one, R::mul(R::mul(three, d.ni), E)), R::mul(d.rho, F)), U[N * ny]);
-        const T t2 = R::mul(R::mul(R::mul(four, d.ni), E), U[N * ny + 1]);
-        const T t3 = R::mul(R::mul(d.ni, E), U[N * ny + 2]);
-        const T t4 = R::mul(R::mul(d.delta, dlt), D);
-        bcol0[w] = R::sub(R::sub(R::add(t1, t2), t3), t4);
-    } else {
-        const T D = d.D0[i], E = d.E0[i], F = d.F0[i];
-        const T t1 = R::mul(R::mul(-d.delta, D), U[(i - 1) * ny]);
-        const T t2 = R::mul(R::add(R::sub(one, R::mul(R::mul(three, d.ni), E)), R::mul(d.rho, F)), U[i * ny]);
-        const T t3 = R::mul(R::mul(d.delta, D), U[(i + 1) * ny]);
-        const T t4 = R::mul(R::mul(d.ni, E), U[i * ny + 2]);
-        const T t5 = R::mul(R::mul(R::mul(four, d.ni), E), U[i * ny + 1]);
-        bcol0[w] = R::add(R::sub(R::add(R::add(t1, t2), t3), t4), t5);
-    }
-    bcolN[w] = d.v_hi[i];
+    if (i < d.nx) boundary1_row<T, X>(d, U, i, bcol0, bcolN, stride);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -250,59 +223,21 @@ __global__ void k_euler(dev_instance<T> d, const T *__restrict__ U, T *__restric
     V[o] = v;
 }
 
-// ------------------------------------------------------------------------------------------
-// HV full-grid stage rhs_intermed_3 (lss_heat_hundsdorfer_verwer_method.hpp:146-171).
-// ------------------------------------------------------------------------------------------
 template <typename T, bool X>
 __global__ void k_hv_stage3(dev_instance<T> d, const T *__restrict__ U, const T *__restrict__ Y1,
                             const T *__restrict__ Y2, T *__restrict__ Y3)
 {
-    using R = ar<X>;
-    const int nx = d.nx, ny = d.ny;
     const int q = 1 + blockIdx.x * blockDim.x + threadIdx.x;
     const int r = 1 + blockIdx.y;
-    if (q > ny - 2 || r > nx - 2) return;
-    const int o = r * ny + q;
-    const T one = T(1);
-    const T th = d.theta;
-    const T M = d.M[o], Z = d.Z[o], P = d.P[o], W = d.W[o];
-    const T t1 = R::mul(R::mul(-th, M), Y1[o - ny]);
-    const T t2 = R::mul(R::add(one, R::mul(th, Z)), Y1[o]);
-    const T t3 = R::mul(R::mul(th, P), Y1[o + ny]);
-    const T t4 = R::mul(R::mul(th, M), U[o - ny]);
-    const T t5 = R::mul(R::mul(th, Z), U[o]);
-    const T t6 = R::mul(R::mul(th, P), U[o + ny]);
-    const T d1 = R::sub(Y2[o + ny + 1], U[o + ny + 1]);
-    const T d2 = R::sub(Y2[o + ny - 1], U[o + ny - 1]);
-    const T d3 = R::sub(Y2[o - ny + 1], U[o - ny + 1]);
-    const T d4 = R::sub(Y2[o - ny - 1], U[o - ny - 1]);
-    const T t7 = R::mul(R::mul(R::mul(d.zeta, d.gamma), d.C[o]), R::add(R::sub(R::sub(d1, d2), d3), d4));
-    const T e1 = R::mul(M, R::sub(Y2[o - ny], U[o - ny]));
-    const T e2 = R::mul(R::add(W, Z), R::sub(Y2[o], U[o]));
-    const T e3 = R::mul(P, R::sub(Y2[o + ny], U[o + ny]));
-    const T e4 = R::mul(d.Mt[o], R::sub(Y2[o - 1], U[o - 1]));
-    const T e5 = R::mul(d.Pt[o], R::sub(Y2[o + 1], U[o + 1]));
-    const T t8 = R::mul(d.zeta, R::add(R::add(R::add(R::sub(e1, e2), e3), e4), e5));
-    Y3[o] = R::add(R::add(R::add(R::sub(R::add(R::sub(R::add(t1, t2), t3), t4), t5), t6), t7), t8);
+    if (q > d.ny - 2 || r > d.nx - 2) return;
+    const int o = r * d.ny + q;
+    Y3[o] = hv3_value<T, X>(d, U, Y1, Y2, o);
 }
 
-// ------------------------------------------------------------------------------------------
-// boundary#2 (explicit_boundary.hpp:202-238): row 0 Dirichlet, row nx-1 from the
-// one-sided Neumann extrapolation with the index_of-remapped column.
-// ------------------------------------------------------------------------------------------
 template <typename T, bool X> __global__ void k_boundary2(dev_instance<T> d, T *__restrict__ V)
 {
-    using R = ar<X>;
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    const int nx = d.nx, ny = d.ny;
-    if (j >= ny) return;
-    const T two = T(2), three = T(3), four = T(4);
-    V[j] = d.s_lo[j];
-    const int jj = d.jmap[j];
-    const int lri = nx - 1;
-    V[lri * ny + j] = R::div(R::sub(R::sub(R::mul(four, V[(lri - 1) * ny + jj]), V[(lri - 2) * ny + jj]),
-                                    R::mul(R::mul(two, d.h1), d.s_hi_neu[j])),
-                             three);
+    if (j < d.ny) boundary2_column<T, X>(d, V, j);
 }
 
 // V(eval_s, eval_v) by bilinear weights (double result).
@@ -424,7 +359,109 @@ template <typename T> int plain_solver<T>::init(instance_tables<T> &&tab, int ar
         LSS_CUDA_TRY(cudaDeviceSynchronize(), "uploading time-dependent tables");
     }
     bil_ = make_bilinear(tab_.x.data(), nx, tab_.y.data(), ny, eval_s, eval_v);
+    return init_exact();
+}
+
+// Lines per CTA of a stage that solves `lines` lines of e rows: as few as put one CTA on every SM (a
+// chain costs the same with one line on its warp as with 32), within the shared memory of a CTA.
+// 0: the rows of `least` lines do not fit.
+static int exact_lines(int lines, int e, int least, int sms, size_t word)
+{
+    int L = least;
+    while (L < 32 && (lines + L - 1) / L > sms) L *= 2;
+    while (L > least && L * static_cast<size_t>(e | 1) * word > EXACT_SMEM) L /= 2;
+    return L * static_cast<size_t>(e | 1) * word > EXACT_SMEM ? 0 : L;
+}
+
+// Thomas solves whose tables are the same in every step: their factors, made once (adi_exact.cuh).  The
+// explicit scheme has no solves; double sweeps, per-step and time-dependent tables and divisors
+// beyond 2^+-64 (FP32: 2^+-24) keep the kernels above.
+template <typename T> int plain_solver<T>::init_exact()
+{
+    exact_s_ = exact_v_ = 0;
+    if (arith_ != LSS_ADI_ARITH_REFERENCE || tab_.double_sweep || tab_.step_tables || tab_.tdep || tab_.scheme == LSS_ADI_EXPLICIT_EULER)
+        return LSS_ADI_OK;
+    const int nx = tab_.nx, ny = tab_.ny;
+    int dev = 0, sms = 0;
+    LSS_CUDA_TRY(cudaGetDevice(&dev), "cudaGetDevice");
+    LSS_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "SM count");
+    const int Ls = exact_lines(ny - 2, nx - 2, 1, sms, sizeof(T)), Lv = exact_lines(nx - 2, ny - 2, 2, sms, sizeof(T));
+    if (!Ls || !Lv) return LSS_ADI_OK;
+    const size_t n = static_cast<size_t>(nx) * ny;
+    dbuf<int> bad;
+    LSS_CUDA_TRY(bad.alloc(1), "allocating line factors");
+    LSS_CUDA_TRY(cudaMemset(bad.p, 0, sizeof(int)), "line factors");
+    LSS_CUDA_TRY(exact_.alloc(8 * n), "allocating line factors");
+    T *q = exact_.p;
+    exact::k_exact_setup<T><<<grid_for(ny - 2, 32), 32>>>(d_.M, d_.Z, d_.P, d_.theta, ny - 2, ny + 1, 1, ny, nx - 2, q, bad.p);
+    exact::k_exact_setup<T><<<grid_for(nx - 2, 32), 32>>>(d_.Mt, d_.W, d_.Pt, d_.theta, nx - 2, ny + 1, ny, 1, ny - 2, q + 4 * n, bad.p);
+    LSS_CUDA_TRY(cudaGetLastError(), "launching the line factors");
+    int out = 0;
+    LSS_CUDA_TRY(cudaMemcpy(&out, bad.p, sizeof(int), cudaMemcpyDeviceToHost), "line factors");
+    if (out) return LSS_ADI_OK;
+    for (const void *k : {reinterpret_cast<const void *>(exact::k_exact_s<T, S_STAGE1>), reinterpret_cast<const void *>(exact::k_exact_s<T, S_STAGE3_CS>),
+                          reinterpret_cast<const void *>(exact::k_exact_s<T, S_STAGE3_MCS>),
+                          reinterpret_cast<const void *>(exact::k_exact_s<T, S_STAGE4_HV>), reinterpret_cast<const void *>(exact::k_exact_v<T>)})
+        LSS_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, EXACT_SMEM), "line solves' shared memory");
+    exact_s_ = Ls;
+    exact_v_ = Lv;
     return LSS_ADI_OK;
+}
+
+// one launch with programmatic stream serialisation
+template <typename... P, typename... A>
+static void launch_dependent(cudaStream_t s, void (*k)(P...), int grid, int block, size_t smem, A &&...args)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k, P(std::forward<A>(args))...);
+}
+
+template <typename T> void plain_solver<T>::enqueue_exact(cudaStream_t s, T *&U, T *&V)
+{
+    const int nx = d_.nx, ny = d_.ny, Ls = exact_s_, Lv = exact_v_;
+    const size_t n = static_cast<size_t>(nx) * ny;
+    T *Y1 = state_.p + 2 * n, *Y2 = state_.p + 3 * n, *Y3 = state_.p + 4 * n;
+    T *bcol0 = state_.p + 7 * n, *bcolN = bcol0 + nx;
+    const T *qs = exact_.p, *qv = exact_.p + 4 * n;
+    auto threads = [](int rows) { return rows <= 1024 ? 128 : 256; };
+    auto S = [&](auto k, const T *A, const T *B, const T *Cc, T *Y, bool bc) {
+        launch_dependent(s, k, grid_for(ny - 2, Ls) + (bc ? 1 : 0), threads((nx - 2) * Ls), Ls * sizeof(T) * ((nx - 2) | 1), d_, qs, Ls, U, A, B, Cc, Y,
+                         bc ? bcol0 : nullptr, bcolN);
+        ++launches_;
+    };
+    auto v_solve = [&](const T *in, const T *inh, T *out, bool last) {
+        launch_dependent(s, exact::k_exact_v<T>, grid_for(nx - 2, Lv), threads((ny - 2) * Lv), Lv * sizeof(T) * ((ny - 2) | 1), d_, qv, Lv, in, inh,
+                         bcol0, bcolN, out, last);
+        ++launches_;
+    };
+    for (int step = 0; step < tab_.steps; ++step) {
+        S(exact::k_exact_s<T, S_STAGE1>, U, nullptr, nullptr, Y1, true);
+        switch (tab_.scheme) {
+        case LSS_ADI_DOUGLAS_RACHFORD: v_solve(U, Y1, V, true); break;
+        case LSS_ADI_CRAIG_SNEYD:
+        case LSS_ADI_MODIFIED_CRAIG_SNEYD:
+            v_solve(U, Y1, Y2, false);
+            if (tab_.scheme == LSS_ADI_CRAIG_SNEYD) S(exact::k_exact_s<T, S_STAGE3_CS>, U, Y1, Y2, Y3, false);
+            else S(exact::k_exact_s<T, S_STAGE3_MCS>, U, Y1, Y2, Y3, false);
+            v_solve(U, Y3, V, true);
+            break;
+        default: // Hundsdorfer-Verwer
+            v_solve(U, Y1, Y2, false);
+            S(exact::k_exact_s<T, S_STAGE4_HV>, Y2, Y1, nullptr, Y3, false);
+            v_solve(Y2, Y3, V, true);
+            break;
+        }
+        std::swap(U, V);
+    }
 }
 
 template <typename T> template <bool X> void plain_solver<T>::enqueue_steps(cudaStream_t s, T *&U, T *&V)
@@ -528,7 +565,9 @@ int plain_solver<T>::forward(const void *payoff, void *out_surface, double *out_
             LSS_CUDA_TRY(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking), "creating capture stream");
             LSS_CUDA_TRY(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal), "beginning graph capture");
             T *u = U0, *v = V0;
-            if (arith_ == LSS_ADI_ARITH_REFERENCE)
+            if (exact_s_)
+                enqueue_exact(cs, u, v);
+            else if (arith_ == LSS_ADI_ARITH_REFERENCE)
                 enqueue_steps<true>(cs, u, v);
             else
                 enqueue_steps<false>(cs, u, v);
@@ -545,7 +584,9 @@ int plain_solver<T>::forward(const void *payoff, void *out_surface, double *out_
         launches_ = graph_launches_;
         if (tab_.steps % 2) std::swap(U, V);
     } else {
-        if (arith_ == LSS_ADI_ARITH_REFERENCE)
+        if (exact_s_)
+            enqueue_exact(s, U, V);
+        else if (arith_ == LSS_ADI_ARITH_REFERENCE)
             enqueue_steps<true>(s, U, V);
         else
             enqueue_steps<false>(s, U, V);
