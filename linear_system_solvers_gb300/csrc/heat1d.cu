@@ -74,7 +74,7 @@ struct h1lane {
 
 struct h1group {
     int n, lanes, steps;
-    int reg;        // 1: the factorised sweep runs in registers (k_h1_reg)
+    int reg;        // 1: the factorised sweep runs in registers (k_h1_reg); 2: in registers, row after row (k_h1_relay)
     long long pt;   // point block: slot s, point t, lane l at pt + (s*n + t)*32 + l
     long long bnd;  // boundary values: step s, side q (0 lower, 1 upper) at bnd + (s*2 + q)*32 + l
     long long src;  // source rows (steps + 1) x n, or -1
@@ -412,7 +412,7 @@ template <typename T> __global__ void __launch_bounds__(128) k_h1_setup_fast(con
     const h1group G = p.groups[g];
     if (lane >= G.lanes) return;
     h1lane &L = p.lanes[static_cast<long long>(g) * LANES + lane];
-    if (G.reg) {
+    if (G.reg == 1) {
         h1_setup_reg<T>(p, G, L, lane);
         return;
     }
@@ -884,6 +884,197 @@ template <bool SRC, bool KEEP> __global__ void __launch_bounds__(LANES, 8) k_h1_
     }
 }
 
+// ------------------------------------------------------------------------------------------
+// FAST, FP32 instances whose rows fit a warp's registers: the operations of the sweep through memory in
+// its order (same bits), with W lanes of R rows per instance as above.  The first and the last solved
+// row are scalars of the lowest and highest lane, the rows between them fill the lanes from the upper
+// end; places below them pass a value through (slope -1 on -0: exact for every value) and hold the first
+// row's u.  Right-hand sides are evaluated by all lanes at once.  A recurrence is run W times by every
+// lane, each time from the value that the lane before ended with: after k rounds the lanes below k
+// are final.
+//
+// What bounds it: 2 W rounds of R dependent multiply-adds and a shuffle (about 90 cycles at R = 16, 3.3 ms
+// for 512 points and 1000 steps) for the longest instances, the issue slots of those rounds for a
+// full GPU.  8192 Black-Scholes calls of 101..512 points and 100..1000 steps: 4.9 ms; the sweep through
+// memory took 22.2 ms, 85 cycles per row of its longest line.
+// ------------------------------------------------------------------------------------------
+constexpr int H1_RELAY_MIN = 8; // points: at least two rows between first and last solved one
+
+template <int R, bool KEEP> __device__ __forceinline__ void h1_relay_unit(const h1params<float> &p, const h1unit un)
+{
+    using T = float;
+    const unsigned all = 0xffffffffu;
+    const int wl = threadIdx.x & 31, W = un.W, li = wl & (W - 1), sub = wl / W;
+    const h1group G = p.groups[un.g];
+    const bool act = sub < un.sub;
+    const int lane = un.lane0 + (act ? sub : 0); // idle sub-warps shadow the first instance and store nothing
+    const h1lane L = p.lanes[static_cast<long long>(un.g) * LANES + lane];
+    const int n = G.n, N = n - 1;
+    const long long NS = static_cast<long long>(n) * LANES;
+    T *base = p.pt + G.pt + lane;
+    const T *WB = base + S_B * NS, *WD = base + S_D * NS, *M = base + S_M * NS, *GG = base + S_G * NS;
+    T *U = base + S_U * NS;
+    const T *BND = p.bnd + G.bnd + lane;
+    T *ALL = KEEP ? p.all + G.all + lane : nullptr;
+    const T th = T(L.theta), omt = T(1) - th, bl = T(L.bl), bh = T(L.bh);
+    const T kap = -omt / th;
+    const bool cn = kap != T(0);
+    const int start = L.start, end = L.end, steps = act ? L.steps : 0;
+    const bool low = li == 0, high = li == W - 1;
+    const T *init = p.init + L.init_off;
+    const int pad = W * R - (end - start - 1);    // places below the rows
+    const int t0 = start + 1 - pad + li * R;      // row of this lane's first place
+    const int pr = min(max(pad - li * R, 0), R);  // places of this lane below the rows
+
+    T wb[R], wd[R], m[R], g[R], u[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const bool in = r >= pr;
+        const int t = in ? t0 + r : start;
+        wb[r] = in ? WB[el(t)] : T(0);
+        wd[r] = in ? WD[el(t)] : T(0);
+        m[r] = in ? M[el(t)] : T(-1);
+        g[r] = in ? GG[el(t)] : T(-1);
+        u[r] = init[t];
+    }
+    // the end row of this lane's side (lane 0: the first, others: the last one)
+    const int te = low ? start : end;
+    const T ewb = WB[el(te)], ewd = WD[el(te)], em = M[el(te)], eg = GG[el(start)];
+    T ue = init[te];
+    T nb = init[low ? start + 1 : end - 1];                                     // its neighbour inside
+    T ob = low ? (start ? init[0] : T(0)) : (end < N ? init[N] : T(0));          // and outside
+    const int side = low ? 0 : 1;
+    T bnew = steps > 0 ? BND[side * LANES] : T(0);
+    T bcur = init[low ? 0 : N];
+    int row = L.forward ? 0 : L.steps;
+    if (KEEP && act) {
+        for (int t = li; t < n; t += W) ALL[(static_cast<long long>(row) * n + t) * LANES] = init[t];
+    }
+    for (int s = 0; s < un.steps; ++s) {
+        const bool live = s < steps;
+        const T bv = bnew;
+        if (s + 1 < steps) bnew = BND[(2 * (s + 1) + side) * LANES];
+        // right-hand sides
+        T c[R];
+        const T first_u = __shfl_sync(all, ue, 0, W), last_u = __shfl_sync(all, ue, W - 1, W);
+        T um = __shfl_up_sync(all, u[R - 1], 1, W), un1 = __shfl_down_sync(all, u[0], 1, W);
+        if (low) um = first_u;
+        if (high) un1 = last_u;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const T u1 = r + 1 < R ? u[r + 1 < R ? r + 1 : 0] : un1;
+            const T v = h1_fma(-m[r], cn ? um : T(0), h1_fma(wd[r], u1, wb[r] * u[r]));
+            c[r] = r >= pr ? v : T(-0.0f);
+            um = u[r];
+        }
+        // first row (lane 0); the order of the sums is that of the sweep through memory
+        T yf;
+        {
+            const T uc = ue, up = nb;
+            yf = h1_fma(em, h1_fma(kap, ob, start ? -bv : T(0)), h1_fma(ewb, uc, ewd * up));
+            if (start == 0) yf = h1_fma(bl, bv, yf);
+            yf += T(0);
+        }
+        // forward recurrence
+        T y = yf;
+        for (int k = 1; k < W; ++k) {
+            T z = y;
+#pragma unroll
+            for (int r = 0; r < R; ++r) z = h1_fma(-m[r], z, c[r]);
+            z = __shfl_up_sync(all, z, 1, W);
+            y = low ? yf : z;
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            y = h1_fma(-m[r], y, c[r]);
+            c[r] = y;
+        }
+        // last row (lane W - 1: y is the row before)
+        T xl;
+        {
+            const T uc = ue, u1 = ob, um2 = nb;
+            xl = h1_fma(bh, bv, h1_fma(em, h1_fma(kap, um2, -y), h1_fma(ewb, uc, ewd * u1)));
+            xl += T(0);
+        }
+        // back substitution
+#pragma unroll
+        for (int r = 0; r < R; ++r) c[r] = r >= pr ? c[r] : T(-0.0f);
+        T x = xl;
+        for (int k = 1; k < W; ++k) {
+            T z = x;
+#pragma unroll
+            for (int r = R - 1; r >= 0; --r) z = h1_fma(-g[r], z, c[r]);
+            z = __shfl_down_sync(all, z, 1, W);
+            x = high ? xl : z;
+        }
+#pragma unroll
+        for (int r = R - 1; r >= 0; --r) {
+            x = h1_fma(-g[r], x, c[r]);
+            c[r] = x;
+        }
+        // x of lane 0: row start + 1; the first row
+        const T xf = h1_fma(-eg, x, yf);
+        const T fill = __shfl_sync(all, xf, 0, W);
+        if (live) {
+#pragma unroll
+            for (int r = 0; r < R; ++r) u[r] = r >= pr ? c[r] : fill;
+            ue = low ? xf : xl;
+            nb = low ? x : c[R - 1];
+            ob = (low ? start == 1 : end < N) ? bv : T(0);
+            bcur = bv;
+        }
+        if (KEEP && live) {
+            row += L.forward ? 1 : -1;
+            T *A1 = ALL + static_cast<long long>(row) * NS;
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                if (r >= pr) A1[el(t0 + r)] = u[r];
+            if (low) A1[el(start)] = ue;
+            if (high) A1[el(end)] = ue;
+            if (low && start == 1) A1[0] = bcur;
+            if (high && end < N) A1[el(N)] = bcur;
+        }
+    }
+    int bad = 0;
+    if (act) {
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            if (r >= pr) {
+                U[el(t0 + r)] = u[r];
+                bad |= !isfinite(u[r]);
+            }
+        if (low || high) {
+            U[el(te)] = ue;
+            bad |= !isfinite(ue);
+            if (low ? start == 1 : end < N) {
+                U[el(low ? 0 : N)] = bcur;
+                bad |= !isfinite(bcur);
+            }
+        }
+    }
+    const unsigned b = __ballot_sync(all, bad);
+    const unsigned mine = (W == 32 ? all : ((1u << W) - 1u) << (sub * W));
+    __syncwarp();
+    if (act && low) {
+        const int i = L.eval_i;
+        p.values[L.inst] = (1.0 - L.eval_w) * static_cast<double>(U[el(i)]) + L.eval_w * static_cast<double>(U[el(i + 1)]);
+        p.status[L.inst] = (b & mine) != 0;
+    }
+}
+
+template <bool KEEP> __global__ void __launch_bounds__(LANES, 16) k_h1_relay(const h1params<float> p)
+{
+    const h1unit un = p.units[blockIdx.x];
+    switch (un.R) {
+    case 4: h1_relay_unit<4, KEEP>(p, un); break;
+    case 8: h1_relay_unit<8, KEEP>(p, un); break;
+    case 10: h1_relay_unit<10, KEEP>(p, un); break;
+    case 12: h1_relay_unit<12, KEEP>(p, un); break;
+    case 14: h1_relay_unit<14, KEEP>(p, un); break;
+    default: h1_relay_unit<H1_RMAX, KEEP>(p, un); break;
+    }
+}
+
 // Lanes per instance and rows per lane for lines of `n` points: the fewest lanes (4 .. 32) whose
 // rows fit 16 per lane -- fewer scan levels per row -- then the fewest rows of the compiled ones.
 static inline void h1_shape(int n, int &W, int &R)
@@ -1038,8 +1229,13 @@ template <typename T> int batch_t<T>::build(std::vector<inst_info> &&inf, std::v
         G.steps = steps;
         // FP64 lines that fit a warp's registers.  Against the sweep through memory (a thread per
         // instance): 4096 Black-Scholes calls of 101..512 points, 100..1000 steps 104 ms -> 7.8 ms.
-        // FP32 keeps the sweep through memory: its results are pinned to that sweep's rounding.
-        G.reg = std::is_same<T, double>::value && arith == LSS_ADI_ARITH_FAST && n <= LANES * H1_RMAX;
+        // FP32 lines without sources keep that sweep's operations and their order (k_h1_relay): 8192 calls
+        // of the same sizes 22.2 ms -> 4.9 ms.  Sources and longer lines stay in memory.
+        G.reg = 0;
+        if (arith == LSS_ADI_ARITH_FAST && n <= LANES * H1_RMAX) {
+            if (std::is_same<T, double>::value) G.reg = 1;
+            else if (!gsrc && n >= H1_RELAY_MIN) G.reg = 2;
+        }
         G.pt = pt;
         pt += static_cast<long long>(NSLOT) * n * LANES;
         G.bnd = bnd;
@@ -1247,6 +1443,10 @@ template <typename T> int batch_t<T>::run(cudaStream_t s)
                 else k_h1_reg<false, false><<<nunits, LANES, 0, s>>>(p);
                 LSS_CUDA_TRY(cudaGetLastError(), "heat1d: launching the time loop");
             }
+        } else if (nunits) {
+            if (keep) k_h1_relay<true><<<nunits, LANES, 0, s>>>(p);
+            else k_h1_relay<false><<<nunits, LANES, 0, s>>>(p);
+            LSS_CUDA_TRY(cudaGetLastError(), "heat1d: launching the time loop");
         }
         const int ctas = sched.ctas, th = h1_warps<T>() * LANES;
         if (!ctas) return LSS_ADI_OK;
