@@ -22,13 +22,18 @@
 
 namespace lss_gb300 {
 
-// slots of the S-direction tables ([t][j] layout, n = nx*ny per slot)
+// slots of the FP32 S-line tables ([t][slot][j], pitch ld)
 enum {
     SL_LA = 0, SL_G, SL_WG, SL_WW, SL_WS, SL_WC, SL_WN, SL_WE,
     SL_S2SC, SL_S2SE, SL_S2IB, SL_S2MZ, SL_X1, SL_X2, SL_X3, SL_X4, SL_X5, SL_IB, SL_COUNT
 };
-// slots of the v-direction tables ([t][i] layout: i fastest)
+// and v-line tables ([t][slot][i]: i fastest)
 enum { VL_LA = 0, VL_G, VL_VC, VL_VN, VL_IB, VL_COUNT };
+// slots of the FP64 line tables: S lines [t][slot][j] (pitch ld), v lines [t][slot][i] (pitch nx)
+enum { DS_LA = 0, DS_G, DS_WG, DS_WW, DS_WS, DS_WQ, DS_WN, DS_WE, DS_IB, DS_WC, DS_COUNT };
+enum { DV_L = 0, DV_U, DV_IB, DV_COUNT };
+template <typename T> __host__ __device__ constexpr int s_slots() { return sizeof(T) == 8 ? static_cast<int>(DS_COUNT) : static_cast<int>(SL_COUNT); }
+template <typename T> __host__ __device__ constexpr int v_slots() { return sizeof(T) == 8 ? static_cast<int>(DV_COUNT) : static_cast<int>(VL_COUNT); }
 // per-instance 1-D arrays along S (nx each).  Adjoint only, coefficient derivatives split into
 // S and v factors: X_HX = S/A (dd^/dr), X_HC = S-factor of c^ (Heston S/A, SABR F^beta/A),
 // X_HA = F^(2 beta)/A^2 and X_HDD = F^(2 beta) A''/A^3 (SABR D(t) terms of a^ and d^)
@@ -40,7 +45,7 @@ enum { Y_SLO = 0, Y_B2C, Y_CHS, Y_HY, Y_BS, Y_EK, Y_ET, Y_ES, Y_HV2, Y_COUNT };
 
 struct bdesc {
     int nx, ny, steps, scheme;
-    int ld, pad0_; // row pitch of the state (FP64: a multiple of 4; FP32: ny)
+    int ld, pad0_; // row pitch of the state and the S-line tables (a multiple of 32 bytes)
     long long o2;  // offset of the instance in the nx*ld arenas
     long long op;  // offset in the nx*ny arena of initial conditions
     int ox, oy;    // offsets in the nx- and ny-sized arenas
@@ -71,8 +76,7 @@ template <typename T> struct bparams {
     const int *layout;                // per CTA: sizes of its warp groups, one hex digit each, lowest first
     T *U, *V, *Y1, *Y2, *Y3;          // state arenas (sum nx*ny each)
     T *B0;                            // nx arena: the explicit v = v_lo boundary column of a step
-    const T *S[SL_COUNT];             // S-direction tables
-    const T *Vt[VL_COUNT];            // v-direction tables
+    const T *S, *Vt;                  // S- and v-direction tables (inst_view)
     const T *X[X_COUNT];              // nx arenas
     const T *Yv[Y_COUNT];             // ny arenas
     const int *imap, *jmap;           // nx / ny arenas
@@ -201,7 +205,7 @@ __device__ __forceinline__ void s_line_slots(T *s, long long slot_stride, int sc
 }
 
 template <typename T>
-__global__ void k_setup_s_lines(setup_params sp, T *S0, long long slot_stride, T *chS_arena)
+__global__ void k_setup_s_lines(setup_params sp, T *S0, T *chS_arena)
 {
     const long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (g >= sp.total_lines) return;
@@ -216,7 +220,7 @@ __global__ void k_setup_s_lines(setup_params sp, T *S0, long long slot_stride, T
     }
     const bdesc d = sp.desc[inst];
     const int j = 1 + static_cast<int>(g - sp.line_start[inst]);
-    const int nx = d.nx, ny = d.ny, e = nx - 2;
+    const int ld = d.ld, e = d.nx - 2;
     const double th = sp.scal[3 * inst], ze = sp.scal[3 * inst + 1], gm = sp.scal[3 * inst + 2];
     const long long N = sp.total_n;
     const double *__restrict__ bM = sp.base, *__restrict__ bP = sp.base + N, *__restrict__ bZ = sp.base + 2 * N,
@@ -226,27 +230,27 @@ __global__ void k_setup_s_lines(setup_params sp, T *S0, long long slot_stride, T
     // DRAM latency per point overlaps the work of the point before (the loop is serial along the
     // line: the set-up of one instance's lines runs on few threads before every step of a
     // time-dependent instance)
-    long long o1 = d.o2 + ny + j;
+    long long o1 = d.o2 + ld + j;
     double nM = bM[o1], nP = bP[o1], nZ = bZ[o1], nMt = bMt[o1], nPt = bPt[o1], nW = bW[o1], nC = bC[o1];
     double gam = 0.0;
     for (int t = 1; t <= e; ++t) {
-        const long long o = d.o2 + (long long)t * ny + j;
+        const long long o = d.o2 + (long long)t * ld + j;
         const double M = nM, P = nP, Z = nZ, Mt = nMt, Pt = nPt, W = nW, C = nC;
         if (t < e) {
-            o1 = o + ny;
+            o1 = o + ld;
             nM = bM[o1]; nP = bP[o1]; nZ = bZ[o1]; nMt = bMt[o1]; nPt = bPt[o1]; nW = bW[o1]; nC = bC[o1];
         }
         const double a = -th * M, b = 1.0 + th * Z, c = -th * P;
         const double beta = (t == 1) ? b : b - a * gam;
         const double ib = 1.0 / beta;
         if (t < e) gam = c / beta;
-        s_line_slots<T>(S0 + o, slot_stride, d.scheme, th, ze, gm, M, P, Z, Mt, Pt, W, C, ib, t < e ? gam : 0.0);
+        s_line_slots<T>(S0 + d.o2 * SL_COUNT + (long long)t * SL_COUNT * ld + j, ld, d.scheme, th, ze, gm, M, P, Z, Mt, Pt, W, C, ib, t < e ? gam : 0.0);
         if (t == e) chS_arena[d.oy + j] = static_cast<T>(c * ib);
     }
 }
 
 template <typename T>
-__global__ void k_setup_v_lines(setup_params sp, T *V0, long long slot_stride, T *chV_arena)
+__global__ void k_setup_v_lines(setup_params sp, T *V0, T *chV_arena)
 {
     const long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (g >= sp.total_lines) return;
@@ -258,24 +262,23 @@ __global__ void k_setup_v_lines(setup_params sp, T *V0, long long slot_stride, T
     const int inst = lo;
     const bdesc d = sp.desc[inst];
     const int i = 1 + static_cast<int>(g - sp.line_start[inst]);
-    const int nx = d.nx, ny = d.ny, e = ny - 2;
+    const int nx = d.nx, e = d.ny - 2;
     const double th = sp.scal[3 * inst];
     const long long N = sp.total_n;
     const double *bMt = sp.base + 3 * N, *bPt = sp.base + 4 * N, *bW = sp.base + 5 * N;
     double gam = 0.0;
     for (int t = 1; t <= e; ++t) {
-        const long long ob = d.o2 + (long long)i * ny + t;  // base tables are [i][j]
-        const long long o = d.o2 + (long long)t * nx + i;   // v tables are [t][i]
+        const long long ob = d.o2 + (long long)i * d.ld + t;  // base tables are [i][j]
         const double a = -th * bMt[ob], b = 1.0 + th * bW[ob], c = -th * bPt[ob];
         const double beta = (t == 1) ? b : b - a * gam;
         const double ib = 1.0 / beta;
         if (t < e) gam = c / beta;
-        T *s = V0 + o;
-        s[VL_LA * slot_stride] = static_cast<T>(a * ib);
-        s[VL_G * slot_stride] = static_cast<T>(t < e ? gam : 0.0);
-        s[VL_VC * slot_stride] = static_cast<T>(th * bW[ob] * ib);
-        s[VL_VN * slot_stride] = static_cast<T>(c * ib);
-        s[VL_IB * slot_stride] = static_cast<T>(ib);
+        T *s = V0 + d.o2 * VL_COUNT + (long long)t * VL_COUNT * nx + i; // v tables are [t][slot][i]
+        s[VL_LA * nx] = static_cast<T>(a * ib);
+        s[VL_G * nx] = static_cast<T>(t < e ? gam : 0.0);
+        s[VL_VC * nx] = static_cast<T>(th * bW[ob] * ib);
+        s[VL_VN * nx] = static_cast<T>(c * ib);
+        s[VL_IB * nx] = static_cast<T>(ib);
         if (t == e) chV_arena[d.ox + i] = static_cast<T>(c * ib);
     }
 }
@@ -290,8 +293,8 @@ __device__ __forceinline__ int setup_instance(const setup_params &sp, long long 
     }
     return lo;
 }
-static __global__ void k_setup_s_delta(setup_params sp, double *S0, long long stride);
-static __global__ void k_setup_v_delta(setup_params sp, double *V0, long long stride);
+static __global__ void k_setup_s_delta(setup_params sp, double *S0);
+static __global__ void k_setup_v_delta(setup_params sp, double *V0);
 
 // ------------------------------------------------------------------------------------------
 // the persistent time-loop kernel
@@ -303,8 +306,13 @@ template <typename T> struct inst_view {
     int nx, ny, ld, e_s, e_v;
     long long o2;
     int ox, oy;
-    __device__ __forceinline__ const T *S(int k) const { return p->S[k] + o2; }
-    __device__ __forceinline__ const T *Vt(int k) const { return p->Vt[k] + o2; }
+    long long so, vo; // line tables
+    int sl, vl;       // elements of a row
+    // line tables of the instance: row t of the S lines holds all its slots, column t of the v lines too (a
+    // row's operands lie within a few KB instead of ten arenas: 5 to 15 % where a GPU full of 256 x 128
+    // instances reads them from HBM)
+    __device__ __forceinline__ const T *S(int k, int t, int j) const { return p->S + so + (long long)t * sl + (k * ld + j); }
+    __device__ __forceinline__ const T *Vt(int k, int t, int i) const { return p->Vt + vo + (long long)t * vl + (k * nx + i); }
     __device__ __forceinline__ const T *X(int k) const { return p->X[k] + ox; }
     __device__ __forceinline__ const T *Yv(int k) const { return p->Yv[k] + oy; }
     __device__ __forceinline__ const int *imap() const { return p->imap + ox; }
@@ -378,113 +386,150 @@ template <typename T> __device__ __forceinline__ void b2_stage(const inst_view<T
 // segment.  The mixed difference (x(t-1,j-1) - x(t-1,j+1)) - (x(t+1,j-1) - x(t+1,j+1)) is formed
 // from a rolling window of the per-row differences x(r,j-1) - x(r,j+1): one subtraction per row.
 //
-// s_line_fwd: right-hand side and forward recurrence y_t = f_t - la_t y_{t-1} of line j over
-// rows t0..t1, starting from y = y_{t0-1}; writes y_t into Y and returns y_{t1}.
-template <typename T, int KIND, int SCH>
-__device__ __forceinline__ T s_line_fwd(const inst_view<T> &v, const T *__restrict__ U, const T *__restrict__ Y1,
-                                        const T *__restrict__ Y2, T *__restrict__ Y, int j, int t0, int t1, T y, T hi)
+// The next rows' operands are loaded before the current ones are used (two rows ahead, eight in the back
+// substitution); the fused multiply-adds are written out, so the rounding hangs on no contraction.
+constexpr int FK = 8; // rows of a block of the back substitution
+template <int KIND, int SCH>
+__device__ __forceinline__ void s_stage(const inst_view<float> &v, const float *U, const float *Y1, const float *Y2, float *Y, int l0, int ls)
 {
-    const int ny = v.ny, e = v.e_s;
-    const long long b = (long long)(t0 - 1) * ny + j;
-    if constexpr (KIND == 1) {
-        // centre column of U (rows t-1, t, t+1), its side columns at row t, per-row differences
-        T u0c = U[b], u1c = U[b + ny];
-        T u1m = U[b + ny - 1], u1p = U[b + ny + 1];
-        T q0 = U[b - 1] - U[b + 1], q1 = u1m - u1p;
-#pragma unroll 4
-        for (int t = t0; t <= t1; ++t) {
-            const long long o = (long long)t * ny + j;
-            const T u2m = U[o + ny - 1], u2c = U[o + ny], u2p = U[o + ny + 1];
-            const T q2 = u2m - u2p;
-            const T mix = q0 - q2;
-            T f = ldg(v.S(SL_WG) + o) * mix;
-            f += ldg(v.S(SL_WW) + o) * u0c;
-            f += ldg(v.S(SL_WS) + o) * u1m;
-            f += ldg(v.S(SL_WC) + o) * u1c;
-            f += ldg(v.S(SL_WN) + o) * u1p;
-            f += ldg(v.S(SL_WE) + o) * u2c;
-            y = f - ldg(v.S(SL_LA) + o) * y;
-            if (t == e) y -= ldg(v.Yv(Y_CHS) + j) * hi;
-            Y[o] = y;
-            u0c = u1c; u1c = u2c;
-            u1m = u2m; u1p = u2p;
-            q0 = q1; q1 = q2;
-        }
-    } else {
-        constexpr bool xt = SCH == LSS_ADI_MODIFIED_CRAIG_SNEYD || SCH == LSS_ADI_HUNDSDORFER_VERWER;
-        constexpr bool hv = SCH == LSS_ADI_HUNDSDORFER_VERWER;
-        // windows: U centre column, Y1 centre column, Delta = Y2 - U (centre column and, at row t,
-        // its side columns), per-row differences of Delta
-        T uc0 = U[b], uc1 = U[b + ny];
-        T y10 = Y1[b], y11 = Y1[b + ny];
-        T d0c = Y2[b] - uc0, d1c = Y2[b + ny] - uc1;
-        T d1m = Y2[b + ny - 1] - U[b + ny - 1], d1p = Y2[b + ny + 1] - U[b + ny + 1];
-        T q0 = (Y2[b - 1] - U[b - 1]) - (Y2[b + 1] - U[b + 1]), q1 = d1m - d1p;
-#pragma unroll 4
-        for (int t = t0; t <= t1; ++t) {
-            const long long o = (long long)t * ny + j;
-            const T uc2 = U[o + ny];
-            const T d2m = Y2[o + ny - 1] - U[o + ny - 1];
-            const T d2p = Y2[o + ny + 1] - U[o + ny + 1];
-            const T q2 = d2m - d2p;
-            const T mix = q0 - q2;
-            T f, y12 = T(0), d2c = T(0);
-            if constexpr (hv || KIND == 2) y12 = Y1[o + ny];
-            if constexpr (xt) d2c = Y2[o + ny] - uc2;
-            if constexpr (hv) {
-                f = ldg(v.S(SL_LA) + o) * y10;
-                f += ldg(v.S(SL_S2SC) + o) * y11;
-                f += ldg(v.S(SL_S2SE) + o) * y12;
-                f += ldg(v.S(SL_S2MZ) + o) * mix;
-                f += ldg(v.S(SL_X1) + o) * d0c;
-                f += ldg(v.S(SL_X2) + o) * d1c;
-                f += ldg(v.S(SL_X3) + o) * d2c;
-                f += ldg(v.S(SL_X4) + o) * d1m;
-                f += ldg(v.S(SL_X5) + o) * d1p;
-            } else {
-                f = ldg(v.S(SL_LA) + o) * uc0;
-                f += ldg(v.S(SL_S2SC) + o) * uc1;
-                f += ldg(v.S(SL_S2SE) + o) * uc2;
-                f += ldg(v.S(SL_S2IB) + o) * y11;
-                f += ldg(v.S(SL_S2MZ) + o) * mix;
-                if constexpr (xt) {
-                    f += ldg(v.S(SL_X1) + o) * d0c;
-                    f += ldg(v.S(SL_X2) + o) * d1c;
-                    f += ldg(v.S(SL_X3) + o) * d2c;
-                    f += ldg(v.S(SL_X4) + o) * d1m;
-                    f += ldg(v.S(SL_X5) + o) * d1p;
-                }
-            }
-            y = f - ldg(v.S(SL_LA) + o) * y;
-            if (t == e) y -= ldg(v.Yv(Y_CHS) + j) * hi;
-            Y[o] = y;
-            uc0 = uc1; uc1 = uc2;
-            y10 = y11; y11 = y12;
-            d0c = d1c; d1c = d2c;
-            d1m = d2m; d1p = d2p;
-            q0 = q1; q1 = q2;
-        }
-    }
-    return y;
-}
-
-template <typename T, int KIND, int SCH>
-__device__ __forceinline__ void s_stage(const inst_view<T> &v, const T *__restrict__ U, const T *__restrict__ Y1,
-                                        const T *__restrict__ Y2, T *__restrict__ Y, int l0, int ls)
-{
-    const int nx = v.nx, ny = v.ny, e = v.e_s;
+    constexpr bool xt = SCH == LSS_ADI_MODIFIED_CRAIG_SNEYD || SCH == LSS_ADI_HUNDSDORFER_VERWER;
+    constexpr bool hv = SCH == LSS_ADI_HUNDSDORFER_VERWER;
+    const int nx = v.nx, ny = v.ny, ld = v.ld, e = v.e_s, last = (nx - 1) * ld;
+    struct row { // tables of row t, state of row t + 1
+        float la, w[10];
+        float um, uc, up;  // KIND 1: U; else Y2 - U (side columns; centre: xt) and
+        float uu, y1;      // U, Y1 at the centre
+    };
     for (int j = 1 + l0; j <= ny - 2; j += ls) {
         const int jj = ldg(v.jmap() + j);
-        const T lo = U[jj], hi = U[(long long)(nx - 1) * ny + jj];
-        T x = s_line_fwd<T, KIND, SCH>(v, U, Y1, Y2, Y, j, 1, e, lo, hi);
-#pragma unroll 4
-        for (int t = e - 1; t >= 1; --t) {
-            const long long o = (long long)t * ny + j;
-            x = Y[o] - ldg(v.S(SL_G) + o) * x;
-            Y[o] = x;
+        const float lo = U[jj], hi = U[last + jj];
+        auto load = [&](int t) -> row {
+            const int o2 = (t + 1) * ld + j;
+            row r;
+            r.la = ldg(v.S(SL_LA, t, j));
+            if constexpr (KIND == 1) {
+                r.w[0] = ldg(v.S(SL_WG, t, j));
+                r.w[1] = ldg(v.S(SL_WW, t, j));
+                r.w[2] = ldg(v.S(SL_WS, t, j));
+                r.w[3] = ldg(v.S(SL_WC, t, j));
+                r.w[4] = ldg(v.S(SL_WN, t, j));
+                r.w[5] = ldg(v.S(SL_WE, t, j));
+                r.um = U[o2 - 1];
+                r.uc = U[o2];
+                r.up = U[o2 + 1];
+            } else {
+                r.w[0] = ldg(v.S(SL_S2SC, t, j));
+                r.w[1] = ldg(v.S(SL_S2SE, t, j));
+                r.w[2] = ldg(v.S(SL_S2MZ, t, j));
+                if constexpr (!hv) r.w[3] = ldg(v.S(SL_S2IB, t, j));
+                if constexpr (xt) {
+                    r.w[4] = ldg(v.S(SL_X1, t, j));
+                    r.w[5] = ldg(v.S(SL_X2, t, j));
+                    r.w[6] = ldg(v.S(SL_X3, t, j));
+                    r.w[7] = ldg(v.S(SL_X4, t, j));
+                    r.w[8] = ldg(v.S(SL_X5, t, j));
+                }
+                r.uu = U[o2];
+                r.um = Y2[o2 - 1] - U[o2 - 1];
+                r.up = Y2[o2 + 1] - U[o2 + 1];
+                if constexpr (xt) r.uc = Y2[o2] - r.uu;
+                r.y1 = Y1[o2];
+            }
+            return r;
+        };
+        // rows t-1, t of the centre columns, side columns at row t, per-row differences of them
+        float u0c, u1c, u1m, u1p, q0, q1, c0 = 0.0f, c1 = 0.0f, y10 = 0.0f, y11 = 0.0f;
+        if constexpr (KIND == 1) {
+            u0c = U[j];
+            u1c = U[ld + j];
+            u1m = U[ld + j - 1];
+            u1p = U[ld + j + 1];
+            q0 = U[j - 1] - U[j + 1];
+        } else {
+            c0 = U[j];
+            c1 = U[ld + j];
+            y10 = Y1[j];
+            y11 = Y1[ld + j];
+            u0c = Y2[j] - c0;
+            u1c = Y2[ld + j] - c1;
+            u1m = Y2[ld + j - 1] - U[ld + j - 1];
+            u1p = Y2[ld + j + 1] - U[ld + j + 1];
+            q0 = (Y2[j - 1] - U[j - 1]) - (Y2[j + 1] - U[j + 1]);
+        }
+        q1 = u1m - u1p;
+        const float chs = ldg(v.Yv(Y_CHS) + j);
+        float y = lo;
+        auto point = [&](const row &r, int t) {
+            const float q2 = r.um - r.up, mix = q0 - q2;
+            float f;
+            if constexpr (KIND == 1) {
+                f = fma_x(r.w[0], mix, mul_x(r.w[1], u0c));
+                f = fma_x(r.w[2], u1m, f);
+                f = fma_x(r.w[3], u1c, f);
+                f = fma_x(r.w[4], u1p, f);
+                f = fma_x(r.w[5], r.uc, f);
+            } else {
+                if constexpr (hv) {
+                    f = fma_x(r.la, y10, mul_x(r.w[0], y11));
+                    f = fma_x(r.w[1], r.y1, f);
+                } else {
+                    f = fma_x(r.la, c0, mul_x(r.w[0], c1));
+                    f = fma_x(r.w[1], r.uu, f);
+                    f = fma_x(r.w[3], y11, f);
+                }
+                f = fma_x(r.w[2], mix, f);
+                if constexpr (xt) {
+                    f = fma_x(r.w[4], u0c, f);
+                    f = fma_x(r.w[5], u1c, f);
+                    f = fma_x(r.w[6], r.uc, f);
+                    f = fma_x(r.w[7], u1m, f);
+                    f = fma_x(r.w[8], u1p, f);
+                }
+                c0 = c1; c1 = r.uu;
+                y10 = y11; y11 = r.y1;
+            }
+            y = fma_x(-r.la, y, f);
+            if (t == e) y = fma_x(-chs, hi, y);
+            Y[t * ld + j] = y;
+            u0c = u1c; u1c = r.uc;
+            u1m = r.um; u1p = r.up;
+            q0 = q1; q1 = q2;
+        };
+        row ra = load(1), rb = load(min(2, e));
+        for (int t = 1; t <= e; t += 2) {
+            const row na = load(min(t + 2, e));
+            point(ra, t);
+            ra = na;
+            if (t + 1 <= e) {
+                const row nb = load(min(t + 3, e));
+                point(rb, t + 1);
+                rb = nb;
+            }
+        }
+        float x = y, yb[FK], gb[FK], yn[FK], gn[FK];
+        auto block = [&](int t, float *yo, float *go) {
+#pragma unroll
+            for (int z = 0; z < FK; ++z) {
+                const int r = max(t - z, 1);
+                yo[z] = Y[r * ld + j];
+                go[z] = ldg(v.S(SL_G, r, j));
+            }
+        };
+        block(e - 1, yb, gb);
+        for (int t = e - 1; t >= 1; t -= FK) {
+            block(t - FK, yn, gn);
+#pragma unroll
+            for (int z = 0; z < FK; ++z) {
+                if (t - z >= 1) {
+                    x = fma_x(-gb[z], x, yb[z]);
+                    Y[(t - z) * ld + j] = x;
+                }
+                yb[z] = yn[z];
+                gb[z] = gn[z];
+            }
         }
         Y[j] = lo;
-        Y[(long long)(nx - 1) * ny + j] = hi;
+        Y[last + j] = hi;
     }
 }
 
@@ -499,46 +544,103 @@ template <typename F> __device__ __forceinline__ void with_scheme(int scheme, F 
     }
 }
 
-// v-line sweep: line i reads row i of `in` (t-1, t, t+1) and `inh` (t); tables are [t][i].
-// v_line_fwd: right-hand side and forward recurrence over t0..t1 from y = y_{t0-1}.
-template <typename T>
-__device__ __forceinline__ T v_line_fwd(const inst_view<T> &v, const T *__restrict__ in, const T *__restrict__ inh,
-                                        T *__restrict__ out, int i, int t0, int t1, T y, T hi)
+// v-line sweep: line i reads row i of `in` (t-1, t, t+1) and `inh` (t); tables are [t][slot][i].  A lane walks
+// its row eight columns at a time (256-bit loads and stores, rows padded to a multiple of eight: whole
+// 32-byte sectors; with half of a sector per access a full GPU ran at half the speed), the next
+// columns and four columns of tables ahead.
+__device__ __forceinline__ void ldv(const float *p, float *o)
 {
-    const int nx = v.nx, ny = v.ny, e = v.e_v;
-    const long long row = (long long)i * ny;
-    T a0 = in[row + t0 - 1], a1 = in[row + t0];
-#pragma unroll 4
-    for (int t = t0; t <= t1; ++t) {
-        const long long ot = (long long)t * nx + i;
-        const T a2 = in[row + t + 1];
-        y = v_point<T>(ldg(v.Vt(VL_LA) + ot), ldg(v.Vt(VL_VC) + ot), ldg(v.Vt(VL_VN) + ot), ldg(v.Vt(VL_IB) + ot), a0,
-                       a1, a2, inh[row + t], y);
-        if (t == e) y = fma_x(-ldg(v.X(X_CHV) + i), hi, y);
-        out[row + t] = y;
-        a0 = a1; a1 = a2;
-    }
-    return y;
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(o[0]), "=f"(o[1]), "=f"(o[2]), "=f"(o[3]), "=f"(o[4]), "=f"(o[5]), "=f"(o[6]), "=f"(o[7])
+                 : "l"(p));
 }
-
-template <typename T>
-__device__ __forceinline__ void v_stage(const inst_view<T> &v, const T *__restrict__ in, const T *__restrict__ inh,
-                                        const T *__restrict__ sb0, T *__restrict__ out, int l0, int ls)
+__device__ __forceinline__ void stv(float *p, const float *o)
 {
-    const int nx = v.nx, ny = v.ny, e = v.e_v;
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(o[0]), "f"(o[1]), "f"(o[2]), "f"(o[3]), "f"(o[4]),
+                 "f"(o[5]), "f"(o[6]), "f"(o[7])
+                 : "memory");
+}
+__device__ __forceinline__ void v_stage(const inst_view<float> &v, const float *in, const float *inh, const float *sb0, float *out, int l0, int ls)
+{
+    const int nx = v.nx, ny = v.ny, ld = v.ld, e = v.e_v;
+    struct cols {
+        float a[8], h[8];
+    };
+    struct tabs {
+        float la[4], vc[4], vn[4], ib[4];
+    };
+    struct bbk {
+        float y[8], g[8];
+    };
     for (int i = 1 + l0; i <= nx - 2; i += ls) {
-        const int ii = ldg(v.imap() + i);
-        const T lo = sb0[ii];
-        const T hi = ldg(v.X(X_VHI) + ii);
-        const long long row = (long long)i * ny;
-        T x = v_line_fwd<T>(v, in, inh, out, i, 1, e, lo, hi);
-#pragma unroll 4
-        for (int t = e - 1; t >= 1; --t) {
-            x = fma_x(-ldg(v.Vt(VL_G) + (long long)t * nx + i), x, out[row + t]);
-            out[row + t] = x;
+        const int ii = ldg(v.imap() + i), row = i * ld;
+        const float lo = sb0[ii], hi = ldg(v.X(X_VHI) + ii), chv = ldg(v.X(X_CHV) + i);
+        auto columns = [&](int t) -> cols { // columns t .. t + 7
+            cols b;
+            const int at = row + min(t, ld - 8);
+            ldv(in + at, b.a);
+            ldv(inh + at, b.h);
+            return b;
+        };
+        auto tables = [&](int t) -> tabs { // of columns t .. t + 3
+            tabs b;
+#pragma unroll
+            for (int z = 0; z < 4; ++z) {
+                const int c = min(max(t + z, 1), e);
+                b.la[z] = ldg(v.Vt(VL_LA, c, i));
+                b.vc[z] = ldg(v.Vt(VL_VC, c, i));
+                b.vn[z] = ldg(v.Vt(VL_VN, c, i));
+                b.ib[z] = ldg(v.Vt(VL_IB, c, i));
+            }
+            return b;
+        };
+        float y = lo, a0 = 0.0f;
+        cols b = columns(0);
+        tabs q = tables(0);
+        for (int t = 0; t <= e; t += 8) {
+            const cols nb = columns(t + 8);
+            float o[8];
+#pragma unroll
+            for (int h = 0; h < 8; h += 4) {
+                const tabs nq = tables(t + h + 4);
+#pragma unroll
+                for (int z = 0; z < 4; ++z) {
+                    const int w = h + z, c = t + w;
+                    const float a2 = w < 7 ? b.a[w < 7 ? w + 1 : 0] : nb.a[0];
+                    if (c >= 1 && c <= e) {
+                        y = v_point<float>(q.la[z], q.vc[z], q.vn[z], q.ib[z], a0, b.a[w], a2, b.h[w], y);
+                        if (c == e) y = fma_x(-chv, hi, y);
+                    }
+                    o[w] = y;
+                    a0 = b.a[w];
+                }
+                q = nq;
+            }
+            stv(out + row + t, o);
+            b = nb;
         }
-        out[row] = lo;
-        out[row + ny - 1] = hi;
+        float x = y;
+        auto back = [&](int t) -> bbk {
+            bbk k;
+            ldv(out + row + max(t, 0), k.y);
+#pragma unroll
+            for (int z = 0; z < 8; ++z) k.g[z] = ldg(v.Vt(VL_G, min(max(t + z, 1), e), i));
+            return k;
+        };
+        const int tl = (ny - 1) / 8 * 8;
+        bbk k = back(tl);
+        for (int t = tl; t >= 0; t -= 8) {
+            const bbk nk = back(t - 8);
+            float o[8];
+#pragma unroll
+            for (int z = 7; z >= 0; --z) {
+                const int c = t + z;
+                if (c >= 1 && c < e) x = fma_x(-k.g[z], x, k.y[z]);
+                o[z] = c >= 1 && c <= e ? x : c == 0 ? lo : c == ny - 1 ? hi : 0.0f;
+            }
+            stv(out + row + t, o);
+            k = nk;
+        }
     }
 }
 
@@ -552,6 +654,10 @@ template <typename T> __device__ __forceinline__ inst_view<T> make_view(const bp
     v.e_s = d.nx - 2;
     v.e_v = d.ny - 2;
     v.o2 = d.o2;
+    v.so = d.o2 * s_slots<T>();
+    v.vo = d.o2 * v_slots<T>();
+    v.sl = d.ld * s_slots<T>();
+    v.vl = d.nx * v_slots<T>();
     v.ox = d.ox;
     v.oy = d.oy;
     return v;
@@ -560,35 +666,35 @@ template <typename T> __device__ __forceinline__ inst_view<T> make_view(const bp
 #include "adi_delta.cuh"
 
 // One time step U -> Vn of scheme SCH with stage outputs in Y1, Y2, Y3; ends with a group barrier.
-template <typename T, int SCH>
-__device__ __forceinline__ void fwd_step(const inst_view<T> &v, const T *U, T *Y1, T *Y2, T *Y3, T *Vn, T *sb0,
+template <int SCH>
+__device__ __forceinline__ void fwd_step(const inst_view<float> &v, const float *U, float *Y1, float *Y2, float *Y3, float *Vn, float *sb0,
                                          double bnc, const grp &g)
 {
     const int l0 = g.t, ls = g.n;
-    b1_stage<T>(v, U, sb0, bnc, l0, ls);
-    s_stage<T, 1, SCH>(v, U, nullptr, nullptr, Y1, l0, ls);
+    b1_stage<float>(v, U, sb0, bnc, l0, ls);
+    s_stage<1, SCH>(v, U, nullptr, nullptr, Y1, l0, ls);
     g.sync();
     if constexpr (SCH == LSS_ADI_DOUGLAS_RACHFORD) {
-        v_stage<T>(v, U, Y1, sb0, Vn, l0, ls);
+        v_stage(v, U, Y1, sb0, Vn, l0, ls);
     } else {
-        v_stage<T>(v, U, Y1, sb0, Y2, l0, ls);
+        v_stage(v, U, Y1, sb0, Y2, l0, ls);
         g.sync();
-        s_stage<T, 2, SCH>(v, U, Y1, Y2, Y3, l0, ls);
+        s_stage<2, SCH>(v, U, Y1, Y2, Y3, l0, ls);
         g.sync();
         if constexpr (SCH == LSS_ADI_HUNDSDORFER_VERWER)
-            v_stage<T>(v, Y2, Y3, sb0, Vn, l0, ls);
+            v_stage(v, Y2, Y3, sb0, Vn, l0, ls);
         else
-            v_stage<T>(v, U, Y3, sb0, Vn, l0, ls);
+            v_stage(v, U, Y3, sb0, Vn, l0, ls);
     }
     g.sync();
-    b2_stage<T>(v, Vn, l0, ls);
+    b2_stage<float>(v, Vn, l0, ls);
     g.sync();
 }
 
 // Persistent forward kernel of the instances of scheme SCH: CTAs of 4 warps split into groups
 // (the layout word of the CTA), each group pulling instances of its class (warps per instance)
 // from the class counter.  Register budget 128 per thread in FP64 (4 CTAs per SM: the sweeps hold
-// the rows that they load ahead), 64 in FP32 (8 CTAs).
+// the rows that they load ahead; FP32, 768 uneven calls: 64.7 ms, 80 and 138 ms with five and six).
 constexpr int BATCH_CTA = 32 * MAX_GROUP_WARPS;
 
 // value at (eval_s, eval_v), corner o of its cell
@@ -604,12 +710,15 @@ template <typename T> __device__ __forceinline__ void load_payoff(const bparams<
     for (int i = g.t / 32; i < d.nx; i += g.n / 32)
         for (int j = g.t & 31; j < d.ny; j += 32) U[i * d.ld + j] = p.payoff[d.op + (long long)i * d.ny + j];
 }
+#ifndef LSS_FWD_MIN_CTAS_F32
+#define LSS_FWD_MIN_CTAS_F32 4
+#endif
 #ifndef LSS_FWD_MIN_CTAS
 #define LSS_FWD_MIN_CTAS 4
 #endif
 
 template <typename T, int SCH>
-__global__ void __launch_bounds__(BATCH_CTA, sizeof(T) == 8 ? LSS_FWD_MIN_CTAS : 8) k_batch_forward(const __grid_constant__ bparams<T> p)
+__global__ void __launch_bounds__(BATCH_CTA, sizeof(T) == 8 ? LSS_FWD_MIN_CTAS : LSS_FWD_MIN_CTAS_F32) k_batch_forward(const __grid_constant__ bparams<T> p)
 {
     __shared__ int s_idx[MAX_GROUP_WARPS];
     __shared__ int s_bad[MAX_GROUP_WARPS];
@@ -625,13 +734,11 @@ __global__ void __launch_bounds__(BATCH_CTA, sizeof(T) == 8 ? LSS_FWD_MIN_CTAS :
         const inst_view<T> v = make_view(p, d);
         T *U = p.U + d.o2, *Vn = p.V + d.o2, *Y1 = p.Y1 + d.o2, *Y2 = p.Y2 + d.o2, *Y3 = p.Y3 + d.o2;
         T *sb0 = p.B0 + d.ox;
-        if constexpr (sizeof(T) == 8) {
-            load_payoff(p, d, U, g);
-            g.sync();
-        }
+        load_payoff(p, d, U, g);
+        g.sync();
         for (int step = 0; step < d.steps; ++step) {
             if constexpr (sizeof(T) == 8) delta_step<SCH>(v, d, U, Y1, Y2, Y3, Vn, sb0, g);
-            else fwd_step<T, SCH>(v, U, Y1, Y2, Y3, Vn, sb0, d.bnc, g);
+            else fwd_step<SCH>(v, U, Y1, Y2, Y3, Vn, sb0, d.bnc, g);
             T *tmp = U;
             U = Vn;
             Vn = tmp;
@@ -791,7 +898,7 @@ __global__ void k_wide_s(const __grid_constant__ bparams<T> p, const T *U, const
     const inst_view<T> v = make_view(p, d);
     with_scheme(d.scheme, [&](auto sch) {
         if constexpr (sizeof(T) == 8) ds_stage<KIND, decltype(sch)::value>(v, d, U, KIND == 1 ? U : Y2, Y1, Y, gtid(), gstride());
-        else s_stage<T, KIND, decltype(sch)::value>(v, U, Y1, Y2, Y, gtid(), gstride());
+        else s_stage<KIND, decltype(sch)::value>(v, U, Y1, Y2, Y, gtid(), gstride());
     });
 }
 // the v stage after the S stage with result `s` (LAST: the step's last one)
@@ -801,7 +908,7 @@ __global__ void k_wide_v(const __grid_constant__ bparams<T> p, const T *U, const
     const bdesc d = p.desc[0];
     const inst_view<T> v = make_view(p, d);
     const bool hv = LAST && d.scheme == LSS_ADI_HUNDSDORFER_VERWER;
-    if constexpr (sizeof(T) == 4) v_stage<T>(v, hv ? Y2 : U, s, b0, out, gtid(), gstride());
+    if constexpr (sizeof(T) == 4) v_stage(v, hv ? Y2 : U, s, b0, out, gtid(), gstride());
     else if constexpr (!LAST) dv_stage<V_FIRST>(v, U, s, nullptr, nullptr, b0, out, gtid(), gstride());
     else if (hv) dv_stage<V_LAST_HV>(v, U, Y1, s, Y2, b0, out, gtid(), gstride());
     else dv_stage<V_LAST>(v, U, s, nullptr, nullptr, b0, out, gtid(), gstride());
@@ -831,7 +938,7 @@ template <typename T> __global__ void k_wide_finish(const __grid_constant__ bpar
     }
 }
 
-static __global__ void k_setup_s_delta(setup_params sp, double *S0, long long stride)
+static __global__ void k_setup_s_delta(setup_params sp, double *S0)
 {
     const long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (g >= sp.total_lines) return;
@@ -852,20 +959,20 @@ static __global__ void k_setup_s_delta(setup_params sp, double *S0, long long st
         const double a = -th * M, b = 1.0 + th * Z, c = -th * P;
         const double ib = 1.0 / fma(-a, gam, b);
         gam = c * ib;
-        double *s = S0 + o;
-        s[DS_LA * stride] = a * ib;
-        s[DS_G * stride] = gam;
-        s[DS_WG * stride] = gm * C * ib;
-        s[DS_WW * stride] = M * ib;
-        s[DS_WS * stride] = Mt * ib;
-        s[DS_WQ * stride] = ((M + P - Z) - W) * ib;
-        s[DS_WC * stride] = -(Z + W) * ib;
-        s[DS_WN * stride] = Pt * ib;
-        s[DS_WE * stride] = P * ib;
-        s[DS_IB * stride] = ib;
+        double *s = S0 + d.o2 * DS_COUNT + (long long)t * DS_COUNT * ld + j;
+        s[DS_LA * ld] = a * ib;
+        s[DS_G * ld] = gam;
+        s[DS_WG * ld] = gm * C * ib;
+        s[DS_WW * ld] = M * ib;
+        s[DS_WS * ld] = Mt * ib;
+        s[DS_WQ * ld] = ((M + P - Z) - W) * ib;
+        s[DS_WC * ld] = -(Z + W) * ib;
+        s[DS_WN * ld] = Pt * ib;
+        s[DS_WE * ld] = P * ib;
+        s[DS_IB * ld] = ib;
     }
 }
-static __global__ void k_setup_v_delta(setup_params sp, double *V0, long long stride)
+static __global__ void k_setup_v_delta(setup_params sp, double *V0)
 {
     const long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (g >= sp.total_lines) return;
@@ -876,18 +983,19 @@ static __global__ void k_setup_v_delta(setup_params sp, double *V0, long long st
     const double th = sp.scal[3 * inst];
     const long long N = sp.total_n, row = d.o2 + (long long)i * d.ld;
     const double *Mt = sp.base + 3 * N + row, *Pt = sp.base + 4 * N + row, *W = sp.base + 5 * N + row;
-    double *L = V0 + d.o2 + i, *U = L + stride, *IB = U + stride;
+    double *L = V0 + d.o2 * DV_COUNT + i, *U = L + DV_U * nx, *IB = L + DV_IB * nx;
+    const long long row_t = (long long)DV_COUNT * nx;
     double ib = 0.0, cp = 0.0;
     for (int t = 1; t <= e; ++t) {
         const double a = -th * Mt[t], b = 1.0 + th * W[t], c = -th * Pt[t];
         const double l = t == 1 ? a : a * ib;
         ib = 1.0 / (t == 1 ? b : fma(-l, cp, b));
-        L[(long long)t * nx] = l;
-        IB[(long long)t * nx] = ib;
-        if (t > 1) U[(long long)(t - 1) * nx] = cp * ib;
+        L[t * row_t] = l;
+        IB[t * row_t] = ib;
+        if (t > 1) U[(t - 1) * row_t] = cp * ib;
         cp = c;
     }
-    U[(long long)e * nx] = cp;
+    U[e * row_t] = cp;
 }
 
 // ------------------------------------------------------------------------------------------
@@ -896,8 +1004,8 @@ static __global__ void k_setup_v_delta(setup_params sp, double *V0, long long st
 template <typename T> struct batch_typed {
     // line tables: delta form (FP64) or the stages on Y1, Y2, Y3 (FP32)
     static constexpr bool DELTA = std::is_same<T, double>::value;
-    static constexpr int S_SLOTS = DELTA ? static_cast<int>(DS_COUNT) : static_cast<int>(SL_COUNT);
-    static constexpr int V_SLOTS = DELTA ? static_cast<int>(DV_COUNT) : static_cast<int>(VL_COUNT);
+    static constexpr int S_SLOTS = s_slots<T>(), V_SLOTS = v_slots<T>();
+    static constexpr int PITCH = 32 / sizeof(T); // rows of the state start on 32-byte sectors
     int count = 0;
     std::vector<bdesc> desc;
     std::vector<int> order;
@@ -958,8 +1066,8 @@ template <typename T> struct batch_typed {
         p.Y1 = state.p + 2 * total_n;
         p.Y2 = state.p + 3 * total_n;
         p.Y3 = state.p + 4 * total_n;
-        for (int s = 0; s < S_SLOTS; ++s) p.S[s] = stab.p + s * total_n;
-        for (int s = 0; s < V_SLOTS; ++s) p.Vt[s] = vtab.p + s * total_n;
+        p.S = stab.p;
+        p.Vt = vtab.p;
         for (int s = 0; s < X_COUNT; ++s) p.X[s] = xarena.p + s * total_x;
         for (int s = 0; s < Y_COUNT; ++s) p.Yv[s] = yarena.p + s * total_y;
         p.imap = d_imap.p;
@@ -1020,7 +1128,7 @@ template <typename T> int batch_typed<T>::create(const lss_adi_problem *ps, int 
         desc[k].ny = ps[k].ny;
         desc[k].steps = ps[k].nt - 1;
         desc[k].scheme = ps[k].scheme;
-        desc[k].ld = DELTA ? (ps[k].ny + 3) / 4 * 4 : ps[k].ny;
+        desc[k].ld = (ps[k].ny + PITCH - 1) / PITCH * PITCH;
         desc[k].o2 = on;
         desc[k].op = of;
         desc[k].ox = static_cast<int>(ox);
@@ -1209,16 +1317,16 @@ template <typename T> int batch_typed<T>::create(const lss_adi_problem *ps, int 
         for (int k = 0; k < n; ++k) { ls[k] = acc; acc += desc[k].ny - 2; }
         LSS_CUDA_TRY(d_ls.upload(ls.data(), n), "batch: line offsets");
         sp.total_lines = acc;
-        if constexpr (DELTA) k_setup_s_delta<<<grid_for(acc, 128), 128>>>(sp, stab.p, total_n);
-        else k_setup_s_lines<T><<<grid_for(acc, 128), 128>>>(sp, stab.p, total_n, yarena.p + Y_CHS * total_y);
+        if constexpr (DELTA) k_setup_s_delta<<<grid_for(acc, 128), 128>>>(sp, stab.p);
+        else k_setup_s_lines<T><<<grid_for(acc, 128), 128>>>(sp, stab.p, yarena.p + Y_CHS * total_y);
         LSS_CUDA_TRY(cudaGetLastError(), "batch: launching S-line set-up");
         LSS_CUDA_TRY(cudaDeviceSynchronize(), "batch: S-line set-up");
         acc = 0;
         for (int k = 0; k < n; ++k) { ls[k] = acc; acc += desc[k].nx - 2; }
         LSS_CUDA_TRY(d_ls.upload(ls.data(), n), "batch: line offsets");
         sp.total_lines = acc;
-        if constexpr (DELTA) k_setup_v_delta<<<grid_for(acc, 128), 128>>>(sp, vtab.p, total_n);
-        else k_setup_v_lines<T><<<grid_for(acc, 128), 128>>>(sp, vtab.p, total_n, xarena.p + X_CHV * total_x);
+        if constexpr (DELTA) k_setup_v_delta<<<grid_for(acc, 128), 128>>>(sp, vtab.p);
+        else k_setup_v_lines<T><<<grid_for(acc, 128), 128>>>(sp, vtab.p, xarena.p + X_CHV * total_x);
         LSS_CUDA_TRY(cudaGetLastError(), "batch: launching v-line set-up");
         LSS_CUDA_TRY(cudaDeviceSynchronize(), "batch: v-line set-up");
     }
@@ -1486,9 +1594,6 @@ template <typename T> int batch_typed<T>::enqueue(int mode, cudaStream_t s)
     if (mode == 1) {
         rc = launch_fwdadj(s);
     } else {
-        if (!DELTA) // (the FP64 kernels read the initial conditions themselves)
-            LSS_CUDA_TRY(cudaMemcpyAsync(state.p, d_payoff.p, total_n * sizeof(T), cudaMemcpyDeviceToDevice, s),
-                         "batch: initial state");
         rc = launch_forward(s);
     }
     return rc;

@@ -33,9 +33,6 @@ __device__ __forceinline__ void st4(double *p, const double *o)
     asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(o[0]), "d"(o[1]), "d"(o[2]), "d"(o[3]) : "memory");
 }
 
-// slots of the FP64 line tables: S lines [t][j] (pitch ld), v lines [t][i] (pitch nx)
-enum { DS_LA = 0, DS_G, DS_WG, DS_WW, DS_WS, DS_WQ, DS_WN, DS_WE, DS_IB, DS_WC, DS_COUNT };
-enum { DV_L = 0, DV_U, DV_IB, DV_COUNT };
 enum { V_FIRST = 0, V_LAST = 1, V_LAST_HV = 2 };
 
 constexpr int BK = 8; // rows of a block of the one-instruction passes
@@ -89,16 +86,16 @@ __device__ __forceinline__ void ds_stage(const inst_view<double> &v, const bdesc
         auto load = [&](int t) -> row {
             const int o = t * ld + j;
             row r;
-            r.la = __ldg(v.S(DS_LA) + o);
-            r.wg = __ldg(v.S(DS_WG) + o);
+            r.la = __ldg(v.S(DS_LA, t, j));
+            r.wg = __ldg(v.S(DS_WG, t, j));
             if constexpr (six) {
-                r.ww = __ldg(v.S(DS_WW) + o);
-                r.ws = __ldg(v.S(DS_WS) + o);
-                r.wc = __ldg(v.S(KIND == 2 && mcs ? DS_WC : DS_WQ) + o);
-                r.wn = __ldg(v.S(DS_WN) + o);
-                r.we = __ldg(v.S(DS_WE) + o);
+                r.ww = __ldg(v.S(DS_WW, t, j));
+                r.ws = __ldg(v.S(DS_WS, t, j));
+                r.wc = __ldg(v.S(KIND == 2 && mcs ? DS_WC : DS_WQ, t, j));
+                r.wn = __ldg(v.S(DS_WN, t, j));
+                r.we = __ldg(v.S(DS_WE, t, j));
             }
-            if constexpr (KIND == 2) r.ib = __ldg(v.S(DS_IB) + o);
+            if constexpr (KIND == 2) r.ib = __ldg(v.S(DS_IB, t, j));
             if constexpr (KIND == 2 && !hv) r.d1 = D1[o];
             r.am = A[o + ld - 1];
             r.ac = A[o + ld];
@@ -155,9 +152,9 @@ __device__ __forceinline__ void ds_stage(const inst_view<double> &v, const bdesc
         auto block = [&](int t, double *yo, double *go) {
 #pragma unroll
             for (int z = 0; z < BK; ++z) {
-                const int o = max(t - z, 1) * ld + j;
-                yo[z] = Y[o];
-                go[z] = __ldg(v.S(DS_G) + o);
+                const int r = max(t - z, 1);
+                yo[z] = Y[r * ld + j];
+                go[z] = __ldg(v.S(DS_G, r, j));
             }
         };
         block(e, yb, gb);
@@ -203,7 +200,7 @@ __device__ __forceinline__ void dv_stage(const inst_view<double> &v, const doubl
                 }
             }
 #pragma unroll
-            for (int z = 0; z < BK; ++z) ll[z] = __ldg(v.Vt(DV_L) + min(t + z, e) * nx + i);
+            for (int z = 0; z < BK; ++z) ll[z] = __ldg(v.Vt(DV_L, min(t + z, e), i));
         };
         double y = d0;
         block(0, db, lb);
@@ -241,9 +238,9 @@ __device__ __forceinline__ void dv_stage(const inst_view<double> &v, const doubl
             }
 #pragma unroll
             for (int z = 0; z < 4; ++z) {
-                const int o = min(max(t, 0) + z, ny - 1) * nx + i;
-                b.u[z] = __ldg(v.Vt(DV_U) + o);
-                b.ib[z] = __ldg(v.Vt(DV_IB) + o);
+                const int c = min(max(t, 0) + z, ny - 1);
+                b.u[z] = __ldg(v.Vt(DV_U, c, i));
+                b.ib[z] = __ldg(v.Vt(DV_IB, c, i));
             }
             return b;
         };
@@ -316,8 +313,8 @@ __device__ __forceinline__ void da_v(const inst_view<double> &v, const double *X
             ld4(XB + row + min(t, ld - 4), b.x);
 #pragma unroll
             for (int z = 0; z < 4; ++z) {
-                b.ib[z] = __ldg(v.Vt(DV_IB) + min(t + z, ny - 1) * nx + i);
-                b.u[z] = __ldg(v.Vt(DV_U) + min(max(t + z - 1, 0), ny - 1) * nx + i);
+                b.ib[z] = __ldg(v.Vt(DV_IB, min(t + z, ny - 1), i));
+                b.u[z] = __ldg(v.Vt(DV_U, min(max(t + z - 1, 0), ny - 1), i));
             }
             return b;
         };
@@ -343,7 +340,7 @@ __device__ __forceinline__ void da_v(const inst_view<double> &v, const double *X
 #pragma unroll
             for (int z = 0; z < BK; z += 4) ld4(DB + row + min(max(t + z, 0), ld - 4), zz + z);
 #pragma unroll
-            for (int z = 0; z < BK; ++z) ll[z] = __ldg(v.Vt(DV_L) + min(max(t + z + 1, 0), ny - 1) * nx + i);
+            for (int z = 0; z < BK; ++z) ll[z] = __ldg(v.Vt(DV_L, min(max(t + z + 1, 0), ny - 1), i));
         };
         const int tl = (ny - 1) / BK * BK;
         back(tl, zb, lb);
@@ -395,10 +392,10 @@ __device__ __forceinline__ void da_s(const inst_view<double> &v, const bdesc &d,
         auto block = [&](int t, double *xo, double *go) {
 #pragma unroll
             for (int k = 0; k < BK; ++k) {
-                const int o = min(t + k, e) * ld + j;
+                const int r = min(t + k, e), o = r * ld + j;
                 xo[k] = XB[o];
                 if constexpr (first_v) xo[k] += DV[o];
-                go[k] = __ldg(v.S(DS_G) + o - ld);
+                go[k] = __ldg(v.S(DS_G, r - 1, j));
             }
         };
         block(1, xb, gb);
@@ -414,7 +411,7 @@ __device__ __forceinline__ void da_s(const inst_view<double> &v, const bdesc &d,
                 gb[k] = gn[k];
             }
         }
-        const double hib = -__ldg(v.S(DS_G) + e * ld + j) * z;
+        const double hib = -__ldg(v.S(DS_G, e, j)) * z;
         // w_t = z_t - la_{t+1} w_{t+1} with the sums, rows t+1, t, t-1 of X and Y in a window
         struct row {
             double z, la, ib, xc, ss, sn, y, m, x0, x1, x2; // z, la_{t+1}, ib, m, x of row t; X, Y of row t-1
@@ -423,8 +420,8 @@ __device__ __forceinline__ void da_s(const inst_view<double> &v, const bdesc &d,
             const int o = t * ld + j, ol = o - ld;
             row r;
             r.z = FB[o];
-            r.la = __ldg(v.S(DS_LA) + o + ld); // the table's row nx-1 is zero
-            r.ib = __ldg(v.S(DS_IB) + o);
+            r.la = __ldg(v.S(DS_LA, t + 1, j)); // the table's row nx-1 is zero
+            r.ib = __ldg(v.S(DS_IB, t, j));
             r.xc = X[ol];
             r.ss = X[ol - 1];
             r.sn = X[ol + 1];
@@ -483,7 +480,7 @@ __device__ __forceinline__ void da_s(const inst_view<double> &v, const bdesc &d,
             ddh = ddc; ddc = ddl;
             ss = r.ss;
         }
-        const double lob = -__ldg(v.S(DS_LA) + ld + j) * w;
+        const double lob = -__ldg(v.S(DS_LA, 1, j)) * w;
         if constexpr (KIND == 2 && hv) { // E's boundary values are U's rows 0 and nx-1
             VB[j] += lob;
             VB[last + j] += hib;
@@ -532,21 +529,21 @@ __device__ __forceinline__ void da_gather(const inst_view<double> &v, const bdes
     for (int q = l0; q < ny; q += ls) {
         const bool lf = q >= 1, rt = q + 1 <= ny - 1;
         auto load = [&](int r) -> raw {
-            const int o = min(max(r, 0), nx - 1) * ld + q;
+            const int t = min(max(r, 0), nx - 1), o = t * ld + q;
             raw a;
             a.f0 = FB[o];
             a.fm = lf ? FB[o - 1] : 0.0;
             a.fp = rt ? FB[o + 1] : 0.0;
-            a.gm = lf ? __ldg(v.S(DS_WG) + o - 1) : 0.0;
-            a.gp = rt ? __ldg(v.S(DS_WG) + o + 1) : 0.0;
+            a.gm = lf ? __ldg(v.S(DS_WG, t, q - 1)) : 0.0;
+            a.gp = rt ? __ldg(v.S(DS_WG, t, q + 1)) : 0.0;
             if constexpr (six) {
-                a.wd = __ldg(v.S(DS_WW) + o);
-                a.wu = __ldg(v.S(DS_WE) + o);
-                a.wm = __ldg(v.S(DS_WC) + o);
-                a.wr = rt ? __ldg(v.S(DS_WS) + o + 1) : 0.0;
-                a.wl = lf ? __ldg(v.S(DS_WN) + o - 1) : 0.0;
+                a.wd = __ldg(v.S(DS_WW, t, q));
+                a.wu = __ldg(v.S(DS_WE, t, q));
+                a.wm = __ldg(v.S(DS_WC, t, q));
+                a.wr = rt ? __ldg(v.S(DS_WS, t, q + 1)) : 0.0;
+                a.wl = lf ? __ldg(v.S(DS_WN, t, q - 1)) : 0.0;
             }
-            if constexpr (KIND == 2 && hv) a.ib = __ldg(v.S(DS_IB) + o);
+            if constexpr (KIND == 2 && hv) a.ib = __ldg(v.S(DS_IB, t, q));
             if constexpr (KIND == 1 || hv) a.vb = VB[o];
             return a;
         };
