@@ -693,8 +693,8 @@ __device__ __forceinline__ void fwd_step(const inst_view<float> &v, const float 
 
 // Persistent forward kernel of the instances of scheme SCH: CTAs of 4 warps split into groups
 // (the layout word of the CTA), each group pulling instances of its class (warps per instance)
-// from the class counter.  Register budget 128 per thread in FP64 (4 CTAs per SM: the sweeps hold
-// the rows that they load ahead; FP32, 768 uneven calls: 64.7 ms, 80 and 138 ms with five and six).
+// from the class counter.  FP64: two CTAs per SM, whose threads hold the rows that the sweeps load ahead
+// (adi_delta.cuh).  FP32: four (768 uneven calls: 64.7 ms; 80 and 138 ms with five and six).
 constexpr int BATCH_CTA = 32 * MAX_GROUP_WARPS;
 
 // value at (eval_s, eval_v), corner o of its cell
@@ -710,15 +710,9 @@ template <typename T> __device__ __forceinline__ void load_payoff(const bparams<
     for (int i = g.t / 32; i < d.nx; i += g.n / 32)
         for (int j = g.t & 31; j < d.ny; j += 32) U[i * d.ld + j] = p.payoff[d.op + (long long)i * d.ny + j];
 }
-#ifndef LSS_FWD_MIN_CTAS_F32
-#define LSS_FWD_MIN_CTAS_F32 4
-#endif
-#ifndef LSS_FWD_MIN_CTAS
-#define LSS_FWD_MIN_CTAS 4
-#endif
 
 template <typename T, int SCH>
-__global__ void __launch_bounds__(BATCH_CTA, sizeof(T) == 8 ? LSS_FWD_MIN_CTAS : LSS_FWD_MIN_CTAS_F32) k_batch_forward(const __grid_constant__ bparams<T> p)
+__global__ void __launch_bounds__(BATCH_CTA, sizeof(T) == 8 ? 2 : 4) k_batch_forward(const __grid_constant__ bparams<T> p)
 {
     __shared__ int s_idx[MAX_GROUP_WARPS];
     __shared__ int s_bad[MAX_GROUP_WARPS];
@@ -767,12 +761,9 @@ __global__ void __launch_bounds__(BATCH_CTA, sizeof(T) == 8 ? LSS_FWD_MIN_CTAS :
 // last segment), followed by the adjoint steps of the segment in reverse order.
 // Results: value, the 5 parameter sensitivities, the final surface (state U arena) and
 // dV/d(initial condition) (state V arena).  A group of w warps works in w consecutive workspace
-// slices.  Register budget 128 per thread (4 CTAs of 4 warps per SM).
-#ifndef LSS_FWDADJ_MIN_CTAS
-#define LSS_FWDADJ_MIN_CTAS 4
-#endif
+// slices.  Two CTAs of 4 warps per SM, as the forward kernel.
 template <int SCH>
-__global__ void __launch_bounds__(BATCH_CTA, LSS_FWDADJ_MIN_CTAS) k_batch_fwdadj(const __grid_constant__ bparams<double> p)
+__global__ void __launch_bounds__(BATCH_CTA, 2) k_batch_fwdadj(const __grid_constant__ bparams<double> p)
 {
     __shared__ int s_idx[MAX_GROUP_WARPS];
     __shared__ int s_bad[MAX_GROUP_WARPS];

@@ -16,11 +16,16 @@
 //
 // What bounds them: an FP64 instruction of a warp takes 64 cycles of its SM sub-partition, whether
 // or not it depends on the one before, so a warp that has its operands in registers saturates its
-// sub-partition alone.  The sweeps therefore load the next rows (S: two, the passes with one
-// instruction per row: eight) before they use the current ones: in-order issue then hides the L2
-// and DRAM latency behind the arithmetic.  The v sweeps walk the rows of the row-major state, a
-// lane per row: they move four columns per access (256-bit loads and stores, rows padded to a
-// multiple of four), 8 L1 wavefronts per column and array instead of 32.
+// sub-partition alone.  A batch's time is that of its largest instances while the GPU is full: their
+// operands come from HBM (about 1 us), which the rows in flight of one warp have to cover.  So a thread
+// takes 255 registers (two CTAs per SM) and holds the next rows: five of the right-hand sides, 16 to
+// 32 of the passes with one instruction per row.  1024 uneven calls (Craig-Sneyd, up to 256 x 128):
+// 187 ms; with two and eight rows at 128 registers and four CTAs per SM 245 ms; sensitivities of 768
+// calls 437 against 552 ms (GPU filled with equal 256 x 128 instances alone: 1.75e10 against 1.95e10
+// point-steps/s).  L2 prefetch instructions instead cost more than they gave (257 ms: their issue
+// slots add to the FP64 chain's).  The v sweeps walk the rows of the row-major state, a lane per row:
+// they move four columns per access (256-bit loads and stores, rows padded to a multiple of four),
+// 8 L1 wavefronts per column and array instead of 32.
 #pragma once
 // Included by adi_batched.cu inside namespace lss_gb300, after inst_view.
 
@@ -35,7 +40,9 @@ __device__ __forceinline__ void st4(double *p, const double *o)
 
 enum { V_FIRST = 0, V_LAST = 1, V_LAST_HV = 2 };
 
-constexpr int BK = 8; // rows of a block of the one-instruction passes
+constexpr int AH = 5;  // rows loaded ahead of the right-hand sides
+constexpr int BK = 16; // rows of a block of the one-instruction passes
+constexpr int VB4 = 4; // blocks of four columns loaded ahead of the v lines' scaled passes
 
 // The explicit v = v_lo column and the rows of S_lo and S_max (b1_stage, b2_stage) in the order of
 // adi_wide.cuh: a single instance in relay order has the same bits.
@@ -136,17 +143,20 @@ __device__ __forceinline__ void ds_stage(const inst_view<double> &v, const bdesc
             a1m = r.am; a1p = r.ap;
             q0 = q1; q1 = q2;
         };
-        row ra = load(1), rb = load(min(2, e));
-        for (int t = 1; t <= e; t += 2) {
-            const row na = load(min(t + 2, e));
-            point(ra, t);
-            ra = na;
-            if (t + 1 <= e) {
-                const row nb = load(min(t + 3, e));
-                point(rb, t + 1);
-                rb = nb;
+        row ring[AH];
+#pragma unroll
+        for (int k = 0; k < AH; ++k) ring[k] = load(min(1 + k, e));
+        int t = 1;
+        for (; t + AH - 1 <= e; t += AH)
+#pragma unroll
+            for (int k = 0; k < AH; ++k) {
+                const row next = load(min(t + k + AH, e));
+                point(ring[k], t + k);
+                ring[k] = next;
             }
-        }
+#pragma unroll
+        for (int k = 0; k < AH - 1; ++k)
+            if (t + k <= e) point(ring[k], t + k);
         // back substitution, blocks of BK rows loaded one block ahead
         double x = hi, yb[BK], gb[BK], yn[BK], gn[BK];
         auto block = [&](int t, double *yo, double *go) {
@@ -158,7 +168,7 @@ __device__ __forceinline__ void ds_stage(const inst_view<double> &v, const bdesc
             }
         };
         block(e, yb, gb);
-        for (int t = e; t >= 1; t -= BK) {
+        for (t = e; t >= 1; t -= BK) {
             block(t - BK, yn, gn);
 #pragma unroll
             for (int z = 0; z < BK; ++z) {
@@ -245,24 +255,29 @@ __device__ __forceinline__ void dv_stage(const inst_view<double> &v, const doubl
             return b;
         };
         const int tl = (ny - 1) / 4 * 4;
-        blk b = back(tl), b2 = back(tl - 4);
-        for (int t = tl; t >= 0; t -= 4) {
-            const blk nb = back(t - 8);
-            double o[4];
+        blk ring[VB4];
 #pragma unroll
-            for (int z = 3; z >= 0; --z) {
-                const int c = t + z;
-                if (c >= 1 && c <= e) {
-                    x = fma(-b.u[z], x, b.y[z]);
-                    o[z] = KIND == V_FIRST ? b.ib[z] * x : fma(b.ib[z], x, b.s[z]);
-                } else {
-                    o[z] = c == 0 ? (KIND == V_FIRST ? d0 : lo) : c == ny - 1 ? (KIND == V_FIRST ? dn : hi) : 0.0;
+        for (int k = 0; k < VB4; ++k) ring[k] = back(tl - 4 * k);
+        for (int t0 = tl; t0 >= 0; t0 -= 4 * VB4)
+#pragma unroll
+            for (int k = 0; k < VB4; ++k) {
+                const int t = t0 - 4 * k;
+                if (t < 0) break;
+                const blk nb = back(t - 4 * VB4), b = ring[k];
+                double o[4];
+#pragma unroll
+                for (int z = 3; z >= 0; --z) {
+                    const int c = t + z;
+                    if (c >= 1 && c <= e) {
+                        x = fma(-b.u[z], x, b.y[z]);
+                        o[z] = KIND == V_FIRST ? b.ib[z] * x : fma(b.ib[z], x, b.s[z]);
+                    } else {
+                        o[z] = c == 0 ? (KIND == V_FIRST ? d0 : lo) : c == ny - 1 ? (KIND == V_FIRST ? dn : hi) : 0.0;
+                    }
                 }
+                st4(out + row + t, o);
+                ring[k] = nb;
             }
-            st4(out + row + t, o);
-            b = b2;
-            b2 = nb;
-        }
     }
 }
 
@@ -319,22 +334,27 @@ __device__ __forceinline__ void da_v(const inst_view<double> &v, const double *X
             return b;
         };
         double z_ = 0.0, zn = 0.0, z0 = 0.0;
-        blk b = fwd(0), b2 = fwd(4);
-        for (int t = 0; t < ny; t += 4) {
-            const blk nb = fwd(t + 8);
-            double o[4];
+        blk ring[VB4];
 #pragma unroll
-            for (int z = 0; z < 4; ++z) {
-                const int c = t + z;
-                if (c >= 1 && c <= e) z_ = fma(-b.u[z], z_, b.ib[z] * b.x[z]);
-                if (c == 0) z0 = b.x[z];
-                if (c == ny - 1) zn = fma(-b.u[z], z_, b.x[z]);
-                o[z] = c <= e ? z_ : 0.0;
+        for (int k = 0; k < VB4; ++k) ring[k] = fwd(4 * k);
+        for (int t0 = 0; t0 < ny; t0 += 4 * VB4)
+#pragma unroll
+            for (int k = 0; k < VB4; ++k) {
+                const int t = t0 + 4 * k;
+                if (t >= ny) break;
+                const blk nb = fwd(t + 4 * VB4), b = ring[k];
+                double o[4];
+#pragma unroll
+                for (int z = 0; z < 4; ++z) {
+                    const int c = t + z;
+                    if (c >= 1 && c <= e) z_ = fma(-b.u[z], z_, b.ib[z] * b.x[z]);
+                    if (c == 0) z0 = b.x[z];
+                    if (c == ny - 1) zn = fma(-b.u[z], z_, b.x[z]);
+                    o[z] = c <= e ? z_ : 0.0;
+                }
+                st4(DB + row + t, o);
+                ring[k] = nb;
             }
-            st4(DB + row + t, o);
-            b = b2;
-            b2 = nb;
-        }
         double w = 0.0, zb[BK], lb[BK], zx[BK], lx[BK];
         auto back = [&](int t, double *zz, double *ll) { // columns t .. t + BK - 1; l of the column after
 #pragma unroll
@@ -440,10 +460,11 @@ __device__ __forceinline__ void da_s(const inst_view<double> &v, const bdesc &d,
         double xh = X[last + j], xc = X[last - ld + j], yh = Y[last + j], yc = Y[last - ld + j];
         double ddh = X[last + j - 1] - X[last + j + 1], ss = X[last - ld + j - 1], ddc = ss - X[last - ld + j + 1];
         double w = 0.0;
-        row nr = load(e);
+        row nr = load(e), nr2 = load(max(e - 1, 1));
         for (int t = e; t >= 1; --t) {
             const row r = nr;
-            nr = load(max(t - 1, 1));
+            nr = nr2;
+            nr2 = load(max(t - 2, 1));
             const int o = t * ld + j;
             w = fma(-r.la, w, r.z);
             const double mu = r.ib * w, ddl = r.ss - r.sn;
@@ -584,12 +605,13 @@ __device__ __forceinline__ void da_gather(const inst_view<double> &v, const bdes
             }
         }
         double up_m = 0.0;
-        raw a0 = load(0), an = load(1);
+        raw a0 = load(0), an = load(1), an2 = load(2);
         part pc = parts(a0);
         double vbc = a0.vb;
         for (int r = 0; r < nx; ++r) {
             const raw a = an;
-            an = load(r + 2);
+            an = an2;
+            an2 = load(r + 3);
             part pn;
             if (r + 1 < nx) pn = parts(a);
             else pn.g = pn.dn = pn.up = pn.mid = pn.e = 0.0;
