@@ -32,20 +32,20 @@ METRIC = "grid-point-steps/s, batched fwd+adjoint vs plain path, FP64 \u22641e-1
 BYTES_PER_GPS_FWD = {"dr": 40, "cs": 96, "mcs": 96, "hv": 96}  # algorithmic bytes per grid-point-step (FP64)
 # Figures of one ncu capture each of the batched kernels on the 1024-instance, 40-step case
 # (--count 1024 --max-time-steps 40; forward: --mode fwd; forward + adjoint: --mode fwdadj
-# --workspace-gb 12, whose plan recomputes a fraction CAPTURE_RF = 0.4898 of the steps), per
+# --workspace-gb 12, whose plan recomputes a fraction CAPTURE_RF = 0.2567 of the steps), per
 # grid-point-step, scaled to a launch by the grid-point-steps it processes.  Forward + adjoint
 # is one forward pass, the recomputation of every checkpoint segment but the last (a fraction rf
 # of the steps) and the adjoint steps, so a figure X of it is X_FWD * (1 + rf) + X_ADJ, with X_ADJ
 # what the forward + adjoint capture (at rf = CAPTURE_RF) leaves after its forward passes.
-CAPTURE_RF = 0.4898
+CAPTURE_RF = 0.2567
 # DRAM bytes read + written (dram__bytes_read.sum + dram__bytes_write.sum): k_batch_forward,
 # k_batch_fwdadj
-DRAM_BYTES_FWD = 339.1
-CAPTURE_DRAM_FWDADJ = 1026.9
+DRAM_BYTES_FWD = 293.1
+CAPTURE_DRAM_FWDADJ = 684.6
 DRAM_BYTES_ADJ = CAPTURE_DRAM_FWDADJ - DRAM_BYTES_FWD * (1.0 + CAPTURE_RF)
 # FP64 instructions, thread level (smsp__sass_thread_inst_executed_op_{dfma,dadd,dmul}_pred_on.sum)
-FP64_INSTR_FWD = 32.07
-CAPTURE_FWDADJ = 139.30
+FP64_INSTR_FWD = 23.32
+CAPTURE_FWDADJ = 93.16
 FP64_INSTR_ADJ = CAPTURE_FWDADJ - FP64_INSTR_FWD * (1.0 + CAPTURE_RF)
 
 
@@ -430,7 +430,7 @@ def main():
                    "global_batch": len(problems_all) if args.strong else len(problems) * world,
                    "grid_point_steps_per_gpu": gps,
                    "threads_per_instance": threads,
-                   "l2": f"inputs larger than L2 (line tables {total_n * 23 * 8 / 1e9:.1f} GB streamed every step)",
+                   "l2": f"inputs larger than L2 (line tables {total_n * 13 * 8 / 1e9:.1f} GB streamed every step)",
                    "parallelism": (f"instance sharding x{world} ({'one batch split by cost' if args.strong else 'a batch per rank'})"
                                    if world > 1 else "single GPU")},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,

@@ -124,14 +124,15 @@ typedef struct lss_adi_problem {
  *   solve the same systems, so LSS_ADI_ARITH_FAST (one precomputed factorisation) serves
  *   both and ignores this bit. */
 #define LSS_ADI_OPT_DOUBLE_SWEEP 2
-/* LINE_PER_THREAD: LSS_ADI_ARITH_FAST single instance: solve every line with one thread (the
- *   batched kernel's arithmetic, bit for bit) instead of the autotuned partitioned line
+/* LINE_PER_THREAD: LSS_ADI_ARITH_FAST single instance: solve every line in the order of one thread
+ *   that walks it (the batched kernel's arithmetic, bit for bit) instead of the partitioned line
  *   solves, which cut each line into chunks to occupy the whole GPU on one instance and
  *   differ from it by rounding only. */
 #define LSS_ADI_OPT_LINE_PER_THREAD 4
 /* WIDE_ADJOINT: lss_adi_adjoint runs the forward + adjoint of this instance as one kernel per
- *   stage over the whole GPU (partitioned line solves unless LINE_PER_THREAD) whatever its
- *   size, instead of one warp group of the batched kernel for instances of up to 256 x 160 points. */
+ *   stage over the whole GPU with partitioned line solves whatever its size.  Without it instances
+ *   of up to 256 x 160 points (and every one with LINE_PER_THREAD) run the recurrences in the batched
+ *   kernel's order, which gives the value the bits of the same instance in a batch. */
 #define LSS_ADI_OPT_WIDE_ADJOINT 8
 
 /*
@@ -197,9 +198,9 @@ int lss_adi_forward_graph(lss_adi_handle *h, const void *payoff, void *out_surfa
  * and SABR (the r sensitivity includes the discount factors D(t) inside a and c).  Instances
  * larger than 256 x 160 points, and SABR with r != 0 (whose S-line tables are rebuilt at every
  * step's time), run the adjoint as one kernel per stage over the whole GPU.
- * Checkpoints every `checkpoint_every` steps; 0 = planned: instances of up to 256 x 160 points
- * take the longest interval the workspace allows (at least ceil(sqrt(steps))), larger ones
- * ceil(sqrt(steps)).  Results do not depend on the interval. */
+ * Checkpoints every `checkpoint_every` steps; 0 = planned: the longest interval whose workspace fits
+ * a quarter of the device and half of its free memory (at least ceil(sqrt(steps))).  Results do
+ * not depend on the interval. */
 int lss_adi_adjoint(lss_adi_handle *h, const void *payoff, double *out_value, double *dv_dparams,
                     void *dv_dpayoff, int checkpoint_every, int flags, void *stream);
 
@@ -208,10 +209,9 @@ int lss_adi_grid(const lss_adi_handle *h, void *x, void *y);
 
 /* Partitioned line solves of a LSS_ADI_ARITH_FAST single instance: every S line is cut into
  * s_chunks and every v line into v_chunks pieces solved concurrently (1 = thread per line;
- * at most 128; at least 4 rows per chunk).  0 for either picks it, with the number of lines
- * per CTA, by timing the sweeps (the autotuner lss_adi_create runs by default); a count set
- * here gets the lines per CTA that give every SM a CTA.  Neither changes the arithmetic of a
- * chunk: results depend on the chunk counts at rounding level only.  out_s / out_v (may be NULL) receive the
+ * at most 128; at least 4 rows per chunk).  0 for either picks it by the line length (the rule
+ * lss_adi_create uses: as many chunks of 4 to 16 rows as one CTA holds).  Results depend on the
+ * chunk counts at rounding level only.  out_s / out_v (may be NULL) receive the
  * counts in use.  LSS_ADI_EUNSUPPORTED for handles on the kernel-per-sweep path.  No
  * counterpart in the reference, whose line solves are serial. */
 int lss_adi_line_chunks(lss_adi_handle *h, int s_chunks, int v_chunks, int *out_s, int *out_v, void *stream);

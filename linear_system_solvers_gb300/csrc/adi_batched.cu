@@ -321,10 +321,8 @@ template <typename T> struct inst_view {
 
 template <typename T> __device__ __forceinline__ T ldg(const T *p) { return __ldg(p); }
 
-// Explicitly rounded products and fused multiply-adds.  The v-line recurrences run in several
-// kernels (rows read in place, rows through shared-memory tiles, partitioned lines), and the
-// autotuner may pick a different variant per instance; written with these, every variant rounds
-// the same way whatever the compiler would contract, so they agree bit for bit.
+// Explicitly rounded products and fused multiply-adds: the FP32 stages, whose results keep their bits,
+// round the same way whatever the compiler would contract.
 __device__ __forceinline__ double mul_x(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ float mul_x(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ double fma_x(double a, double b, double c) { return __fma_rn(a, b, c); }

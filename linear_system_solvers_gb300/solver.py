@@ -112,7 +112,7 @@ class ImplicitHestonSolver:
             pass
 
     def line_chunks(self, s_chunks: int = 0, v_chunks: int = 0, stream: int = 0):
-        """Chunks per S line / v line of the partitioned solves (0 = autotune); returns those in use."""
+        """Chunks per S line / v line of the partitioned solves (0 = by the line length); returns those in use."""
         a, b = ctypes.c_int(), ctypes.c_int()
         L.check(self.lib.lss_adi_line_chunks(self._h, int(s_chunks), int(v_chunks), ctypes.byref(a), ctypes.byref(b),
                                              ctypes.c_void_p(stream)))
