@@ -384,9 +384,10 @@ template <typename T> __device__ __forceinline__ void b2_stage(const inst_view<T
 // segment.  The mixed difference (x(t-1,j-1) - x(t-1,j+1)) - (x(t+1,j-1) - x(t+1,j+1)) is formed
 // from a rolling window of the per-row differences x(r,j-1) - x(r,j+1): one subtraction per row.
 //
-// The next rows' operands are loaded before the current ones are used (two rows ahead, eight in the back
+// The next rows' operands are loaded before the current ones are used (five rows ahead, 16 in the back
 // substitution); the fused multiply-adds are written out, so the rounding hangs on no contraction.
-constexpr int FK = 8; // rows of a block of the back substitution
+constexpr int FA = 5;  // rows loaded ahead of the right-hand sides
+constexpr int FK = 16; // rows of a block of the back substitution
 template <int KIND, int SCH>
 __device__ __forceinline__ void s_stage(const inst_view<float> &v, const float *U, const float *Y1, const float *Y2, float *Y, int l0, int ls)
 {
@@ -493,17 +494,20 @@ __device__ __forceinline__ void s_stage(const inst_view<float> &v, const float *
             u1m = r.um; u1p = r.up;
             q0 = q1; q1 = q2;
         };
-        row ra = load(1), rb = load(min(2, e));
-        for (int t = 1; t <= e; t += 2) {
-            const row na = load(min(t + 2, e));
-            point(ra, t);
-            ra = na;
-            if (t + 1 <= e) {
-                const row nb = load(min(t + 3, e));
-                point(rb, t + 1);
-                rb = nb;
+        row ring[FA];
+#pragma unroll
+        for (int k = 0; k < FA; ++k) ring[k] = load(min(1 + k, e));
+        int t = 1;
+        for (; t + FA - 1 <= e; t += FA)
+#pragma unroll
+            for (int k = 0; k < FA; ++k) {
+                const row next = load(min(t + k + FA, e));
+                point(ring[k], t + k);
+                ring[k] = next;
             }
-        }
+#pragma unroll
+        for (int k = 0; k < FA - 1; ++k)
+            if (t + k <= e) point(ring[k], t + k);
         float x = y, yb[FK], gb[FK], yn[FK], gn[FK];
         auto block = [&](int t, float *yo, float *go) {
 #pragma unroll
@@ -514,7 +518,7 @@ __device__ __forceinline__ void s_stage(const inst_view<float> &v, const float *
             }
         };
         block(e - 1, yb, gb);
-        for (int t = e - 1; t >= 1; t -= FK) {
+        for (t = e - 1; t >= 1; t -= FK) {
             block(t - FK, yn, gn);
 #pragma unroll
             for (int z = 0; z < FK; ++z) {
@@ -545,7 +549,7 @@ template <typename F> __device__ __forceinline__ void with_scheme(int scheme, F 
 // v-line sweep: line i reads row i of `in` (t-1, t, t+1) and `inh` (t); tables are [t][slot][i].  A lane walks
 // its row eight columns at a time (256-bit loads and stores, rows padded to a multiple of eight: whole
 // 32-byte sectors; with half of a sector per access a full GPU ran at half the speed), the next
-// columns and four columns of tables ahead.
+// 16 columns and eight columns of tables ahead.
 __device__ __forceinline__ void ldv(const float *p, float *o)
 {
     asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -593,14 +597,16 @@ __device__ __forceinline__ void v_stage(const inst_view<float> &v, const float *
             return b;
         };
         float y = lo, a0 = 0.0f;
-        cols b = columns(0);
-        tabs q = tables(0);
+        cols b = columns(0), b2 = columns(8);
+        tabs qr[2] = {tables(0), tables(4)};
         for (int t = 0; t <= e; t += 8) {
-            const cols nb = columns(t + 8);
+            const cols nb = b2;
+            b2 = columns(t + 16);
             float o[8];
 #pragma unroll
             for (int h = 0; h < 8; h += 4) {
-                const tabs nq = tables(t + h + 4);
+                const tabs q = qr[h / 4];
+                qr[h / 4] = tables(t + h + 8);
 #pragma unroll
                 for (int z = 0; z < 4; ++z) {
                     const int w = h + z, c = t + w;
@@ -612,7 +618,6 @@ __device__ __forceinline__ void v_stage(const inst_view<float> &v, const float *
                     o[w] = y;
                     a0 = b.a[w];
                 }
-                q = nq;
             }
             stv(out + row + t, o);
             b = nb;
@@ -626,9 +631,10 @@ __device__ __forceinline__ void v_stage(const inst_view<float> &v, const float *
             return k;
         };
         const int tl = (ny - 1) / 8 * 8;
-        bbk k = back(tl);
+        bbk k = back(tl), k2 = back(tl - 8);
         for (int t = tl; t >= 0; t -= 8) {
-            const bbk nk = back(t - 8);
+            const bbk nk = k2;
+            k2 = back(t - 16);
             float o[8];
 #pragma unroll
             for (int z = 7; z >= 0; --z) {
@@ -692,7 +698,9 @@ __device__ __forceinline__ void fwd_step(const inst_view<float> &v, const float 
 // Persistent forward kernel of the instances of scheme SCH: CTAs of 4 warps split into groups
 // (the layout word of the CTA), each group pulling instances of its class (warps per instance)
 // from the class counter.  FP64: two CTAs per SM, whose threads hold the rows that the sweeps load ahead
-// (adi_delta.cuh).  FP32: four (768 uneven calls: 64.7 ms; 80 and 138 ms with five and six).
+// (adi_delta.cuh).  FP32: three, 168 registers (768 uneven calls 49.9 ms with five rows ahead, 51.8 with
+// four, 71 with six; two rows ahead with four CTAs of 128 registers 64.7 ms, a GPU full of equal 256 x 128
+// instances alone 301 against 367 us a step).
 constexpr int BATCH_CTA = 32 * MAX_GROUP_WARPS;
 
 // value at (eval_s, eval_v), corner o of its cell
@@ -710,7 +718,7 @@ template <typename T> __device__ __forceinline__ void load_payoff(const bparams<
 }
 
 template <typename T, int SCH>
-__global__ void __launch_bounds__(BATCH_CTA, sizeof(T) == 8 ? 2 : 4) k_batch_forward(const __grid_constant__ bparams<T> p)
+__global__ void __launch_bounds__(BATCH_CTA, sizeof(T) == 8 ? 2 : 3) k_batch_forward(const __grid_constant__ bparams<T> p)
 {
     __shared__ int s_idx[MAX_GROUP_WARPS];
     __shared__ int s_bad[MAX_GROUP_WARPS];
