@@ -266,17 +266,30 @@ __global__ void k_exact_setup(const T *low, const T *diag, const T *up, T theta,
     if (l >= lines) return;
     T gam = T(0);
     int out = 0;
-    for (int t = 1; t <= e; ++t) {
-        const long long o = first + l * next + (t - 1) * st;
-        const T av = R::mul(-theta, low[o]);
-        const T bv = R::add(T(1), R::mul(theta, diag[o]));
-        const T cv = -R::mul(theta, up[o]);
+    long long o = first + l * next;
+    T nl = low[o], nd = diag[o], nu = up[o]; // the next row's coefficients, loaded before this row's division
+    for (int t = 1; t <= e; ++t, o += st) {
+        const T av = R::mul(-theta, nl);
+        const T bv = R::add(T(1), R::mul(theta, nd));
+        const T cv = -R::mul(theta, nu);
+        if (t < e) {
+            nl = low[o + st];
+            nd = diag[o + st];
+            nu = up[o + st];
+        }
         const T beta = t == 1 ? bv : R::sub(bv, R::mul(av, gam));
-        gam = R::div(cv, beta);
-        out |= !divisor_ok(beta);
+        const T r = R::div(T(1), beta);
+        const bool ok = divisor_ok(beta);
+        if (ok && in_range(cv)) {
+            const T q0 = R::mul(cv, r);
+            gam = fma_rn(fma_rn(-beta, q0, cv), r, q0);
+        } else {
+            gam = R::div(cv, beta);
+        }
+        out |= !ok;
         rec[4 * o] = av;
         rec[4 * o + 1] = beta;
-        rec[4 * o + 2] = R::div(T(1), beta);
+        rec[4 * o + 2] = r;
         rec[4 * o + 3] = gam;
     }
     if (out) atomicOr(bad, 1);

@@ -391,7 +391,10 @@ template <typename T> int plain_solver<T>::init_exact()
     dbuf<int> bad;
     LSS_CUDA_TRY(bad.alloc(1), "allocating line factors");
     LSS_CUDA_TRY(cudaMemset(bad.p, 0, sizeof(int)), "line factors");
-    LSS_CUDA_TRY(exact_.alloc(8 * n), "allocating line factors");
+    if (exact_.alloc(8 * n) != cudaSuccess) { // no room beside the tables: the kernels above
+        (void)cudaGetLastError();
+        return LSS_ADI_OK;
+    }
     T *q = exact_.p;
     exact::k_exact_setup<T><<<grid_for(ny - 2, 32), 32>>>(d_.M, d_.Z, d_.P, d_.theta, ny - 2, ny + 1, 1, ny, nx - 2, q, bad.p);
     exact::k_exact_setup<T><<<grid_for(nx - 2, 32), 32>>>(d_.Mt, d_.W, d_.Pt, d_.theta, nx - 2, ny + 1, ny, 1, ny - 2, q + 4 * n, bad.p);
