@@ -167,7 +167,7 @@ template <typename T> __device__ __forceinline__ void ref_split(T th, T A, T B, 
     c = R::mul(-th, D);
 }
 
-template <typename T, bool DS, int PF> __global__ void __launch_bounds__(128) k_h1_ref(const h1params<T> p)
+template <typename T, bool DS, int PF> __device__ __forceinline__ void h1_ref_body(const h1params<T> &p)
 {
     using R = ar<true>;
     const int g = blockIdx.x * (blockDim.x / LANES) + threadIdx.x / LANES;
@@ -394,6 +394,10 @@ template <typename T, bool DS, int PF> __global__ void __launch_bounds__(128) k_
     p.values[L.inst] = (1.0 - L.eval_w) * static_cast<double>(U[el(i)]) + L.eval_w * static_cast<double>(U[el(i + 1)]);
     p.status[L.inst] = bad;
 }
+// FP64 asks for two CTAs per SM: with 168 registers, the compiler's own choice, its spills cost 16 %
+// (65536 Black-Scholes calls 1346 ms against 1164).
+template <typename T, bool DS, int PF> __global__ void __launch_bounds__(128) k_h1_ref(const h1params<T> p) { h1_ref_body<T, DS, PF>(p); }
+template <bool DS, int PF> __global__ void __launch_bounds__(128, 2) k_h1_ref64(const h1params<double> p) { h1_ref_body<double, DS, PF>(p); }
 
 // ------------------------------------------------------------------------------------------
 // FAST: one factorisation per instance (set-up), then per step one fused right-hand-side +
@@ -1455,10 +1459,13 @@ template <typename T> int batch_t<T>::run(cudaStream_t s)
         else if (src) k_h1_fast<T, H1_PF, true, false><<<ctas, th, 0, s>>>(p);
         else k_h1_fast<T, H1_PF, false, false><<<ctas, th, 0, s>>>(p);
     }
-    else if (ds)
-        k_h1_ref<T, true, 4><<<blocks, 128, 0, s>>>(p);
-    else
-        k_h1_ref<T, false, 4><<<blocks, 128, 0, s>>>(p);
+    else if constexpr (std::is_same<T, double>::value) {
+        if (ds) k_h1_ref64<true, 4><<<blocks, 128, 0, s>>>(p);
+        else k_h1_ref64<false, 4><<<blocks, 128, 0, s>>>(p);
+    } else {
+        if (ds) k_h1_ref<T, true, 4><<<blocks, 128, 0, s>>>(p);
+        else k_h1_ref<T, false, 4><<<blocks, 128, 0, s>>>(p);
+    }
     LSS_CUDA_TRY(cudaGetLastError(), "heat1d: launching the time loop");
     return LSS_ADI_OK;
 }
