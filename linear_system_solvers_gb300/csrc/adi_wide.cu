@@ -228,7 +228,8 @@ template <typename T> struct line_solver {
         c.PreG = q; q += chunks;
         c.GA = q; q += static_cast<long long>(sp.tiles) * sp.groups() * wp.ls;
     }
-    // Partition: `ps`, `pv` chunks per S / v line (0: chosen by choose_split).
+    // Partition: `ps`, `pv` chunks per S / v line (0: chosen by choose_split).  The products and the cleared
+    // table sets are on the device when it returns: no stream of the caller is ordered behind the set-up's.
     int set_chunks(int ps, int pv)
     {
         wp.s = choose_split(nx - 2, false, ps);
@@ -249,6 +250,7 @@ template <typename T> struct line_solver {
         }
         products(nullptr, false);
         LSS_CUDA_TRY(cudaGetLastError(), "wide: chunk products");
+        LSS_CUDA_TRY(cudaStreamSynchronize(nullptr), "wide: chunk products");
         return LSS_ADI_OK;
     }
 
