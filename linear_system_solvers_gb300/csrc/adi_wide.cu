@@ -17,37 +17,6 @@
 namespace lss_gb300 {
 namespace wide {
 
-// Partition of a line's `rows` rows, `chunks` > 0 forcing the chunk count.  Short chunks as long as
-// they fit one CTA: the time of a small instance is the chain of one chunk and the composition, and
-// few lines per CTA spread the FP64 work over more SMs (one 32-byte sector of doubles per row of an
-// S stage, at 4 lines).  Measured per step (S and v stages of one split, others alike): 400 x 200 HV
-// 35.5 us with S (4 lines, 100 chunks of 4), 46 us with (8, 50 of 8), 59 us with (4, 64 of 4, two
-// tiles); 1000 x 500 HV 64 us with v (8, 63 of 8), 75 us with (8, 32 of 16), 107 us with S (4, 63 of
-// 16) instead of (4, 125 of 8); 4096 x 2048 HV 0.84 ms with S (8, 32 of 16, eight tiles) or v (4, 64
-// of 16, two tiles), 0.88 ms with 8 rows per chunk.  At least five rows per S chunk (four per v
-// chunk, boundary rows included).
-static split choose_split(int rows, bool vec, int chunks)
-{
-    split s;
-    const int sizes_s[] = {5, 8, 16}, sizes_v[] = {4, 8, 16};
-    const int *sizes = vec ? sizes_v : sizes_s;
-    const int most = chunks > 0 ? chunks : vec ? 64 : 128;
-    s.R = 16;
-    for (int k = 2; k >= 0; --k)
-        if ((rows + sizes[k] - 1) / sizes[k] <= most) s.R = sizes[k];
-    s.PC = chunks > 0 ? chunks : (rows + s.R - 1) / s.R;
-    s.L = vec ? 8 : 4;
-    if (chunks <= 0 && s.PC > most) { // longer lines: tiles
-        s.PC = vec ? 64 : 32;
-        s.L = vec ? 4 : 8;
-    }
-    while (s.L > 1 && s.L * s.PC > MAX_CTA) s.L /= 2;
-    s.tiles = (rows + s.R * s.PC - 1) / (s.R * s.PC);
-    s.gs = 1;
-    while (s.gs * s.gs < s.PC) ++s.gs;
-    return s;
-}
-
 template <typename T> struct line_solver {
     int nx = 0, ny = 0, ld = 0, steps = 0, scheme = 0, sms = 0;
     long long n = 0;
@@ -218,15 +187,14 @@ template <typename T> struct line_solver {
     // chunk products of both sweeps of both directions
     long long carry_need() const
     {
-        auto words = [](const split &q) { return static_cast<long long>(q.tiles) * (2 * q.PC + q.groups()); };
-        return 2LL * wp.ls * (words(wp.s) + words(wp.v));
+        return 2 * (carry_table(wp.s, wp.ls) + carry_table(wp.v, wp.lv));
     }
-    void carve(carry_tab<T> &c, const split &sp, T *&q) const
+    template <typename Q> static void carve(carry_tab<Q> &c, const split &sp, int stride, Q *&q)
     {
-        const long long chunks = static_cast<long long>(sp.tiles) * sp.PC * wp.ls;
+        const long long chunks = static_cast<long long>(sp.tiles) * sp.PC * stride;
         c.A = q; q += chunks;
         c.PreG = q; q += chunks;
-        c.GA = q; q += static_cast<long long>(sp.tiles) * sp.groups() * wp.ls;
+        c.GA = q; q += static_cast<long long>(sp.tiles) * sp.groups() * stride;
     }
     // Partition: `ps`, `pv` chunks per S / v line (0: chosen by choose_split).  The products and the cleared
     // table sets are on the device when it returns: no stream of the caller is ordered behind the set-up's.
@@ -234,12 +202,13 @@ template <typename T> struct line_solver {
     {
         wp.s = choose_split(nx - 2, false, ps);
         wp.v = choose_split(ny, true, pv);
-        wp.ls = std::max(nx, ld);
+        wp.ls = ld;
+        wp.lv = nx;
         const long long need = carry_need();
         if (static_cast<long long>(carry_mem.n) < need) LSS_CUDA_TRY(carry_mem.alloc(need), "wide: allocating chunk products");
         T *q = carry_mem.p;
-        for (carry_tab<T> *c : {&wp.sf, &wp.sb}) carve(*c, wp.s, q);
-        for (carry_tab<T> *c : {&wp.vf, &wp.vb}) carve(*c, wp.v, q);
+        for (carry_tab<T> *c : {&wp.sf, &wp.sb}) carve(*c, wp.s, wp.ls, q);
+        for (carry_tab<T> *c : {&wp.vf, &wp.vb}) carve(*c, wp.v, wp.lv, q);
         if (graph) cudaGraphExecDestroy(graph);
         graph = nullptr;
         if (tdep) {
@@ -279,7 +248,7 @@ template <typename T> struct line_solver {
         const int lines = s_lines ? ny : nx, grid = grid_for(lines, sp.L) * sp.tiles;
         const long long ts = s_lines ? ld : 1, st = s_lines ? 1 : ld;
         launch(s, k_wide_products<T>, grid, dim3(sp.L * sp.PC), sizeof(T) * sp.L * sp.PC, fac, ts, st, lines, first, last,
-               s_lines ? 1 : 0, shift, sp, fwd, out, wp.ls);
+               s_lines ? 1 : 0, shift, sp, fwd, out, s_lines ? wp.ls : wp.lv);
     }
     void products(cudaStream_t s, bool s_lines)
     {
@@ -296,8 +265,7 @@ template <typename T> struct line_solver {
     // four CTAs per SM, while the sets stay within half of L2 (64 MB).
     int set_groups()
     {
-        const long long chunks = static_cast<long long>(wp.s.tiles) * (2 * wp.s.PC + wp.s.groups()) * wp.ls;
-        const long long words = (W_COUNT * n + 2 * nx + (td_adjoint ? 4 : 2) * chunks + 3) / 4 * 4;
+        const long long words = (W_COUNT * n + 2 * nx + (td_adjoint ? 4 : 2) * carry_table(wp.s, wp.ls) + 3) / 4 * 4;
         const long long fit = (64LL << 20) / (words * static_cast<long long>(sizeof(double))), ctas = grid_for(ny - 2, wp.s.L);
         const long long fill = (4LL * sms + ctas - 1) / ctas;
         td_group = static_cast<int>(std::max(1LL, std::min({fit, fill, static_cast<long long>(TDEP_STEPS), static_cast<long long>(steps)})));
@@ -308,20 +276,13 @@ template <typename T> struct line_solver {
         td_set.xb = td_sets.p + W_COUNT * n;
         td_set.stride = words;
         double *q = td_set.xb + 2 * nx;
-        carve_set(td_set.sf, q);
-        carve_set(td_set.sb, q);
+        carve(td_set.sf, wp.s, wp.ls, q);
+        carve(td_set.sb, wp.s, wp.ls, q);
         if (td_adjoint) {
-            carve_set(td_set.sz, q);
-            carve_set(td_set.sw, q);
+            carve(td_set.sz, wp.s, wp.ls, q);
+            carve(td_set.sw, wp.s, wp.ls, q);
         }
         return LSS_ADI_OK;
-    }
-    void carve_set(carry_tab<double> &c, double *&q) const
-    {
-        const long long chunks = static_cast<long long>(wp.s.tiles) * wp.s.PC * wp.ls;
-        c.A = q; q += chunks;
-        c.PreG = q; q += chunks;
-        c.GA = q; q += static_cast<long long>(wp.s.tiles) * wp.s.groups() * wp.ls;
     }
     static carry_tab<double> shifted(const carry_tab<double> &c, long long o) { return {c.A + o, c.PreG + o, c.GA + o}; }
 
@@ -579,8 +540,8 @@ struct line_adjoint : wide_adjoint_base {
         const long long need = w.carry_need();
         if (static_cast<long long>(carry_adj.n) < need) LSS_CUDA_TRY(carry_adj.alloc(need), "wide adjoint: allocating chunk products");
         double *q = carry_adj.p;
-        for (carry_tab<double> *c : {&ap.sz, &ap.sw}) w.carve(*c, w.wp.s, q);
-        for (carry_tab<double> *c : {&ap.vz, &ap.vw}) w.carve(*c, w.wp.v, q);
+        for (carry_tab<double> *c : {&ap.sz, &ap.sw}) w.carve(*c, w.wp.s, w.wp.ls, q);
+        for (carry_tab<double> *c : {&ap.vz, &ap.vw}) w.carve(*c, w.wp.v, w.wp.lv, q);
         if (!w.tdep) s_products(nullptr);
         w.product(nullptr, false, w.wp.V[W_VU], 1, w.ny - 1, -1, true, ap.vz);
         w.product(nullptr, false, w.wp.V[W_VL], 0, w.ny - 2, 1, false, ap.vw);

@@ -36,19 +36,10 @@
 // length R of a chunk, one memory latency per pass and the composition.
 #pragma once
 
+#include "adi_split.hpp"
+
 namespace lss_gb300 {
 namespace wide {
-
-constexpr int MAX_CTA = 512; // threads per CTA (128 registers each)
-
-// One direction's partition.
-struct split {
-    int L = 8, PC = 1; // lines per CTA, chunks per line
-    int R = 4;         // rows per chunk (compiled: 5, 8, 16 for S lines, 4, 8, 16 for v lines)
-    int gs = 1;        // chunks per group of the composition
-    int tiles = 1;
-    __host__ __device__ int groups() const { return (PC + gs - 1) / gs; }
-};
 
 // chunk products of one sweep: chunk tile * PC + c of line l at [(tile * PC + c) * ls + l], in the
 // sweep's order (the back sweeps run the chunks from the last to the first)
@@ -69,7 +60,7 @@ template <typename T> struct wparams {
     const T *yslo, *yb2c;                        // ny
     const int *imap, *jmap;
     carry_tab<T> sf, sb, vf, vb; // S forward / back, v forward / back
-    int ls;                      // line stride of the carry tables
+    int ls, lv;                  // line strides of the S and the v carry tables
     split s, v;
 };
 
@@ -108,7 +99,6 @@ template <typename T> struct carry {
     T *b, *a, *gb, *ga;
     int L, PC, gs, ng, lane, c;
 };
-__host__ __device__ inline int carry_words(const split &s) { return 2 * s.L * (s.PC + s.groups()); }
 template <typename T> __device__ __forceinline__ carry<T> make_carry(T *raw, const split &s, int sweep, int lane, int c)
 {
     carry<T> k;
@@ -345,8 +335,8 @@ __global__ void __launch_bounds__(MAX_CTA) k_wide_v(const __grid_constant__ wpar
     const carry<T> kb = make_carry(reinterpret_cast<T *>(raw), sp, 1, lane, c);
     pdl_launch();
     T preg, bpreg;
-    carry_load(kf, p.vf, p.ls, 0, i, preg);
-    carry_load(kb, p.vb, p.ls, sp.tiles - 1, i, bpreg);
+    carry_load(kf, p.vf, p.lv, 0, i, preg);
+    carry_load(kb, p.vb, p.lv, sp.tiles - 1, i, bpreg);
     const int ii = p.imap[i];
     const T hi = p.xvhi[ii];
     // columns past the row's end are read at its last four, with the tables taken as zero there
@@ -373,7 +363,7 @@ __global__ void __launch_bounds__(MAX_CTA) k_wide_v(const __grid_constant__ wpar
         const int t0 = (tile * sp.PC + c) * R;
         if (tile > 0) {
             __syncthreads();
-            carry_load(kf, p.vf, p.ls, tile, i, preg);
+            carry_load(kf, p.vf, p.lv, tile, i, preg);
         }
         if (R > 8 || tile > 0) tables(t0);
 #pragma unroll
@@ -414,7 +404,7 @@ __global__ void __launch_bounds__(MAX_CTA) k_wide_v(const __grid_constant__ wpar
         const bool again = tile + 1 < sp.tiles;
         if (again) {
             __syncthreads();
-            carry_load(kb, p.vb, p.ls, tile, i, bpreg);
+            carry_load(kb, p.vb, p.lv, tile, i, bpreg);
             tables(t0);
 #pragma unroll
             for (int r = 0; r < R; r += 4) ld4(out + col(t0 + r), f + r);
@@ -845,8 +835,8 @@ __global__ void __launch_bounds__(MAX_CTA) k_wadj_v(const __grid_constant__ wpar
     const carry<double> kb = make_carry(reinterpret_cast<double *>(raw), sp, 1, lane, c);
     pdl_launch();
     double preg, bpreg;
-    carry_load(kf, q.vz, p.ls, 0, i, preg);
-    carry_load(kb, q.vw, p.ls, sp.tiles - 1, i, bpreg);
+    carry_load(kf, q.vz, p.lv, 0, i, preg);
+    carry_load(kb, q.vw, p.lv, sp.tiles - 1, i, bpreg);
     auto col = [&](int t) -> long long { return row + min(t, ld - 4); };
     // b2^T: rows nx-2 and nx-3 take the extrapolated row's adjoint
     const double fold = KIND == V_FIRST ? 0.0 : il == nx - 2 ? 4.0 / 3.0 : il == nx - 3 ? -1.0 / 3.0 : 0.0;
@@ -857,7 +847,7 @@ __global__ void __launch_bounds__(MAX_CTA) k_wadj_v(const __grid_constant__ wpar
         const int t0 = (tile * sp.PC + c) * R;
         if (tile > 0) {
             __syncthreads();
-            carry_load(kf, q.vz, p.ls, tile, i, preg);
+            carry_load(kf, q.vz, p.lv, tile, i, preg);
         }
         double ib[R];
 #pragma unroll
@@ -907,7 +897,7 @@ __global__ void __launch_bounds__(MAX_CTA) k_wadj_v(const __grid_constant__ wpar
         const int t0 = (tile * sp.PC + c) * R;
         if (tile + 1 < sp.tiles) {
             __syncthreads();
-            carry_load(kb, q.vw, p.ls, tile, i, bpreg);
+            carry_load(kb, q.vw, p.lv, tile, i, bpreg);
 #pragma unroll
             for (int r = 0; r < R; r += 4) ld4(DB + col(t0 + r), f + r);
         }
