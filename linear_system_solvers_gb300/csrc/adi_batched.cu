@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "adi_batched.hpp"
+#include "adi_index.hpp"
 
 namespace lss_gb300 {
 
@@ -307,12 +308,11 @@ template <typename T> struct inst_view {
     long long o2;
     int ox, oy;
     long long so, vo; // line tables
-    int sl, vl;       // elements of a row
     // line tables of the instance: row t of the S lines holds all its slots, column t of the v lines too (a
     // row's operands lie within a few KB instead of ten arenas: 5 to 15 % where a GPU full of 256 x 128
     // instances reads them from HBM)
-    __device__ __forceinline__ const T *S(int k, int t, int j) const { return p->S + so + (long long)t * sl + (k * ld + j); }
-    __device__ __forceinline__ const T *Vt(int k, int t, int i) const { return p->Vt + vo + (long long)t * vl + (k * nx + i); }
+    __device__ __forceinline__ const T *S(int k, int t, int j) const { return p->S + so + table_at<s_slots<T>()>(t, k, j, ld); }
+    __device__ __forceinline__ const T *Vt(int k, int t, int i) const { return p->Vt + vo + table_at<v_slots<T>()>(t, k, i, nx); }
     __device__ __forceinline__ const T *X(int k) const { return p->X[k] + ox; }
     __device__ __forceinline__ const T *Yv(int k) const { return p->Yv[k] + oy; }
     __device__ __forceinline__ const int *imap() const { return p->imap + ox; }
@@ -660,8 +660,6 @@ template <typename T> __device__ __forceinline__ inst_view<T> make_view(const bp
     v.o2 = d.o2;
     v.so = d.o2 * s_slots<T>();
     v.vo = d.o2 * v_slots<T>();
-    v.sl = d.ld * s_slots<T>();
-    v.vl = d.nx * v_slots<T>();
     v.ox = d.ox;
     v.oy = d.oy;
     return v;
@@ -956,17 +954,18 @@ static __global__ void k_setup_s_delta(setup_params sp, double *S0)
         const double a = -th * M, b = 1.0 + th * Z, c = -th * P;
         const double ib = 1.0 / fma(-a, gam, b);
         gam = c * ib;
-        double *s = S0 + d.o2 * DS_COUNT + (long long)t * DS_COUNT * ld + j;
-        s[DS_LA * ld] = a * ib;
-        s[DS_G * ld] = gam;
-        s[DS_WG * ld] = gm * C * ib;
-        s[DS_WW * ld] = M * ib;
-        s[DS_WS * ld] = Mt * ib;
-        s[DS_WQ * ld] = ((M + P - Z) - W) * ib;
-        s[DS_WC * ld] = -(Z + W) * ib;
-        s[DS_WN * ld] = Pt * ib;
-        s[DS_WE * ld] = P * ib;
-        s[DS_IB * ld] = ib;
+        double *row = S0 + d.o2 * DS_COUNT;
+        auto slot = [&](int k) -> double & { return row[table_at<DS_COUNT>(t, k, j, ld)]; };
+        slot(DS_LA) = a * ib;
+        slot(DS_G) = gam;
+        slot(DS_WG) = gm * C * ib;
+        slot(DS_WW) = M * ib;
+        slot(DS_WS) = Mt * ib;
+        slot(DS_WQ) = ((M + P - Z) - W) * ib;
+        slot(DS_WC) = -(Z + W) * ib;
+        slot(DS_WN) = Pt * ib;
+        slot(DS_WE) = P * ib;
+        slot(DS_IB) = ib;
     }
 }
 static __global__ void k_setup_v_delta(setup_params sp, double *V0)
