@@ -198,9 +198,9 @@ int lss_adi_forward_graph(lss_adi_handle *h, const void *payoff, void *out_surfa
  * and SABR (the r sensitivity includes the discount factors D(t) inside a and c).  Instances
  * larger than 256 x 160 points, and SABR with r != 0 (whose S-line tables are rebuilt at every
  * step's time), run the adjoint as one kernel per stage over the whole GPU.
- * Checkpoints every `checkpoint_every` steps; 0 = planned: the longest interval whose workspace fits
- * a quarter of the device and half of its free memory (at least ceil(sqrt(steps))).  Results do
- * not depend on the interval. */
+ * Checkpoints every `checkpoint_every` steps; 0 = planned at the handle's first such call: the longest
+ * interval whose workspace fits a sixteenth of the device and half of its free memory (at least
+ * ceil(sqrt(steps))).  The handle keeps the workspace.  Results do not depend on the interval. */
 int lss_adi_adjoint(lss_adi_handle *h, const void *payoff, double *out_value, double *dv_dparams,
                     void *dv_dpayoff, int checkpoint_every, int flags, void *stream);
 

@@ -42,9 +42,11 @@ template <typename T> struct dbuf {
     cudaError_t alloc(size_t count)
     {
         release();
-        n = count;
         if (count == 0) return cudaSuccess;
-        return cudaMalloc(reinterpret_cast<void **>(&p), count * sizeof(T));
+        const cudaError_t e = cudaMalloc(reinterpret_cast<void **>(&p), count * sizeof(T));
+        if (e == cudaSuccess) n = count;
+        else p = nullptr;
+        return e;
     }
     cudaError_t upload(const T *src, size_t count, cudaStream_t s = nullptr)
     {

@@ -483,7 +483,8 @@ struct line_adjoint : wide_adjoint_base {
     line_solver<double> w;
     dbuf<double> ws, factors, carry_adj, grads;
     adj_params ap{};
-    long long held = 0, nacc = 0;
+    long long nacc = 0;
+    int planned = 0; // interval of checkpoint_every = 0, kept while its workspace is held
 
     int init(const lss_adi_problem &p)
     {
@@ -614,6 +615,37 @@ struct line_adjoint : wide_adjoint_base {
         return (nseg + 4LL * (c + 1) + 2 + 6) * w.n + w.nx + 2LL * w.ny + 5 * nacc;
     }
 
+    // Checkpoint interval and workspace of a run.  every = 0: the longest interval within a sixteenth of the
+    // device and half of what is free (no step is recomputed when one segment holds the whole time
+    // loop), at least ceil(sqrt(steps)).  It is chosen once and kept: what other users of the device hold
+    // does not make a call allocate again.  Where its workspace cannot be had after all, the shortest is taken.
+    int reserve(int every, int &c)
+    {
+        const int steps = w.steps, least = std::max(1, static_cast<int>(std::ceil(std::sqrt(static_cast<double>(steps)))));
+        const bool keep = every <= 0 && planned > 0 && static_cast<long long>(ws.n) == need(planned);
+        c = every > 0 ? std::min(every, steps) : keep ? planned : least;
+        if (every <= 0 && !keep) {
+            size_t free_b = 0, total_b = 0;
+            LSS_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b), "wide adjoint: device memory");
+            const double held_b = static_cast<double>(ws.n) * sizeof(double);
+            const double most = std::min(static_cast<double>(total_b) / 16, 0.5 * (static_cast<double>(free_b) + held_b));
+            for (int k = steps; k > c; --k)
+                if (static_cast<double>(need(k)) * sizeof(double) <= most) {
+                    c = k;
+                    break;
+                }
+        }
+        cudaError_t e = static_cast<long long>(ws.n) == need(c) ? cudaSuccess : ws.alloc(need(c));
+        if (e == cudaErrorMemoryAllocation && every <= 0 && c > least) {
+            (void)cudaGetLastError();
+            c = least;
+            e = ws.alloc(need(c));
+        }
+        LSS_CUDA_TRY(e, "wide adjoint: allocating workspace");
+        if (every <= 0) planned = c;
+        return LSS_ADI_OK;
+    }
+
     int run(const void *payoff, double *out_value, double *dv_dparams, void *dv_dpayoff, int checkpoint_every, int flags,
             void *stream) override
     {
@@ -626,32 +658,17 @@ struct line_adjoint : wide_adjoint_base {
             LSS_CUDA_TRY(cudaMemcpyAsync(w.pay.p, payoff, bytes, dev ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s),
                          "lss_adi_adjoint: copying the terminal condition");
         nacc = std::max<long long>(static_cast<long long>(grid_for(w.ny - 1, w.wp.s.L)) * w.wp.s.L * w.wp.s.PC, w.nx);
-        // the longest interval within a quarter of the device (and half of what is free): no step is
-        // recomputed when one segment holds the whole time loop
-        int c = checkpoint_every > 0 ? std::min(checkpoint_every, steps)
-                                     : std::max(1, static_cast<int>(std::ceil(std::sqrt(static_cast<double>(steps)))));
-        if (checkpoint_every <= 0) {
-            size_t free_b = 0, total_b = 0;
-            LSS_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b), "wide adjoint: device memory");
-            const double held_b = static_cast<double>(ws.n) * sizeof(double);
-            const double most = std::min(0.25 * static_cast<double>(total_b), 0.5 * (static_cast<double>(free_b) + held_b));
-            for (int k = steps; k > c; --k)
-                if (static_cast<double>(need(k)) * sizeof(double) <= most) {
-                    c = k;
-                    break;
-                }
-        }
-        if (static_cast<long long>(ws.n) < need(c) || held != need(c)) {
-            LSS_CUDA_TRY(ws.alloc(need(c)), "wide adjoint: allocating workspace");
-            held = need(c);
-        }
-        // the boundary rows and columns that no kernel writes are read as zeros
-        LSS_CUDA_TRY(cudaMemsetAsync(ws.p, 0, need(c) * sizeof(double), s), "wide adjoint: clearing");
+        int c = 0;
+        int rc = reserve(checkpoint_every, c);
+        if (rc) return rc;
         const int nseg = (steps + c - 1) / c;
         double *CK = ws.p, *SEG = CK + nseg * n, *W0 = SEG + 4LL * (c + 1) * n, *W1 = W0 + n;
         arrays a;
         a.VB = W1 + n; a.DB = a.VB + n; a.FB = a.DB + n; a.MU = a.FB + n; a.DV = a.MU + n; a.D2B = a.DV + n;
         a.LV = a.D2B + n; a.LS = a.LV + w.nx; a.HS = a.LS + w.ny; a.ACC = a.HS + w.ny;
+        // read where no kernel writes: VB and FB (boundary rows and columns) and the sums.  The states and
+        // increments are written wherever they are read, so the checkpoints need no clearing.
+        LSS_CUDA_TRY(cudaMemsetAsync(a.VB, 0, (need(c) - (a.VB - ws.p)) * sizeof(double), s), "wide adjoint: clearing");
         auto slot = [&](int m, int k) { return SEG + (4LL * m + k) * n; };
         const long long flat = static_cast<long long>(w.nx) * w.ny;
         w.launches = 0;
