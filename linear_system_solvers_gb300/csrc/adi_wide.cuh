@@ -60,8 +60,9 @@ template <typename T> struct wparams {
     const T *yslo, *yb2c;                        // ny
     const int *imap, *jmap;
     carry_tab<T> sf, sb, vf, vb; // S forward / back, v forward / back
-    int ls, lv;                  // line strides of the S and the v carry tables
+    int ls;                      // line stride of the S carry tables
     split s, v;
+    int lv;                      // line stride of the v carry tables
 };
 
 enum { W_LA = 0, W_G, W_WG, W_WW, W_WS, W_WQ, W_WN, W_WE, W_IB, W_WC, W_COUNT };
