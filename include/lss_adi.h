@@ -207,11 +207,14 @@ int lss_adi_adjoint(lss_adi_handle *h, const void *payoff, double *out_value, do
 /* Grid of the handle: x (nx) = S_i, y (ny) = v_j, in the precision's type (host). */
 int lss_adi_grid(const lss_adi_handle *h, void *x, void *y);
 
-/* Partitioned line solves of a LSS_ADI_ARITH_FAST single instance: every S line is cut into
- * s_chunks and every v line into v_chunks pieces solved concurrently (1 = thread per line;
- * at most 128; at least 4 rows per chunk).  0 for either picks it by the line length (the rule
- * lss_adi_create uses: as many chunks of 4 to 16 rows as one CTA holds).  Results depend on the
- * chunk counts at rounding level only.  out_s / out_v (may be NULL) receive the
+/* Partitioned line solves of a LSS_ADI_ARITH_FAST single instance: s_chunks pieces of every S line and
+ * v_chunks of every v line are solved concurrently, each of at most 16 rows; a line of more than
+ * 16 x count rows is walked in several tiles of that many pieces (at most 128; at least 4 rows per
+ * piece; 1 = one piece at a time).  0 for either picks it by the line length (the rule lss_adi_create
+ * uses: pieces of 4 to 16 rows, as many as one CTA holds).  Results depend on the counts at
+ * rounding level only.  The adjoint of the handle follows, except for instances of up to
+ * 256 x 160 points, which keep the batched kernel's order (LSS_ADI_OPT_WIDE_ADJOINT).  A handle of
+ * LSS_ADI_OPT_LINE_PER_THREAD becomes a partitioned one.  out_s / out_v (may be NULL) receive the
  * counts in use.  LSS_ADI_EUNSUPPORTED for handles on the kernel-per-sweep path.  No
  * counterpart in the reference, whose line solves are serial. */
 int lss_adi_line_chunks(lss_adi_handle *h, int s_chunks, int v_chunks, int *out_s, int *out_v, void *stream);

@@ -187,9 +187,8 @@ int lss_adi_adjoint(lss_adi_handle *h, const void *payoff, double *out_value, do
         std::unique_ptr<wide_adjoint_base> a;
         int rc = make_wide_adjoint(h->prob, a);
         if (rc) return rc;
-        if (h->wide) { // the forward's chunk counts, so both passes solve alike
-            int ps = 0, pv = 0;
-            h->wide->current_chunks(ps, pv);
+        int ps = 0, pv = 0;
+        if (h->wide && h->wide->asked_chunks(ps, pv)) { // so both passes solve alike
             rc = a->set_chunks(ps, pv, stream);
             if (rc) return rc;
         }
@@ -222,8 +221,7 @@ int lss_adi_line_chunks(lss_adi_handle *h, int s_chunks, int v_chunks, int *out_
     int rc = h->wide->chunks(s_chunks, v_chunks, &ps, &pv, stream);
     if (rc) return rc;
     if (h->adj) {
-        h->wide->current_chunks(ps, pv);
-        rc = h->adj->set_chunks(ps, pv, stream);
+        rc = h->adj->set_chunks(s_chunks, v_chunks, stream);
         if (rc) return rc;
     }
     if (out_s) *out_s = ps;

@@ -1797,11 +1797,7 @@ template <typename T> struct wide_solver : wide_solver_base {
         }
         return parts->chunks(s_chunks, v_chunks, out_s, out_v, stream);
     }
-    void current_chunks(int &s_chunks, int &v_chunks) const override
-    {
-        s_chunks = v_chunks = 1;
-        if (parts) parts->current_chunks(s_chunks, v_chunks);
-    }
+    bool asked_chunks(int &s_chunks, int &v_chunks) const override { return parts && parts->asked_chunks(s_chunks, v_chunks); }
 };
 
 int make_wide_solver(const lss_adi_problem &p, std::unique_ptr<wide_solver_base> &out)

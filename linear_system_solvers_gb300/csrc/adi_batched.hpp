@@ -18,7 +18,8 @@ struct wide_solver_base {
                         bool use_graph) = 0;
     virtual int grid(void *x, void *y) const = 0;
     virtual int chunks(int s_chunks, int v_chunks, int *out_s, int *out_v, void *stream) = 0;
-    virtual void current_chunks(int &s_chunks, int &v_chunks) const = 0;
+    // true once lss_adi_line_chunks has set counts (0: chosen by the line's length)
+    virtual bool asked_chunks(int &s_chunks, int &v_chunks) const = 0;
 };
 int make_wide_solver(const lss_adi_problem &p, std::unique_ptr<wide_solver_base> &out);
 // the same with the line solves partitioned over the whole GPU (adi_wide.cu)
@@ -27,7 +28,7 @@ int make_partitioned_solver(const lss_adi_problem &p, std::unique_ptr<wide_solve
 // Forward + adjoint of one parametric FP64 instance (behind lss_adi_adjoint, adi_wide.cu).
 struct wide_adjoint_base {
     virtual ~wide_adjoint_base() = default;
-    virtual int set_chunks(int s_chunks, int v_chunks, void *stream) = 0; // 0: chosen by the line's length
+    virtual int set_chunks(int s_chunks, int v_chunks, void *stream) = 0; // counts of lss_adi_line_chunks
     virtual int run(const void *payoff, double *out_value, double *dv_dparams, void *dv_dpayoff, int checkpoint_every, int flags,
                     void *stream) = 0;
 };

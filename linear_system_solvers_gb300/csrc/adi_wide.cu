@@ -420,6 +420,8 @@ template <typename T> struct line_solver {
 template <typename T> struct line_front : wide_solver_base {
     line_solver<T> w;
     std::vector<T> x, y, pay0;
+    int ask_s = 0, ask_v = 0;
+    bool asked = false;
 
     int init(const lss_adi_problem &p)
     {
@@ -465,15 +467,18 @@ template <typename T> struct line_front : wide_solver_base {
         w.serial = 0; // chunk counts ask for partitioned solves
         int rc = w.set_chunks(s_chunks, v_chunks);
         if (rc) return rc;
-        LSS_CUDA_TRY(cudaDeviceSynchronize(), "lss_adi_line_chunks");
+        ask_s = s_chunks;
+        ask_v = v_chunks;
+        asked = true;
         if (out_s) *out_s = w.wp.s.PC;
         if (out_v) *out_v = w.wp.v.PC;
         return LSS_ADI_OK;
     }
-    void current_chunks(int &s_chunks, int &v_chunks) const override
+    bool asked_chunks(int &s_chunks, int &v_chunks) const override
     {
-        s_chunks = w.wp.s.PC;
-        v_chunks = w.wp.v.PC;
+        s_chunks = ask_s;
+        v_chunks = ask_v;
+        return asked;
     }
 };
 
@@ -527,16 +532,24 @@ struct line_adjoint : wide_adjoint_base {
         // instance in a batch.  (One warp group of the batched kernel took 119 ms for a 128 x 64 x 200
         // Craig-Sneyd call with sensitivities.)  Larger ones, and those of LSS_ADI_OPT_WIDE_ADJOINT, are
         // partitioned; LINE_PER_THREAD asks for relay order at any size.
-        const bool small = p.nx <= 256 && static_cast<long long>(p.nx) * p.ny <= 40960 && !time_dependent(p);
-        w.serial = (p.options & LSS_ADI_OPT_LINE_PER_THREAD) || (small && !(p.options & LSS_ADI_OPT_WIDE_ADJOINT));
-        return set_chunks(0, 0, nullptr);
+        small = p.nx <= 256 && static_cast<long long>(p.nx) * p.ny <= 40960 && !time_dependent(p) && !(p.options & LSS_ADI_OPT_WIDE_ADJOINT);
+        w.serial = small || (p.options & LSS_ADI_OPT_LINE_PER_THREAD);
+        return partition(0, 0);
     }
     double tau0 = 0.0, dtau = 0.0;
+    bool small = false; // relay order whatever chunk counts the forward solve was given
 
+    // Counts set for the forward solve ask for partitioned solves here too, of instances that are not small.
     int set_chunks(int ps, int pv, void *stream) override
     {
         LSS_CUDA_TRY(cudaStreamSynchronize(static_cast<cudaStream_t>(stream)), "lss_adi_adjoint: chunk counts");
-        if (w.serial) ps = pv = 0; // (relay order: the same result for every count)
+        w.serial = small;
+        return partition(small ? 0 : ps, small ? 0 : pv);
+    }
+    // Partition of both passes.  Counts of 0 give the adjoint the lines per CTA of choose_split as well (handing
+    // it the forward's counts as set ones gave tiled lines 4 instead of 8 lines per S stage).
+    int partition(int ps, int pv)
+    {
         int rc = w.set_chunks(ps, pv);
         if (rc) return rc;
         const long long need = w.carry_need();
