@@ -960,10 +960,11 @@ static __global__ void k_setup_s_delta(setup_params sp, double *S0)
         slot(DS_G) = gam;
         slot(DS_WG) = gm * C * ib;
         slot(DS_WW) = M * ib;
-        slot(DS_WS) = Mt * ib;
-        slot(DS_WQ) = ((M + P - Z) - W) * ib;
+        const double ws = Mt * ib, wn = Pt * ib;
+        slot(DS_WS) = ws;
+        slot(DS_WQ) = center_weight<double>(M, P, Z, Mt, Pt, W, ib, ws, wn, t, j);
         slot(DS_WC) = -(Z + W) * ib;
-        slot(DS_WN) = Pt * ib;
+        slot(DS_WN) = wn;
         slot(DS_WE) = P * ib;
         slot(DS_IB) = ib;
     }

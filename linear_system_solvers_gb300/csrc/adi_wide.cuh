@@ -520,14 +520,15 @@ __global__ void __launch_bounds__(MAX_CTA) k_wide_products(const T *fac, long lo
 // S-line tables of one line per thread (double arithmetic), from M, P, Z, Mt, Pt, W, C (pitch ld)
 template <typename T>
 __device__ __forceinline__ void s_slots(T *s, long long n, double M, double P, double Z, double Mt, double Pt, double W, double C,
-                                        double gm, double ib)
+                                        double gm, double ib, int t, int j)
 {
+    const T ws = static_cast<T>(Mt * ib), wn = static_cast<T>(Pt * ib);
     s[W_WG * n] = static_cast<T>(gm * C * ib);
     s[W_WW * n] = static_cast<T>(M * ib);
-    s[W_WS * n] = static_cast<T>(Mt * ib);
-    s[W_WQ * n] = static_cast<T>(((M + P - Z) - W) * ib);
+    s[W_WS * n] = ws;
+    s[W_WQ * n] = center_weight<T>(M, P, Z, Mt, Pt, W, ib, ws, wn, t, j);
     s[W_WC * n] = static_cast<T>(-(Z + W) * ib);
-    s[W_WN * n] = static_cast<T>(Pt * ib);
+    s[W_WN * n] = wn;
     s[W_WE * n] = static_cast<T>(P * ib);
 }
 template <typename T>
@@ -554,7 +555,7 @@ __global__ void k_wide_setup_s(const double *base, long long n, int nx, int ny, 
         s[W_LA * n] = static_cast<T>(a * ib);
         s[W_G * n] = static_cast<T>(gam);
         s[W_IB * n] = static_cast<T>(ib);
-        s_slots(s, n, v[0], v[1], v[2], v[3], v[4], v[5], v[6], gm, ib);
+        s_slots(s, n, v[0], v[1], v[2], v[3], v[4], v[5], v[6], gm, ib, t, j);
     }
 }
 template <typename T>
@@ -718,7 +719,7 @@ __global__ void __launch_bounds__(MAX_CTA) k_wide_tdep(const __grid_constant__ t
                 S[W_IB * q.n + o] = ib;
                 S[W_G * q.n + o] = gam;
                 S[W_LA * q.n + o] = la;
-                s_slots(S + o, q.n, m[r], pp[r], z, q.mt[o], q.pt[o], q.w[o], dc * q.cs[o], q.gm, ib);
+                s_slots(S + o, q.n, m[r], pp[r], z, q.mt[o], q.pt[o], q.w[o], dc * q.cs[o], q.gm, ib, t, j);
                 if (r == 0) la1 = la;
                 else prl *= -la;
                 prb *= -gam;
