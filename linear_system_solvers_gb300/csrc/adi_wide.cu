@@ -200,8 +200,8 @@ template <typename T> struct line_solver {
     // table sets are on the device when it returns: no stream of the caller is ordered behind the set-up's.
     int set_chunks(int ps, int pv)
     {
-        wp.s = choose_split(nx - 2, false, ps);
-        wp.v = choose_split(ny, true, pv);
+        wp.s = choose_split(nx - 2, ny - 2, false, ps, sms, sizeof(T));
+        wp.v = choose_split(ny, nx - 2, true, pv, sms, sizeof(T));
         wp.ls = ld;
         wp.lv = nx;
         const long long need = carry_need();

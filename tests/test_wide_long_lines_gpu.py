@@ -32,3 +32,14 @@ def test_device_memory_and_result(lss, nx, ny, model):
     assert np.all(np.isfinite(ref))
     assert rel_err(got, ref) < 1e-9
     assert abs(val - rval) <= 1e-9 * max(1.0, abs(rval))
+
+
+@pytest.mark.parametrize("precision", ["f64", "f32"])
+@pytest.mark.parametrize("nx,ny", [(2600, 306), (2600, 308), (2600, 1218), (2600, 1220)])
+def test_both_sides_of_the_lines_that_fill_the_gpu(lss, nx, ny, precision):
+    """S lines of several tiles with 2, 4 and 8 lines per CTA: the split solves the thread-per-line systems."""
+    p = lss.HestonProblem(scheme="hv", nx=nx, ny=ny, nt=3, maturity=1e-6, rho=-0.2)
+    got, _ = lss.ImplicitHestonSolver(p, precision=precision).solve()
+    ref, _ = lss.ImplicitHestonSolver(dataclasses.replace(p, line_per_thread=True), precision=precision).solve()
+    assert np.all(np.isfinite(ref))
+    assert rel_err(got, ref) < (1e-10 if precision == "f64" else 1e-4)
