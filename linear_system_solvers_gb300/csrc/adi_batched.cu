@@ -376,6 +376,16 @@ template <typename T> __device__ __forceinline__ void b2_stage(const inst_view<T
     }
 }
 
+// Rows that a thread of the batched kernels loads ahead: AH of the right-hand sides, blocks of BK in the
+// one-instruction passes, VB4 blocks of four columns in the v lines' scaled passes (FP64), two blocks of
+// eight columns or none (FP32).
+struct deep {
+    static constexpr int AH = 5, BK = 16, VB4 = 4;
+};
+struct shallow {
+    static constexpr int AH = 1, BK = 4, VB4 = 1;
+};
+
 // Stages of the FP32 instances, written on Y1, Y2, Y3 (their values keep that form's rounding; FP64
 // runs in delta form, adi_delta.cuh).
 //
@@ -386,13 +396,12 @@ template <typename T> __device__ __forceinline__ void b2_stage(const inst_view<T
 //
 // The next rows' operands are loaded before the current ones are used (five rows ahead, 16 in the back
 // substitution); the fused multiply-adds are written out, so the rounding hangs on no contraction.
-constexpr int FA = 5;  // rows loaded ahead of the right-hand sides
-constexpr int FK = 16; // rows of a block of the back substitution
-template <int KIND, int SCH>
+template <int KIND, int SCH, typename DEPTH = deep>
 __device__ __forceinline__ void s_stage(const inst_view<float> &v, const float *U, const float *Y1, const float *Y2, float *Y, int l0, int ls)
 {
     constexpr bool xt = SCH == LSS_ADI_MODIFIED_CRAIG_SNEYD || SCH == LSS_ADI_HUNDSDORFER_VERWER;
     constexpr bool hv = SCH == LSS_ADI_HUNDSDORFER_VERWER;
+    constexpr int FA = DEPTH::AH, FK = DEPTH::BK;
     const int nx = v.nx, ny = v.ny, ld = v.ld, e = v.e_s, last = (nx - 1) * ld;
     struct row { // tables of row t, state of row t + 1
         float la, w[10];
@@ -562,8 +571,10 @@ __device__ __forceinline__ void stv(float *p, const float *o)
                  "f"(o[5]), "f"(o[6]), "f"(o[7])
                  : "memory");
 }
+template <typename DEPTH = deep>
 __device__ __forceinline__ void v_stage(const inst_view<float> &v, const float *in, const float *inh, const float *sb0, float *out, int l0, int ls)
 {
+    constexpr bool ahead = DEPTH::VB4 > 1;
     const int nx = v.nx, ny = v.ny, ld = v.ld, e = v.e_v;
     struct cols {
         float a[8], h[8];
@@ -597,16 +608,29 @@ __device__ __forceinline__ void v_stage(const inst_view<float> &v, const float *
             return b;
         };
         float y = lo, a0 = 0.0f;
-        cols b = columns(0), b2 = columns(8);
-        tabs qr[2] = {tables(0), tables(4)};
+        cols b, b2;
+        tabs qr[2];
+        if constexpr (ahead) {
+            b = columns(0);
+            b2 = columns(8);
+            qr[0] = tables(0);
+            qr[1] = tables(4);
+        }
         for (int t = 0; t <= e; t += 8) {
-            const cols nb = b2;
-            b2 = columns(t + 16);
+            cols nb;
+            if constexpr (ahead) {
+                nb = b2;
+                b2 = columns(t + 16);
+            } else {
+                b = columns(t);
+                nb.a[0] = in[row + min(t + 8, ld - 1)];
+            }
             float o[8];
 #pragma unroll
             for (int h = 0; h < 8; h += 4) {
+                if constexpr (!ahead) qr[h / 4] = tables(t + h);
                 const tabs q = qr[h / 4];
-                qr[h / 4] = tables(t + h + 8);
+                if constexpr (ahead) qr[h / 4] = tables(t + h + 8);
 #pragma unroll
                 for (int z = 0; z < 4; ++z) {
                     const int w = h + z, c = t + w;
@@ -620,7 +644,7 @@ __device__ __forceinline__ void v_stage(const inst_view<float> &v, const float *
                 }
             }
             stv(out + row + t, o);
-            b = nb;
+            if constexpr (ahead) b = nb;
         }
         float x = y;
         auto back = [&](int t) -> bbk {
@@ -631,10 +655,16 @@ __device__ __forceinline__ void v_stage(const inst_view<float> &v, const float *
             return k;
         };
         const int tl = (ny - 1) / 8 * 8;
-        bbk k = back(tl), k2 = back(tl - 8);
+        bbk k = back(tl), k2;
+        if constexpr (ahead) k2 = back(tl - 8);
         for (int t = tl; t >= 0; t -= 8) {
-            const bbk nk = k2;
-            k2 = back(t - 16);
+            bbk nk;
+            if constexpr (ahead) {
+                nk = k2;
+                k2 = back(t - 16);
+            } else if (t >= 8) {
+                nk = back(t - 8);
+            }
             float o[8];
 #pragma unroll
             for (int z = 7; z >= 0; --z) {
@@ -668,25 +698,25 @@ template <typename T> __device__ __forceinline__ inst_view<T> make_view(const bp
 #include "adi_delta.cuh"
 
 // One time step U -> Vn of scheme SCH with stage outputs in Y1, Y2, Y3; ends with a group barrier.
-template <int SCH>
+template <int SCH, typename DEPTH>
 __device__ __forceinline__ void fwd_step(const inst_view<float> &v, const float *U, float *Y1, float *Y2, float *Y3, float *Vn, float *sb0,
                                          double bnc, const grp &g)
 {
     const int l0 = g.t, ls = g.n;
     b1_stage<float>(v, U, sb0, bnc, l0, ls);
-    s_stage<1, SCH>(v, U, nullptr, nullptr, Y1, l0, ls);
+    s_stage<1, SCH, DEPTH>(v, U, nullptr, nullptr, Y1, l0, ls);
     g.sync();
     if constexpr (SCH == LSS_ADI_DOUGLAS_RACHFORD) {
-        v_stage(v, U, Y1, sb0, Vn, l0, ls);
+        v_stage<DEPTH>(v, U, Y1, sb0, Vn, l0, ls);
     } else {
-        v_stage(v, U, Y1, sb0, Y2, l0, ls);
+        v_stage<DEPTH>(v, U, Y1, sb0, Y2, l0, ls);
         g.sync();
-        s_stage<2, SCH>(v, U, Y1, Y2, Y3, l0, ls);
+        s_stage<2, SCH, DEPTH>(v, U, Y1, Y2, Y3, l0, ls);
         g.sync();
         if constexpr (SCH == LSS_ADI_HUNDSDORFER_VERWER)
-            v_stage(v, Y2, Y3, sb0, Vn, l0, ls);
+            v_stage<DEPTH>(v, Y2, Y3, sb0, Vn, l0, ls);
         else
-            v_stage(v, U, Y3, sb0, Vn, l0, ls);
+            v_stage<DEPTH>(v, U, Y3, sb0, Vn, l0, ls);
     }
     g.sync();
     b2_stage<float>(v, Vn, l0, ls);
@@ -715,8 +745,8 @@ template <typename T> __device__ __forceinline__ void load_payoff(const bparams<
         for (int j = g.t & 31; j < d.ny; j += 32) U[i * d.ld + j] = p.payoff[d.op + (long long)i * d.ny + j];
 }
 
-template <typename T, int SCH>
-__global__ void __launch_bounds__(BATCH_CTA, sizeof(T) == 8 ? 2 : 3) k_batch_forward(const __grid_constant__ bparams<T> p)
+template <typename T, int SCH, typename DEPTH>
+__global__ void __launch_bounds__(BATCH_CTA, sizeof(T) == 8 && DEPTH::AH == deep::AH ? 2 : 3) k_batch_forward(const __grid_constant__ bparams<T> p)
 {
     __shared__ int s_idx[MAX_GROUP_WARPS];
     __shared__ int s_bad[MAX_GROUP_WARPS];
@@ -735,8 +765,8 @@ __global__ void __launch_bounds__(BATCH_CTA, sizeof(T) == 8 ? 2 : 3) k_batch_for
         load_payoff(p, d, U, g);
         g.sync();
         for (int step = 0; step < d.steps; ++step) {
-            if constexpr (sizeof(T) == 8) delta_step<SCH>(v, d, U, Y1, Y2, Y3, Vn, sb0, g);
-            else fwd_step<SCH>(v, U, Y1, Y2, Y3, Vn, sb0, d.bnc, g);
+            if constexpr (sizeof(T) == 8) delta_step<SCH, DEPTH>(v, d, U, Y1, Y2, Y3, Vn, sb0, g);
+            else fwd_step<SCH, DEPTH>(v, U, Y1, Y2, Y3, Vn, sb0, d.bnc, g);
             T *tmp = U;
             U = Vn;
             Vn = tmp;
@@ -1027,6 +1057,7 @@ template <typename T> struct batch_typed {
     // (one launch per scheme present: each specialisation gets its own register allocation)
     struct group_plan {
         int grid = 0;
+        bool small = false; // forward: every instance has small lines
         int start[MAX_GROUP_WARPS + 1] = {}, cnt[MAX_GROUP_WARPS + 1] = {};
         long long need[MAX_GROUP_WARPS + 1] = {};
         std::vector<int> order, layout;
@@ -1342,6 +1373,14 @@ template <typename T> int batch_typed<T>::prepare_adjoint(cudaStream_t s)
     return make_plan(1);
 }
 
+// Instances that run with `shallow`, where no instance of their scheme is larger: most of what `deep` loads
+// ahead lies past the ends of their lines, and its registers leave fewer instances on an SM.  Forward,
+// 50 steps, ms with deep / shallow (and with the kernels before rows were loaded ahead): FP64 DR 20000 of
+// 8 x 8 8.2 / 6.7 (7.0), 1000 of 8 x 100 4.9 / 3.6 (4.3), 20000 of 64 x 16 53 / 46, but 1000 Craig-Sneyd of
+// 64 x 16 7.0 / 7.2; FP32 DR 20000 of 8 x 8 3.0 / 1.8 (1.4), of 16 x 16 4.5 / 3.8 (4.2), but 1000
+// Craig-Sneyd of 24 x 16 0.93 / 1.0.
+template <typename T> static bool small_lines(const bdesc &d) { return static_cast<long long>(d.nx) * d.ny <= (sizeof(T) == 8 ? 900 : 256); }
+
 // Workspace (doubles) of one instance checkpointed every c steps: nseg checkpoints, the stage
 // increments of one segment (4 arrays per step plus the segment's end), two scratch states, six
 // adjoint arrays and three line-end vectors.
@@ -1453,19 +1492,26 @@ template <typename T> int batch_typed<T>::make_plan(int mode)
         work[sc][cls[k]] += static_cast<double>(gps[k]) * slots / (2.0 * lines);
         warps_wanted[sc] += cls[k];
     }
-    int per_sm = 0;
+    int per_sm = 0, per_sm_small = 0;
     if constexpr (std::is_same<T, double>::value) {
         if (mode == 1)
             LSS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_fwdadj<LSS_ADI_CRAIG_SNEYD>, BATCH_CTA, 0),
                          "occupancy");
     }
-    if (mode == 0)
-        LSS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_forward<T, LSS_ADI_CRAIG_SNEYD>, BATCH_CTA, 0),
+    if (mode == 0) {
+        LSS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_forward<T, LSS_ADI_CRAIG_SNEYD, deep>, BATCH_CTA, 0),
                      "occupancy");
-    const int resident = sms * std::max(1, per_sm);
+        LSS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_small, k_batch_forward<T, LSS_ADI_CRAIG_SNEYD, shallow>, BATCH_CTA, 0),
+                     "occupancy");
+    }
     int grid[NSCHEMES];
-    for (int sc = 0; sc < NSCHEMES; ++sc)
+    for (int sc = 0; sc < NSCHEMES; ++sc) {
+        bool &small = mp.sch[sc].small;
+        small = mode == 0;
+        for (int k = 0; k < count; ++k) small = small && (desc[k].scheme != sc || small_lines<T>(desc[k]));
+        const int resident = sms * std::max(1, small ? per_sm_small : per_sm);
         grid[sc] = std::max(1, std::min(resident, (warps_wanted[sc] + MAX_GROUP_WARPS - 1) / MAX_GROUP_WARPS));
+    }
     mp.per_warp = 0;
     for (int sc = 0; sc < NSCHEMES; ++sc)
         for (int c = 0; c <= MAX_GROUP_WARPS; ++c) mp.sch[sc].need[c] = 0;
@@ -1547,12 +1593,17 @@ template <typename T> int batch_typed<T>::launch_forward(cudaStream_t s)
         const group_plan &g = plan[0].sch[sc];
         if (!g.grid) continue;
         const bparams<T> p = params_for(0, sc);
-        switch (sc) {
-        case LSS_ADI_DOUGLAS_RACHFORD: k_batch_forward<T, LSS_ADI_DOUGLAS_RACHFORD><<<g.grid, BATCH_CTA, 0, s>>>(p); break;
-        case LSS_ADI_CRAIG_SNEYD: k_batch_forward<T, LSS_ADI_CRAIG_SNEYD><<<g.grid, BATCH_CTA, 0, s>>>(p); break;
-        case LSS_ADI_MODIFIED_CRAIG_SNEYD: k_batch_forward<T, LSS_ADI_MODIFIED_CRAIG_SNEYD><<<g.grid, BATCH_CTA, 0, s>>>(p); break;
-        default: k_batch_forward<T, LSS_ADI_HUNDSDORFER_VERWER><<<g.grid, BATCH_CTA, 0, s>>>(p); break;
-        }
+        auto launch = [&](auto depth) {
+            using D = decltype(depth);
+            switch (sc) {
+            case LSS_ADI_DOUGLAS_RACHFORD: k_batch_forward<T, LSS_ADI_DOUGLAS_RACHFORD, D><<<g.grid, BATCH_CTA, 0, s>>>(p); break;
+            case LSS_ADI_CRAIG_SNEYD: k_batch_forward<T, LSS_ADI_CRAIG_SNEYD, D><<<g.grid, BATCH_CTA, 0, s>>>(p); break;
+            case LSS_ADI_MODIFIED_CRAIG_SNEYD: k_batch_forward<T, LSS_ADI_MODIFIED_CRAIG_SNEYD, D><<<g.grid, BATCH_CTA, 0, s>>>(p); break;
+            default: k_batch_forward<T, LSS_ADI_HUNDSDORFER_VERWER, D><<<g.grid, BATCH_CTA, 0, s>>>(p); break;
+            }
+        };
+        if (g.small) launch(shallow{});
+        else launch(deep{});
         LSS_CUDA_TRY(cudaGetLastError(), "batch: launching k_batch_forward");
         ++launches;
     }

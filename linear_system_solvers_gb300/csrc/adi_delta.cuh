@@ -40,9 +40,7 @@ __device__ __forceinline__ void st4(double *p, const double *o)
 
 enum { V_FIRST = 0, V_LAST = 1, V_LAST_HV = 2 };
 
-constexpr int AH = 5;  // rows loaded ahead of the right-hand sides
-constexpr int BK = 16; // rows of a block of the one-instruction passes
-constexpr int VB4 = 4; // blocks of four columns loaded ahead of the v lines' scaled passes
+constexpr int BK = deep::BK, VB4 = deep::VB4; // of the adjoint's passes
 
 // The explicit v = v_lo column and the rows of S_lo and S_max (b1_stage, b2_stage) in the order of
 // adi_wide.cuh: a single instance in relay order has the same bits.
@@ -69,12 +67,13 @@ __device__ __forceinline__ void db2_stage(const inst_view<double> &v, double *Vn
 }
 
 // One S stage.  KIND 1: A = U.  KIND 2: A = D2.  Y: the increment, rows 0 and nx-1 included.
-template <int KIND, int SCH>
+template <int KIND, int SCH, typename DEPTH = deep>
 __device__ __forceinline__ void ds_stage(const inst_view<double> &v, const bdesc &d, const double *U, const double *A, const double *D1,
                                          double *Y, int l0, int ls)
 {
     constexpr bool hv = SCH == LSS_ADI_HUNDSDORFER_VERWER, mcs = SCH == LSS_ADI_MODIFIED_CRAIG_SNEYD;
     constexpr bool six = KIND == 1 || hv || mcs; // the six-point operator enters
+    constexpr int AH = DEPTH::AH, BK = DEPTH::BK;
     const int nx = v.nx, ny = v.ny, ld = v.ld, e = nx - 2, last = (nx - 1) * ld;
     const double zeta = d.a_zeta, zt = d.a_zeta - d.a_theta;
     struct row {
@@ -186,10 +185,12 @@ __device__ __forceinline__ void ds_stage(const inst_view<double> &v, const bdesc
 }
 
 // One v stage (KIND, see adi_wide.cuh): right-hand side D (+ E), boundary column sb0.
-template <int KIND>
+template <int KIND, typename DEPTH = deep>
 __device__ __forceinline__ void dv_stage(const inst_view<double> &v, const double *U, const double *D, const double *E, const double *D2,
                                          const double *sb0, double *out, int l0, int ls)
 {
+    constexpr int BK = DEPTH::BK, VB4 = DEPTH::VB4;
+    static_assert(BK % 4 == 0, "columns move four at a time");
     const int nx = v.nx, ny = v.ny, ld = v.ld, e = ny - 2;
     for (int i = 1 + l0; i <= nx - 2; i += ls) {
         const int row = i * ld;
@@ -669,24 +670,24 @@ __device__ __forceinline__ void da_b1(const inst_view<double> &v, const bdesc &d
 }
 
 // One forward step U -> Vn by group g, stage increments in D1, D2, D3; ends with a group barrier.
-template <int SCH>
+template <int SCH, typename DEPTH = deep>
 __device__ __forceinline__ void delta_step(const inst_view<double> &v, const bdesc &d, const double *U, double *D1, double *D2, double *D3,
                                            double *Vn, double *sb0, const grp &g)
 {
     const int l0 = g.t, ls = g.n;
     db1_stage(v, d, U, sb0, l0, ls);
-    ds_stage<1, SCH>(v, d, U, U, nullptr, D1, l0, ls);
+    ds_stage<1, SCH, DEPTH>(v, d, U, U, nullptr, D1, l0, ls);
     if constexpr (SCH != LSS_ADI_DOUGLAS_RACHFORD) d2_edges(v, U, D2, l0, ls);
     g.sync();
     if constexpr (SCH == LSS_ADI_DOUGLAS_RACHFORD) {
-        dv_stage<V_LAST>(v, U, D1, nullptr, nullptr, sb0, Vn, l0, ls);
+        dv_stage<V_LAST, DEPTH>(v, U, D1, nullptr, nullptr, sb0, Vn, l0, ls);
     } else {
-        dv_stage<V_FIRST>(v, U, D1, nullptr, nullptr, sb0, D2, l0, ls);
+        dv_stage<V_FIRST, DEPTH>(v, U, D1, nullptr, nullptr, sb0, D2, l0, ls);
         g.sync();
-        ds_stage<2, SCH>(v, d, U, D2, D1, D3, l0, ls);
+        ds_stage<2, SCH, DEPTH>(v, d, U, D2, D1, D3, l0, ls);
         g.sync();
-        if constexpr (SCH == LSS_ADI_HUNDSDORFER_VERWER) dv_stage<V_LAST_HV>(v, U, D1, D3, D2, sb0, Vn, l0, ls);
-        else dv_stage<V_LAST>(v, U, D3, nullptr, nullptr, sb0, Vn, l0, ls);
+        if constexpr (SCH == LSS_ADI_HUNDSDORFER_VERWER) dv_stage<V_LAST_HV, DEPTH>(v, U, D1, D3, D2, sb0, Vn, l0, ls);
+        else dv_stage<V_LAST, DEPTH>(v, U, D3, nullptr, nullptr, sb0, Vn, l0, ls);
     }
     g.sync();
     db2_stage(v, Vn, l0, ls);
