@@ -308,11 +308,13 @@ template <typename T> struct inst_view {
     long long o2;
     int ox, oy;
     long long so, vo; // line tables
+    table_index<s_slots<T>()> si;
+    table_index<v_slots<T>()> vi;
     // line tables of the instance: row t of the S lines holds all its slots, column t of the v lines too (a
     // row's operands lie within a few KB instead of ten arenas: 5 to 15 % where a GPU full of 256 x 128
     // instances reads them from HBM)
-    __device__ __forceinline__ const T *S(int k, int t, int j) const { return p->S + so + table_at<s_slots<T>()>(t, k, j, ld); }
-    __device__ __forceinline__ const T *Vt(int k, int t, int i) const { return p->Vt + vo + table_at<v_slots<T>()>(t, k, i, nx); }
+    __device__ __forceinline__ const T *S(int k, int t, int j) const { return p->S + so + si.at(t, k, j); }
+    __device__ __forceinline__ const T *Vt(int k, int t, int i) const { return p->Vt + vo + vi.at(t, k, i); }
     __device__ __forceinline__ const T *X(int k) const { return p->X[k] + ox; }
     __device__ __forceinline__ const T *Yv(int k) const { return p->Yv[k] + oy; }
     __device__ __forceinline__ const int *imap() const { return p->imap + ox; }
@@ -688,8 +690,10 @@ template <typename T> __device__ __forceinline__ inst_view<T> make_view(const bp
     v.e_s = d.nx - 2;
     v.e_v = d.ny - 2;
     v.o2 = d.o2;
-    v.so = d.o2 * s_slots<T>();
-    v.vo = d.o2 * v_slots<T>();
+    v.si = table_index<s_slots<T>()>(d.ld);
+    v.vi = table_index<v_slots<T>()>(d.nx);
+    v.so = d.o2 * s_slots<T>() + v.si.base();
+    v.vo = d.o2 * v_slots<T>() + v.vi.base();
     v.ox = d.ox;
     v.oy = d.oy;
     return v;
@@ -984,8 +988,9 @@ static __global__ void k_setup_s_delta(setup_params sp, double *S0)
         const double a = -th * M, b = 1.0 + th * Z, c = -th * P;
         const double ib = 1.0 / fma(-a, gam, b);
         gam = c * ib;
-        double *row = S0 + d.o2 * DS_COUNT;
-        auto slot = [&](int k) -> double & { return row[table_at<DS_COUNT>(t, k, j, ld)]; };
+        const table_index<DS_COUNT> si(ld);
+        double *tab = S0 + d.o2 * DS_COUNT + si.base();
+        auto slot = [&](int k) -> double & { return tab[si.at(t, k, j)]; };
         slot(DS_LA) = a * ib;
         slot(DS_G) = gam;
         slot(DS_WG) = gm * C * ib;

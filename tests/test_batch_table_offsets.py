@@ -28,4 +28,4 @@ def test_offsets_of_the_largest_grids():
 def test_kernels_reach_their_tables_through_it():
     src = open(os.path.join(CSRC, "adi_batched.cu")).read()
     view = re.search(r"struct inst_view \{.*?\n\};", src, re.S).group(0)
-    assert "table_at<s_slots<T>()>(t, k, j, ld)" in view and "table_at<v_slots<T>()>(t, k, i, nx)" in view
+    assert "si.at(t, k, j)" in view and "vi.at(t, k, i)" in view
