@@ -97,14 +97,15 @@ typedef struct lss_heat1d_batch lss_heat1d_batch;
 /* Builds a batch of independent problems (any sizes, steps, boundary kinds) and uploads it.
  * arith: LSS_ADI_ARITH_REFERENCE (the reference's operation order, IEEE divisions, no
  * contraction: bit-identical to its host policy) or LSS_ADI_ARITH_FAST (one factorisation per
- * instance, reciprocal pivots, FMA: within rounding of the reference).  options: LSS_HEAT1D_OPT_*. */
+ * instance, reciprocal pivots, FMA: within rounding of the reference; in FP64 the sweep of lines of up to
+ * 100 points is chosen by the whole book, so their last bits may differ between books).  options: LSS_HEAT1D_OPT_*. */
 int lss_heat1d_batch_create(const lss_heat1d_tables *problems, int count, int precision, int arith, int options,
                             lss_heat1d_batch **b);
 int lss_heat1d_batch_create_bs(const lss_heat1d_bs *problems, int count, int precision, int arith, int options,
                                lss_heat1d_batch **b);
 
-/* Runs every instance's whole time loop: one kernel launch (device-resident, asynchronous on
- * `stream`).  The initial conditions are those uploaded by create or the last run_host. */
+/* Runs every instance's whole time loop: one kernel launch, or two where the book has lines for both
+ * sweeps of the FAST arithmetic (device-resident, asynchronous on `stream`).  The initial conditions are those uploaded by create or the last run_host. */
 int lss_heat1d_batch_run(lss_heat1d_batch *b, void *stream);
 
 /* End-to-end step: uploads `initials` (concatenated n values per instance in creation order,

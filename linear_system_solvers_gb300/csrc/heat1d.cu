@@ -880,10 +880,17 @@ template <bool SRC, bool KEEP> __global__ void __launch_bounds__(LANES, 8) k_h1_
     const h1unit un = p.units[blockIdx.x];
     switch (un.R) {
     case 4: h1_reg_unit<double, 4, SRC, KEEP>(p, un, scan, sq); break;
+    case 5: h1_reg_unit<double, 5, SRC, KEEP>(p, un, scan, sq); break;
+    case 6: h1_reg_unit<double, 6, SRC, KEEP>(p, un, scan, sq); break;
+    case 7: h1_reg_unit<double, 7, SRC, KEEP>(p, un, scan, sq); break;
     case 8: h1_reg_unit<double, 8, SRC, KEEP>(p, un, scan, sq); break;
+    case 9: h1_reg_unit<double, 9, SRC, KEEP>(p, un, scan, sq); break;
     case 10: h1_reg_unit<double, 10, SRC, KEEP>(p, un, scan, sq); break;
+    case 11: h1_reg_unit<double, 11, SRC, KEEP>(p, un, scan, sq); break;
     case 12: h1_reg_unit<double, 12, SRC, KEEP>(p, un, scan, sq); break;
+    case 13: h1_reg_unit<double, 13, SRC, KEEP>(p, un, scan, sq); break;
     case 14: h1_reg_unit<double, 14, SRC, KEEP>(p, un, scan, sq); break;
+    case 15: h1_reg_unit<double, 15, SRC, KEEP>(p, un, scan, sq); break;
     default: h1_reg_unit<double, H1_RMAX, SRC, KEEP>(p, un, scan, sq); break;
     }
 }
@@ -1071,23 +1078,19 @@ template <bool KEEP> __global__ void __launch_bounds__(LANES, 16) k_h1_relay(con
     const h1unit un = p.units[blockIdx.x];
     switch (un.R) {
     case 4: h1_relay_unit<4, KEEP>(p, un); break;
+    case 5: h1_relay_unit<5, KEEP>(p, un); break;
+    case 6: h1_relay_unit<6, KEEP>(p, un); break;
+    case 7: h1_relay_unit<7, KEEP>(p, un); break;
     case 8: h1_relay_unit<8, KEEP>(p, un); break;
+    case 9: h1_relay_unit<9, KEEP>(p, un); break;
     case 10: h1_relay_unit<10, KEEP>(p, un); break;
+    case 11: h1_relay_unit<11, KEEP>(p, un); break;
     case 12: h1_relay_unit<12, KEEP>(p, un); break;
+    case 13: h1_relay_unit<13, KEEP>(p, un); break;
     case 14: h1_relay_unit<14, KEEP>(p, un); break;
+    case 15: h1_relay_unit<15, KEEP>(p, un); break;
     default: h1_relay_unit<H1_RMAX, KEEP>(p, un); break;
     }
-}
-
-// Lanes per instance and rows per lane for lines of `n` points: the fewest lanes (4 .. 32) whose
-// rows fit 16 per lane -- fewer scan levels per row -- then the fewest rows of the compiled ones.
-static inline void h1_shape(int n, int &W, int &R)
-{
-    W = 4;
-    while (W * H1_RMAX < n) W *= 2;
-    R = H1_RMAX;
-    for (int c : {14, 12, 10, 8, 4})
-        if (W * c >= n) R = c;
 }
 
 // scatter of per-instance contiguous tables into the interleaved group layout (the instance of
@@ -1194,6 +1197,16 @@ template <typename T> struct batch_t : batch_base {
         p.nwarps = sched.ctas * sched.warps_per_cta;
         return p;
     }
+    // most rows that an instance of a group solves in registers (k_h1_relay: between its first and last)
+    int group_rows(size_t g) const
+    {
+        int rows = 0;
+        for (int l = 0; l < groups[g].lanes; ++l) {
+            const h1lane &L = lanes[g * LANES + l];
+            rows = std::max(rows, L.end - L.start + 1);
+        }
+        return groups[g].reg == 2 ? rows - 2 : rows;
+    }
     int build(std::vector<inst_info> &&inf, std::vector<host_tables<T>> &tabs);
     int run(cudaStream_t s);
     int launches() const override { return arith == LSS_ADI_ARITH_FAST ? (nunits > 0) + (sched.ctas > 0) : 1; }
@@ -1231,8 +1244,8 @@ template <typename T> int batch_t<T>::build(std::vector<inst_info> &&inf, std::v
         }
         G.lanes = l;
         G.steps = steps;
-        // FP64 lines that fit a warp's registers.  Against the sweep through memory (a thread per
-        // instance): 4096 Black-Scholes calls of 101..512 points, 100..1000 steps 104 ms -> 7.8 ms.
+        // FP64 lines that fit a warp's registers (but see memory_limit).  Against the sweep through memory (a
+        // thread per instance): 4096 Black-Scholes calls of 101..512 points, 100..1000 steps 104 ms -> 7.8 ms.
         // FP32 lines without sources keep that sweep's operations and their order (k_h1_relay): 8192 calls
         // of the same sizes 22.2 ms -> 4.9 ms.  Sources and longer lines stay in memory.
         G.reg = 0;
@@ -1285,6 +1298,18 @@ template <typename T> int batch_t<T>::build(std::vector<inst_info> &&inf, std::v
         L.lo_lin = f.lo_lin;
         L.hi_lin = f.hi_lin;
         L.init_off = init_off[i];
+    }
+    // FP64 groups of short lines in a book that fills the GPU go back to the sweep through memory
+    {
+        int dev = 0, sms = 0;
+        LSS_CUDA_TRY(cudaGetDevice(&dev), "heat1d: device");
+        LSS_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "heat1d: SM count");
+        std::vector<group_cost> cost;
+        for (size_t g = 0; g < groups.size(); ++g)
+            if (groups[g].reg == 1) cost.push_back({groups[g].n, group_rows(g), groups[g].lanes, groups[g].steps});
+        const int limit = memory_limit(cost, sms, H1_RMAX);
+        for (h1group &G : groups)
+            if (G.reg == 1 && G.n <= limit) G.reg = 0;
     }
     // flat host arrays in creation order
     std::vector<T> coef_flat, init_flat(total_init), bnd_flat, src_flat;
@@ -1396,6 +1421,14 @@ template <typename T> int batch_t<T>::build(std::vector<inst_info> &&inf, std::v
         // lines that fit a warp's registers: one unit per 32 / W instances of a group, costliest first
         std::vector<h1unit> units;
         std::vector<int> mem_groups;
+        double warps = 0.0; // of the FP64 groups on the fewest lanes
+        for (size_t g = 0; g < groups.size(); ++g)
+            if (groups[g].reg == 1) {
+                int W = 0, R = 0;
+                register_shape(group_rows(g), 4, H1_RMAX, W, R);
+                warps += (groups[g].lanes * W + 31) / 32;
+            }
+        const bool idle = warps <= 8.0 * sms; // two warps per SM sub-partition
         for (size_t g = 0; g < groups.size(); ++g) {
             const h1group &G = groups[g];
             if (!G.reg) {
@@ -1403,7 +1436,10 @@ template <typename T> int batch_t<T>::build(std::vector<inst_info> &&inf, std::v
                 continue;
             }
             int W = 0, R = 0;
-            h1_shape(G.n, W, R);
+            const int rows = group_rows(g);
+            int least = G.reg == 1 ? 4 : 2;
+            if (G.reg == 1 && idle) register_shape(G.n, 4, H1_RMAX, least, R);
+            register_shape(rows, least, H1_RMAX, W, R);
             for (int l = 0; l < G.lanes; l += 32 / W) {
                 h1unit u{static_cast<int>(g), l, std::min(32 / W, G.lanes - l), W, R, 0};
                 for (int q = 0; q < u.sub; ++q) u.steps = std::max(u.steps, lanes[g * LANES + l + q].steps);
