@@ -101,7 +101,7 @@ template <typename T> struct h1params {
     const h1unit *units;   // factorised sweep in registers: one warp per unit
     const int *warp_first; // factorised sweep through memory: the groups of warp w are
     const int *warp_group; // warp_group[warp_first[w] .. warp_first[w + 1])
-    int nwarps;
+    int nwarps, warps_per_cta; // (a CTA is launched with the warps that have groups)
 };
 
 __device__ __forceinline__ long long el(int t) { return static_cast<long long>(t) * LANES; }
@@ -636,8 +636,9 @@ __device__ __forceinline__ void h1_fast_group(const h1params<T> p, const int g, 
 template <typename T, int PF, bool SRC, bool KEEP>
 __global__ void __launch_bounds__(h1_warps<T>() * LANES, 1) k_h1_fast(const h1params<T> p)
 {
-    const int w = blockIdx.x * (blockDim.x / LANES) + threadIdx.x / LANES;
+    const int w = blockIdx.x * p.warps_per_cta + threadIdx.x / LANES;
     const int lane = threadIdx.x % LANES;
+    asm volatile("griddepcontrol.launch_dependents;"); // the sweep in registers of the same run may start
     if (w >= p.nwarps) return;
     const int q1 = p.warp_first[w + 1];
     for (int q = p.warp_first[w]; q < q1; ++q) h1_fast_group<T, PF, SRC, KEEP>(p, p.warp_group[q], lane);
@@ -668,6 +669,10 @@ __global__ void __launch_bounds__(h1_warps<T>() * LANES, 1) k_h1_fast(const h1pa
 // ------------------------------------------------------------------------------------------
 constexpr int H1_SCAN = 5; // log2(32)
 constexpr int H1_RMAX = 16;    // rows per lane that fit the registers (l, g, u and the sweep's values)
+
+// Launched behind the sweep through memory, a sweep in registers runs beside it (the two share no instance);
+// it ends after it, so that its end is the run's.
+__device__ __forceinline__ void end_of_run() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Factors of one instance per thread, in double, written over the group's slots: l -> S_M,
 // g -> S_G, q -> S_K (zero on rows that are not solved).  Groups of larger lines keep k_h1_setup_fast.
@@ -893,6 +898,7 @@ template <bool SRC, bool KEEP> __global__ void __launch_bounds__(LANES, 8) k_h1_
     case 15: h1_reg_unit<double, 15, SRC, KEEP>(p, un, scan, sq); break;
     default: h1_reg_unit<double, H1_RMAX, SRC, KEEP>(p, un, scan, sq); break;
     }
+    end_of_run();
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1091,6 +1097,7 @@ template <bool KEEP> __global__ void __launch_bounds__(LANES, 16) k_h1_relay(con
     case 15: h1_relay_unit<15, KEEP>(p, un); break;
     default: h1_relay_unit<H1_RMAX, KEEP>(p, un); break;
     }
+    end_of_run();
 }
 
 // scatter of per-instance contiguous tables into the interleaved group layout (the instance of
@@ -1195,6 +1202,7 @@ template <typename T> struct batch_t : batch_base {
         p.warp_first = d_wfirst.p;
         p.warp_group = d_wgroup.p;
         p.nwarps = sched.ctas * sched.warps_per_cta;
+        p.warps_per_cta = sched.warps_per_cta;
         return p;
     }
     // most rows that an instance of a group solves in registers (k_h1_relay: between its first and last)
@@ -1475,27 +1483,33 @@ template <typename T> int batch_t<T>::run(cudaStream_t s)
     const int blocks = grid_for(static_cast<long long>(groups.size()) * LANES, 128);
     const bool keep = d_all.p != nullptr, src = d_src.p != nullptr;
     if (arith == LSS_ADI_ARITH_FAST) {
-        if constexpr (std::is_same<T, double>::value) {
-            if (nunits) {
-                if (keep && src) k_h1_reg<true, true><<<nunits, LANES, 0, s>>>(p);
-                else if (keep) k_h1_reg<false, true><<<nunits, LANES, 0, s>>>(p);
-                else if (src) k_h1_reg<true, false><<<nunits, LANES, 0, s>>>(p);
-                else k_h1_reg<false, false><<<nunits, LANES, 0, s>>>(p);
-                LSS_CUDA_TRY(cudaGetLastError(), "heat1d: launching the time loop");
-            }
-        } else if (nunits) {
-            if (keep) k_h1_relay<true><<<nunits, LANES, 0, s>>>(p);
-            else k_h1_relay<false><<<nunits, LANES, 0, s>>>(p);
+        const int ctas = sched.ctas, th = sched.warps_used() * LANES;
+        if (ctas) {
+            if (keep && src) k_h1_fast<T, H1_PF, true, true><<<ctas, th, 0, s>>>(p);
+            else if (keep) k_h1_fast<T, H1_PF, false, true><<<ctas, th, 0, s>>>(p);
+            else if (src) k_h1_fast<T, H1_PF, true, false><<<ctas, th, 0, s>>>(p);
+            else k_h1_fast<T, H1_PF, false, false><<<ctas, th, 0, s>>>(p);
             LSS_CUDA_TRY(cudaGetLastError(), "heat1d: launching the time loop");
         }
-        const int ctas = sched.ctas, th = h1_warps<T>() * LANES;
-        if (!ctas) return LSS_ADI_OK;
-        if (keep && src) k_h1_fast<T, H1_PF, true, true><<<ctas, th, 0, s>>>(p);
-        else if (keep) k_h1_fast<T, H1_PF, false, true><<<ctas, th, 0, s>>>(p);
-        else if (src) k_h1_fast<T, H1_PF, true, false><<<ctas, th, 0, s>>>(p);
-        else k_h1_fast<T, H1_PF, false, false><<<ctas, th, 0, s>>>(p);
+        if (!nunits) return LSS_ADI_OK;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(nunits);
+        cfg.blockDim = dim3(LANES);
+        cfg.stream = s;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = ctas ? 1 : 0;
+        void (*k)(const h1params<T>);
+        if constexpr (std::is_same<T, double>::value)
+            k = keep && src ? k_h1_reg<true, true> : keep ? k_h1_reg<false, true> : src ? k_h1_reg<true, false> : k_h1_reg<false, false>;
+        else
+            k = keep ? k_h1_relay<true> : k_h1_relay<false>;
+        LSS_CUDA_TRY(cudaLaunchKernelEx(&cfg, k, p), "heat1d: launching the time loop");
+        return LSS_ADI_OK;
     }
-    else if constexpr (std::is_same<T, double>::value) {
+    if constexpr (std::is_same<T, double>::value) {
         if (ds) k_h1_ref64<true, 4><<<blocks, 128, 0, s>>>(p);
         else k_h1_ref64<false, 4><<<blocks, 128, 0, s>>>(p);
     } else {

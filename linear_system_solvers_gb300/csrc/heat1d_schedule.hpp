@@ -29,6 +29,15 @@ struct warp_schedule {
     int warps_per_cta = 0;
     std::vector<int> first; // per warp (ctas * warps_per_cta + 1 entries): start of its list in `group`
     std::vector<int> group; // group indices, warp after warp
+    // warps of a CTA up to the last that has groups in any: the others are not launched and leave their
+    // registers to what runs beside
+    int warps_used() const
+    {
+        int used = 0;
+        for (size_t w = 0; w + 1 < first.size(); ++w)
+            if (first[w + 1] > first[w]) used = std::max(used, static_cast<int>(w) % warps_per_cta + 1);
+        return used;
+    }
 };
 
 // work[g]: cost of group g (points x time steps).  sms: SMs of the device; warps_per_cta: a

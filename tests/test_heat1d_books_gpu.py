@@ -45,3 +45,18 @@ def test_every_number_of_solved_rows(lss, oracle, n, lo, hi):
     b = lss.tabulated_batch([t] * 3, "f64", "fast")
     b.run_host()
     assert rel_err(b.solution(2), oracle.solve_1d(p, "f64")) < 1e-10
+
+
+@pytest.mark.parametrize("precision", ["f64", "f32"])
+def test_both_sweeps_of_a_book_end_with_the_run(lss, precision):
+    """Lines for both sweeps in one book, which run beside each other: runs that follow at once on the same
+    stream, and a read of the results queued behind them, see the values of each sweep alone."""
+    short, long_lines = book(lss, 500, 400, nt=40), book(lss, 700, 30, nt=40)
+    b = lss.black_scholes_batch(short + long_lines, precision)
+    assert b.launch_count() == 2
+    want = np.concatenate([lss.black_scholes_batch(q, precision).run_host()[0] for q in (short, long_lines)])
+    for _ in range(20):
+        for _ in range(3):
+            b.run()
+        v, st = b.results()
+        assert not st.any() and np.array_equal(v, want)
