@@ -20,6 +20,7 @@
 
 #include "adi_batched.hpp"
 #include "adi_index.hpp"
+#include "adi_threads.hpp"
 
 namespace lss_gb300 {
 
@@ -1185,104 +1186,93 @@ template <typename T> int batch_typed<T>::create(const lss_adi_problem *ps, int 
     std::vector<double> scal(3 * static_cast<size_t>(n));
     std::vector<T> pay(static_cast<size_t>(total_flat));
     const unsigned nthr = std::max(1u, std::min(32u, std::thread::hardware_concurrency()));
-    std::vector<std::thread> pool;
-    std::vector<int> errs(nthr, 0);
-    for (unsigned w = 0; w < nthr; ++w) {
-        pool.emplace_back([&, w]() {
-            try {
-                for (int k = static_cast<int>(w); k < n; k += static_cast<int>(nthr)) {
-                    instance_tables<T> tt;
-                    build_tables_for<T>(ps[k], tt);
-                    const bdesc &d = desc[k];
-                    const size_t nn = static_cast<size_t>(d.nx) * d.ny;
-                    for (int s = 0; s < 7; ++s)
-                        for (int i = 0; i < d.nx; ++i) {
-                            double *dst = base.data() + s * static_cast<size_t>(total_n) + d.o2 + static_cast<size_t>(i) * d.ld;
-                            const T *src = tt.coef.data() + s * nn + static_cast<size_t>(i) * d.ny;
-                            for (int j = 0; j < d.ny; ++j) dst[j] = static_cast<double>(src[j]);
-                        }
-                    std::copy(tt.payoff.begin(), tt.payoff.end(), pay.begin() + d.op);
-                    const double th = tt.sc.theta, ni = tt.sc.ni, dl = tt.sc.delta, rk = tt.sc.rho;
-                    scal[3 * k] = th;
-                    scal[3 * k + 1] = static_cast<double>(tt.sc.zeta);
-                    scal[3 * k + 2] = static_cast<double>(tt.sc.gamma);
-                    for (int i = 0; i < d.nx; ++i) {
-                        const double D = tt.coef_v0[i], E = tt.coef_v0[d.nx + i], F = tt.coef_v0[2 * d.nx + i];
-                        xh[XB_M * total_x + d.ox + i] = static_cast<T>(-dl * D);
-                        xh[XB_C * total_x + d.ox + i] = static_cast<T>(1.0 - 3.0 * ni * E + rk * F);
-                        xh[XB_P * total_x + d.ox + i] = static_cast<T>(dl * D);
-                        xh[XB_2 * total_x + d.ox + i] = static_cast<T>(-ni * E);
-                        xh[XB_1 * total_x + d.ox + i] = static_cast<T>(4.0 * ni * E);
-                        xh[X_VHI * total_x + d.ox + i] = tt.v_hi[i];
-                        imh[d.ox + i] = tt.imap[i];
-                    }
-                    const double h1 = tt.sc.h1;
-                    {
-                        // coefficient derivatives (adjoint), double
-                        sinh_map<double> g;
-                        g.init(ps[k]);
-                        const double sg = ps[k].sigma, bt = ps[k].sabr_beta;
-                        for (int i = 0; i < d.nx; ++i) {
-                            const s_factors q = derivative_s(ps[k], g, static_cast<double>(tt.sc.h1) * i);
-                            xh[X_HX * total_x + d.ox + i] = static_cast<T>(q.hx);
-                            xh[X_HC * total_x + d.ox + i] = static_cast<T>(q.hc);
-                            xh[X_HA * total_x + d.ox + i] = static_cast<T>(q.ha);
-                            xh[X_HDD * total_x + d.ox + i] = static_cast<T>(q.hdd);
-                        }
-                        for (int j = 0; j < d.ny; ++j) {
-                            const v_factors q = derivative_v(ps[k], g, static_cast<double>(tt.sc.h2) * j);
-                            yh[Y_HY * total_y + d.oy + j] = static_cast<T>(q.hy);
-                            yh[Y_BS * total_y + d.oy + j] = static_cast<T>(q.bs);
-                            yh[Y_EK * total_y + d.oy + j] = static_cast<T>(q.ek);
-                            yh[Y_ET * total_y + d.oy + j] = static_cast<T>(q.et);
-                            yh[Y_ES * total_y + d.oy + j] = static_cast<T>(q.es);
-                            yh[Y_HV2 * total_y + d.oy + j] = static_cast<T>(q.hv2);
-                        }
-                        desc[k].model = ps[k].model;
-                        desc[k].a_alphat = static_cast<double>(tt.sc.alpha);
-                        desc[k].a_omb = 1.0 - bt;
-                        const double kk = static_cast<double>(tt.sc.k);
-                        desc[k].a_tau0 = ps[k].forward ? ps[k].maturity - kk : kk;
-                        desc[k].a_dtau = ps[k].forward ? -kk : kk;
-                        desc[k].a_delta = static_cast<double>(tt.sc.delta);
-                        desc[k].a_halfk = 0.5 * static_cast<double>(tt.sc.k);
-                        desc[k].a_ni = static_cast<double>(tt.sc.ni);
-                        desc[k].a_betat = static_cast<double>(tt.sc.beta);
-                        desc[k].a_sigma = sg;
-                        desc[k].a_rho = ps[k].rho;
-                        desc[k].a_theta = static_cast<double>(tt.sc.theta);
-                        desc[k].a_zeta = static_cast<double>(tt.sc.zeta);
-                        desc[k].a_gamma = static_cast<double>(tt.sc.gamma);
-                        desc[k].a_k = static_cast<double>(tt.sc.k);
-                        desc[k].ck = std::max(1, static_cast<int>(std::ceil(std::sqrt(static_cast<double>(d.steps)))));
-                    }
-                    for (int j = 0; j < d.ny; ++j) {
-                        yh[Y_SLO * total_y + d.oy + j] = tt.s_lo[j];
-                        yh[Y_B2C * total_y + d.oy + j] = static_cast<T>(2.0 * h1 * static_cast<double>(tt.s_hi_neu[j]) / 3.0);
-                        jmh[d.oy + j] = tt.jmap[j];
-                    }
-                    // modified Craig-Sneyd with zeta == theta adds (zeta - theta) * (...) = 0: it is
-                    // Craig-Sneyd (the reference's surfaces are bit-identical), so run the CS stencil
-                    if (ps[k].scheme == LSS_ADI_MODIFIED_CRAIG_SNEYD && tt.sc.zeta == tt.sc.theta)
-                        desc[k].scheme = LSS_ADI_CRAIG_SNEYD;
-                    const double DN = tt.coef_v0[d.nx - 1];
-                    desc[k].bnc = -dl * (2.0 * h1 * static_cast<double>(tt.s_hi_neu[0])) * DN;
-                    const bilinear b = make_bilinear(tt.x.data(), d.nx, tt.y.data(), d.ny, ps[k].eval_s, ps[k].eval_v);
-                    desc[k].i0 = b.i0;
-                    desc[k].j0 = b.j0;
-                    desc[k].w00 = b.w00;
-                    desc[k].w10 = b.w10;
-                    desc[k].w01 = b.w01;
-                    desc[k].w11 = b.w11;
+    run_shares(nthr, [&](unsigned w) {
+        for (int k = static_cast<int>(w); k < n; k += static_cast<int>(nthr)) {
+            instance_tables<T> tt;
+            build_tables_for<T>(ps[k], tt);
+            const bdesc &d = desc[k];
+            const size_t nn = static_cast<size_t>(d.nx) * d.ny;
+            for (int s = 0; s < 7; ++s)
+                for (int i = 0; i < d.nx; ++i) {
+                    double *dst = base.data() + s * static_cast<size_t>(total_n) + d.o2 + static_cast<size_t>(i) * d.ld;
+                    const T *src = tt.coef.data() + s * nn + static_cast<size_t>(i) * d.ny;
+                    for (int j = 0; j < d.ny; ++j) dst[j] = static_cast<double>(src[j]);
                 }
-            } catch (...) {
-                errs[w] = 1;
+            std::copy(tt.payoff.begin(), tt.payoff.end(), pay.begin() + d.op);
+            const double th = tt.sc.theta, ni = tt.sc.ni, dl = tt.sc.delta, rk = tt.sc.rho;
+            scal[3 * k] = th;
+            scal[3 * k + 1] = static_cast<double>(tt.sc.zeta);
+            scal[3 * k + 2] = static_cast<double>(tt.sc.gamma);
+            for (int i = 0; i < d.nx; ++i) {
+                const double D = tt.coef_v0[i], E = tt.coef_v0[d.nx + i], F = tt.coef_v0[2 * d.nx + i];
+                xh[XB_M * total_x + d.ox + i] = static_cast<T>(-dl * D);
+                xh[XB_C * total_x + d.ox + i] = static_cast<T>(1.0 - 3.0 * ni * E + rk * F);
+                xh[XB_P * total_x + d.ox + i] = static_cast<T>(dl * D);
+                xh[XB_2 * total_x + d.ox + i] = static_cast<T>(-ni * E);
+                xh[XB_1 * total_x + d.ox + i] = static_cast<T>(4.0 * ni * E);
+                xh[X_VHI * total_x + d.ox + i] = tt.v_hi[i];
+                imh[d.ox + i] = tt.imap[i];
             }
-        });
-    }
-    for (auto &t : pool) t.join();
-    for (int e : errs)
-        if (e) return set_error(LSS_ADI_ENOMEM, "batch: host table construction failed");
+            const double h1 = tt.sc.h1;
+            {
+                // coefficient derivatives (adjoint), double
+                sinh_map<double> g;
+                g.init(ps[k]);
+                const double sg = ps[k].sigma, bt = ps[k].sabr_beta;
+                for (int i = 0; i < d.nx; ++i) {
+                    const s_factors q = derivative_s(ps[k], g, static_cast<double>(tt.sc.h1) * i);
+                    xh[X_HX * total_x + d.ox + i] = static_cast<T>(q.hx);
+                    xh[X_HC * total_x + d.ox + i] = static_cast<T>(q.hc);
+                    xh[X_HA * total_x + d.ox + i] = static_cast<T>(q.ha);
+                    xh[X_HDD * total_x + d.ox + i] = static_cast<T>(q.hdd);
+                }
+                for (int j = 0; j < d.ny; ++j) {
+                    const v_factors q = derivative_v(ps[k], g, static_cast<double>(tt.sc.h2) * j);
+                    yh[Y_HY * total_y + d.oy + j] = static_cast<T>(q.hy);
+                    yh[Y_BS * total_y + d.oy + j] = static_cast<T>(q.bs);
+                    yh[Y_EK * total_y + d.oy + j] = static_cast<T>(q.ek);
+                    yh[Y_ET * total_y + d.oy + j] = static_cast<T>(q.et);
+                    yh[Y_ES * total_y + d.oy + j] = static_cast<T>(q.es);
+                    yh[Y_HV2 * total_y + d.oy + j] = static_cast<T>(q.hv2);
+                }
+                desc[k].model = ps[k].model;
+                desc[k].a_alphat = static_cast<double>(tt.sc.alpha);
+                desc[k].a_omb = 1.0 - bt;
+                const double kk = static_cast<double>(tt.sc.k);
+                desc[k].a_tau0 = ps[k].forward ? ps[k].maturity - kk : kk;
+                desc[k].a_dtau = ps[k].forward ? -kk : kk;
+                desc[k].a_delta = static_cast<double>(tt.sc.delta);
+                desc[k].a_halfk = 0.5 * static_cast<double>(tt.sc.k);
+                desc[k].a_ni = static_cast<double>(tt.sc.ni);
+                desc[k].a_betat = static_cast<double>(tt.sc.beta);
+                desc[k].a_sigma = sg;
+                desc[k].a_rho = ps[k].rho;
+                desc[k].a_theta = static_cast<double>(tt.sc.theta);
+                desc[k].a_zeta = static_cast<double>(tt.sc.zeta);
+                desc[k].a_gamma = static_cast<double>(tt.sc.gamma);
+                desc[k].a_k = static_cast<double>(tt.sc.k);
+                desc[k].ck = std::max(1, static_cast<int>(std::ceil(std::sqrt(static_cast<double>(d.steps)))));
+            }
+            for (int j = 0; j < d.ny; ++j) {
+                yh[Y_SLO * total_y + d.oy + j] = tt.s_lo[j];
+                yh[Y_B2C * total_y + d.oy + j] = static_cast<T>(2.0 * h1 * static_cast<double>(tt.s_hi_neu[j]) / 3.0);
+                jmh[d.oy + j] = tt.jmap[j];
+            }
+            // modified Craig-Sneyd with zeta == theta adds (zeta - theta) * (...) = 0: it is
+            // Craig-Sneyd (the reference's surfaces are bit-identical), so run the CS stencil
+            if (ps[k].scheme == LSS_ADI_MODIFIED_CRAIG_SNEYD && tt.sc.zeta == tt.sc.theta)
+                desc[k].scheme = LSS_ADI_CRAIG_SNEYD;
+            const double DN = tt.coef_v0[d.nx - 1];
+            desc[k].bnc = -dl * (2.0 * h1 * static_cast<double>(tt.s_hi_neu[0])) * DN;
+            const bilinear b = make_bilinear(tt.x.data(), d.nx, tt.y.data(), d.ny, ps[k].eval_s, ps[k].eval_v);
+            desc[k].i0 = b.i0;
+            desc[k].j0 = b.j0;
+            desc[k].w00 = b.w00;
+            desc[k].w10 = b.w10;
+            desc[k].w01 = b.w01;
+            desc[k].w11 = b.w11;
+        }
+    });
 
     // longest instances first
     order.resize(n);

@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "adi_batched.hpp"
+#include "adi_threads.hpp"
 #include "adi_wide.cuh"
 
 namespace lss_gb300 {
@@ -108,13 +109,8 @@ template <typename T> struct line_solver {
                         for (int j = 0; j < ny; ++j) dst[j] = static_cast<double>(src[j]);
                     }
             };
-            if (flat < 100000 || nthr == 1) {
-                fill(0, 1);
-            } else {
-                std::vector<std::thread> pool;
-                for (unsigned w = 0; w < nthr; ++w) pool.emplace_back(fill, w, nthr);
-                for (auto &t : pool) t.join();
-            }
+            const unsigned shares = flat < 100000 ? 1 : nthr;
+            run_shares(shares, [&](unsigned w) { fill(w, shares); });
             LSS_CUDA_TRY(base.upload(hb.data(), hb.size()), "wide: uploading coefficient tables");
         }
         if (!td_case) k_wide_setup_s<T><<<grid_for(ny - 2, 32), 32>>>(base.p, n, nx, ny, ld, th, gm, stab.p);

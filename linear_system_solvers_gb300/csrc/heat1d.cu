@@ -26,6 +26,7 @@
 
 #include "adi_common.hpp"
 #include "adi_device.cuh"
+#include "adi_threads.hpp"
 #include "heat1d_schedule.hpp"
 
 #include <algorithm>
@@ -1693,12 +1694,9 @@ static int create_bs(const lss_heat1d_bs *ps, int count, int arith, int options,
     std::vector<host_tables<T>> tabs(count);
     const unsigned hw = std::max(1u, std::min(64u, std::thread::hardware_concurrency()));
     const int nthr = static_cast<int>(std::min<long long>(hw, count));
-    std::vector<std::thread> pool;
-    for (int w = 0; w < nthr; ++w)
-        pool.emplace_back([&, w]() {
-            for (int i = w; i < count; i += nthr) bs_tables<T>(ps[i], tabs[i], info[i]);
-        });
-    for (auto &t : pool) t.join();
+    run_shares(static_cast<unsigned>(nthr), [&](unsigned w) {
+        for (int i = static_cast<int>(w); i < count; i += nthr) bs_tables<T>(ps[i], tabs[i], info[i]);
+    });
     auto bt = std::make_unique<batch_t<T>>();
     bt->precision = std::is_same<T, double>::value ? LSS_ADI_FP64 : LSS_ADI_FP32;
     bt->arith = arith;
