@@ -326,16 +326,14 @@ template <typename T> __device__ __forceinline__ T ldg(const T *p) { return __ld
 
 // Explicitly rounded products and fused multiply-adds: the FP32 stages, whose results keep their bits,
 // round the same way whatever the compiler would contract.
-__device__ __forceinline__ double mul_x(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ float mul_x(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ double fma_x(double a, double b, double c) { return __fma_rn(a, b, c); }
 __device__ __forceinline__ float fma_x(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 
 // One point of the v-line forward recurrence: y_t = la a0 + vc a1 + vn a2 + ib h - la y_{t-1}
 // (a0, a1, a2: `in` at t-1, t, t+1; h: `inh` at t).
-template <typename T> __device__ __forceinline__ T v_point(T la, T vc, T vn, T ib, T a0, T a1, T a2, T h, T y)
+__device__ __forceinline__ float v_point(float la, float vc, float vn, float ib, float a0, float a1, float a2, float h, float y)
 {
-    T f = mul_x(la, a0);
+    float f = mul_x(la, a0);
     f = fma_x(vc, a1, f);
     f = fma_x(vn, a2, f);
     f = fma_x(ib, h, f);
@@ -639,7 +637,7 @@ __device__ __forceinline__ void v_stage(const inst_view<float> &v, const float *
                     const int w = h + z, c = t + w;
                     const float a2 = w < 7 ? b.a[w < 7 ? w + 1 : 0] : nb.a[0];
                     if (c >= 1 && c <= e) {
-                        y = v_point<float>(q.la[z], q.vc[z], q.vn[z], q.ib[z], a0, b.a[w], a2, b.h[w], y);
+                        y = v_point(q.la[z], q.vc[z], q.vn[z], q.ib[z], a0, b.a[w], a2, b.h[w], y);
                         if (c == e) y = fma_x(-chv, hi, y);
                     }
                     o[w] = y;
@@ -1048,7 +1046,6 @@ template <typename T> struct batch_typed {
     dbuf<int> d_order, d_counter, d_status, d_final, d_imap, d_jmap;
     dbuf<double> d_values;
     dbuf<T> state, stab, vtab, xarena, yarena;
-    std::vector<std::vector<T>> payoff_host;
     dbuf<T> d_payoff; // concatenated initial conditions (sum n)
     long long launches = 0;
     // forward + adjoint
@@ -1307,13 +1304,6 @@ template <typename T> int batch_typed<T>::create(const lss_adi_problem *ps, int 
     LSS_CUDA_TRY(cudaMemset(d_grads.p, 0, d_grads.n * sizeof(double)), "batch: clearing gradients");
     adjoint_ok = std::is_same<T, double>::value;
     adjoint_why = adjoint_ok ? "" : "the adjoint is FP64 only";
-    for (int k = 0; k < n && adjoint_ok; ++k) {
-        // time-dependent tables are rebuilt per step by the host-sequenced wide kernels only
-        if (time_dependent(ps[k]) && n > 1) {
-            adjoint_ok = false;
-            adjoint_why = "SABR with r != 0 (time-dependent coefficients) runs as a single instance only";
-        }
-    }
 
     // factorise on the device from the base tables
     {
