@@ -32,16 +32,16 @@ METRIC = "grid-point-steps/s, batched fwd+adjoint vs plain path, FP64 \u22641e-1
 BYTES_PER_GPS_FWD = {"dr": 40, "cs": 96, "mcs": 96, "hv": 96}  # algorithmic bytes per grid-point-step (FP64)
 # Figures of one ncu capture each of the batched kernels on the 1024-instance, 40-step case
 # (--count 1024 --max-time-steps 40; forward: --mode fwd; forward + adjoint: --mode fwdadj
-# --workspace-gb 12, whose plan recomputes a fraction CAPTURE_RF = 0.2567 of the steps), per
-# grid-point-step, scaled to a launch by the grid-point-steps it processes.  Forward + adjoint
+# --workspace-gb 12, whose plan recomputes a fraction CAPTURE_RF = 0.2567 of the steps), both at the
+# 128 threads per instance that the autotuner takes there (its third launch), per grid-point-step, scaled to a launch by the grid-point-steps it processes.  Forward + adjoint
 # is one forward pass, the recomputation of every checkpoint segment but the last (a fraction rf
 # of the steps) and the adjoint steps, so a figure X of it is X_FWD * (1 + rf) + X_ADJ, with X_ADJ
 # what the forward + adjoint capture (at rf = CAPTURE_RF) leaves after its forward passes.
 CAPTURE_RF = 0.2567
 # DRAM bytes read + written (dram__bytes_read.sum + dram__bytes_write.sum): k_batch_forward,
 # k_batch_fwdadj
-DRAM_BYTES_FWD = 293.1
-CAPTURE_DRAM_FWDADJ = 684.6
+DRAM_BYTES_FWD = 252.1
+CAPTURE_DRAM_FWDADJ = 684.7
 DRAM_BYTES_ADJ = CAPTURE_DRAM_FWDADJ - DRAM_BYTES_FWD * (1.0 + CAPTURE_RF)
 # FP64 instructions, thread level (smsp__sass_thread_inst_executed_op_{dfma,dadd,dmul}_pred_on.sum)
 FP64_INSTR_FWD = 23.32
@@ -1094,7 +1094,7 @@ def time_plain_path(lss, problems, stream, batched_value, mode, m=64):
         out = {"value": plain_a, "unit": "grid-point-steps/s", "sample_instances": len(sub),
                "how": "lss_adi_adjoint per instance with LSS_ADI_OPT_WIDE_ADJOINT (forward + adjoint, the same "
                       "work as the batched run, each instance on the whole GPU: kernel per stage, partitioned "
-                      "line solves, autotuned chunks)",
+                      "line solves, chunks by the line lengths)",
                "batched_over_plain": batched_value / plain_a, "forward_only": out}
     return out
 

@@ -210,7 +210,7 @@ int lss_adi_grid(const lss_adi_handle *h, void *x, void *y);
 /* Partitioned line solves of a LSS_ADI_ARITH_FAST single instance: s_chunks pieces of every S line and
  * v_chunks of every v line are solved concurrently, each of at most 16 rows; a line of more than
  * 16 x count rows is walked in several tiles of that many pieces (at most 128; at least 4 rows per
- * piece; 1 = one piece at a time).  0 for either picks it by the line length (the rule lss_adi_create
+ * piece; 1 = one piece at a time).  0 for either picks it by the lines (the rule lss_adi_create
  * uses: pieces of 4 to 16 rows, as many as one CTA holds).  Results depend on the counts at
  * rounding level only.  The adjoint of the handle follows, except for instances of up to
  * 256 x 160 points, which keep the batched kernel's order (LSS_ADI_OPT_WIDE_ADJOINT).  A handle of
@@ -258,9 +258,9 @@ int lss_adi_batch_surface(lss_adi_batch *b, int index, void *out_surface);
 /* dV/d(initial condition grid) of instance `index` after a mode-1 run (host, FP64, Nx*Ny). */
 int lss_adi_batch_payoff_gradient(lss_adi_batch *b, int index, void *out);
 
-/* Lines-per-CTA autotuner: runs `mode` once per CTA size (32, 64, 128, 256 threads per
+/* Lines-per-CTA autotuner: runs `mode` once per group size (32, 64, 128 threads per
  * instance; each thread owns one S-line or v-line at a time) and keeps the fastest for later runs of
- * that mode.  With *threads_per_instance > 0 on entry it sets that size without timing; on
+ * that mode.  With *threads_per_instance = 32, 64, 96 or 128 on entry it sets that size without timing; on
  * return it holds the size in use.  The runs overwrite the batch's results. */
 int lss_adi_batch_autotune(lss_adi_batch *b, int mode, int *threads_per_instance, void *stream);
 

@@ -230,8 +230,8 @@ __global__ void k_setup_s_lines(setup_params sp, T *S0, T *chS_arena)
                  *__restrict__ bW = sp.base + 5 * N, *__restrict__ bC = sp.base + 6 * N;
     // the next point's coefficients are loaded before this point's eighteen stores, so that one
     // DRAM latency per point overlaps the work of the point before (the loop is serial along the
-    // line: the set-up of one instance's lines runs on few threads before every step of a
-    // time-dependent instance)
+    // line, and an instance has few lines; made once, for FP32 batches and FP32 instances with a
+    // thread per line)
     long long o1 = d.o2 + ld + j;
     double nM = bM[o1], nP = bP[o1], nZ = bZ[o1], nMt = bMt[o1], nPt = bPt[o1], nW = bW[o1], nC = bC[o1];
     double gam = 0.0;
@@ -1839,8 +1839,9 @@ template <typename T> struct wide_solver : wide_solver_base {
 
 int make_wide_solver(const lss_adi_problem &p, std::unique_ptr<wide_solver_base> &out)
 {
-    // time-dependent coefficients (no batched kernel to agree with) run partitioned, in one chunk per line
-    // where a thread per line is asked for
+    // time-dependent coefficients (no batched kernel to agree with) run partitioned; where a thread per
+    // line is asked for, in relay order: the chunks of a line one after the other, with a thread per
+    // line's operations
     if (!(p.options & LSS_ADI_OPT_LINE_PER_THREAD) || time_dependent(p)) return make_partitioned_solver(p, out);
     try {
         if (p.precision == LSS_ADI_FP64) {

@@ -10,9 +10,10 @@
 // step 23 FP64 instructions for Craig-Sneyd (32 when written on Y1, Y2, Y3), ten S and three v
 // tables (instead of 18 and five).  F is evaluated with differences along the S line,
 //   F(U) = M (U_{t-1} - U_t) + P (U_{t+1} - U_t) + M~ U_{j-1} + P~ U_{j+1} + (M + P - Z - W) U_t + mixed,
-// one subtraction more than with the weight -(Z + W): the terms of size k / h^2 U cancel exactly, and
-// the step's rounding against extended precision is 10 to 300 times below that of the operator
-// written out (and of the reference order) on grids of 100 x 50 to 2050 x 9.
+// one subtraction more than with the weight -(Z + W): the terms of size k / h^2 U cancel exactly.  The
+// rounding of F itself, against extended precision, is 10 to 300 times below that of the operator
+// written out on grids of 100 x 50 to 2050 x 9 (the state is still rounded once a step, which bounds
+// what a whole solve gains); the centre weight is formed from the row's reaction term, by center_weight.
 //
 // What bounds them: an FP64 instruction of a warp takes 64 cycles of its SM sub-partition, whether
 // or not it depends on the one before, so a warp that has its operands in registers saturates its

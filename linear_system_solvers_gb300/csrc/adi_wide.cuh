@@ -14,7 +14,8 @@
 // tables, every S stage reads the same six right-hand-side tables, and a time step takes about
 // two thirds of the FP64 operations of the stages written on Y1, Y2, Y3.  F is evaluated with
 // differences along the S line, M (U_{t-1} - U_t) + P (U_{t+1} - U_t) + (M + P - Z - W) U_t + ...: the
-// terms of size k / h^2 U cancel exactly (rounding 10 to 300 times below the operator written out).
+// terms of size k / h^2 U cancel exactly (the rounding of F, not of the whole solve, is 10 to 300
+// times below that of the operator written out; the centre weight: center_weight).
 //
 // Line solves.  S lines in row-scaled factors (tables already divided by the pivot):
 //   y_t = f_t - la_t y_{t-1},  x_t = y_t - g_t x_{t+1}          (x_0 = lo, x_{nx-1} = hi)

@@ -18,10 +18,11 @@
 //   FAST:      1 WB, 2 WD (right-hand-side weights of u_t, u_{t+1} scaled by the pivot reciprocal;
 //              the weight of u_{t-1} is -(1-theta)/theta * M), 3 M (a_t / beta_t), 4 G (gamma_t),
 //              5 KR (k / beta_t), 6 U, 7 Y (forward sweep); slot 0 keeps A_ (unused)
-//   FAST, FP64, n <= 512 (sweep in registers, k_h1_reg): 3 l, 4 g, 5 q (h1_setup_reg), 6 final U
+//   FAST, FP64, groups whose sweep is in registers (k_h1_reg; up to 512 points): 3 l, 4 g, 5 q (h1_setup_reg), 6 final U
 // Per-step boundary values (2 per step) and source rows are interleaved the same way.  The
-// whole time loop of an instance runs in one thread of one launch: there is no exchange
-// between instances and no per-step launch.
+// whole time loop of an instance runs in one launch, on one thread (through memory) or on the
+// lanes of one warp (in registers): there is no exchange between instances and no per-step
+// launch.  A batch with lines for both sweeps has one launch of each, side by side.
 #include "lss_heat1d.h"
 
 #include "adi_common.hpp"
@@ -913,7 +914,7 @@ template <bool SRC, bool KEEP> __global__ void __launch_bounds__(LANES, 8) k_h1_
 //
 // What bounds it: 2 W rounds of R dependent multiply-adds and a shuffle (about 90 cycles at R = 16, 3.3 ms
 // for 512 points and 1000 steps) for the longest instances, the issue slots of those rounds for a
-// full GPU.  8192 Black-Scholes calls of 101..512 points and 100..1000 steps: 4.9 ms; the sweep through
+// full GPU.  8192 Black-Scholes calls of 101..512 points and 100..1000 steps: 4.7 ms; the sweep through
 // memory took 22.2 ms, 85 cycles per row of its longest line.
 // ------------------------------------------------------------------------------------------
 constexpr int H1_RELAY_MIN = 8; // points: at least two rows between first and last solved one
@@ -1254,9 +1255,9 @@ template <typename T> int batch_t<T>::build(std::vector<inst_info> &&inf, std::v
         G.lanes = l;
         G.steps = steps;
         // FP64 lines that fit a warp's registers (but see memory_limit).  Against the sweep through memory (a
-        // thread per instance): 4096 Black-Scholes calls of 101..512 points, 100..1000 steps 104 ms -> 7.8 ms.
+        // thread per instance): 4096 Black-Scholes calls of 101..512 points, 100..1000 steps 104 ms -> 7.7 ms.
         // FP32 lines without sources keep that sweep's operations and their order (k_h1_relay): 8192 calls
-        // of the same sizes 22.2 ms -> 4.9 ms.  Sources and longer lines stay in memory.
+        // of the same sizes 22.2 ms -> 4.7 ms.  Sources and longer lines stay in memory.
         G.reg = 0;
         if (arith == LSS_ADI_ARITH_FAST && n <= LANES * H1_RMAX) {
             if (std::is_same<T, double>::value) G.reg = 1;

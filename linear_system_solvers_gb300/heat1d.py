@@ -12,7 +12,7 @@ Mirrors the reference's 1-D implicit front end
   and solves on the device.  ``solve()`` returns the final values, ``solve_all()`` every time
   level (the reference's solve(container_2d&)).
 * ``BlackScholesBatch`` runs many parametric Black-Scholes problems (the model of the
-  reference's 1-D tests) in one launch.
+  reference's 1-D tests) in one launch, two where short and long lines meet.
 
 The CUDA library is the only compute path; a missing library fails the import.
 """

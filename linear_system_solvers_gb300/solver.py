@@ -48,7 +48,7 @@ class HestonProblem:
     fp64_tables: bool = False  # FP32 only: tables and index_of remaps built in double
     solver: str = "tlu"  # tridiagonal_method_enum: "tlu" ThomasLUSolver | "ds" DoubleSweepSolver
     line_per_thread: bool = False  # fast single instance: no partitioned line solves (batched-kernel bits)
-    wide_adjoint: bool = False  # adjoint(): whole-GPU kernel-per-stage path at any size (not one CTA)
+    wide_adjoint: bool = False  # adjoint(): partitioned line solves at any size (small ones: relay order, batch bits)
 
     # fields that choose how the device runs a problem, not which PDE it is
     EXECUTION_FIELDS = ("eval_s", "eval_v", "fp64_tables", "line_per_thread", "wide_adjoint")
@@ -112,7 +112,7 @@ class ImplicitHestonSolver:
             pass
 
     def line_chunks(self, s_chunks: int = 0, v_chunks: int = 0, stream: int = 0):
-        """Chunks per S line / v line of the partitioned solves (0 = by the line length); returns those in use."""
+        """Chunks per S line / v line of the partitioned solves (0 = by lines and their length); returns those in use."""
         a, b = ctypes.c_int(), ctypes.c_int()
         L.check(self.lib.lss_adi_line_chunks(self._h, int(s_chunks), int(v_chunks), ctypes.byref(a), ctypes.byref(b),
                                              ctypes.c_void_p(stream)))
