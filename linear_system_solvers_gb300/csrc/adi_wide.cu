@@ -575,7 +575,7 @@ struct line_adjoint : wide_adjoint_base {
         });
     }
     struct arrays {
-        double *VB, *DB, *FB, *MU, *DV, *D2B, *LV, *LS, *HS, *ACC;
+        double *VB, *DB, *FB[2], *MU, *DV, *D2B, *LV, *LS, *HS, *ACC; // FB: first and second S stage
     };
     template <int KIND, int SCH>
     void adj_s(cudaStream_t s, const arrays &a, const double *U, const double *Vn, const double *D1, const double *D2, const double *Y,
@@ -584,14 +584,14 @@ struct line_adjoint : wide_adjoint_base {
         const split &sp = w.wp.s;
         w.shaped<true>([&](auto r, auto ser) {
             w.launch(s, k_wadj_s<decltype(r)::value, KIND, SCH, decltype(ser)::value>, grid_for(w.ny - 1, sp.L), dim3(sp.L * sp.PC),
-                     2 * sizeof(double) * carry_words(sp), w.wp, ap, U, Vn, D1, D2, Y, XB, a.DV, a.VB, a.FB, a.MU, a.LS, a.HS, a.ACC,
-                     nacc, tau, da, dc);
+                     2 * sizeof(double) * carry_words(sp), w.wp, ap, U, Vn, D1, D2, Y, XB, a.DV, a.VB, a.FB[KIND - 1], a.MU, a.LS, a.HS,
+                     a.ACC, nacc, tau, da, dc);
         });
     }
     template <int KIND, int SCH> void gather(cudaStream_t s, const arrays &a, const double *U, double tau, double da)
     {
         const int grid = grid_for(static_cast<long long>(w.nx) * w.ny, 256);
-        w.launch(s, k_wadj_gather<KIND, SCH>, grid, dim3(256), 0, w.wp, ap, U, a.FB, a.D2B, a.VB, a.LS, a.HS, a.LV, a.ACC, nacc, tau, da);
+        w.launch(s, k_wadj_gather<KIND, SCH>, grid, dim3(256), 0, w.wp, ap, U, a.FB[KIND - 1], a.D2B, a.VB, a.LS, a.HS, a.LV, a.ACC, nacc, tau, da);
     }
     template <int SCH>
     void adjoint_step(cudaStream_t s, const arrays &a, int m, const double *U, const double *D1, const double *D2, const double *D3,
@@ -618,11 +618,25 @@ struct line_adjoint : wide_adjoint_base {
         gather<1, SCH>(s, a, U, tau, da);
     }
 
+    // Relay order: the parameter sums are made from the arrays of all steps of a segment (k_wadj_lines).
+    bool by_lines() const { return w.serial && !w.tdep; }
+    static int padded(int k) { return (k + 31) / 32 * 32; }
     // Workspace (doubles) at checkpoint interval c
     long long need(int c) const
     {
         const long long nseg = (w.steps + c - 1) / c;
-        return (nseg + 4LL * (c + 1) + 2 + 6) * w.n + w.nx + 2LL * w.ny + 5 * nacc;
+        const long long base = (nseg + 4LL * (c + 1) + 2) * w.n + 2LL * w.ny;
+        if (by_lines()) return base + (3 + 4LL * c) * w.n + c * (w.nx + 8LL * padded(w.ny - 2) + 3LL * padded(w.nx)) + 5 * 128;
+        return base + 6 * w.n + w.nx + 5 * nacc;
+    }
+    template <int SCH> void sum_lines(cudaStream_t s, const line_sums &g, bool end)
+    {
+        const int lines = grid_for(static_cast<long long>(g.len) * g.lp, 128);
+        constexpr bool dr = SCH == LSS_ADI_DOUGLAS_RACHFORD;
+        if constexpr (!dr) k_wadj_lines<2, SCH><<<lines, 128, 0, s>>>(w.wp, ap, g);
+        k_wadj_lines<1, SCH><<<lines, 128, 0, s>>>(w.wp, ap, g);
+        k_wadj_rows<<<grid_for(static_cast<long long>(g.len) * g.rp, 128), 128, 0, s>>>(w.wp, ap, g);
+        k_wadj_fold<dr><<<5, g.threads, 0, s>>>(w.wp, ap, g, end, grads.p);
     }
 
     // Checkpoint interval and workspace of a run.  every = 0: the longest interval within a sixteenth of the
@@ -673,9 +687,28 @@ struct line_adjoint : wide_adjoint_base {
         if (rc) return rc;
         const int nseg = (steps + c - 1) / c;
         double *CK = ws.p, *SEG = CK + nseg * n, *W0 = SEG + 4LL * (c + 1) * n, *W1 = W0 + n;
+        const bool lines = by_lines();
+        const long long each = lines ? c : 1; // steps whose adjoint arrays are kept
+        line_sums ls{};
         arrays a;
-        a.VB = W1 + n; a.DB = a.VB + n; a.FB = a.DB + n; a.MU = a.FB + n; a.DV = a.MU + n; a.D2B = a.DV + n;
-        a.LV = a.D2B + n; a.LS = a.LV + w.nx; a.HS = a.LS + w.ny; a.ACC = a.HS + w.ny;
+        a.MU = W1 + n; a.D2B = a.MU + n;
+        double *DB = a.D2B + n, *DV = DB + each * n;
+        ls.terms = DV + each * n;
+        ls.lp = lines ? padded(w.ny - 2) : 0;
+        ls.rp = lines ? padded(w.nx) : 0;
+        ls.rows = ls.terms + 8LL * ls.lp * each;
+        a.VB = ls.rows + 3LL * ls.rp * each;
+        double *FB = a.VB + n, *LV = FB + (lines ? 2 * each : 1) * n;
+        a.LS = LV + each * w.nx; a.HS = a.LS + w.ny; a.ACC = a.HS + w.ny;
+        ls.seg = SEG; ls.FB = FB; ls.DB = DB; ls.DV = DV; ls.LV = LV; ls.acc = a.ACC; ls.n = n; ls.dtau = dtau;
+        ls.threads = 32 * std::max(1, std::min(4, (w.ny - 2 + 31) / 32)); // of the batch's warp groups
+        if (lines) a.ACC = nullptr;
+        auto arrays_of = [&](int k) { // of step k of a segment
+            const long long at = lines ? k : 0;
+            a.DB = DB + at * n; a.DV = DV + at * n; a.LV = LV + at * w.nx;
+            a.FB[1] = FB + (lines ? 2 * at : 0) * n;
+            a.FB[0] = lines ? a.FB[1] + n : FB;
+        };
         // read where no kernel writes: VB and FB (boundary rows and columns) and the sums.  The states and
         // increments are written wherever they are read, so the checkpoints need no clearing.
         LSS_CUDA_TRY(cudaMemsetAsync(a.VB, 0, (need(c) - (a.VB - ws.p)) * sizeof(double), s), "wide adjoint: clearing");
@@ -705,6 +738,7 @@ struct line_adjoint : wide_adjoint_base {
             for (int k = 0; k < len && g < nseg - 1; ++k)
                 w.forward_step(s, n0 + k, k == 0 ? u0 : slot(k, 0), slot(k, 1), slot(k, 2), slot(k, 3), slot(k + 1, 0));
             for (int k = len - 1; k >= 0; --k) {
+                arrays_of(k);
                 const double *U = k == 0 ? u0 : slot(k, 0), *D1 = slot(k, 1), *D2 = slot(k, 2), *D3 = slot(k, 3), *Vn = slot(k + 1, 0);
                 switch (w.scheme) {
                 case LSS_ADI_DOUGLAS_RACHFORD: adjoint_step<LSS_ADI_DOUGLAS_RACHFORD>(s, a, n0 + k, U, D1, D2, D3, Vn); break;
@@ -713,8 +747,16 @@ struct line_adjoint : wide_adjoint_base {
                 default: adjoint_step<LSS_ADI_HUNDSDORFER_VERWER>(s, a, n0 + k, U, D1, D2, D3, Vn); break;
                 }
             }
+            if (!lines) continue;
+            ls.u0 = u0; ls.len = len; ls.tau = tau0 + dtau * n0;
+            switch (w.scheme) {
+            case LSS_ADI_DOUGLAS_RACHFORD: sum_lines<LSS_ADI_DOUGLAS_RACHFORD>(s, ls, g == 0); break;
+            case LSS_ADI_CRAIG_SNEYD: sum_lines<LSS_ADI_CRAIG_SNEYD>(s, ls, g == 0); break;
+            case LSS_ADI_MODIFIED_CRAIG_SNEYD: sum_lines<LSS_ADI_MODIFIED_CRAIG_SNEYD>(s, ls, g == 0); break;
+            default: sum_lines<LSS_ADI_HUNDSDORFER_VERWER>(s, ls, g == 0); break;
+            }
         }
-        k_wadj_reduce<<<5, 1024, 0, s>>>(a.ACC, nacc, grads.p);
+        if (!lines) k_wadj_reduce<<<5, 1024, 0, s>>>(a.ACC, nacc, grads.p);
         LSS_CUDA_TRY(cudaGetLastError(), "wide adjoint: launching");
         if (out_value)
             LSS_CUDA_TRY(cudaMemcpyAsync(out_value, w.value.p, sizeof(double), cudaMemcpyDeviceToHost, s), "lss_adi_adjoint: value");

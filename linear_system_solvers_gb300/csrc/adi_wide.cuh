@@ -1046,6 +1046,24 @@ __global__ void __launch_bounds__(MAX_CTA) k_wadj_s(const __grid_constant__ wpar
         };
         if constexpr (SER) relay<double, false>(kb, in, sweep);
         else sweep(compose<double, false>(kb, w, bpreg, in));
+        auto store = [&](int t, long long o, double w, double mu) {
+            if (!act) return;
+            FB[o] = w;
+            if constexpr (KIND == 2 && !hv) MU[o] = mu; // adjoint of D1
+            if (t == 1) {
+                const double l = -p.S[W_LA][o] * w;
+                if constexpr (KIND == 2 && hv) VB[j] += l;
+                else LS[j] = KIND == 1 && !dr && !hv ? LS[j] + l : l;
+            }
+        };
+        if (acc == nullptr) { // the sums: k_wadj_lines
+#pragma unroll
+            for (int r = R - 1; r >= 0; --r) {
+                const long long o = at(t0 + r);
+                if (t0 + r <= e) store(t0 + r, o, f[r], p.S[W_IB][o] * f[r]);
+            }
+            continue;
+        }
         // X: the operand of the explicit terms (U, or D2), Y: the stage's result; rows t+1, t, t-1
         const double *X = KIND == 1 ? U : D2;
         double xh = X[at(t0 + R)], xc = X[at(t0 + R - 1)], yh = Y[at(t0 + R)], yc = Y[at(t0 + R - 1)];
@@ -1060,15 +1078,7 @@ __global__ void __launch_bounds__(MAX_CTA) k_wadj_s(const __grid_constant__ wpar
             const double xl = X[ol], yl = Y[ol], sl = X[ol - 1], ddl = sl - X[ol + 1];
             if (t <= e) {
                 const double mu = p.S[W_IB][o] * w;
-                if (act) {
-                    FB[o] = w;
-                    if constexpr (KIND == 2 && !hv) MU[o] = mu; // adjoint of D1
-                    if (t == 1) {
-                        const double l = -p.S[W_LA][o] * w;
-                        if constexpr (KIND == 2 && hv) VB[j] += l;
-                        else LS[j] = KIND == 1 && !dr && !hv ? LS[j] + l : l;
-                    }
-                }
+                store(t, o, w, mu);
                 const double mx = mu * q.hx[t], mc = q.sabr ? mu * q.hc[t] : mx;
                 const double dy = yh - yl;
                 s.Y = fma(mx, dy, s.Y);
@@ -1112,7 +1122,7 @@ __global__ void __launch_bounds__(MAX_CTA) k_wadj_s(const __grid_constant__ wpar
             ss = sl;
         }
     }
-    if (!act) return;
+    if (!act || acc == nullptr) return;
     // the line's sums: theta weighs the terms in Y, dw (1 for the first stage) those in X
     const double th = q.theta, wx = KIND == 1 ? 1.0 : q.dw, we = KIND == 1 ? 1.0 : q.zeta;
     const double A = th * s.Y + wx * s.A;
@@ -1139,7 +1149,7 @@ __global__ void __launch_bounds__(MAX_CTA) k_wadj_s(const __grid_constant__ wpar
 // Cross-line adjoints of an S stage, one thread per grid point (p, q).  KIND 2: adjoint of D2 (for HV
 // on top of the state's adjoint, next = U + D2 + ...; rows 0 and nx-1 are -U).  KIND 1: F^T into the
 // state's adjoint, the S lines' boundary values (index_of remap) and the explicit v = v_lo column
-// with its parameter sensitivities (acc slots of the rows).
+// with its parameter sensitivities (acc slots of the rows; without acc k_wadj_rows has them).
 template <int KIND, int SCH>
 __global__ void __launch_bounds__(256) k_wadj_gather(const __grid_constant__ wparams<double> p, const __grid_constant__ adj_params a,
                                                      const double *U, const double *FB, double *D2B, double *VB, const double *LS,
@@ -1175,7 +1185,7 @@ __global__ void __launch_bounds__(256) k_wadj_gather(const __grid_constant__ wpa
     double x = dn + up;
     if constexpr (six) {
         mid = fma(W(W_WS, o + 1, rt), F(o + 1, rt), fma(W(W_WN, o - 1, lf), F(o - 1, lf), p.S[W_WC][o] * FB[o]));
-        x += KIND == 2 && mcs ? p.zt * mid : mid;
+        x += KIND == 2 && mcs ? __dmul_rn(p.zt, mid) : mid; // rounded by itself, as there
     }
     if constexpr (KIND == 2) {
         const double d = hv ? fma(p.zeta, x, -(p.S[W_IB][o] * FB[o])) : mcs ? x : p.zeta * x;
@@ -1202,7 +1212,7 @@ __global__ void __launch_bounds__(256) k_wadj_gather(const __grid_constant__ wpa
             else {
                 const double below = r >= 1 ? p.xbp[r - 1] : 0.0, above = r + 1 <= nx - 2 ? p.xbm[r + 1] : 0.0;
                 v += fma(below, B0(r - 1), fma(p.xbc[r], bb, above * B0(r + 1)));
-                if (bb != 0.0) {
+                if (acc != nullptr && bb != 0.0) {
                     const double u0 = U[o], u1 = U[o + 1], u2 = U[o + 2];
                     const double ee = a.ni * bb * (4.0 * u1 - 3.0 * u0 - u2);
                     double hd = a.hx[r];
@@ -1215,6 +1225,166 @@ __global__ void __launch_bounds__(256) k_wadj_gather(const __grid_constant__ wpa
             }
         }
         VB[o] = v;
+    }
+}
+
+// Parameter sums of an adjoint in relay order, from the arrays of the steps of a checkpoint segment: with the
+// operations of the batched kernel (da_s, da_b1) in its order, so that the gradients have the bits of the
+// same instance in a batch, on a warp group of its own class.  They are small against their terms where the
+// scheme has growing modes: with a thread per chunk and its own partial sums, 4 of 240 small calls came out
+// more than 1e-13 from the batch's.  The stages, where the sums were a chain of every step, are left with
+// the solves (k_wadj_s without acc), and the sums of all steps of a segment are made at once: 128 x 64 x
+// 200 Craig-Sneyd 23.4 ms with sensitivities, 26.1 ms with the sums in the stages.
+struct line_sums {
+    const double *u0, *seg;                     // state of the segment's first step; U, D1, D2, D3 of step k at seg + 4 k n
+    const double *FB, *DB, *DV, *LV;            // FB: stages 2 and 1 of step k at FB + 2 k n
+    double *terms, *rows, *acc;                 // terms of line l: [step][stage][4][lp]; of row p: [step][3][rp]
+    long long n;
+    int len, lp, rp, threads;                   // steps; lines, rows of a multiple of 32; threads of the batch's group
+    double tau, dtau;                           // time of step 0 of the segment
+    __device__ __forceinline__ const double *U(int k) const { return k == 0 ? u0 : seg + 4LL * k * n; }
+};
+
+// What bounds it: a line's FP64 instructions (25 per row); a thread per line and step, so the whole GPU has work.
+template <int KIND, int SCH>
+__global__ void __launch_bounds__(128) k_wadj_lines(const __grid_constant__ wparams<double> p, const __grid_constant__ adj_params q,
+                                                    const __grid_constant__ line_sums g)
+{
+    constexpr bool hv = SCH == LSS_ADI_HUNDSDORFER_VERWER, mcs = SCH == LSS_ADI_MODIFIED_CRAIG_SNEYD, dr = SCH == LSS_ADI_DOUGLAS_RACHFORD;
+    constexpr bool xt = KIND == 2 && (hv || mcs); // D2 terms besides the mixed one
+    constexpr bool first_v = KIND == 1 && !dr;
+    const int nx = p.nx, ny = p.ny, ld = p.ld, e = nx - 2;
+    const long long last = (nx - 1LL) * ld, id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const int k = static_cast<int>(id / g.lp), l = static_cast<int>(id % g.lp), j = l + 1;
+    if (k >= g.len || j > ny - 2) return;
+    const bool sabr = q.sabr;
+    const double *U = g.U(k), *Vn = g.U(k + 1), *D1 = g.seg + (4LL * k + 1) * g.n, *D2 = D1 + g.n, *D3 = D2 + g.n;
+    const double *X = KIND == 1 ? U : D2, *Y = KIND == 1 ? D1 : D3;
+    const double *FB = g.FB + (2LL * k + (KIND == 1 ? 1 : 0)) * g.n, *M = (first_v ? g.DV : g.DB) + k * g.n;
+    double sY = 0, sB = 0, sE = 0, sA = 0, sC = 0, sQ = 0, sS = 0, sYa = 0, sYd = 0, sAa = 0, sDd = 0, vd = 0, v0 = 0, vm = 0;
+    double xh = X[last + j], xc = X[last - ld + j], yh = Y[last + j], yc = Y[last - ld + j];
+    double ddh = X[last + j - 1] - X[last + j + 1], ss = X[last - ld + j - 1], ddc = ss - X[last - ld + j + 1];
+#pragma unroll 4
+    for (int t = e; t >= 1; --t) {
+        const long long o = (long long)t * ld + j, ol = o - ld;
+        const double mu = p.S[W_IB][o] * FB[o];
+        const double xl = X[ol], sl = X[ol - 1], yl = Y[ol], ddl = sl - X[ol + 1], m = M[o];
+        double x0, x1, x2;
+        if constexpr (first_v) {
+            x0 = D2[o - 1]; x1 = D2[o]; x2 = D2[o + 1];
+        } else {
+            x0 = Vn[o - 1] - U[o - 1]; x1 = Vn[o] - U[o]; x2 = Vn[o + 1] - U[o + 1];
+            if constexpr (hv) { x0 -= D2[o - 1]; x1 -= D2[o]; x2 -= D2[o + 1]; }
+        }
+        const double mx = mu * q.hx[t], mc = sabr ? mu * q.hc[t] : mx;
+        const double dy = yh - yl;
+        sY = fma(mx, dy, sY);
+        sB = fma(mu, yc, sB);
+        sE = fma(mc, ddl - ddh, sE);
+        double dx = 0.0;
+        if constexpr (KIND == 1 || xt) {
+            dx = KIND == 2 && mcs ? -xh - xl : xh - xl;
+            sA = fma(mx, dx, sA);
+            sC = fma(mu, xc, sC);
+            sQ = fma(mu, ddc, sQ);
+            sS = fma(mu, ss - xc, sS);
+        }
+        if (sabr) {
+            const double ma = mu * q.ha[t], md = mu * q.hdd[t];
+            sYa = fma(ma, yl + yh - 2.0 * yc, sYa);
+            sYd = fma(md, dy, sYd);
+            if constexpr (KIND == 1 || xt) {
+                sAa = fma(ma, xl + (KIND == 2 && mcs ? -xh : xh) - 2.0 * xc, sAa);
+                sDd = fma(md, dx, sDd);
+            }
+        }
+        vd = fma(m, x2 - x0, vd);
+        v0 = fma(m, x1, v0);
+        vm = fma(m, x0 - x1, vm);
+        xh = xc; xc = xl;
+        yh = yc; yc = yl;
+        ddh = ddc; ddc = ddl;
+        ss = sl;
+    }
+    const double th = q.theta, wx = KIND == 1 ? 1.0 : hv ? q.zeta : q.zeta - q.theta, we = KIND == 1 ? 1.0 : q.zeta;
+    const double A = th * sY + wx * sA, B = -(th * sB + 2.0 * wx * sC), Q = -wx * sQ, D = wx * (2.0 * sS - sQ);
+    const double E = we * q.gamma * sE;
+    const double es = q.es[j], bs = q.bs[j], hy = q.hy[j], tau = g.tau + g.dtau * k;
+    double g0 = q.delta * A + q.halfk * B;
+    if (sabr)
+        g0 += tau * q.omb * (q.hv2[j] * (2.0 * q.delta * (th * sYd + wx * sDd) - 2.0 * q.alphat * (th * sYa + wx * sAa)) -
+                             q.rho * q.sigma * hy * E);
+    const double nq = q.ni * (Q + th * vd);
+    double *o = g.terms + (2LL * k + (KIND == 1 ? 1 : 0)) * 4 * g.lp + l;
+    o[0] = g0 - q.halfk * th * v0;
+    o[g.lp] = nq;
+    o[2 * g.lp] = es * nq + q.betat * bs * (D + th * (2.0 * vm + vd)) + q.rho * hy * E;
+    o[3 * g.lp] = E;
+}
+
+// Terms of the explicit v = v_lo column (da_b1), a thread per row and step.
+static __global__ void __launch_bounds__(128) k_wadj_rows(const __grid_constant__ wparams<double> p, const __grid_constant__ adj_params q,
+                                                          const __grid_constant__ line_sums g)
+{
+    const int nx = p.nx, ld = p.ld;
+    const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const int k = static_cast<int>(id / g.rp), i = static_cast<int>(id % g.rp);
+    if (k >= g.len) return;
+    const double *U = g.U(k) + (long long)i * ld, *LV = g.LV + (long long)k * nx;
+    double bb = 0.0, x = 0.0, ee = 0.0;
+    if (i >= 1 && i <= nx - 2) {
+        bb = p.imap[i] == i ? LV[i] : 0.0;
+        if (i + 1 <= nx - 2 && p.imap[i + 1] == i) bb += LV[i + 1];
+    }
+    if (bb != 0.0) {
+        const double u0 = U[0], tau = g.tau + g.dtau * k;
+        ee = q.ni * bb * (4.0 * U[1] - 3.0 * u0 - U[2]);
+        double hd = q.hx[i];
+        if (q.sabr) hd += 2.0 * q.omb * tau * q.hv2[0] * q.hdd[i];
+        x = q.delta * hd * (U[ld] - U[-ld]) - q.k * u0;
+    }
+    double *o = g.rows + 3LL * k * g.rp + i;
+    o[0] = bb;
+    o[g.rp] = x;
+    o[2 * g.rp] = ee;
+}
+
+// The terms added up over the steps, last step first, as the batch's group does: thread l0 has the lines 1 + l0,
+// 1 + l0 + threads, ... of stage 2, those of stage 1, then the rows l0, l0 + threads, ...  A CTA per sum
+// (r, kappa, theta, sigma, rho).  What bounds it: one chain of
+// additions, and L2 latency.
+template <bool DR> __global__ void __launch_bounds__(128) k_wadj_fold(const __grid_constant__ wparams<double> p, const __grid_constant__ adj_params q,
+                                                                      const __grid_constant__ line_sums g, bool end, double *grads)
+{
+    __shared__ double red[4];
+    const int what = blockIdx.x, l0 = threadIdx.x, ls = g.threads, lines = p.ny - 2, nx = p.nx;
+    // what each line's term is: added, or times a factor of the line
+    const int term = what == 0 ? 0 : what == 3 ? 2 : what == 4 ? 3 : 1;
+    const double *col = what == 1 ? q.ek : what == 2 ? q.et : q.es;
+    const double sh = q.sigma;
+    double acc = g.acc[128 * what + l0];
+    for (int k = g.len - 1; k >= 0; --k) {
+        for (int st = DR ? 1 : 0; st < 2; ++st) {
+            const double *t = g.terms + ((2LL * k + st) * 4 + term) * g.lp;
+            for (int l = l0; l < lines; l += ls) {
+                if (what == 0 || what == 3) acc += t[l];
+                else acc = fma(what == 4 ? sh * q.hy[l + 1] : col[l + 1], t[l], acc);
+            }
+        }
+        const double *b = g.rows + 3LL * k * g.rp;
+        if (what < 4)
+            for (int i = l0; i < nx; i += ls)
+                if (b[i] != 0.0) acc = what == 0 ? fma(b[i], b[g.rp + i], acc) : fma(b[2 * g.rp + i], col[0], acc);
+    }
+    g.acc[128 * what + l0] = acc;
+    if (!end) return;
+    for (int off = 16; off > 0; off >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, off);
+    if (l0 % 32 == 0) red[l0 / 32] = acc;
+    __syncthreads();
+    if (l0 == 0) {
+        double sum = 0.0;
+        for (int w = 0; w < ls / 32; ++w) sum += red[w];
+        grads[what == 0 ? 4 : what - 1] = sum;
     }
 }
 
