@@ -996,7 +996,7 @@ static __global__ void k_setup_s_delta(setup_params sp, double *S0)
         slot(DS_WW) = M * ib;
         const double ws = Mt * ib, wn = Pt * ib;
         slot(DS_WS) = ws;
-        slot(DS_WQ) = center_weight<double>(M, P, Z, Mt, Pt, W, ib, ws, wn, t, j);
+        slot(DS_WQ) = center_weight<double>((M + P - Z) + ((Mt + Pt) - W), ib, ws, wn, t, j);
         slot(DS_WC) = -(Z + W) * ib;
         slot(DS_WN) = wn;
         slot(DS_WE) = P * ib;

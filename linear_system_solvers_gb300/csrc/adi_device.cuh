@@ -105,17 +105,17 @@ __device__ __forceinline__ T s_rhs(const dev_instance<T> &d, int t, int j, const
 
 // Weight of U_t in the explicit operator with differences along the S line, (M + P - Z) - W times ib, for
 // the neighbours' weights ws = M~ ib and wn = P~ ib as they are stored: the row's sum is the reaction
-// term, and the weight is formed from it.  Written as -W plus the reaction it is rounded by the same
+// term r = (M + P - Z) + ((M~ + P~) - W), and the weight is formed from it.  Written as -W plus the reaction it is rounded by the same
 // amount wherever W has the same exponent (W is a multiple of its last place, the reaction a constant), a
 // reaction of up to eps W that adds up over the steps: SABR 12 x 3000 (W = 1.3e4) was 6.7e-12 off extended
 // precision after 10 steps, so 1.5e-13.  A reaction of less than 2^20 last places does not get different
 // roundings from the change of ib along the line; there the weight is rounded up or down in proportion (a
 // hash of row t and column j is added below the last place of T).
 template <typename T>
-__device__ __forceinline__ T center_weight(double M, double P, double Z, double Mt, double Pt, double W, double ib, T ws, T wn, int t, int j)
+__device__ __forceinline__ T center_weight(double r, double ib, T ws, T wn, int t, int j)
 {
     constexpr int digits = sizeof(T) == 8 ? 52 : 23;
-    const double sum = static_cast<double>(ws) + static_cast<double>(wn), r = (M + P - Z) + ((Mt + Pt) - W);
+    const double sum = static_cast<double>(ws) + static_cast<double>(wn);
     auto exponent = [](double x) { return (__double2hiint(x) >> 20) & 0x7ff; };
     const int last = exponent(sum) - digits; // exponent field of the last place of the sum in T
     if (exponent(r) + exponent(ib) - 1023 >= last + 20 || last <= 0) return static_cast<T>(fma(r, ib, -sum));

@@ -524,8 +524,8 @@ struct line_adjoint : wide_adjoint_base {
         ap.sabr = p.model == LSS_ADI_SABR;
         tau0 = p.forward ? p.maturity - ap.k : ap.k;
         dtau = p.forward ? -ap.k : ap.k;
-        // Up to 256 x 160 points the recurrences run in relay order: the value has the bits of the same
-        // instance in a batch.  (One warp group of the batched kernel took 119 ms for a 128 x 64 x 200
+        // Up to 256 x 160 points the recurrences run in relay order: value and gradients have the bits of
+        // the same instance in a batch (gradients: see line_sums).  (One warp group of the batched kernel took 119 ms for a 128 x 64 x 200
         // Craig-Sneyd call with sensitivities.)  Larger ones, and those of LSS_ADI_OPT_WIDE_ADJOINT, are
         // partitioned; LINE_PER_THREAD asks for relay order at any size.
         small = p.nx <= 256 && static_cast<long long>(p.nx) * p.ny <= 40960 && !time_dependent(p) && !(p.options & LSS_ADI_OPT_WIDE_ADJOINT);

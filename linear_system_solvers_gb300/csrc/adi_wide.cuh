@@ -518,16 +518,16 @@ __global__ void __launch_bounds__(MAX_CTA) k_wide_products(const T *fac, long lo
         const_cast<T *>(out.GA)[(long long)(tile * sp.groups() + at / sp.gs) * ls + l] = in_group * pr;
 }
 
-// S-line tables of one line per thread (double arithmetic), from M, P, Z, Mt, Pt, W, C (pitch ld)
+// S-line tables of one line per thread (double arithmetic), from M, P, Z, Mt, Pt, W, C (pitch ld) and mpz, M + P - Z
 template <typename T>
-__device__ __forceinline__ void s_slots(T *s, long long n, double M, double P, double Z, double Mt, double Pt, double W, double C,
-                                        double gm, double ib, int t, int j)
+__device__ __forceinline__ void s_slots(T *s, long long n, double M, double P, double Z, double mpz, double Mt, double Pt, double W,
+                                        double C, double gm, double ib, int t, int j)
 {
     const T ws = static_cast<T>(Mt * ib), wn = static_cast<T>(Pt * ib);
     s[W_WG * n] = static_cast<T>(gm * C * ib);
     s[W_WW * n] = static_cast<T>(M * ib);
     s[W_WS * n] = ws;
-    s[W_WQ * n] = center_weight<T>(M, P, Z, Mt, Pt, W, ib, ws, wn, t, j);
+    s[W_WQ * n] = center_weight<T>(mpz + ((Mt + Pt) - W), ib, ws, wn, t, j);
     s[W_WC * n] = static_cast<T>(-(Z + W) * ib);
     s[W_WN * n] = wn;
     s[W_WE * n] = static_cast<T>(P * ib);
@@ -556,7 +556,7 @@ __global__ void k_wide_setup_s(const double *base, long long n, int nx, int ny, 
         s[W_LA * n] = static_cast<T>(a * ib);
         s[W_G * n] = static_cast<T>(gam);
         s[W_IB * n] = static_cast<T>(ib);
-        s_slots(s, n, v[0], v[1], v[2], v[3], v[4], v[5], v[6], gm, ib, t, j);
+        s_slots(s, n, v[0], v[1], v[2], v[0] + v[1] - v[2], v[3], v[4], v[5], v[6], gm, ib, t, j);
     }
 }
 template <typename T>
@@ -720,7 +720,7 @@ __global__ void __launch_bounds__(MAX_CTA) k_wide_tdep(const __grid_constant__ t
                 S[W_IB * q.n + o] = ib;
                 S[W_G * q.n + o] = gam;
                 S[W_LA * q.n + o] = la;
-                s_slots(S + o, q.n, m[r], pp[r], z, q.mt[o], q.pt[o], q.w[o], dc * q.cs[o], q.gm, ib, t, j);
+                s_slots(S + o, q.n, m[r], pp[r], z, -q.z0, q.mt[o], q.pt[o], q.w[o], dc * q.cs[o], q.gm, ib, t, j);
                 if (r == 0) la1 = la;
                 else prl *= -la;
                 prb *= -gam;
@@ -811,7 +811,8 @@ __global__ void k_wide_end(const T *U, int nx, int ny, int ld, bilinear b, T *su
 // adjoint passes through the step unchanged but for its ends and F's transpose, so one array VB
 // is updated in place.  Parameter sensitivities of an S solve (I - theta A1) Y = rhs(X) are
 // mu . (d rhs X + theta dA1 Y), mu = ib w; of a v solve w . theta dA2 x.  Both are accumulated by the
-// S kernels, where the coefficient derivatives' v factors are constant along a thread's line.
+// S kernels, where the coefficient derivatives' v factors are constant along a thread's line (in relay
+// order by k_wadj_lines, for all steps of a segment).
 // ------------------------------------------------------------------------------------------
 struct adj_params {
     const double *hx, *hc, *ha, *hdd;          // nx
