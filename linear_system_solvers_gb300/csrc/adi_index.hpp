@@ -14,7 +14,8 @@ namespace lss_gb300 {
 // row fits an int, counted from the row's middle slot.  FP32 (18 slots): 64 bits; its v tables (five)
 // unsigned numbers.  The choice is the kernels': with 64-bit or unsigned rows the FP64 ones lose 3 to 5 %
 // (20000 Craig-Sneyd calls of 64 x 16 126.5 against 119.9 ms), with signed v rows FP32 Douglas-Rachford
-// 40 % (768 uneven calls 72 against 52 ms).
+// 40 % (768 uneven calls 72 against 52 ms).  Against rows counted in ints, which the longest do not fit, the
+// FP32 kernels take 1 to 3 % longer (604 Craig-Sneyd calls 50.2 and 49.2 ms).
 template <int SLOTS> struct table_index {
     static constexpr bool half = SLOTS == 10, wide = SLOTS == 18, plain = SLOTS == 3;
     static_assert(half || wide || plain || SLOTS == 5, "elements of a row");
