@@ -618,15 +618,17 @@ struct line_adjoint : wide_adjoint_base {
         gather<1, SCH>(s, a, U, tau, da);
     }
 
-    // Relay order: the parameter sums are made from the arrays of all steps of a segment (k_wadj_lines).
+    // Relay order: the parameter sums are made from the arrays of a run of steps of a segment (k_wadj_lines).
     bool by_lines() const { return w.serial && !w.tdep; }
+    // Steps of a run: 256 MB of arrays, at least 32 steps (128 x 64 x 200 24.4 ms with runs of 32, 23.4 with one).
+    int run_of(int c) const { return static_cast<int>(std::min<long long>(c, std::max(32LL, (1LL << 23) / w.n))); }
     static int padded(int k) { return (k + 31) / 32 * 32; }
     // Workspace (doubles) at checkpoint interval c
     long long need(int c) const
     {
         const long long nseg = (w.steps + c - 1) / c;
         const long long base = (nseg + 4LL * (c + 1) + 2) * w.n + 2LL * w.ny;
-        if (by_lines()) return base + (3 + 4LL * c) * w.n + c * (w.nx + 8LL * padded(w.ny - 2) + 3LL * padded(w.nx)) + 5 * 128;
+        if (by_lines()) return base + (3 + 4LL * run_of(c)) * w.n + run_of(c) * (w.nx + 8LL * padded(w.ny - 2) + 3LL * padded(w.nx)) + 5 * 128;
         return base + 6 * w.n + w.nx + 5 * nacc;
     }
     template <int SCH> void sum_lines(cudaStream_t s, const line_sums &g, bool end)
@@ -688,7 +690,7 @@ struct line_adjoint : wide_adjoint_base {
         const int nseg = (steps + c - 1) / c;
         double *CK = ws.p, *SEG = CK + nseg * n, *W0 = SEG + 4LL * (c + 1) * n, *W1 = W0 + n;
         const bool lines = by_lines();
-        const long long each = lines ? c : 1; // steps whose adjoint arrays are kept
+        const int each = lines ? run_of(c) : 1; // steps whose adjoint arrays are kept
         line_sums ls{};
         arrays a;
         a.MU = W1 + n; a.D2B = a.MU + n;
@@ -699,12 +701,12 @@ struct line_adjoint : wide_adjoint_base {
         ls.rows = ls.terms + 8LL * ls.lp * each;
         a.VB = ls.rows + 3LL * ls.rp * each;
         double *FB = a.VB + n, *LV = FB + (lines ? 2 * each : 1) * n;
-        a.LS = LV + each * w.nx; a.HS = a.LS + w.ny; a.ACC = a.HS + w.ny;
-        ls.seg = SEG; ls.FB = FB; ls.DB = DB; ls.DV = DV; ls.LV = LV; ls.acc = a.ACC; ls.n = n; ls.dtau = dtau;
+        a.LS = LV + static_cast<long long>(each) * w.nx; a.HS = a.LS + w.ny; a.ACC = a.HS + w.ny;
+        ls.FB = FB; ls.DB = DB; ls.DV = DV; ls.LV = LV; ls.acc = a.ACC; ls.n = n; ls.tau = tau0; ls.dtau = dtau;
         ls.threads = 32 * std::max(1, std::min(4, (w.ny - 2 + 31) / 32)); // of the batch's warp groups
         if (lines) a.ACC = nullptr;
         auto arrays_of = [&](int k) { // of step k of a segment
-            const long long at = lines ? k : 0;
+            const long long at = k % each;
             a.DB = DB + at * n; a.DV = DV + at * n; a.LV = LV + at * w.nx;
             a.FB[1] = FB + (lines ? 2 * at : 0) * n;
             a.FB[0] = lines ? a.FB[1] + n : FB;
@@ -746,14 +748,15 @@ struct line_adjoint : wide_adjoint_base {
                 case LSS_ADI_MODIFIED_CRAIG_SNEYD: adjoint_step<LSS_ADI_MODIFIED_CRAIG_SNEYD>(s, a, n0 + k, U, D1, D2, D3, Vn); break;
                 default: adjoint_step<LSS_ADI_HUNDSDORFER_VERWER>(s, a, n0 + k, U, D1, D2, D3, Vn); break;
                 }
-            }
-            if (!lines) continue;
-            ls.u0 = u0; ls.len = len; ls.tau = tau0 + dtau * n0;
-            switch (w.scheme) {
-            case LSS_ADI_DOUGLAS_RACHFORD: sum_lines<LSS_ADI_DOUGLAS_RACHFORD>(s, ls, g == 0); break;
-            case LSS_ADI_CRAIG_SNEYD: sum_lines<LSS_ADI_CRAIG_SNEYD>(s, ls, g == 0); break;
-            case LSS_ADI_MODIFIED_CRAIG_SNEYD: sum_lines<LSS_ADI_MODIFIED_CRAIG_SNEYD>(s, ls, g == 0); break;
-            default: sum_lines<LSS_ADI_HUNDSDORFER_VERWER>(s, ls, g == 0); break;
+                if (!lines || k % each != 0) continue;
+                ls.u0 = U; ls.seg = slot(k, 0); ls.len = std::min(each, len - k); ls.n0 = n0 + k;
+                const bool end = ls.n0 == 0;
+                switch (w.scheme) {
+                case LSS_ADI_DOUGLAS_RACHFORD: sum_lines<LSS_ADI_DOUGLAS_RACHFORD>(s, ls, end); break;
+                case LSS_ADI_CRAIG_SNEYD: sum_lines<LSS_ADI_CRAIG_SNEYD>(s, ls, end); break;
+                case LSS_ADI_MODIFIED_CRAIG_SNEYD: sum_lines<LSS_ADI_MODIFIED_CRAIG_SNEYD>(s, ls, end); break;
+                default: sum_lines<LSS_ADI_HUNDSDORFER_VERWER>(s, ls, end); break;
+                }
             }
         }
         if (!lines) k_wadj_reduce<<<5, 1024, 0, s>>>(a.ACC, nacc, grads.p);

@@ -812,7 +812,7 @@ __global__ void k_wide_end(const T *U, int nx, int ny, int ld, bilinear b, T *su
 // is updated in place.  Parameter sensitivities of an S solve (I - theta A1) Y = rhs(X) are
 // mu . (d rhs X + theta dA1 Y), mu = ib w; of a v solve w . theta dA2 x.  Both are accumulated by the
 // S kernels, where the coefficient derivatives' v factors are constant along a thread's line (in relay
-// order by k_wadj_lines, for all steps of a segment).
+// order by k_wadj_lines, for a run of steps).
 // ------------------------------------------------------------------------------------------
 struct adj_params {
     const double *hx, *hc, *ha, *hdd;          // nx
@@ -1229,20 +1229,21 @@ __global__ void __launch_bounds__(256) k_wadj_gather(const __grid_constant__ wpa
     }
 }
 
-// Parameter sums of an adjoint in relay order, from the arrays of the steps of a checkpoint segment: with the
+// Parameter sums of an adjoint in relay order, from the arrays of a run of steps of a checkpoint segment: with the
 // operations of the batched kernel (da_s, da_b1) in its order, so that the gradients have the bits of the
 // same instance in a batch, on a warp group of its own class.  They are small against their terms where the
 // scheme has growing modes: with a thread per chunk and its own partial sums, 4 of 240 small calls came out
 // more than 1e-13 from the batch's.  The stages, where the sums were a chain of every step, are left with
-// the solves (k_wadj_s without acc), and the sums of all steps of a segment are made at once: 128 x 64 x
+// the solves (k_wadj_s without acc), and the sums of many steps are made at once: 128 x 64 x
 // 200 Craig-Sneyd 23.4 ms with sensitivities, 26.1 ms with the sums in the stages.
 struct line_sums {
-    const double *u0, *seg;                     // state of the segment's first step; U, D1, D2, D3 of step k at seg + 4 k n
+    const double *u0, *seg;                     // state of the first step; U, D1, D2, D3 of step k at seg + 4 k n
     const double *FB, *DB, *DV, *LV;            // FB: stages 2 and 1 of step k at FB + 2 k n
     double *terms, *rows, *acc;                 // terms of line l: [step][stage][4][lp]; of row p: [step][3][rp]
     long long n;
     int len, lp, rp, threads;                   // steps; lines, rows of a multiple of 32; threads of the batch's group
-    double tau, dtau;                           // time of step 0 of the segment
+    int n0;                                     // number of the first of them
+    double tau, dtau;                           // time of step 0, of a step
     __device__ __forceinline__ const double *U(int k) const { return k == 0 ? u0 : seg + 4LL * k * n; }
 };
 
@@ -1310,7 +1311,7 @@ __global__ void __launch_bounds__(128) k_wadj_lines(const __grid_constant__ wpar
     const double th = q.theta, wx = KIND == 1 ? 1.0 : hv ? q.zeta : q.zeta - q.theta, we = KIND == 1 ? 1.0 : q.zeta;
     const double A = th * sY + wx * sA, B = -(th * sB + 2.0 * wx * sC), Q = -wx * sQ, D = wx * (2.0 * sS - sQ);
     const double E = we * q.gamma * sE;
-    const double es = q.es[j], bs = q.bs[j], hy = q.hy[j], tau = g.tau + g.dtau * k;
+    const double es = q.es[j], bs = q.bs[j], hy = q.hy[j], tau = g.tau + g.dtau * (g.n0 + k);
     double g0 = q.delta * A + q.halfk * B;
     if (sabr)
         g0 += tau * q.omb * (q.hv2[j] * (2.0 * q.delta * (th * sYd + wx * sDd) - 2.0 * q.alphat * (th * sYa + wx * sAa)) -
@@ -1338,7 +1339,7 @@ static __global__ void __launch_bounds__(128) k_wadj_rows(const __grid_constant_
         if (i + 1 <= nx - 2 && p.imap[i + 1] == i) bb += LV[i + 1];
     }
     if (bb != 0.0) {
-        const double u0 = U[0], tau = g.tau + g.dtau * k;
+        const double u0 = U[0], tau = g.tau + g.dtau * (g.n0 + k);
         ee = q.ni * bb * (4.0 * U[1] - 3.0 * u0 - U[2]);
         double hd = q.hx[i];
         if (q.sabr) hd += 2.0 * q.omb * tau * q.hv2[0] * q.hdd[i];

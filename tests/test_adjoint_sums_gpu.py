@@ -50,11 +50,13 @@ def test_edges_of_warps_and_rows(nx, ny, nt, scheme):
                             alpha_scale=10.0, beta_scale=24.0)])
 
 
+@pytest.mark.parametrize("every", [0, 7, 40])
 @pytest.mark.parametrize("scheme", ["dr", "cs", "hv"])
-def test_sabr_gradients_have_the_bits_of_the_batch(scheme):
+def test_sabr_gradients_have_the_bits_of_the_batch(scheme, every):
+    """Their terms hold the time of the step, in segments of any length."""
     same([lss.HestonProblem(model="sabr", sigma=0.4, rho=-0.3, sabr_beta=0.5, rate=0.0, strike=0.05, maturity=2.0, s_lo=0.0,
-                            s_hi=0.2, v_lo=0.0, v_hi=1.0, nx=60, ny=40, nt=21, scheme=scheme, nonuniform=True, acc_point=0.05,
-                            alpha_scale=10.0, beta_scale=24.0, eval_s=0.05, eval_v=0.2)])
+                            s_hi=0.2, v_lo=0.0, v_hi=1.0, nx=60, ny=40, nt=75, scheme=scheme, nonuniform=True, acc_point=0.05,
+                            alpha_scale=10.0, beta_scale=24.0, eval_s=0.05, eval_v=0.2)], checkpoint_every=every)
 
 
 @pytest.mark.parametrize("every", [1, 4, 19, 20, 50])
@@ -69,3 +71,11 @@ def test_line_per_thread_of_more_lines_than_a_group_has_threads():
     p = lss.HestonProblem(nx=300, ny=280, nt=5, scheme="cs", rho=-0.2, nonuniform=True, acc_point=100.0, alpha_scale=10.0,
                           beta_scale=24.0, line_per_thread=True)
     same([p])
+
+
+def test_more_steps_than_a_run():
+    """300 x 300 points: runs of 93 steps."""
+    p = lss.HestonProblem(nx=300, ny=300, nt=121, maturity=0.2, scheme="dr", rho=-0.2, nonuniform=True, acc_point=100.0,
+                          alpha_scale=10.0, beta_scale=24.0, line_per_thread=True)
+    same([p])
+    same([p], checkpoint_every=100)
