@@ -303,14 +303,15 @@ static __global__ void k_setup_v_delta(setup_params sp, double *V0);
 // ------------------------------------------------------------------------------------------
 // One instance's view of the arenas.  The arena base pointers stay in the kernel's parameter
 // space (__grid_constant__), so they cost no registers; only the offsets are carried.
-template <typename T> struct inst_view {
+// FAR: FP32 rows of any length (adi_index.hpp).
+template <typename T, bool FAR = false> struct inst_view {
     const bparams<T> *p;
     int nx, ny, ld, e_s, e_v;
     long long o2;
     int ox, oy;
     long long so, vo; // line tables
-    table_index<s_slots<T>()> si;
-    table_index<v_slots<T>()> vi;
+    table_index<s_slots<T>(), FAR> si;
+    table_index<v_slots<T>(), FAR> vi;
     // line tables of the instance: row t of the S lines holds all its slots, column t of the v lines too (a
     // row's operands lie within a few KB instead of ten arenas: 5 to 15 % where a GPU full of 256 x 128
     // instances reads them from HBM)
@@ -343,8 +344,8 @@ __device__ __forceinline__ float v_point(float la, float vc, float vn, float ib,
 // boundary#1: the v = v_lo column, explicit (explicit_boundary.hpp:39-84); result in smem
 // Work distribution of every stage: items l0, l0 + ls, ... (threads of one CTA in the
 // batched kernel; all threads of a grid in the per-stage kernels of the wide path).
-template <typename T>
-__device__ __forceinline__ void b1_stage(const inst_view<T> &v, const T *__restrict__ U, T *__restrict__ sb0, double bnc,
+template <typename T, bool FAR>
+__device__ __forceinline__ void b1_stage(const inst_view<T, FAR> &v, const T *__restrict__ U, T *__restrict__ sb0, double bnc,
                                          int l0, int ls)
 {
     const int nx = v.nx, ld = v.ld, N = nx - 1;
@@ -365,7 +366,7 @@ __device__ __forceinline__ void b1_stage(const inst_view<T> &v, const T *__restr
 }
 
 // boundary#2: row S_lo and the S_max extrapolation row (explicit_boundary.hpp:202-238)
-template <typename T> __device__ __forceinline__ void b2_stage(const inst_view<T> &v, T *Vn, int l0, int ls)
+template <typename T, bool FAR> __device__ __forceinline__ void b2_stage(const inst_view<T, FAR> &v, T *Vn, int l0, int ls)
 {
     const int nx = v.nx, ny = v.ny, ld = v.ld, lri = nx - 1;
     const T four3 = T(4.0 / 3.0), third = T(1.0 / 3.0);
@@ -382,9 +383,15 @@ template <typename T> __device__ __forceinline__ void b2_stage(const inst_view<T
 // eight columns or none (FP32).
 struct deep {
     static constexpr int AH = 5, BK = 16, VB4 = 4;
+    static constexpr bool FAR = false;
+};
+// FP32 rows of tables beyond NEAR_PITCH (the kernels of one instance with a thread per line always take it)
+struct deep_far : deep {
+    static constexpr bool FAR = true;
 };
 struct shallow {
     static constexpr int AH = 1, BK = 4, VB4 = 1;
+    static constexpr bool FAR = false;
 };
 
 // Stages of the FP32 instances, written on Y1, Y2, Y3 (their values keep that form's rounding; FP64
@@ -397,8 +404,8 @@ struct shallow {
 //
 // The next rows' operands are loaded before the current ones are used (five rows ahead, 16 in the back
 // substitution); the fused multiply-adds are written out, so the rounding hangs on no contraction.
-template <int KIND, int SCH, typename DEPTH = deep>
-__device__ __forceinline__ void s_stage(const inst_view<float> &v, const float *U, const float *Y1, const float *Y2, float *Y, int l0, int ls)
+template <int KIND, int SCH, typename DEPTH = deep, bool FAR>
+__device__ __forceinline__ void s_stage(const inst_view<float, FAR> &v, const float *U, const float *Y1, const float *Y2, float *Y, int l0, int ls)
 {
     constexpr bool xt = SCH == LSS_ADI_MODIFIED_CRAIG_SNEYD || SCH == LSS_ADI_HUNDSDORFER_VERWER;
     constexpr bool hv = SCH == LSS_ADI_HUNDSDORFER_VERWER;
@@ -572,8 +579,8 @@ __device__ __forceinline__ void stv(float *p, const float *o)
                  "f"(o[5]), "f"(o[6]), "f"(o[7])
                  : "memory");
 }
-template <typename DEPTH = deep>
-__device__ __forceinline__ void v_stage(const inst_view<float> &v, const float *in, const float *inh, const float *sb0, float *out, int l0, int ls)
+template <typename DEPTH = deep, bool FAR>
+__device__ __forceinline__ void v_stage(const inst_view<float, FAR> &v, const float *in, const float *inh, const float *sb0, float *out, int l0, int ls)
 {
     constexpr bool ahead = DEPTH::VB4 > 1;
     const int nx = v.nx, ny = v.ny, ld = v.ld, e = v.e_v;
@@ -679,9 +686,9 @@ __device__ __forceinline__ void v_stage(const inst_view<float> &v, const float *
     }
 }
 
-template <typename T> __device__ __forceinline__ inst_view<T> make_view(const bparams<T> &p, const bdesc &d)
+template <bool FAR, typename T> __device__ __forceinline__ inst_view<T, FAR> make_view(const bparams<T> &p, const bdesc &d)
 {
-    inst_view<T> v;
+    inst_view<T, FAR> v;
     v.p = &p;
     v.nx = d.nx;
     v.ny = d.ny;
@@ -689,8 +696,8 @@ template <typename T> __device__ __forceinline__ inst_view<T> make_view(const bp
     v.e_s = d.nx - 2;
     v.e_v = d.ny - 2;
     v.o2 = d.o2;
-    v.si = table_index<s_slots<T>()>(d.ld);
-    v.vi = table_index<v_slots<T>()>(d.nx);
+    v.si = table_index<s_slots<T>(), FAR>(d.ld);
+    v.vi = table_index<v_slots<T>(), FAR>(d.nx);
     v.so = d.o2 * s_slots<T>() + v.si.base();
     v.vo = d.o2 * v_slots<T>() + v.vi.base();
     v.ox = d.ox;
@@ -702,7 +709,7 @@ template <typename T> __device__ __forceinline__ inst_view<T> make_view(const bp
 
 // One time step U -> Vn of scheme SCH with stage outputs in Y1, Y2, Y3; ends with a group barrier.
 template <int SCH, typename DEPTH>
-__device__ __forceinline__ void fwd_step(const inst_view<float> &v, const float *U, float *Y1, float *Y2, float *Y3, float *Vn, float *sb0,
+__device__ __forceinline__ void fwd_step(const inst_view<float, DEPTH::FAR> &v, const float *U, float *Y1, float *Y2, float *Y3, float *Vn, float *sb0,
                                          double bnc, const grp &g)
 {
     const int l0 = g.t, ls = g.n;
@@ -762,7 +769,7 @@ __global__ void __launch_bounds__(BATCH_CTA, sizeof(T) == 8 && DEPTH::AH == deep
         g.sync();
         if (inst < 0) break;
         const bdesc d = p.desc[inst];
-        const inst_view<T> v = make_view(p, d);
+        const auto v = make_view<DEPTH::FAR>(p, d);
         T *U = p.U + d.o2, *Vn = p.V + d.o2, *Y1 = p.Y1 + d.o2, *Y2 = p.Y2 + d.o2, *Y3 = p.Y3 + d.o2;
         T *sb0 = p.B0 + d.ox;
         load_payoff(p, d, U, g);
@@ -816,7 +823,7 @@ __global__ void __launch_bounds__(BATCH_CTA, 2) k_batch_fwdadj(const __grid_cons
         g.sync();
         if (inst < 0) break;
         const bdesc d = p.desc[inst];
-        const inst_view<double> v = make_view(p, d);
+        const inst_view<double> v = make_view<false>(p, d);
         const int nx = d.nx, ny = d.ny;
         const long long n = (long long)nx * d.ld;
         const int c = d.ck;
@@ -911,7 +918,7 @@ __device__ __forceinline__ int gstride() { return gridDim.x * blockDim.x; }
 template <typename T> __global__ void k_wide_b1(const __grid_constant__ bparams<T> p, const T *U, T *b0, T *Y2)
 {
     const bdesc d = p.desc[0];
-    const inst_view<T> v = make_view(p, d);
+    const auto v = make_view<sizeof(T) == 4>(p, d);
     if constexpr (sizeof(T) == 8) {
         db1_stage(v, d, U, b0, gtid(), gstride());
         d2_edges(v, U, Y2, gtid(), gstride());
@@ -923,7 +930,7 @@ template <typename T, int KIND>
 __global__ void k_wide_s(const __grid_constant__ bparams<T> p, const T *U, const T *Y1, const T *Y2, T *Y)
 {
     const bdesc d = p.desc[0];
-    const inst_view<T> v = make_view(p, d);
+    const auto v = make_view<sizeof(T) == 4>(p, d);
     with_scheme(d.scheme, [&](auto sch) {
         if constexpr (sizeof(T) == 8) ds_stage<KIND, decltype(sch)::value>(v, d, U, KIND == 1 ? U : Y2, Y1, Y, gtid(), gstride());
         else s_stage<KIND, decltype(sch)::value>(v, U, Y1, Y2, Y, gtid(), gstride());
@@ -934,7 +941,7 @@ template <typename T, bool LAST>
 __global__ void k_wide_v(const __grid_constant__ bparams<T> p, const T *U, const T *Y1, const T *Y2, const T *s, const T *b0, T *out)
 {
     const bdesc d = p.desc[0];
-    const inst_view<T> v = make_view(p, d);
+    const auto v = make_view<sizeof(T) == 4>(p, d);
     const bool hv = LAST && d.scheme == LSS_ADI_HUNDSDORFER_VERWER;
     if constexpr (sizeof(T) == 4) v_stage(v, hv ? Y2 : U, s, b0, out, gtid(), gstride());
     else if constexpr (!LAST) dv_stage<V_FIRST>(v, U, s, nullptr, nullptr, b0, out, gtid(), gstride());
@@ -944,7 +951,7 @@ __global__ void k_wide_v(const __grid_constant__ bparams<T> p, const T *U, const
 template <typename T> __global__ void k_wide_b2(const __grid_constant__ bparams<T> p, T *Vn)
 {
     const bdesc d = p.desc[0];
-    const inst_view<T> v = make_view(p, d);
+    const auto v = make_view<sizeof(T) == 4>(p, d);
     if constexpr (sizeof(T) == 8) db2_stage(v, Vn, gtid(), gstride());
     else b2_stage<T>(v, Vn, gtid(), gstride());
 }
@@ -1061,6 +1068,7 @@ template <typename T> struct batch_typed {
     struct group_plan {
         int grid = 0;
         bool small = false; // forward: every instance has small lines
+        bool far = false;   // FP32: rows of tables that need 64-bit offsets (adi_index.hpp)
         int start[MAX_GROUP_WARPS + 1] = {}, cnt[MAX_GROUP_WARPS + 1] = {};
         long long need[MAX_GROUP_WARPS + 1] = {};
         std::vector<int> order, layout;
@@ -1493,7 +1501,11 @@ template <typename T> int batch_typed<T>::make_plan(int mode)
     for (int sc = 0; sc < NSCHEMES; ++sc) {
         bool &small = mp.sch[sc].small;
         small = mode == 0;
-        for (int k = 0; k < count; ++k) small = small && (desc[k].scheme != sc || small_lines<T>(desc[k]));
+        mp.sch[sc].far = false;
+        for (int k = 0; k < count; ++k) {
+            small = small && (desc[k].scheme != sc || small_lines<T>(desc[k]));
+            mp.sch[sc].far = mp.sch[sc].far || (desc[k].scheme == sc && desc[k].ld > NEAR_PITCH);
+        }
         const int resident = sms * std::max(1, small ? per_sm_small : per_sm);
         grid[sc] = std::max(1, std::min(resident, (warps_wanted[sc] + MAX_GROUP_WARPS - 1) / MAX_GROUP_WARPS));
     }
@@ -1587,8 +1599,13 @@ template <typename T> int batch_typed<T>::launch_forward(cudaStream_t s)
             default: k_batch_forward<T, LSS_ADI_HUNDSDORFER_VERWER, D><<<g.grid, BATCH_CTA, 0, s>>>(p); break;
             }
         };
-        if (g.small) launch(shallow{});
-        else launch(deep{});
+        bool far = false;
+        if constexpr (sizeof(T) == 4) {
+            far = g.far;
+            if (far) launch(deep_far{});
+        }
+        if (!far && g.small) launch(shallow{});
+        else if (!far) launch(deep{});
         LSS_CUDA_TRY(cudaGetLastError(), "batch: launching k_batch_forward");
         ++launches;
     }

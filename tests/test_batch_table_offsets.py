@@ -21,8 +21,17 @@ def test_offsets_of_the_largest_grids():
             for t in (0, 1, rows - 1):
                 for slot in (0, slots - 1):
                     cases.append((t, slot, pitch - 1, pitch, slots))
+    near = (2**31 - 1) // 18 // 8 * 8 # the longest pitch of the FP32 kernels with int rows; v tables of any length
+    for nx, pitch in ((8, near), (1000, 104), (1 << 26, 8)):
+        for t in (0, 1, nx - 1):
+            cases += [(t, 0, pitch - 1, pitch, 180), (t, 17, pitch - 1, pitch, 180)]
+    for pitch, rows in ((1 << 28, 4), (4, 1 << 28)):
+        cases += [(t, slot, pitch - 1, pitch, 50) for t in (0, rows - 1) for slot in (0, 4)]
     res = subprocess.run([out], input="\n".join(" ".join(map(str, c)) for c in cases), check=True, capture_output=True, text=True)
-    assert [int(x) for x in res.stdout.split()] == [(t * slots + slot) * pitch + q for t, slot, q, pitch, slots in cases]
+    got = [int(x) for x in res.stdout.split()]
+    slots_of = lambda s: {180: 18, 50: 5}.get(s, s)
+    assert got[:-1] == [(t * slots_of(slots) + slot) * pitch + q for t, slot, q, pitch, slots in cases]
+    assert near <= got[-1] and 18 * got[-1] < 2**31
 
 
 def test_kernels_reach_their_tables_through_it():
